@@ -697,7 +697,7 @@ struct DfsArgs {
     unsigned long long budget_ns;  // per-launch wall-clock budget (0 = unlimited)
     uint32_t* tasks;             // stolen-range queue [task_cap][16 words]
     uint32_t task_cap;
-    unsigned int* qctr;          // [8]: tasks reserved, tickets issued, -, completed, -, -, seeds issued
+    unsigned int* qctr;          // [kQWords]: kQReserved, kQTickets, kQDone
     uint32_t epoch;              // per-launch tag written as a task's ready flag (never 0)
     uint32_t force_split;        // publish unstarted work at every chunk, waited for or not (tests)
     uint32_t shard, num_shards;  // this engine expands the seed groups whose key hashes to shard (seed_shard)
@@ -818,304 +818,17 @@ struct RunBitsCount : RunBits {
 };
 
 
-// Number of x in the intersection of the resolved lists bn[ids[0..nl)] with x
-// not among the matched core vertices m[t], t in the bit set excl (positions
-// whose vertex can lie in these lists).  Warp-cooperative; the result is
-// warp-uniform.  One list: its length minus the excluded vertices it holds.
-// Several: the shortest list is scanned 32 elements at a time and each
-// element probed in the others.
-template <class RB>
-__device__ unsigned long long isect_count(const uint4* bn, const uint8_t* ids, uint32_t nl, const uint32_t* m,
-                                          uint32_t excl, const uint32_t* __restrict__ pool,
-                                          const uint32_t* __restrict__ dval, uint32_t lane,
-                                          unsigned long long& bytes, const RB& rb) {
-    if (nl == 1) {
-        const uint4 r = bn[ids[0]];
-        bool in = false;
-        if (lane < 16 && ((excl >> lane) & 1u)) {
-            // a vertex held by two positions (a self-loop seed edge) is excluded once
-            bool dup = false;
-            for (uint32_t e = excl & ((1u << lane) - 1u); e; e &= e - 1) dup |= m[__ffs(e) - 1] == m[lane];
-            if (!dup) in = rb.has(ids[0], r, pool, dval, m[lane]);
-            bytes += 32u * (33u - __clz(r.y | 1u));
-        }
-        return (unsigned long long)(r.y + r.w) - __popc(__ballot_sync(kFull, in));
-    }
-    uint32_t g = 0, glen = 0xffffffffu;
-    for (uint32_t i = 0; i < nl; ++i) {
-        const uint4 r = bn[ids[i]];
-        if (r.y + r.w < glen) { glen = r.y + r.w; g = i; }
-    }
-    const uint4 gr = bn[ids[g]];
-    unsigned long long c = 0;
-    for (uint32_t base = 0; base < glen; base += 32) {
-        const uint32_t idx = base + lane;
-        bool ok = idx < glen;
-        if (ok) {
-            const uint32_t x = idx < gr.y ? __ldg(pool + gr.x + idx) : __ldg(dval + gr.z + (idx - gr.y));
-            bytes += 4;
-            for (uint32_t e = excl; e; e &= e - 1) ok &= (x != m[__ffs(e) - 1]);
-            for (uint32_t i = 0; i < nl && ok; ++i) {
-                if (i == g) continue;
-                const uint4 r = bn[ids[i]];
-                bytes += 32u * (33u - __clz(r.y | 1u));
-                ok = rb.has(ids[i], r, pool, dval, x);
-            }
-        }
-        c += __popc(__ballot_sync(kFull, ok));
-    }
-    return c;
-}
+// Tail counts (EdgePlan's subsets).  At the position being evaluated the prefix
+// is fixed: a subset whose lists all hang off it has one count per prefix
+// (s_tc), recounted only when a position it reads changed since (`dirty`, the
+// shallowest position whose vertex changed; kClean: none); the others are
+// counted per candidate, one lane each.
+constexpr uint32_t kPairLaneMax = 0xffffffffu;  // pair counting: longest shorter list counted per lane ($CGB_PAIR_LANE_MAX)
+constexpr uint32_t kClean = 0xffu;
+constexpr uint32_t kNoPos = 0xffffffffu;
 
-// Positions owning the lists bn[ids[0..nl)]: without self-loops a matched
-// vertex never lies in its own lists, so excluding it needs no test.
-__device__ __forceinline__ uint32_t owner_mask(const EdgePlan& P, const uint8_t* ids, uint32_t nl) {
-    uint32_t o = 0;
-    for (uint32_t i = 0; i < nl; ++i) o |= 1u << P.bn_pos[ids[i]];
-    return o;
-}
-
-// Injective assignments of a label group of k <= 3 tail vertices from the
-// sizes sc[mask] of the intersections of its members' candidate sets
-// (inclusion-exclusion over coinciding members).
-__device__ __forceinline__ unsigned long long group_count(const unsigned long long* sc, uint32_t k) {
-    if (k == 1) return sc[1];
-    if (k == 2) return sc[1] * sc[2] - sc[3];
-    return sc[1] * sc[2] * sc[4] - sc[3] * sc[4] - sc[5] * sc[2] - sc[6] * sc[1] + 2 * sc[7];
-}
-
-// Number of injective assignments of the tail vertices given the matched core
-// m[0..n_core): per label group, inclusion-exclusion over the sizes of the
-// members' candidate sets and of their intersections (core vertices
-// excluded); groups multiply.  Warp-cooperative, warp-uniform result.
-template <class RB>
-__device__ unsigned long long tail_count_warp(const EdgePlan& P, const uint32_t* m, uint4* bn, const uint4* rec,
-                                              uint32_t dvcap, const uint32_t* __restrict__ pool,
-                                              const uint32_t* __restrict__ dval, bool self_loops, uint32_t lane,
-                                              unsigned long long& bytes, const RB& rb) {
-    const uint32_t nc = P.n_core, n = P.n;
-    // resolve every tail BN record once
-    for (uint32_t k = P.bn_off[nc] + lane; k < P.bn_off[n]; k += 32) {
-        const size_t at = (size_t)P.bn_dir[k] * dvcap + m[P.bn_pos[k]];
-        uint4 r = rec[at];
-        if (!P.bn_dvis[k]) r.w = 0;
-        bn[k] = r;
-        rb.note(k, at);
-        bytes += 16;
-    }
-    __syncwarp();
-    unsigned long long prod = 1;
-    uint32_t t = nc;
-    while (t < n && prod) {
-        uint32_t e = t;
-        while (e < n && P.tail_gid[e] == P.tail_gid[t]) ++e;
-        const uint32_t k = e - t;
-        unsigned long long sc[8];
-        for (uint32_t mask = 1; mask < (1u << k); ++mask) {
-            uint8_t ids[kMaxBN];
-            uint32_t nl = 0;
-            for (uint32_t i = 0; i < k; ++i)
-                if (mask & (1u << i))
-                    for (uint32_t q = P.bn_off[t + i]; q < P.bn_off[t + i + 1]; ++q) ids[nl++] = (uint8_t)q;
-            const uint32_t ex = P.excl[t] & ~(self_loops ? 0u : owner_mask(P, ids, nl));
-            sc[mask] = isect_count(bn, ids, nl, m, ex, pool, dval, lane, bytes, rb);
-        }
-        prod *= group_count(sc, k);
-        t = e;
-    }
-    return prod;
-}
-
-// At the last core depth j = n_core - 1 the prefix m[0..j) is fixed while all
-// candidates of position j are scanned.  Subsets of a tail group whose lists
-// hang only off prefix vertices have counts that do not depend on the
-// candidate: tail_prepare computes them once per prefix (excluding the prefix
-// vertices); tail_eval then only subtracts whether the candidate itself lies
-// in the set, and intersects the subsets with lists at position j per
-// candidate.
-constexpr unsigned long long kDynamic = ~0ull;
-constexpr uint32_t kPairLaneMax = 64;  // pair counting: longest shorter list a lane scans alone ($CGB_PAIR_LANE_MAX)
-constexpr uint32_t kClean = 0xffu;  // tail cache up to date
-
-// Recounts only the entries that depend on a position >= dirty (the shallowest
-// position whose vertex changed since the last call): an entry's count
-// depends on the positions of its lists' backward neighbours and of the
-// excluded core vertices, so e.g. a subset hanging off positions 0 and 1
-// is counted once per (m[0], m[1]), not once per prefix.  Positions >= j
-// are not matched yet: subsets with a list there are left kDynamic.
-template <class RB>
-__device__ void tail_prepare(const EdgePlan& P, const uint32_t* m, uint4* bn, unsigned long long* cache,
-                             uint32_t dirty, uint32_t j, const uint4* rec, uint32_t dvcap,
-                             const uint32_t* __restrict__ pool, const uint32_t* __restrict__ dval, bool self_loops,
-                             uint32_t lane, unsigned long long& bytes, const RB& rb) {
-    const uint32_t nc = P.n_core, n = P.n;
-    for (uint32_t k = P.bn_off[nc] + lane; k < P.bn_off[n]; k += 32) {
-        if (P.bn_pos[k] >= j || P.bn_pos[k] < dirty) continue;  // records of unchanged owners are current
-        const size_t at = (size_t)P.bn_dir[k] * dvcap + m[P.bn_pos[k]];
-        uint4 r = rec[at];
-        if (!P.bn_dvis[k]) r.w = 0;
-        bn[k] = r;
-        rb.note(k, at);
-        bytes += 16;
-    }
-    __syncwarp();
-    uint32_t t = nc;
-    while (t < n) {
-        uint32_t e = t;
-        while (e < n && P.tail_gid[e] == P.tail_gid[t]) ++e;
-        const uint32_t k = e - t;
-        for (uint32_t mask = 1; mask < (1u << k); ++mask) {
-            uint8_t ids[kMaxBN];
-            uint32_t nl = 0, dep = 0;
-            bool dynamic = false;
-            for (uint32_t i = 0; i < k; ++i)
-                if (mask & (1u << i))
-                    for (uint32_t q = P.bn_off[t + i]; q < P.bn_off[t + i + 1]; ++q) {
-                        ids[nl++] = (uint8_t)q;
-                        dynamic |= P.bn_pos[q] >= j;
-                        dep = max(dep, (uint32_t)P.bn_pos[q]);
-                    }
-            const uint32_t ex = P.excl[t] & ((1u << j) - 1u) & ~(self_loops ? 0u : owner_mask(P, ids, nl));
-            if (ex) dep = max(dep, 31u - __clz(ex));
-            if (!dynamic && dep < dirty) continue;  // still valid
-            const unsigned long long v = dynamic ? kDynamic : isect_count(bn, ids, nl, m, ex, pool, dval, lane, bytes, rb);
-            if (lane == 0) cache[t * 8 + mask] = v;
-        }
-        t = e;
-    }
-    __syncwarp();
-}
-
-// Tail count for the core embedding m[0..n_core) (m[j] = the candidate).
-template <class RB>
-__device__ unsigned long long tail_eval(const EdgePlan& P, const uint32_t* m, uint4* bn,
-                                        const unsigned long long* cache, const uint4* rec, uint32_t dvcap,
-                                        const uint32_t* __restrict__ pool, const uint32_t* __restrict__ dval,
-                                        bool self_loops, uint32_t lane, unsigned long long& bytes,
-                                        const RB& rb) {
-    const uint32_t nc = P.n_core, n = P.n, j = nc - 1;
-    const uint32_t c = m[j];
-    for (uint32_t k = P.bn_off[nc] + lane; k < P.bn_off[n]; k += 32) {
-        if (P.bn_pos[k] != j) continue;
-        const size_t at = (size_t)P.bn_dir[k] * dvcap + c;
-        uint4 r = rec[at];
-        if (!P.bn_dvis[k]) r.w = 0;
-        bn[k] = r;
-        rb.note(k, at);
-        bytes += 16;
-    }
-    __syncwarp();
-    unsigned long long prod = 1;
-    uint32_t t = nc;
-    while (t < n && prod) {
-        uint32_t e = t;
-        while (e < n && P.tail_gid[e] == P.tail_gid[t]) ++e;
-        const uint32_t k = e - t;
-        unsigned long long sc[8];
-        for (uint32_t mask = 1; mask < (1u << k); ++mask) {
-            uint8_t ids[kMaxBN];
-            uint32_t nl = 0;
-            for (uint32_t i = 0; i < k; ++i)
-                if (mask & (1u << i))
-                    for (uint32_t q = P.bn_off[t + i]; q < P.bn_off[t + i + 1]; ++q) ids[nl++] = (uint8_t)q;
-            const unsigned long long cv = cache[t * 8 + mask];
-            if (cv != kDynamic && !((P.excl[t] >> j) & 1u)) {
-                sc[mask] = cv;  // the candidate cannot lie in these lists (another label)
-            } else if (cv != kDynamic) {
-                bool in = true;
-                if (lane < nl) {
-                    const uint4 r = bn[ids[lane]];
-                    in = rb.has(ids[lane], r, pool, dval, c);
-                    bytes += 32u * (33u - __clz(r.y | 1u));
-                }
-                sc[mask] = cv - (__all_sync(kFull, in) ? 1ull : 0ull);
-            } else {
-                const uint32_t ex = P.excl[t] & ~(self_loops ? 0u : owner_mask(P, ids, nl));
-                sc[mask] = isect_count(bn, ids, nl, m, ex, pool, dval, lane, bytes, rb);
-            }
-        }
-        prod *= group_count(sc, k);
-        t = e;
-    }
-    return prod;
-}
-
-// Tail count for the candidate c of the last core position, evaluated by
-// one lane (plans with tail_lane): every cached subset count is prefix-only
-// and c is removed from it when c lies in all of the subset's lists (only
-// for groups sharing the last core vertex's label).  A group whose one list
-// hangs off the last core position (tail_lane 2, cached as kDynamic) counts
-// c's own list: its length minus the excluded prefix vertices it holds (c
-// is not in its own list: no self-loops on this path).  Lanes diverge only
-// in the loads and searches.
-template <bool kLane2, class RB>
-__device__ unsigned long long tail_eval_lane(const EdgePlan& P, const uint4* bn, const unsigned long long* cache,
-                                             const uint4* __restrict__ rec, uint32_t dvcap, const uint32_t* m,
-                                             const uint32_t* __restrict__ pool, const uint32_t* __restrict__ dval,
-                                             uint32_t c, unsigned long long& bytes, const RB& rb) {
-    const uint32_t nc = P.n_core, n = P.n, j = nc - 1;
-    unsigned long long prod = 1;
-    uint32_t t = nc;
-    while (t < n && prod) {
-        uint32_t e = t;
-        while (e < n && P.tail_gid[e] == P.tail_gid[t]) ++e;
-        const uint32_t k = e - t;
-        const bool same_label = (P.excl[t] >> j) & 1u;
-        unsigned long long sc[8];
-        for (uint32_t mask = 1; mask < (1u << k); ++mask) {
-            unsigned long long cv = cache[t * 8 + mask];
-            if (kLane2 && cv == kDynamic) {
-                const uint32_t q = P.bn_off[t];
-                const size_t at = (size_t)P.bn_dir[q] * dvcap + c;
-                uint4 r = rec[at];
-                if (!P.bn_dvis[q]) r.w = 0;
-                rb.touch(at);
-                bytes += 16;
-                cv = (unsigned long long)r.y + r.w;
-                const uint32_t ex = P.excl[t] & ((1u << j) - 1u);
-                if (ex) {
-                    const uint32_t sl = rb.slot_at(at);
-                    for (uint32_t b = ex; b; b &= b - 1) {
-                        bytes += 32u * (33u - __clz(r.y | 1u));
-                        cv -= rb.has_slot(sl, r, pool, dval, m[__ffs(b) - 1]) ? 1ull : 0ull;
-                    }
-                }
-            } else if (same_label) {
-                bool in = true;
-                for (uint32_t i = 0; i < k && in; ++i)
-                    if (mask & (1u << i))
-                        for (uint32_t q = P.bn_off[t + i]; q < P.bn_off[t + i + 1] && in; ++q) {
-                            const uint4 r = bn[q];
-                            bytes += 32u * (33u - __clz(r.y | 1u));
-                            in = rb.has(q, r, pool, dval, c);
-                        }
-                cv -= in ? 1ull : 0ull;
-            }
-            sc[mask] = cv;
-        }
-        prod *= group_count(sc, k);
-        t = e;
-    }
-    return prod;
-}
-
-// Tail count of a plan with tail_const: every subset is prefix-only and no
-// candidate of the last core position can lie in a tail list, so the count
-// is the product of the cached group counts.
-__device__ unsigned long long tail_const_value(const EdgePlan& P, const unsigned long long* cache) {
-    unsigned long long prod = 1;
-    uint32_t t = P.n_core;
-    while (t < P.n && prod) {
-        uint32_t e = t;
-        while (e < P.n && P.tail_gid[e] == P.tail_gid[t]) ++e;
-        prod *= group_count(cache + t * 8, e - t);
-        t = e;
-    }
-    return prod;
-}
-
-// Level sums (plans with sum_from): the product of the lengths of c's own
-// lists towards the tail vertices in sum_tails (1 when there are none).
+// Product of the lengths of c's own lists towards the tail vertices in
+// sum_tails (1 when there are none): the weight of c in a level sum.
 template <class RB>
 __device__ __forceinline__ unsigned long long sum_lens(const EdgePlan& P, const uint4* __restrict__ rec,
                                                        uint32_t dvcap, uint32_t c, const RB& rb) {
@@ -1131,22 +844,145 @@ __device__ __forceinline__ unsigned long long sum_lens(const EdgePlan& P, const 
     return v;
 }
 
+// One value per lane with `on`, for its own candidate c at position d, over the
+// lists of one subset (bits of `lists`, bn index sub_base + bit).  Lists of
+// positions below d hang off the prefix (resolved in bn, the same for every
+// lane); the others are c's own (their record is read here).
+//   !sum: the number of x in every list with x not among the vertices matched
+//         at the positions in ex (position d holds c);
+//   sum:  the sum of sum_lens(x) over the one list.
+// The lanes' shortest lists are laid end to end and walked 32 entries at a
+// time by the whole warp, each entry with its owner's c (binary lifting over
+// the prefix sums): a walk takes ceil(total / 32) steps whatever the lists'
+// lengths, where one candidate at a time leaves most lanes idle (lists of a
+// handful of entries) and one lane per candidate waits for the longest list.
+template <class RB>
+__device__ __forceinline__ unsigned long long flat_lists(const EdgePlan& P, uint32_t lists, uint32_t d, bool sum,
+                                                         bool on, uint32_t c, uint32_t ex, const uint32_t* m,
+                                                         const uint4* bn, const uint4* __restrict__ rec,
+                                                         uint32_t dvcap, const uint32_t* __restrict__ pool,
+                                                         const uint32_t* __restrict__ dval, uint32_t lane,
+                                                         uint32_t& bytes, const RB& rb) {
+    // this lane's shortest list: record fields x, y, z, length, bn index
+    uint32_t gx = 0, gy = 0, gz = 0, glen = 0xffffffffu, gq = 0;
+    for (uint32_t b = lists; b; b &= b - 1) {
+        const uint32_t q = P.sub_base + __ffs(b) - 1;
+        uint4 r = make_uint4(0, 0, 0, 0);
+        if (P.bn_pos[q] < d) {
+            r = bn[q];
+        } else if (on) {
+            const size_t at = (size_t)P.bn_dir[q] * dvcap + c;
+            r = rec[at];
+            if (!P.bn_dvis[q]) r.w = 0;
+            rb.touch(at);
+            bytes += 16;
+        }
+        if (r.y + r.w < glen) {
+            glen = r.y + r.w;
+            gx = r.x; gy = r.y; gz = r.z; gq = q;
+        }
+    }
+    if (!on) glen = 0;
+    unsigned long long res = 0;
+    // 32 lists of at most 2^26 entries fit a 32-bit position; longer ones go one lane at a time
+    uint32_t todo = __ballot_sync(kFull, glen != 0);
+    const bool huge = __reduce_max_sync(kFull, glen) > (1u << 26);
+    while (todo) {
+        const uint32_t part = huge ? (todo & (0u - todo)) : todo;
+        todo &= ~part;
+        const uint32_t len = ((part >> lane) & 1u) ? glen : 0u;
+        uint32_t incl = len;  // prefix sums of the lanes' lengths
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFull, incl, o);
+            if (lane >= (uint32_t)o) incl += v;
+        }
+        const uint32_t total = __shfl_sync(kFull, incl, 31);
+        const uint32_t first = incl - len;
+        for (uint32_t b0 = 0; b0 < total; b0 += 32) {
+            const uint32_t i = b0 + lane;
+            uint32_t o = 0;  // owner of entry i: the number of lanes whose lists end at or before i
+#pragma unroll
+            for (uint32_t step = 16; step >= 1; step >>= 1)
+                if (__shfl_sync(kFull, incl, o + step - 1) <= i) o += step;
+            const uint32_t off = i - __shfl_sync(kFull, first, o);
+            const uint32_t ox = __shfl_sync(kFull, gx, o), oy = __shfl_sync(kFull, gy, o);
+            const uint32_t oz = __shfl_sync(kFull, gz, o);
+            const uint32_t oc = __shfl_sync(kFull, c, o), oq = __shfl_sync(kFull, gq, o);
+            bool ok = i < total;
+            uint32_t x = 0;
+            if (ok) {
+                x = off < oy ? __ldg(pool + ox + off) : __ldg(dval + oz + (off - oy));
+                bytes += 4;
+            }
+            if (sum) {
+                unsigned long long v = ok ? sum_lens(P, rec, dvcap, x, rb) : 0ull;
+                // inclusive sums within each owner's stretch, read at its last entry here
+#pragma unroll
+                for (int s = 1; s < 32; s <<= 1) {
+                    const unsigned long long u = __shfl_up_sync(kFull, v, s);
+                    const uint32_t uo = __shfl_up_sync(kFull, o, s);
+                    if (lane >= (uint32_t)s && uo == o) v += u;
+                }
+                const bool any = len && first < b0 + 32u && incl > b0;
+                const unsigned long long got = __shfl_sync(kFull, v, any ? min(incl - b0, 32u) - 1u : 0u);
+                if (any) res += got;
+            } else {
+                if (ok) {
+                    for (uint32_t e = ex; e; e &= e - 1) {
+                        const uint32_t t = __ffs(e) - 1;
+                        ok &= x != (t == d ? oc : m[t]);
+                    }
+                    for (uint32_t b = lists; b && ok; b &= b - 1) {
+                        const uint32_t q = P.sub_base + __ffs(b) - 1;
+                        if (q == oq) continue;
+                        uint4 r;
+                        uint32_t sl;
+                        if (P.bn_pos[q] < d) {
+                            r = bn[q];
+                            sl = rb.slot ? rb.bslot[q] : kNoSlot;
+                        } else {
+                            const size_t at = (size_t)P.bn_dir[q] * dvcap + oc;
+                            r = rec[at];
+                            if (!P.bn_dvis[q]) r.w = 0;
+                            sl = rb.slot_at(at);
+                        }
+                        bytes += 32u * (33u - __clz(r.y | 1u));
+                        ok = rb.has_slot(sl, r, pool, dval, x);
+                    }
+                }
+                const uint32_t bal = __ballot_sync(kFull, ok);
+                if (len && first < b0 + 32u && incl > b0) {
+                    const uint32_t lo = first > b0 ? first - b0 : 0u, hi = min(incl - b0, 32u);
+                    res += __popc(bal >> lo & (0xffffffffu >> (32u - (hi - lo))));
+                }
+            }
+        }
+    }
+    return res;
+}
+
 // Level-sum table: slots of {key, value}; key 0 = empty, K << 1 = claimed
 // by a warp computing the value, K << 1 | 1 = value published, with
 // K = (plan << 27 | vertex) + 1.  Zeroed before every launch, so values never
 // outlive the index state they were computed on.  A lookup probes
 // kLsumProbes slots; a warp that finds its key busy or every probe taken by
 // other keys computes the value itself (nobody waits).
+// A slot is read and published by one 16-byte access (single-copy atomic), so
+// key and value need no order between them: relaxed, because an acquire at
+// device scope drops the SM's whole L1, which the searches of the other 31
+// resident warps live in.
 constexpr uint32_t kLsumProbes = 4;
 constexpr uint32_t kLsumNone = 0xffffffffu;
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
+__device__ __forceinline__ void lsum_load(const unsigned long long* slot, unsigned long long& k,
+                                          unsigned long long& v) {
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(k), "=l"(v) : "l"(slot) : "memory");
 }
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void lsum_publish(unsigned long long* slot, unsigned long long K, unsigned long long v) {
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
+                 ::"l"(slot), "l"((K << 1) | 1ull), "l"(v) : "memory");
 }
 
 // One thread: the published value of K (hit = true), or the slot this
@@ -1156,17 +992,16 @@ __device__ __forceinline__ uint32_t lsum_find(unsigned long long* tab, uint32_t 
     uint32_t s = (uint32_t)((K * 0x9e3779b97f4a7c15ull) >> 32) & mask;
     for (uint32_t probe = 0; probe < kLsumProbes; ++probe, s = (s + 1) & mask) {
         unsigned long long* slot = tab + 2 * (size_t)s;
-        unsigned long long k = ld_acquire_u64(slot);
+        unsigned long long k, v;
+        lsum_load(slot, k, v);
         if (k == 0) {
-            const unsigned long long prev = atomicCAS(slot, 0ull, K << 1);
-            if (prev == 0) return s;
-            k = prev;
-            if (k & 1ull) k = ld_acquire_u64(slot);  // published meanwhile: read with acquire
+            if (atomicCAS(slot, 0ull, K << 1) == 0) return s;
+            lsum_load(slot, k, v);  // claimed or published meanwhile
         }
         if ((k >> 1) == K) {
             if (k & 1ull) {
                 hit = true;
-                val = *(volatile const unsigned long long*)(slot + 1);
+                val = v;
             }
             return kLsumNone;  // published, or being computed by another warp
         }
@@ -1174,18 +1009,24 @@ __device__ __forceinline__ uint32_t lsum_find(unsigned long long* tab, uint32_t 
     return kLsumNone;
 }
 
-// Product of the cached prefix-only group counts (groups whose lists hang
-// off the last core position are cached as kDynamic and left out).
-__device__ unsigned long long tail_static_product(const EdgePlan& P, const unsigned long long* cache) {
-    unsigned long long prod = 1;
-    uint32_t t = P.n_core;
-    while (t < P.n && prod) {
-        uint32_t e = t;
-        while (e < P.n && P.tail_gid[e] == P.tail_gid[t]) ++e;
-        if (cache[t * 8 + 1] != kDynamic) prod *= group_count(cache + t * 8, e - t);
-        t = e;
+// One thread: the published value of K, without claiming its slot.
+__device__ __forceinline__ bool lsum_peek(const unsigned long long* tab, uint32_t mask, unsigned long long K,
+                                          unsigned long long& val) {
+    uint32_t s = (uint32_t)((K * 0x9e3779b97f4a7c15ull) >> 32) & mask;
+    for (uint32_t probe = 0; probe < kLsumProbes; ++probe, s = (s + 1) & mask) {
+        unsigned long long k, v;
+        lsum_load(tab + 2 * (size_t)s, k, v);
+        if (k == ((K << 1) | 1ull)) {
+            val = v;
+            return true;
+        }
+        if (k == 0) return false;
     }
-    return prod;
+    return false;
+}
+// key of the subtree memo of plan ei at vertex x (level sums use the same table without the top bit)
+__device__ __forceinline__ unsigned long long memo_key(uint32_t ei, uint32_t x) {
+    return ((1ull << 42) | ((unsigned long long)ei << 27) | x) + 1ull;
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
@@ -1193,20 +1034,31 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
     return x;
 }
 
-// Work units of the DFS: seeds (delta edges) from a counter, and stolen
-// ranges from a ring of tasks.  A task is 16 words: w0 = ei | depth << 16 |
-// generator << 24, w1/w2 = [lo, hi) of the generator list, w3 = ready tag,
-// w4..15 = the matched prefix.  A warp without a seed takes one ticket
-// (atomicAdd on the ticket counter) and waits for task number `ticket`;
-// tasks are numbered by an atomicAdd in the same order, so every task has
-// exactly one consumer and neither side contends on a CAS.  While tickets outnumber reserved
-// tasks, a busy warp publishes all the work it has not started at its
-// shallowest level (top of its stack), so the biggest remaining subtrees
-// move first.  Termination: a warp leaves when completed == seeds + reserved
-// (completed read first); a unit's reservations happen before its
-// completion, so equality means no unit is active and none can be created
-// (and every reserved task was consumed, so the waiting warp's ticket will
-// never be filled).
+// Work units of the DFS: seeds (delta edges) from a counter, ranges handed
+// over inside a block through shared memory, and ranges handed to other blocks
+// through a ring of tasks in device memory.  A task is 16 words: w0 = ei |
+// depth << 16 | generator << 24, w1/w2 = [lo, hi) of the generator list, w3 =
+// ready tag (ring only), w4..15 = the matched prefix.  At every chunk a busy
+// warp that sees a waiting one publishes all the work it has not started at
+// its shallowest level (top of its stack), so the biggest remaining subtrees
+// move first: to a warp of its own block if one waits (s_wait; the task goes
+// into that warp's mailbox), else to the ring while tickets outnumber reserved
+// tasks.
+// One waiting warp per block (s_poller) holds a ring ticket (atomicAdd on the
+// ticket counter) and waits for task number `ticket`; tasks are numbered by an
+// atomicAdd in the same order, so every task has exactly one consumer and
+// neither side contends on a CAS.  The other waiting warps spin on their
+// mailbox in shared memory.  What bounds a launch with little work is how fast
+// that work spreads: with all 4,736 resident warps polling the ring and the
+// termination counters (ld.acquire at device scope, which also drops the SM's
+// L1), the counters' L2 slice saturated and a donor's own look at them took
+// 15,000 cycles.
+// Termination: completed == seeds + reserved, completed read first.  s_live
+// counts a block's unfinished units (high word; a mailbox task counts from its
+// donation) and its finished seeds and ring tasks not yet reported (low word);
+// they are reported when no unit of the block is unfinished, so a reported
+// unit has no part left anywhere but in the ring, where its reservation came
+// before its report: equality means no unit is active and none can be created.
 // Device-scope acquire load / release increment (cheaper than full fences).
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
     unsigned int v;
@@ -1218,7 +1070,24 @@ __device__ __forceinline__ void add_release(unsigned int* p, unsigned int v) {
 }
 
 constexpr uint32_t kTaskWords = 16;
+// DFS queue counters (words); the polled ones on lines of their own
+constexpr uint32_t kQReserved = 0, kQTickets = 1, kQDone = 32, kQBusy = 40, kQWords = 64;
+// Tail vertices with up to this many lists stay in the tail where they hang off
+// the last core vertex (single-query engine).  R-MAT 1M/10M, 9-vertex dense,
+// matching per batch: none 14.4 ms, up to three lists 14.0, all 16.4 (four
+// lists: enumerating the vertex narrows its candidates list by list, which the
+// per-candidate count does not share between candidates); R-MAT 100k/1M, a
+// 6-vertex sparse pattern: none 0.50 ms, up to three 0.26.
+constexpr uint32_t kFoldLists = 3;
+constexpr unsigned long long kLiveUnit = 1ull << 32;  // one unfinished unit in s_live
 constexpr uint32_t kNoTicket = 0xffffffffu;
+
+// tasks reserved (x) and tickets issued (y) in one load
+__device__ __forceinline__ uint2 ld_relaxed_u2(const unsigned int* q) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(q) : "memory");
+    return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+}
 constexpr uint32_t kNoVertex = 0xffffffffu;  // m[1] of a grouped unit: matches no candidate
 
 // First index of the ascending X[0..n) whose value is >= c (> c when upper),
@@ -1258,9 +1127,9 @@ struct SeedGroup {
         if (n <= 32) return __popc(__ballot_sync(kFull, xv == c));
         return warp_bound(x, n, c, true, lane) - warp_bound(x, n, c, false, lane);
     }
-    // sum over the lanes with `on` of the multiplicity of their own c: only
-    // the values of X inside the chunk's range [cmin, cmax] are looked at
-    __device__ __forceinline__ uint32_t mult_sum(uint32_t c, bool on, uint32_t lane) const {
+    // per lane with `on`, the multiplicity of its own c: only the values of X
+    // inside the chunk's range [cmin, cmax] are looked at
+    __device__ __forceinline__ uint32_t mult_lane(uint32_t c, bool on, uint32_t lane) const {
         const uint32_t cmin = __reduce_min_sync(kFull, on ? c : 0xffffffffu);
         const uint32_t cmax = __reduce_max_sync(kFull, on ? c : 0u);
         if (cmin > cmax) return 0;
@@ -1285,9 +1154,7 @@ struct SeedGroup {
                 for (; p < hi && __ldg(x + p) == c; ++p) ++r;
             }
         }
-        r = on ? r : 0u;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(kFull, r, o);
-        return r;
+        return on ? r : 0u;
     }
 };
 // Ready tag of ticket t in launch `epoch`: the epoch's low 20 bits and the
@@ -1318,8 +1185,8 @@ constexpr uint32_t kCandMask = (1u << kCandBits) - 1u;
 // kMulti = true: the plans of every registered query in global memory
 // (a.plans, one per (query, edge); a.qe of them), seed table searched in
 // global memory, each warp's current plan copied to shared memory when its
-// unit changes plan.  kSums = false compiles the level sums and the
-// per-lane pendant tails (tail_lane 2) out: the kernel is bound by
+// unit changes plan.  kSums = false compiles the level sums,
+// memos and pair counting out: the kernel is bound by
 // instruction fetch, and their code doubled its fetch stalls on patterns
 // whose plans never use them.
 template <bool kMulti, bool kFoot = false, bool kSums = true>
@@ -1328,10 +1195,17 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     __shared__ uint4 s_bn[kDfsWarps][kMaxBN];
     __shared__ uint32_t s_rbs[kDfsWarps][kMaxBN];  // run bit-set slot of each resolved record
     __shared__ uint32_t s_m[kDfsWarps][kMaxQV];
-    __shared__ unsigned long long s_tc[kDfsWarps][kMaxQV * 8];
+    __shared__ unsigned long long s_tc[kDfsWarps][cgb::kMaxSub];  // counts of the subsets off the prefix
     __shared__ uint32_t s_pre[kMulti ? 1 : kMaxQE + 1];
     __shared__ uint32_t s_lo[kMulti ? 1 : kMaxQE];
     __shared__ __align__(16) EdgePlan s_plan[kMulti ? kDfsWarps : cgb::kMaxQEKeyed];
+    __shared__ uint32_t s_box[kDfsWarps][kTaskWords];  // mailboxes: tasks from this block's busy warps
+    __shared__ uint32_t s_boxfull[kDfsWarps];
+    __shared__ uint32_t s_wait;                        // bit w: warp w waits on its mailbox
+    __shared__ uint32_t s_poller;                      // a warp of this block waits on the ring
+    __shared__ uint32_t s_over;                        // the launch has no work left
+    __shared__ unsigned long long s_live;              // unfinished units << 32 | finished, unreported
+    __shared__ unsigned long long s_stat[kDfsWarps][3];  // tail counts, bytes, busy cycles
 
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t w = threadIdx.x >> 5;
@@ -1346,6 +1220,14 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         uint32_t* dst = reinterpret_cast<uint32_t*>(s_plan);
         for (uint32_t t = threadIdx.x; t < a.qe * (uint32_t)(sizeof(EdgePlan) / 4); t += blockDim.x)
             dst[t] = __ldg(src + t);
+    }
+    if (threadIdx.x < kDfsWarps) {
+        s_boxfull[threadIdx.x] = 0;
+        s_stat[threadIdx.x][0] = s_stat[threadIdx.x][1] = s_stat[threadIdx.x][2] = 0;
+    }
+    if (threadIdx.x == 0) {
+        s_wait = s_poller = s_over = 0;
+        s_live = 0;
     }
     __syncthreads();
     auto pre_at = [&](uint32_t e) -> uint32_t { return kMulti ? __ldg(a.seed_pre + e) : s_pre[e]; };
@@ -1364,51 +1246,107 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     rb.words = a.rb_words;
     rb.bslot = s_rbs[w];
     if constexpr (kFoot) rb.touched = a.touched;
-    volatile unsigned int* vq = a.qctr;  // [0] tasks reserved, [1] tickets issued, [3] completed, [6] seeds
-
+    volatile unsigned int* vq = a.qctr;
+    volatile uint32_t* vfull = s_boxfull;
     // per-depth state held by lane == depth
     uint32_t st_ncand = 0, st_pos = 0, st_next = 0, st_len = 0, st_gen = 0;
     uint32_t st_hs = 0;  // grouped units: X multiplicity of the vertices at hit positions < depth
     unsigned long long cnt = 0;  // lane-local partial count of the current edge
-    unsigned long long n_seeds = 0, n_chunks = 0, n_tested = 0, n_tail = 0, n_tasks = 0;
-    unsigned long long n_bytes = 0;  // algorithmic bytes: seed keys, records, list words, probe sectors
+    // statistics: 32-bit counts in registers; tail counts and bytes (seed keys,
+    // records, list words, probe sectors) gathered in shared memory, bytes
+    // from a per-lane count emptied every 64 steps and at every unit's end
+    uint32_t n_seeds = 0, n_chunks = 0, n_tested = 0, n_tasks = 0, n_bytes = 0;
+    auto count_tails = [&](uint32_t v) { s_stat[w][0] += v; };
+    auto flush_bytes = [&]() {
+        const uint32_t b = __reduce_add_sync(kFull, n_bytes >> 2);
+        n_bytes &= 3u;
+        if (lane == 0) s_stat[w][1] += 4ull * b;
+    };
     int cur_ei = -1;
     const unsigned long long t_start = global_ns();
     uint32_t steps = 0;
     bool out_of_time = false;
+    bool no_seed = false;         // lane 0: every seed has been taken
+    bool waiting = false;         // lane 0: this warp's bit of s_wait was set
     uint32_t ticket = kNoTicket;  // lane 0: ticket of the task ring this warp waits on
     uint32_t dirty = 0;  // shallowest position changed since the tail cache was filled (kClean: none)
-    unsigned long long lsum = 0;  // one-position level sum over G of the current m[p]
     bool mb = false;              // counting a subtree memo (EdgePlan::memo_from) to publish
     bool mb_split = false;        // part of that subtree went to other warps: count it, publish nothing
     uint32_t mb_slot = kLsumNone;
     unsigned long long mb_base = 0;  // lane-local count when the memo's subtree was entered
-    uint32_t ls_dirty = 0;        // shallowest position changed since lsum was computed (kClean: none)
-    unsigned long long tail_const = 0;  // tail count of the current prefix (plans with tail_const)
+    unsigned long long tail_k = 0;  // product of the tail groups that depend on the current prefix alone
     uint32_t idle_spins = 0;
+    bool first_seed = true;
+    uint32_t kind = 0;
+    uint32_t unit_clk = 0;  // kMulti: clock at the current unit's start
 
     for (;;) {
-        // ---- acquire a unit: 1 = seed, 2 = task, 3 = all done, 0 = nothing yet
-        uint32_t kind = 0, item = 0;
+        // ---- acquire a unit: 1 = seed, 2 = ring task, 3 = all done, 4 = mailbox task, 0 = nothing yet
+        if (kind) {
+            // the unit before is finished; its report waits until no unit of the block is unfinished
+            flush_bytes();
+            if (lane == 0) {
+                if (kMulti) s_stat[w][2] += (uint32_t)clock() - unit_clk;
+                const unsigned long long dv = (kind != 4 ? 1ull : 0ull) - kLiveUnit;
+                const unsigned long long nv = atomicAdd(&s_live, dv) + dv;
+                if (nv < kLiveUnit && nv && atomicCAS(&s_live, nv, 0ull) == nv)
+                    add_release(a.qctr + kQDone, (unsigned int)nv);
+            }
+        }
+        kind = 0;
+        uint32_t item = 0;
         if (lane == 0) {
-            if (ticket == kNoTicket && vq[6] < total) {  // vq[6] mirrors work_next without incrementing it
-                item = atomicAdd(a.work_next, 1u);
-                if (item < total) kind = 1;
-                else atomicMax((unsigned int*)&a.qctr[6], total);
+            if (!no_seed) {
+                // the first seed of every warp is fixed (no atomic when there are fewer seeds than warps)
+                item = first_seed ? blockIdx.x + gridDim.x * w : gridDim.x * kDfsWarps + atomicAdd(a.work_next, 1u);
+                first_seed = false;
+                if (item < total) {
+                    kind = 1;
+                    atomicAdd(&s_live, kLiveUnit);
+                } else {
+                    no_seed = true;
+                }
             }
             if (!kind) {
-                // no seed left: hold one ticket of the task ring and wait for its task
-                if (ticket == kNoTicket) ticket = atomicAdd((unsigned int*)&a.qctr[1], 1u);
-                const volatile uint32_t* tk = a.tasks + (size_t)(ticket & (a.task_cap - 1u)) * kTaskWords;
-                if (tk[3] == task_tag(epoch, ticket)) {
-                    kind = 2;
-                    item = ticket;
-                    ticket = kNoTicket;
-                } else if ((idle_spins & 3u) == 3u) {
-                    // completed is read with acquire before reserved (see termination above)
-                    const unsigned int done = ld_acquire((const unsigned int*)&a.qctr[3]);
-                    const unsigned int made = ld_acquire((const unsigned int*)&a.qctr[0]);
-                    if (done == total + made && vq[6] >= total) kind = 3;
+                if (!a.steal) {
+                    kind = 3;  // nothing is ever shared
+                } else if (ticket == kNoTicket) {
+                    if (!waiting) {
+                        atomicOr(&s_wait, 1u << w);
+                        waiting = true;
+                    }
+                    if (vfull[w]) {
+                        kind = 4;
+                        waiting = false;
+                    } else if (*(volatile uint32_t*)&s_over) {
+                        kind = 3;
+                    } else if (!*(volatile uint32_t*)&s_poller && atomicCAS(&s_poller, 0u, 1u) == 0u) {
+                        // wait on the ring for the block instead, unless a busy
+                        // warp has just taken this warp's bit to fill its mailbox
+                        if ((atomicAnd(&s_wait, ~(1u << w)) >> w) & 1u) {
+                            waiting = false;
+                            ticket = atomicAdd(a.qctr + kQTickets, 1u);
+                        } else {
+                            *(volatile uint32_t*)&s_poller = 0;
+                        }
+                    }
+                }
+                if (ticket != kNoTicket) {
+                    const volatile uint32_t* tk = a.tasks + (size_t)(ticket & (a.task_cap - 1u)) * kTaskWords;
+                    if (tk[3] == task_tag(epoch, ticket)) {
+                        kind = 2;
+                        item = ticket;
+                        ticket = kNoTicket;
+                        atomicAdd(&s_live, kLiveUnit);
+                        *(volatile uint32_t*)&s_poller = 0;
+                    } else if ((idle_spins & 3u) == 3u && vq[kQDone] == total + vq[kQReserved]) {
+                        // a plain look said done: again in order, completed read with acquire before reserved
+                        const unsigned int done = ld_acquire(a.qctr + kQDone);
+                        if (done == total + ld_acquire(a.qctr + kQReserved)) {
+                            *(volatile uint32_t*)&s_over = 1;
+                            kind = 3;
+                        }
+                    }
                 }
             }
         }
@@ -1416,7 +1354,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         item = __shfl_sync(kFull, item, 0);
         if (kind == 3) break;
         if (kind == 0) {
-            __nanosleep(idle_spins < 64 ? 128u : 1024u);
+            __nanosleep(idle_spins < 16 ? 40u : 200u);
             ++idle_spins;
             if ((idle_spins & 255u) == 0) {
                 const bool late = a.budget_ns && (global_ns() - t_start) > a.budget_ns;
@@ -1425,6 +1363,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
             continue;
         }
         idle_spins = 0;
+        if (kMulti) unit_clk = (uint32_t)clock();
 
         int ei = 0;
         uint32_t jbase = 2, tgen = 0, tlo = 0, thi = 0;
@@ -1447,25 +1386,22 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                 // a grouped edge runs one DFS per first vertex: only the first
                 // seed of each run of equal first vertices starts one
                 const uint64_t prev = a.dkeys[e_lo + (item - e_pre) - 1];
-                if (((prev ^ key) >> a.B & vmask) == 0) {
-                    if (lane == 0) add_release((unsigned int*)&a.qctr[3], 1u);
-                    continue;
-                }
+                if (((prev ^ key) >> a.B & vmask) == 0) continue;
             }
-            if (a.num_shards > 1 && seed_shard((uint32_t)ei, (uint32_t)((key >> a.B) & vmask), a.num_shards) != a.shard) {
-                if (lane == 0) add_release((unsigned int*)&a.qctr[3], 1u);
+            if (a.num_shards > 1 && seed_shard((uint32_t)ei, (uint32_t)((key >> a.B) & vmask), a.num_shards) != a.shard)
                 continue;
-            }
             if (lane == 0) {
                 m[0] = (uint32_t)((key >> a.B) & vmask);
                 m[1] = grouped_at(ei) ? kNoVertex : (uint32_t)(key & vmask);
                 n_bytes += 8;
             }
         } else {
-            // lane 0 saw the ticket's ready tag: the task's words are published
-            volatile uint32_t* tk = a.tasks + (size_t)(item & (a.task_cap - 1u)) * kTaskWords;
-            __threadfence();
+            // lane 0 saw the ticket's ready tag, or its mailbox full: the task's words are published
+            volatile uint32_t* tk = kind == 4 ? s_box[w] : a.tasks + (size_t)(item & (a.task_cap - 1u)) * kTaskWords;
+            if (kind == 4) __threadfence_block(); else __threadfence();
             const uint32_t wv = lane < kTaskWords ? tk[lane] : 0;
+            __syncwarp();
+            if (kind == 4 && lane == 0) vfull[w] = 0;
             const uint32_t w0 = __shfl_sync(kFull, wv, 0);
             ei = (int)(w0 & 0xffffu);
             jbase = (w0 >> 16) & 0xffu;
@@ -1493,6 +1429,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         const bool tail_cache = a.tail_cache && !(P.flags & cgb::kPlanNoTailCache);
         const uint32_t nc = P.n_core;
         const bool has_tail = nc < P.n;
+        const bool serial = has_tail && (!tail_cache || (P.flags & cgb::kPlanWarpTail));
         SeedGroup X{nullptr, 0u, kNoVertex};
         // weight of a grouped embedding with hs hits (1 inside a memo's subtree,
         // whose count is weighted once when it is complete)
@@ -1504,17 +1441,8 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
             X.x = a.dval + xr.z;
             X.n = xr.w;
             if (X.n <= 32 && lane < X.n) X.xv = __ldg(X.x + lane);
-            if (lane == 0) n_bytes += 16 + 4ull * min(X.n, 32u);
+            if (lane == 0) n_bytes += 16 + 4 * min(X.n, 32u);
         }
-        if (kind == 1 && nc == 2) {  // the seed edge alone is the core: only the tail remains
-            const unsigned long long tc =
-                (P.n == 2) ? 1ull : tail_count_warp(P, m, bn, a.rec, a.dvcap, a.pool, a.dval, self_loops, lane, n_bytes, rb);
-            if (lane == 0) { cnt += P.grouped ? tc * X.n : tc; ++n_tail; }
-            __syncwarp();
-            if (lane == 0) add_release((unsigned int*)&a.qctr[3], 1u);
-            continue;
-        }
-
         // set up depth j: resolve BN records, choose the shortest list as generator
         auto setup = [&](uint32_t j) {
             const uint32_t o0 = P.bn_off[j], o1 = P.bn_off[j + 1];
@@ -1540,13 +1468,21 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         };
 
         dirty = 0;  // new unit: every cached tail count is stale
-        ls_dirty = 0;
-        const bool level_sum = kSums && P.sum_from && !a.vb && !self_loops && (tail_cache || !has_tail);
+        const bool level_sum = kSums && P.sum_from && !a.vb && !self_loops && (!serial);
         const bool memo_on = kSums && P.memo_from && a.lsum_tab && !a.vb && !self_loops;
-        const bool pair_on = kSums && P.pair_last && !a.vb && !self_loops && (tail_cache || !has_tail);
+        const bool pair_on = kSums && P.pair_last && !a.vb && !self_loops && (!serial);
+        const bool sum_on = level_sum && !P.sum_dense;  // one-position sums, through the table
+        const bool peek_on = memo_on && P.memo_from == P.memo_pos + 1;
+        // position whose chunks are evaluated per lane besides the last one
+        const uint32_t dpre = (pair_on || (sum_on && nc > 3)) ? nc - 2 : kNoPos;
+        // depths where a chunk's passing candidates are partly counted at once:
+        // only what is not scanned yet is ever shared from them
+        const uint32_t counted = (dpre != kNoPos ? 1u << dpre : 0u) | (peek_on ? 1u << P.memo_pos : 0u);
         mb = false;
-        setup(jbase);
-        if (kind == 2 && lane == jbase) { st_gen = tgen; st_next = tlo; st_len = thi; }
+        if (nc > 2) {
+            setup(jbase);
+            if (kind != 1 && lane == jbase) { st_gen = tgen; st_next = tlo; st_len = thi; }
+        }
         if (P.grouped) {
             uint32_t h = 0;
             for (uint32_t p = 2; p < jbase; ++p)
@@ -1555,435 +1491,441 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         }
         __syncwarp();
         uint32_t j = jbase;
-        while (j >= jbase) {
-            if (a.budget_ns && ((++steps & 1023u) == 0)) {
-                // bounded run: give up (and report) once the budget is spent
-                unsigned long long now = global_ns();
-                out_of_time = __shfl_sync(kFull, (now - t_start) > a.budget_ns ? 1 : 0, 0) != 0;
-                if (out_of_time) break;
-            }
-            const uint32_t ncand = __shfl_sync(kFull, st_ncand, j);
-            const uint32_t pos = __shfl_sync(kFull, st_pos, j);
-            if (pos < ncand) {
-                if (lane == j) st_pos = pos + 1;
-                if (lane == 0) m[j] = s_cand[w][j][pos] & kCandMask;
-                __syncwarp();
-                dirty = min(dirty, j);
-                ls_dirty = min(ls_dirty, j);
-                if (P.grouped) {
-                    uint32_t h = __shfl_sync(kFull, st_hs, j);
-                    if ((P.hit_mask >> j) & 1u) h += X.mult(m[j], lane);
-                    if (lane == j + 1) st_hs = h;
-                }
-                ++j;
-                setup(j);
-                continue;
-            }
-            const uint32_t gnext = __shfl_sync(kFull, st_next, j);
-            uint32_t glen = __shfl_sync(kFull, st_len, j);
-            if (memo_on && !mb && j == P.memo_from && gnext == 0 && glen > 0) {
-                // the whole level below m[memo_pos]: its count from the table,
-                // or counted here (unweighted) and published at the level's end
-                const uint4 gr = bn[P.bn_off[j] + __shfl_sync(kFull, st_gen, j)];
-                if (glen == gr.y + gr.w) {
-                    const unsigned long long K =
-                        ((1ull << 42) | ((unsigned long long)ei << 27) | m[P.memo_pos]) + 1ull;
-                    uint32_t claim = kLsumNone;
-                    bool hit = false;
-                    unsigned long long hv = 0;
-                    if (lane == 0) claim = lsum_find(a.lsum_tab, a.lsum_mask, K, hit, hv);
-                    if (__shfl_sync(kFull, hit ? 1u : 0u, 0)) {
-                        unsigned long long v = __shfl_sync(kFull, hv, 0);
-                        if (P.grouped) v *= gw(__shfl_sync(kFull, st_hs, j));
-                        if (lane == 0) { cnt += v; ++n_tail; }
-                        if (lane == j) st_next = glen;
-                        __syncwarp();
-                        continue;
-                    }
-                    claim = __shfl_sync(kFull, claim, 0);
-                    if (claim != kLsumNone) {
-                        mb = true;
-                        mb_split = false;
-                        mb_slot = claim;
-                        mb_base = cnt;
-                    }
+        for (;;) {
+            if ((++steps & 63u) == 0) {
+                flush_bytes();
+                if (a.budget_ns && (steps & 1023u) == 0) {
+                    // bounded run: give up (and report) once the budget is spent
+                    unsigned long long now = global_ns();
+                    out_of_time = __shfl_sync(kFull, (now - t_start) > a.budget_ns ? 1 : 0, 0) != 0;
+                    if (out_of_time) break;
                 }
             }
-            if (level_sum && P.sum_dense && a.wsum && j == P.sum_from && gnext == 0 && glen > 0 &&
-                glen == bn[P.bn_off[j]].y + bn[P.bn_off[j]].w) {
-                // positions [j, n_core) counted at once: the product of the
-                // precomputed sums of the positions owned by prefix positions
-                unsigned long long v = 1;
-                if (lane >= j && lane < nc) {
-                    const uint32_t p = P.bn_pos[P.bn_off[lane]];
-                    if (p < j) {
-                        v = __ldg(a.wsum + (size_t)(P.wslot + lane - j) * a.dvcap + m[p]);
-                        n_bytes += 8;
-                    }
-                }
-                for (int o = 16; o > 0; o >>= 1) v *= __shfl_xor_sync(kFull, v, o);
-                if (has_tail) {
-                    if (dirty <= P.tail_dep)
-                        tail_prepare(P, m, bn, s_tc[w], dirty, j, a.rec, a.dvcap, a.pool, a.dval, self_loops, lane,
-                                     n_bytes, rb);
-                    dirty = kClean;
-                    v *= tail_static_product(P, s_tc[w]);
-                }
-                if (P.grouped) v *= gw(__shfl_sync(kFull, st_hs, j));
-                if (lane == 0) { cnt += v; ++n_tail; }
-                if (lane == j) st_next = glen;
-                __syncwarp();
-                continue;
-            }
-            if (level_sum && !P.sum_dense && j == nc - 1 && gnext == 0 && glen > 0) {
-                // the whole last level at once (not a stolen part of it): the
-                // level sum over G, less the matched prefix vertices in G
-                const uint32_t o0 = P.bn_off[j];
-                const uint4 gr = bn[o0];
-                if (glen == gr.y + gr.w) {
-                    if (ls_dirty <= P.bn_pos[o0]) {
-                        // the sum over G of the owner m[p]: from the table, or
-                        // scanned (and published when this warp claimed its slot)
-                        const unsigned long long K = (((unsigned long long)ei << 27) | m[P.bn_pos[o0]]) + 1ull;
-                        uint32_t claim = kLsumNone;
-                        bool hit = false;
-                        unsigned long long hv = 0;
-                        if (a.lsum_tab && lane == 0) claim = lsum_find(a.lsum_tab, a.lsum_mask, K, hit, hv);
-                        if (__shfl_sync(kFull, hit ? 1u : 0u, 0)) {
-                            lsum = __shfl_sync(kFull, hv, 0);
-                        } else {
-                            unsigned long long sv = 0;
-                            for (uint32_t idx = lane; idx < glen; idx += 32) {
-                                const uint32_t c =
-                                    idx < gr.y ? __ldg(a.pool + gr.x + idx) : __ldg(a.dval + gr.z + (idx - gr.y));
-                                sv += sum_lens(P, a.rec, a.dvcap, c, rb);
-                                n_bytes += 4;
-                            }
-                            lsum = warp_sum(sv);
-                            if (lane == 0 && claim != kLsumNone) {
-                                a.lsum_tab[2 * (size_t)claim + 1] = lsum;
-                                st_release_u64(a.lsum_tab + 2 * (size_t)claim, (K << 1) | 1ull);
-                            }
-                        }
-                        ls_dirty = kClean;
-                    }
-                    unsigned long long corr = 0;
-                    bool hit = false;
-                    if (lane < j && ((P.sum_same >> lane) & 1u)) {
-                        const uint32_t x = m[lane];
-                        if (x != kNoVertex && rb.has(o0, gr, a.pool, a.dval, x)) {
-                            hit = true;
-                            corr = sum_lens(P, a.rec, a.dvcap, x, rb);
-                        }
-                    }
-                    corr = warp_sum(corr);
-                    const uint32_t nhit = __popc(__ballot_sync(kFull, hit));
-                    unsigned long long v = lsum - corr;
-                    if (has_tail) {
-                        if (dirty <= P.tail_dep)
-                            tail_prepare(P, m, bn, s_tc[w], dirty, nc - 1, a.rec, a.dvcap, a.pool, a.dval,
-                                         self_loops, lane,
-                                         n_bytes, rb);
-                        dirty = kClean;
-                        v *= tail_static_product(P, s_tc[w]);
-                    }
-                    if (P.grouped) v *= gw(__shfl_sync(kFull, st_hs, j));
-                    if (lane == 0) { cnt += v; n_tail += glen - nhit; }
-                    if (lane == j) st_next = glen;
+            // What this step evaluates: `ok` lanes, each with a candidate c at
+            // position d, worth v0 times its tail count; or (node) no candidate
+            // at all: lane 0 stands for the whole subtree below the prefix m[0..d).
+            bool node = nc == 2, ok = false;
+            uint32_t c = 0, d = j, gnext = 0, glen = 0;
+            unsigned long long v0 = 1;
+            if (nc > 2) {
+                const uint32_t ncand = __shfl_sync(kFull, st_ncand, j);
+                const uint32_t pos = __shfl_sync(kFull, st_pos, j);
+                if (pos < ncand) {
+                    if (lane == j) st_pos = pos + 1;
+                    if (lane == 0) m[j] = s_cand[w][j][pos] & kCandMask;
                     __syncwarp();
+                    dirty = min(dirty, j);
+                    if (P.grouped) {
+                        uint32_t h = __shfl_sync(kFull, st_hs, j);
+                        if ((P.hit_mask >> j) & 1u) h += X.mult(m[j], lane);
+                        if (lane == j + 1) st_hs = h;
+                    }
+                    ++j;
+                    setup(j);
                     continue;
                 }
-            }
-            if (gnext < glen) {
-                const uint32_t g = __shfl_sync(kFull, st_gen, j);
-                // While warps wait for tasks, hand the work not yet started at the
-                // shallowest level of this unit to the queue: at a depth d < j
-                // the buffered survivors not yet descended plus the unscanned
-                // generator range, at d = j the range after this chunk.  The
-                // survivors are a contiguous stretch of the generator (their
-                // offsets in their chunk ride in the top bits of s_cand), so
-                // one range [lo, hi) of depth d's generator describes it all.
-                if (a.steal) {  // checked at every chunk: a waiting warp is served within one chunk's time
-                    uint32_t want = 0;  // some warp holds a ticket no task has been reserved for
-                    if (lane == 0) want = (a.force_split || (int)(vq[1] - vq[0]) > 0) ? 1u : 0u;
-                    if (__shfl_sync(kFull, want, 0)) {
-                        bool has = false;
-                        if (lane >= jbase && lane < j) has = st_next < st_len || st_pos < st_ncand;
-                        // at a pair-counting depth a chunk's passing candidates were
-                        // partly counted already: only its unscanned range is shared
-                        if (pair_on && lane == nc - 2 && lane >= jbase && lane < j) has = st_next < st_len;
-                        if (lane == j) has = glen > gnext + 32u;
-                        const uint32_t hb = __ballot_sync(kFull, has);
-                        uint32_t slot = 0xffffffffu;
-                        if (hb && lane == 0) {
-                            // reserve the next task number while tickets wait for one (always, under
-                            // force_split).  atomicAdd never fails, so concurrent producers may
-                            // overshoot the demand by a few tasks; those wait in the ring for the
-                            // next idle warps, and the slack keeps the ring from lapping its head.
-                            const unsigned int t = vq[0], hd = vq[1];
-                            if ((a.force_split || (int)(hd - t) > 0) && (int)(t - hd) < (int)(a.task_cap - kTaskSlack))
-                                slot = atomicAdd((unsigned int*)&a.qctr[0], 1u);
+                gnext = __shfl_sync(kFull, st_next, j);
+                glen = __shfl_sync(kFull, st_len, j);
+                if (gnext >= glen) {
+                    if (mb && j == P.memo_from) {
+                        // the memo's subtree is complete: publish its count, weight it once
+                        const unsigned long long S = warp_sum(cnt - mb_base);
+                        if (lane == 0 && !mb_split)
+                            lsum_publish(a.lsum_tab + 2 * (size_t)mb_slot, memo_key((uint32_t)ei, m[P.memo_pos]), S);
+                        const unsigned long long wv =
+                            P.grouped ? (unsigned long long)(X.n - __shfl_sync(kFull, st_hs, j)) : 1ull;
+                        cnt = mb_base + (lane == 0 ? S * wv : 0ull);
+                        mb = false;
+                    }
+                    if (j == jbase) break;
+                    --j;
+                    continue;
+                }
+                if (kSums && gnext == 0 && (memo_on || level_sum)) {
+                    const uint4 gr = bn[P.bn_off[j] + __shfl_sync(kFull, st_gen, j)];
+                    if (glen == gr.y + gr.w) {
+                        if (memo_on && !mb && j == P.memo_from) {
+                            // the whole level below m[memo_pos]: its count from the table,
+                            // or counted here (unweighted) and published at the level's end
+                            uint32_t claim = kLsumNone;
+                            bool hit = false;
+                            unsigned long long hv = 0;
+                            if (lane == 0)
+                                claim = lsum_find(a.lsum_tab, a.lsum_mask, memo_key((uint32_t)ei, m[P.memo_pos]), hit, hv);
+                            if (__shfl_sync(kFull, hit ? 1u : 0u, 0)) {
+                                unsigned long long v = __shfl_sync(kFull, hv, 0);
+                                if (P.grouped) v *= gw(__shfl_sync(kFull, st_hs, j));
+                                if (lane == 0) { cnt += v; count_tails(1); }
+                                if (lane == j) st_next = glen;
+                                __syncwarp();
+                                continue;
+                            }
+                            claim = __shfl_sync(kFull, claim, 0);
+                            if (claim != kLsumNone) {
+                                mb = true;
+                                mb_split = false;
+                                mb_slot = claim;
+                                mb_base = cnt;
+                            }
                         }
-                        slot = __shfl_sync(kFull, slot, 0);
-                        if (slot != 0xffffffffu) {
-                            const uint32_t d = __ffs(hb) - 1;
-                            if (mb && d >= P.memo_from) mb_split = true;  // the memo's count is no longer all here
-                            uint32_t lo = 0, hi = 0;
-                            if (lane == d) {
-                                if (d == j) {
-                                    lo = gnext + 32u;
-                                    hi = glen;
-                                } else if (pair_on && d == nc - 2) {
-                                    lo = st_next;  // the buffered survivors stay with this warp
-                                    hi = st_len;
-                                } else {
-                                    lo = st_pos < st_ncand ? st_next - 32u + (s_cand[w][d][st_pos] >> kCandBits)
-                                                           : st_next;
-                                    hi = st_len;
+                        if (level_sum && P.sum_dense && a.wsum && j == P.sum_from) {
+                            // positions [j, n_core) counted at once: the product of the
+                            // precomputed sums of the positions owned by prefix positions
+                            if (lane >= j && lane < nc) {
+                                const uint32_t p = P.bn_pos[P.bn_off[lane]];
+                                if (p < j) {
+                                    v0 = __ldg(a.wsum + (size_t)(P.wslot + lane - j) * a.dvcap + m[p]);
+                                    n_bytes += 8;
                                 }
                             }
-                            lo = __shfl_sync(kFull, lo, d);
-                            hi = __shfl_sync(kFull, hi, d);
-                            const uint32_t gd = __shfl_sync(kFull, st_gen, d);
-                            uint32_t* tk = a.tasks + (size_t)(slot & (a.task_cap - 1u)) * kTaskWords;
-                            uint32_t v = 0;
-                            if (lane == 0) v = (uint32_t)ei | (d << 16) | (gd << 24);
-                            else if (lane == 1) v = lo;
-                            else if (lane == 2) v = hi;
-                            else if (lane >= 4 && lane < 4 + kMaxQV) v = (lane - 4 < d) ? m[lane - 4] : 0u;
-                            if (lane < kTaskWords && lane != 3) tk[lane] = v;
-                            __threadfence();
-                            __syncwarp();
-                            if (lane == 0) *(volatile uint32_t*)(tk + 3) = task_tag(epoch, slot);
-                            if (lane == d) {
-                                if (d == j) st_len = gnext + 32u;
-                                else if (pair_on && d == nc - 2) st_len = st_next;
-                                else { st_len = st_next; st_ncand = st_pos; }
-                            }
-                            if (d == j) glen = gnext + 32u;
+                            for (int o = 16; o > 0; o >>= 1) v0 *= __shfl_xor_sync(kFull, v0, o);
+                            node = true;
+                        } else if (sum_on && nc == 3) {
+                            node = true;  // the last core position right below the seed
                         }
                     }
                 }
-                const uint32_t o0 = P.bn_off[j], o1 = P.bn_off[j + 1];
-                const uint4 gr = bn[o0 + g];
-                const uint32_t idx = gnext + lane;
-                bool ok = idx < glen;
-                uint32_t c = 0;
-                if (ok) {
-                    c = idx < gr.y ? __ldg(a.pool + gr.x + idx) : __ldg(a.dval + gr.z + (idx - gr.y));
-                    n_bytes += 4;
-                    for (uint32_t t = 0; t < j; ++t) ok &= (c != m[t]);
-                    if (ok && a.vb)  // the valid bits are a sound superset: a clear bit cannot match
-                        ok = (__ldg(a.vb + ((size_t)ei * a.qv + P.vs[j]) * a.vb_stride + (c >> 5)) >> (c & 31)) & 1u;
-                }
-                if (ok) {
-                    // Each candidate is searched in every other backward list,
-                    // stopping at the first miss.  All lanes search the same list
-                    // with the same trip count, so the branch-free search keeps
-                    // the warp converged, and the first steps of every lane hit
-                    // the same words.
-                    for (uint32_t k = o0; k < o1 && ok; ++k) {
-                        if (k == o0 + g) continue;
-                        const uint4 r = bn[k];
-                        const uint32_t sl = rb.slot ? s_rbs[w][k] : kNoSlot;
-                        if (sl != kNoSlot) {
-                            n_bytes += 4;
-                            ok = (__ldg(rb.bits + (size_t)sl * rb.words + (c >> 5)) >> (c & 31)) & 1u;
-                        } else {
-                            n_bytes += 32u * (33u - __clz(r.y | 1u));
-                            ok = sorted_has_bl(a.pool + r.x, r.y, c);
-                        }
-                        if (!ok && r.w) {
-                            n_bytes += 32u * (33u - __clz(r.w | 1u));
-                            ok = sorted_has_bl(a.dval + r.z, r.w, c);
-                        }
-                    }
-                    ++n_tested;
-                }
-                ++n_chunks;
-                if (j == nc - 1) {
-                    // grouped units weigh each embedding by |X| minus the X
-                    // multiplicity of its hit-position vertices
-                    const uint32_t hs = P.grouped ? __shfl_sync(kFull, st_hs, j) : 0u;
-                    const bool hit_last = P.grouped && ((P.hit_mask >> j) & 1u);
-                    if (has_tail && P.tail_const && tail_cache) {
-                        // the tail count depends on the prefix only: one value per prefix
-                        const uint32_t bal = __ballot_sync(kFull, ok);
-                        if (bal) {
-                            if (dirty <= P.tail_dep) {
-                                tail_prepare(P, m, bn, s_tc[w], dirty, nc - 1, a.rec, a.dvcap, a.pool, a.dval,
-                                             self_loops, lane, n_bytes, rb);
-                                tail_const = tail_const_value(P, s_tc[w]);
-                            }
-                            dirty = kClean;
-                            unsigned long long wsum = __popc(bal);
-                            if (P.grouped) {
-                                wsum *= gw(hs);
-                                if (hit_last) wsum -= X.mult_sum(c, ok, lane);
-                            }
-                            if (lane == 0) { cnt += wsum * tail_const; n_tail += __popc(bal); }
-                        }
-                    } else if (has_tail && P.tail_lane && (P.tail_lane == 1 || (kSums && !self_loops)) &&
-                               tail_cache && !hit_last) {
-                        // the tail depends on the candidate only through prefix-only
-                        // lists: every lane counts its own candidate's tail
-                        const uint32_t bal = __ballot_sync(kFull, ok);
-                        if (bal) {
-                            if (dirty <= P.tail_dep)
-                                tail_prepare(P, m, bn, s_tc[w], dirty, nc - 1, a.rec, a.dvcap, a.pool, a.dval,
-                                             self_loops, lane, n_bytes, rb);
-                            dirty = kClean;
-                            if (ok) {
-                                const unsigned long long tc =
-                                    tail_eval_lane<kSums>(P, bn, s_tc[w], a.rec, a.dvcap, m, a.pool, a.dval, c, n_bytes,
-                                                          rb);
-                                cnt += P.grouped ? tc * gw(hs) : tc;
-                            }
-                            if (lane == 0) n_tail += __popc(bal);
-                        }
-                    } else if (has_tail) {
-                        // every surviving candidate completes a core embedding: count its tail
-                        uint32_t bal = __ballot_sync(kFull, ok);
-                        while (bal) {
-                            const int l = __ffs(bal) - 1;
-                            bal &= bal - 1;
-                            const uint32_t cl = __shfl_sync(kFull, c, l);
-                            if (dirty <= P.tail_dep && tail_cache) {
-                                // first embedding since the prefix changed: recount the stale prefix-only subsets
-                                tail_prepare(P, m, bn, s_tc[w], dirty, nc - 1, a.rec, a.dvcap, a.pool, a.dval,
-                                             self_loops, lane, n_bytes, rb);
-                            }
-                            dirty = kClean;
-                            if (lane == 0) m[j] = cl;
-                            __syncwarp();
-                            const unsigned long long tc =
-                                tail_cache
-                                    ? tail_eval(P, m, bn, s_tc[w], a.rec, a.dvcap, a.pool, a.dval, self_loops, lane,
-                                                n_bytes, rb)
-                                    : tail_count_warp(P, m, bn, a.rec, a.dvcap, a.pool, a.dval, self_loops, lane,
-                                                      n_bytes, rb);
-                            unsigned long long wt = 1;
-                            if (P.grouped) wt = gw(hs) - (hit_last ? X.mult(cl, lane) : 0u);
-                            if (lane == 0) { cnt += tc * wt; ++n_tail; }
-                            __syncwarp();
-                        }
-                    } else if (P.grouped) {
-                        const uint32_t nok = __popc(__ballot_sync(kFull, ok));
-                        unsigned long long wsum = (unsigned long long)nok * gw(hs);
-                        if (hit_last) wsum -= X.mult_sum(c, ok, lane);
-                        if (lane == 0) cnt += wsum;
-                    } else {
-                        cnt += ok ? 1ull : 0ull;
-                    }
-                } else {
-                    bool desc = ok;  // survivors buffered for the descent
-                    if (pair_on && j == nc - 2) {
-                        // each lane counts its candidate's last level: |A ∩ B|,
-                        // A = the prefix list of the last position, B = the
-                        // candidate's own; candidates whose shorter list is long
-                        // descend as usual
-                        const uint32_t ka = P.pair_a, kb = P.pair_b;
+                if (!node) {
+                    // While warps wait for tasks, hand the work not yet started at the
+                    // shallowest level of this unit to one of them: at a depth d < j
+                    // the buffered survivors not yet descended plus the unscanned
+                    // generator range, at d = j the range after this chunk.  The
+                    // survivors are a contiguous stretch of the generator (their
+                    // offsets in their chunk ride in the top bits of s_cand), so
+                    // one range [lo, hi) of depth d's generator describes it all.
+                    if (a.steal) {  // checked at every chunk: a waiting warp is served within one chunk's time
+                        // 2: a warp of this block waits; 1: some block holds a ticket no task has been reserved for
+                        uint32_t want = 0;
                         if (lane == 0) {
-                            const size_t at = (size_t)P.bn_dir[ka] * a.dvcap + m[P.bn_pos[ka]];
-                            uint4 r = a.rec[at];
-                            if (!P.bn_dvis[ka]) r.w = 0;
-                            bn[ka] = r;
-                            rb.note(ka, at);
+                            if (a.force_split) {
+                                want = 1u;
+                            } else if (*(volatile uint32_t*)&s_wait) {
+                                want = 2u;
+                            } else {
+                                const uint2 q = ld_relaxed_u2(a.qctr);
+                                want = (int)(q.y - q.x) > 0 ? 1u : 0u;
+                            }
                         }
-                        __syncwarp();
-                        const uint4 ra = bn[ka];
-                        const uint32_t la = ra.y + ra.w;
-                        unsigned long long pc = 0;
-                        bool counted = false;
-                        if (ok) {
-                            const size_t atb = (size_t)P.bn_dir[kb] * a.dvcap + c;
-                            uint4 rq = a.rec[atb];
-                            if (!P.bn_dvis[kb]) rq.w = 0;
-                            rb.touch(atb);
-                            n_bytes += 16;
-                            const uint32_t lq = rq.y + rq.w;
-                            if (min(la, lq) <= a.pair_lane_max) {
-                                counted = true;
-                                const uint32_t slq = rb.slot_at(atb);
-                                if (lq <= la) {
-                                    for (uint32_t i = 0; i < lq; ++i) {
-                                        const uint32_t x = i < rq.y ? __ldg(a.pool + rq.x + i) : __ldg(a.dval + rq.z + (i - rq.y));
-                                        pc += rb.has(ka, ra, a.pool, a.dval, x) ? 1ull : 0ull;
+                        want = __shfl_sync(kFull, want, 0);
+                        if (want) {
+                            bool has = false;
+                            if (lane >= jbase && lane < j) has = st_next < st_len || st_pos < st_ncand;
+                            // at a depth of `counted` a chunk's passing candidates were partly
+                            // counted already: only its unscanned range is shared
+                            if (lane >= jbase && lane < j && ((counted >> lane) & 1u)) has = st_next < st_len;
+                            if (lane == j) has = glen > gnext + 32u;
+                            const uint32_t hb = __ballot_sync(kFull, has);
+                            uint32_t slot = 0xffffffffu;
+                            if (hb && lane == 0) {
+                                if (want == 2u) {
+                                    const uint32_t wm = *(volatile uint32_t*)&s_wait;
+                                    const uint32_t t = wm ? __ffs(wm) - 1 : 0u;
+                                    if (wm && ((atomicAnd(&s_wait, ~(1u << t)) >> t) & 1u)) {
+                                        slot = t;
+                                        atomicAdd(&s_live, kLiveUnit);
                                     }
                                 } else {
-                                    for (uint32_t i = 0; i < la; ++i) {
-                                        const uint32_t x = i < ra.y ? __ldg(a.pool + ra.x + i) : __ldg(a.dval + ra.z + (i - ra.y));
-                                        pc += rb.has_slot(slq, rq, a.pool, a.dval, x) ? 1ull : 0ull;
+                                    // reserve the next task number while tickets wait for one (always, under
+                                    // force_split).  atomicAdd never fails, so concurrent producers may
+                                    // overshoot the demand by a few tasks; those wait in the ring for the
+                                    // next idle warps, and the slack keeps the ring from lapping its head.
+                                    const uint2 q = ld_relaxed_u2(a.qctr);
+                                    if ((a.force_split || (int)(q.y - q.x) > 0) &&
+                                        (int)(q.x - q.y) < (int)(a.task_cap - kTaskSlack))
+                                        slot = atomicAdd(a.qctr + kQReserved, 1u);
+                                }
+                            }
+                            slot = __shfl_sync(kFull, slot, 0);
+                            if (slot != 0xffffffffu) {
+                                const uint32_t d = __ffs(hb) - 1;
+                                if (mb && d >= P.memo_from) mb_split = true;  // the memo's count is no longer all here
+                                uint32_t lo = 0, hi = 0;
+                                if (lane == d) {
+                                    if (d == j) {
+                                        lo = gnext + 32u;
+                                        hi = glen;
+                                    } else if ((counted >> d) & 1u) {
+                                        lo = st_next;  // the buffered survivors stay with this warp
+                                        hi = st_len;
+                                    } else {
+                                        lo = st_pos < st_ncand ? st_next - 32u + (s_cand[w][d][st_pos] >> kCandBits)
+                                                               : st_next;
+                                        hi = st_len;
                                     }
                                 }
-                                for (uint32_t e = P.pair_excl; e; e &= e - 1) {
-                                    const uint32_t x = m[__ffs(e) - 1];
-                                    if (x != kNoVertex && rb.has(ka, ra, a.pool, a.dval, x) &&
-                                        rb.has_slot(slq, rq, a.pool, a.dval, x))
-                                        --pc;
+                                lo = __shfl_sync(kFull, lo, d);
+                                hi = __shfl_sync(kFull, hi, d);
+                                const uint32_t gd = __shfl_sync(kFull, st_gen, d);
+                                uint32_t* tk =
+                                    want == 2u ? s_box[slot] : a.tasks + (size_t)(slot & (a.task_cap - 1u)) * kTaskWords;
+                                uint32_t v = 0;
+                                if (lane == 0) v = (uint32_t)ei | (d << 16) | (gd << 24);
+                                else if (lane == 1) v = lo;
+                                else if (lane == 2) v = hi;
+                                else if (lane >= 4 && lane < 4 + kMaxQV) v = (lane - 4 < d) ? m[lane - 4] : 0u;
+                                if (lane < kTaskWords && lane != 3) tk[lane] = v;
+                                if (want == 2u) __threadfence_block(); else __threadfence();
+                                __syncwarp();
+                                if (lane == 0) {
+                                    if (want == 2u) vfull[slot] = 1;
+                                    else *(volatile uint32_t*)(tk + 3) = task_tag(epoch, slot);
+                                }
+                                if (lane == d) {
+                                    if (d == j) st_len = gnext + 32u;
+                                    else if ((counted >> d) & 1u) st_len = st_next;
+                                    else { st_len = st_next; st_ncand = st_pos; }
+                                }
+                                if (d == j) glen = gnext + 32u;
+                            }
+                        }
+                    }
+                    const uint32_t g = __shfl_sync(kFull, st_gen, j);
+                    const uint32_t o0 = P.bn_off[j], o1 = P.bn_off[j + 1];
+                    const uint4 gr = bn[o0 + g];
+                    const uint32_t idx = gnext + lane;
+                    ok = idx < glen;
+                    if (ok) {
+                        c = idx < gr.y ? __ldg(a.pool + gr.x + idx) : __ldg(a.dval + gr.z + (idx - gr.y));
+                        n_bytes += 4;
+                        for (uint32_t t = 0; t < j; ++t) ok &= (c != m[t]);
+                        if (ok && a.vb)  // the valid bits are a sound superset: a clear bit cannot match
+                            ok = (__ldg(a.vb + ((size_t)ei * a.qv + P.vs[j]) * a.vb_stride + (c >> 5)) >> (c & 31)) & 1u;
+                    }
+                    if (ok) {
+                        // Each candidate is searched in every other backward list,
+                        // stopping at the first miss.  All lanes search the same list
+                        // with the same trip count, so the branch-free search keeps
+                        // the warp converged, and the first steps of every lane hit
+                        // the same words.
+                        for (uint32_t k = o0; k < o1 && ok; ++k) {
+                            if (k == o0 + g) continue;
+                            const uint4 r = bn[k];
+                            n_bytes += 32u * (33u - __clz(r.y | 1u));
+                            ok = rb.has(k, r, a.pool, a.dval, c);
+                        }
+                        ++n_tested;
+                    }
+                    ++n_chunks;
+                    if (j != nc - 1) {
+                        bool desc = ok;  // survivors buffered for the descent
+                        if (kSums && j == dpre) {
+                            // counted below, per lane; pair counting leaves candidates
+                            // whose shorter list is long to the descent
+                            desc = false;
+                            if (pair_on && a.pair_lane_max != kPairLaneMax) {
+                                const size_t ata = (size_t)P.bn_dir[P.pair_a] * a.dvcap + m[P.bn_pos[P.pair_a]];
+                                const size_t atb = (size_t)P.bn_dir[P.pair_b] * a.dvcap + c;
+                                uint4 ra = a.rec[ata], rq = ok ? a.rec[atb] : make_uint4(0, 0, 0, 0);
+                                const uint32_t la = ra.y + (P.bn_dvis[P.pair_a] ? ra.w : 0u);
+                                const uint32_t lq = rq.y + (P.bn_dvis[P.pair_b] ? rq.w : 0u);
+                                desc = ok && min(la, lq) > a.pair_lane_max;
+                                ok = ok && !desc;
+                            }
+                        } else if (kSums && peek_on && j == P.memo_pos && !mb) {
+                            // subtrees below this position already counted by some warp
+                            bool hit = false;
+                            unsigned long long hv = 0;
+                            if (ok) hit = lsum_peek(a.lsum_tab, a.lsum_mask, memo_key((uint32_t)ei, c), hv);
+                            unsigned long long wt = 1;
+                            if (P.grouped) {
+                                wt = X.n - __shfl_sync(kFull, st_hs, j);
+                                if ((P.hit_mask >> j) & 1u) wt -= X.mult_lane(c, hit, lane);
+                            }
+                            if (hit) cnt += hv * wt;
+                            desc = ok && !hit;
+                            ok = false;
+                        } else {
+                            ok = false;
+                        }
+                        const uint32_t bal = __ballot_sync(kFull, desc);
+                        if (desc) s_cand[w][j][__popc(bal & ((1u << lane) - 1u))] = c | (lane << kCandBits);
+                        if (lane == j) { st_ncand = __popc(bal); st_pos = 0; }
+                    }
+                }
+            }
+            if (node) ok = lane == 0;
+            // the positions from n_core - 1 (one-position sums) or sum_from on are
+            // counted by their sums, pendants included
+            const bool summed = kSums && (sum_on ? node || j == dpre : node && nc > 2);
+            uint32_t bal = __ballot_sync(kFull, ok);
+            bool dead = false;  // no candidate of this level has a tail
+            while (bal) {
+                // one pass over the subsets for all lanes, or (serial) one embedding at a time
+                bool on = ok;
+                uint32_t de = d;
+                if (serial && !node) {
+                    const uint32_t l = __ffs(bal) - 1;
+                    if (lane == l) m[j] = c;
+                    __syncwarp();
+                    on = lane == l;
+                    de = nc;
+                    dirty = tail_cache ? min(dirty, j) : 0u;
+                }
+                bal = serial && !node ? bal & (bal - 1u) : 0u;
+                const uint32_t dmask = (1u << de) - 1u;
+                const bool refresh = dirty < de && ((P.tail_reads & dmask) >> dirty) != 0;
+                unsigned long long prod = on ? v0 : 0ull;
+                if (refresh || dirty == 0) tail_k = 1;
+                if (refresh) {
+                    // records of the tail's (and the pair's) lists off changed prefix positions
+                    for (uint32_t k = (pair_on ? P.sub_base : P.bn_off[nc]) + lane; k < P.bn_off[P.n]; k += 32) {
+                        const uint32_t p = P.bn_pos[k];
+                        if (p >= de || p < dirty) continue;
+                        const size_t at = (size_t)P.bn_dir[k] * a.dvcap + m[p];
+                        uint4 r = a.rec[at];
+                        if (!P.bn_dvis[k]) r.w = 0;
+                        bn[k] = r;
+                        rb.note(k, at);
+                        n_bytes += 16;
+                    }
+                    __syncwarp();
+                }
+                if (refresh || (P.sub_any >> de)) {
+                    unsigned long long acc = 1, sc[3];
+                    for (uint32_t i = 0; i < P.n_sub; ++i) {
+                        const uint32_t sk = P.sub_kind[i];
+                        const bool is_sum = kSums && (sk & cgb::kSubSum), is_pair = kSums && (sk & cgb::kSubPair);
+                        if (kSums && ((is_sum && !(sum_on && summed)) || (is_pair && !(pair_on && j == dpre)) ||
+                                      (summed && (sk & cgb::kSubPend))))
+                            continue;
+                        const bool live = is_sum || is_pair || (P.sub_group[i] >> de) != 0;
+                        if (!live && !refresh) continue;
+                        const uint32_t lists = P.sub_lists[i], pos = P.sub_pos[i];
+                        const uint32_t ex = P.sub_excl[i] & ~(self_loops ? 0u : pos) & (dmask | 1u << de);
+                        const bool stat = !is_sum && !(pos >> de);  // lists off the prefix only: cached
+                        unsigned long long v;
+                        if (stat && !(refresh && ((pos | (ex & dmask)) >> dirty))) {
+                            v = s_tc[w][i];
+                        } else {
+                            bool fon = stat ? lane == 0 : prod != 0;
+                            uint32_t fc = c, claim = kLsumNone;
+                            unsigned long long hv = 0, K = 0;
+                            bool hit = false;
+                            uint32_t fd = de;
+                            if (is_sum) {
+                                // the sum over the list of its owner (this lane's candidate, or
+                                // one vertex for the whole step): from the table, or walked here
+                                // (and published when this lane claimed its slot)
+                                const uint32_t p = P.bn_pos[P.sub_base];
+                                if (p < de) { fc = m[p]; fon = lane == 0; }
+                                fd = 0;
+                                K = (((unsigned long long)ei << 27) | fc) + 1ull;
+                                if (fon && a.lsum_tab) claim = lsum_find(a.lsum_tab, a.lsum_mask, K, hit, hv);
+                                fon = fon && !hit;
+                            }
+                            if (!is_sum && !(lists & (lists - 1u))) {
+                                // one list: its length less the excluded vertices in it
+                                const uint32_t q = P.sub_base + __ffs(lists) - 1;
+                                uint4 r = make_uint4(0, 0, 0, 0);
+                                uint32_t sl = kNoSlot;
+                                if (stat) {
+                                    r = bn[q];
+                                    sl = rb.slot ? rb.bslot[q] : kNoSlot;
+                                } else if (fon) {
+                                    const size_t at = (size_t)P.bn_dir[q] * a.dvcap + c;
+                                    r = a.rec[at];
+                                    if (!P.bn_dvis[q]) r.w = 0;
+                                    if (ex) sl = rb.slot_at(at);
+                                    rb.touch(at);
+                                    n_bytes += 16;
+                                }
+                                v = (unsigned long long)r.y + r.w;
+                                for (uint32_t e = stat ? ex & dmask : ex; e; e &= e - 1) {
+                                    const uint32_t t = __ffs(e) - 1;
+                                    const uint32_t x = t == de ? c : m[t];
+                                    // a vertex held by two positions (a self-loop seed edge) is excluded once
+                                    bool dup = x == kNoVertex;
+                                    if (self_loops)
+                                        for (uint32_t e2 = ex & ((1u << t) - 1u); e2; e2 &= e2 - 1) dup |= m[__ffs(e2) - 1] == x;
+                                    if (!dup && v) v -= rb.has_slot(sl, r, a.pool, a.dval, x) ? 1ull : 0ull;
+                                }
+                            } else {
+                                v = flat_lists(P, lists, fd, is_sum, fon, fc, stat ? ex & dmask : ex, m, bn, a.rec, a.dvcap,
+                                               a.pool, a.dval, lane, n_bytes, rb);
+                            }
+                            if (stat) {
+                                v = __shfl_sync(kFull, v, 0);
+                                if (lane == 0) s_tc[w][i] = v;
+                                __syncwarp();
+                            } else if (is_sum) {
+                                if (claim != kLsumNone) lsum_publish(a.lsum_tab + 2 * (size_t)claim, K, v);
+                                if (hit) v = hv;
+                                const uint32_t p = P.bn_pos[P.sub_base];
+                                if (p < de) v = __shfl_sync(kFull, v, 0);
+                                // less the matched prefix vertices in the list
+                                const size_t at = (size_t)P.bn_dir[P.sub_base] * a.dvcap + fc;
+                                for (uint32_t e = P.sum_same & (dmask | 1u << de); e; e &= e - 1) {
+                                    const uint32_t t = __ffs(e) - 1;
+                                    const uint32_t x = t == de ? c : m[t];
+                                    if (!on || x == kNoVertex) continue;
+                                    uint4 r = a.rec[at];
+                                    if (!P.bn_dvis[P.sub_base]) r.w = 0;
+                                    if (rb.has_slot(rb.slot_at(at), r, a.pool, a.dval, x))
+                                        v -= sum_lens(P, a.rec, a.dvcap, x, rb);
                                 }
                             }
                         }
-                        const uint32_t cb = __ballot_sync(kFull, counted);
-                        if (cb) {
-                            unsigned long long tc = 1;
-                            if (has_tail) {
-                                if (dirty <= P.tail_dep)
-                                    tail_prepare(P, m, bn, s_tc[w], dirty, nc - 2, a.rec, a.dvcap, a.pool, a.dval,
-                                                 self_loops, lane, n_bytes, rb);
-                                dirty = kClean;
-                                tc = tail_static_product(P, s_tc[w]);
-                                // the cache is marked current: so must be the prefix's tail
-                                // count that the descending candidates' last level reads
-                                if (P.tail_const) tail_const = tc;
+                        if (stat && on && ((ex >> de) & 1u) && v) {
+                            // the candidate itself may lie in every list of the subset
+                            bool in = true;
+                            for (uint32_t b = lists; b && in; b &= b - 1) {
+                                const uint32_t q = P.sub_base + __ffs(b) - 1;
+                                n_bytes += 32u * (33u - __clz(bn[q].y | 1u));
+                                in = rb.has(q, bn[q], a.pool, a.dval, c);
                             }
-                            const unsigned long long wgt = P.grouped ? gw(__shfl_sync(kFull, st_hs, j)) : 1ull;
-                            if (counted) cnt += pc * tc * wgt;
-                            if (lane == 0) n_tail += __popc(cb);
+                            v -= in ? 1ull : 0ull;
                         }
-                        desc = ok && !counted;
+                        // inclusion-exclusion over the members that coincide
+                        const uint32_t mem = sk & 7u;
+                        if (!(mem & (mem - 1u))) {
+                            acc = mem == 1u ? v : acc * v;
+                            sc[mem >> 1] = v;
+                        } else if (mem == 7u) {
+                            acc += 2 * v;
+                        } else {
+                            acc -= (sk & cgb::kSubThree) ? v * sc[mem == 3u ? 2 : mem == 5u ? 1 : 0] : v;
+                        }
+                        if (sk & cgb::kSubLast) {
+                            if (live) prod *= acc;
+                            else tail_k *= acc;
+                        }
                     }
-                    const uint32_t bal = __ballot_sync(kFull, desc);
-                    if (desc) s_cand[w][j][__popc(bal & ((1u << lane) - 1u))] = c | (lane << kCandBits);
-                    if (lane == j) { st_ncand = __popc(bal); st_pos = 0; }
                 }
-                if (lane == j) st_next = gnext + 32;
-                __syncwarp();
-                continue;
-            }
-            if (mb && j == P.memo_from) {
-                // the memo's subtree is complete: publish its count, weight it once
-                const unsigned long long S = warp_sum(cnt - mb_base);
-                if (lane == 0 && !mb_split) {
-                    const unsigned long long K =
-                        ((1ull << 42) | ((unsigned long long)ei << 27) | m[P.memo_pos]) + 1ull;
-                    a.lsum_tab[2 * (size_t)mb_slot + 1] = S;
-                    st_release_u64(a.lsum_tab + 2 * (size_t)mb_slot, (K << 1) | 1ull);
+                dirty = kClean;
+                if (tail_k == 0) dead = true;
+                unsigned long long wt = 1;
+                if (P.grouped) {
+                    wt = gw(__shfl_sync(kFull, st_hs, d));
+                    if (!node && ((P.hit_mask >> d) & 1u)) wt -= X.mult_lane(c, on, lane);
                 }
-                const unsigned long long wv =
-                    P.grouped ? (unsigned long long)(X.n - __shfl_sync(kFull, st_hs, j)) : 1ull;
-                cnt = mb_base + (lane == 0 ? S * wv : 0ull);
-                mb = false;
+                if (on) cnt += prod * tail_k * wt;
+                const uint32_t non = __popc(__ballot_sync(kFull, on));
+                if (lane == 0) count_tails(non);
             }
-            --j;
+            if (nc == 2) break;
+            // a level whose prefix-only tail count is 0 adds nothing however it goes on
+            if (lane == j) st_next = node || (dead && !serial) ? glen : gnext + 32u;
+            __syncwarp();
         }
         if (out_of_time) {
             if (lane == 0) atomicOr(a.err, 8u);
             break;
         }
-        if (lane == 0) add_release((unsigned int*)&a.qctr[3], 1u);
     }
     if (out_of_time && lane == 0) atomicOr(a.err, 8u);
     const unsigned long long c = warp_sum(cnt);
     if (cur_ei >= 0 && lane == 0 && c) atomicAdd(a.counts + cur_ei, c);
-    const unsigned long long tested = warp_sum(n_tested), tails = warp_sum(n_tail), bytes = warp_sum(n_bytes);
+    const unsigned long long tested = warp_sum(n_tested);
+    flush_bytes();
     if (lane == 0) {
         atomicAdd(a.stats + 0, n_seeds);
         atomicAdd(a.stats + 1, n_chunks);
         atomicAdd(a.stats + 2, tested);
-        atomicAdd(a.stats + 3, tails);
-        atomicAdd(a.stats + 4, bytes);
+        atomicAdd(a.stats + 3, s_stat[w][0]);
+        atomicAdd(a.stats + 4, s_stat[w][1]);
         atomicAdd(a.stats + 7, n_tasks);
+        // cycles spent on units (the autotuner's measure of a plan's work)
+        if (kMulti) atomicAdd((unsigned long long*)(a.qctr + kQBusy), s_stat[w][2]);
     }
 }
 
@@ -2208,6 +2150,7 @@ struct cgb_handle {
     cgb_config cfg{};
     int device = 0;
     int num_sms = 148;
+    int clock_khz = 0;
     int dfs_occupancy = 0;  // resident DFS blocks per SM
     uint32_t dfs_epoch = 0; // launch counter used as the task ready tag
     cudaStream_t stream = nullptr;
@@ -2258,7 +2201,7 @@ struct cgb_handle {
     unsigned long long* d_counts = nullptr;  // [kMaxQE]
     unsigned long long* d_stats = nullptr;   // [8]
     uint32_t* d_tasks = nullptr;             // stolen-range queue
-    unsigned int* d_qctr = nullptr;          // queue counters [8]
+    unsigned int* d_qctr = nullptr;          // DFS queue counters [kQWords]
     unsigned long long last_stats[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     void* d_temp = nullptr; size_t temp_cap = 0;
 
@@ -2747,6 +2690,7 @@ cgb_status cgb_create(const cgb_config* cfg, cgb_handle** out) {
 #define CKC(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { *out = h; return fail(h, CGB_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); } } while (0)
     CKC(cudaSetDevice(h->device));
     CKC(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device));
+    CKC(cudaDeviceGetAttribute(&h->clock_khz, cudaDevAttrClockRate, h->device));
     CKC(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
     CKC(cudaMalloc(&h->d_scal, 4 * sizeof(unsigned long long)));
@@ -2763,7 +2707,7 @@ cgb_status cgb_create(const cgb_config* cfg, cgb_handle** out) {
     CKC(cudaMalloc(&h->d_counts, kMaxQE * sizeof(unsigned long long)));
     CKC(cudaMalloc(&h->d_stats, 8 * sizeof(unsigned long long)));
     CKC(cudaMalloc(&h->d_tasks, (size_t)kTaskCap * kTaskWords * sizeof(uint32_t)));
-    CKC(cudaMalloc(&h->d_qctr, 8 * sizeof(unsigned int)));
+    CKC(cudaMalloc(&h->d_qctr, kQWords * sizeof(unsigned int)));
     CKC(cudaMemset(h->d_tasks, 0, (size_t)kTaskCap * kTaskWords * sizeof(uint32_t)));
     CKC(cudaMalloc(&h->d_qe_dirs, 2 * kMaxQE));
     CKC(cudaMalloc(&h->d_edge_ok, kMaxQE));
@@ -2857,7 +2801,7 @@ cgb_status cgb_build_index(cgb_handle* h, const uint64_t* keys, uint64_t n, uint
     for (uint32_t d = 0; d < h->nd; ++d) avg[d] = nodes[d] ? (float)card[d] / (float)nodes[d] : 0.f;
     cgb::plan_edges(h->q, avg, h->plans, !(h->cfg.flags & CGB_FLAG_ENUMERATE_TAIL),
                     !(h->cfg.flags & CGB_FLAG_PLAIN_CORE_ORDER), !(h->cfg.flags & CGB_FLAG_NO_SEED_GROUPS),
-                    !(h->cfg.flags & CGB_FLAG_WARP_TAIL), !(h->cfg.flags & CGB_FLAG_NO_LEVEL_SUM), true);
+                    !(h->cfg.flags & CGB_FLAG_WARP_TAIL), !(h->cfg.flags & CGB_FLAG_NO_LEVEL_SUM), true, kFoldLists);
     h->n_wsum = 0;
     h->wjobs_for = nullptr;  // the plans changed: rebuild the level-sum jobs
     for (uint32_t e = 0; e < h->q.qe; ++e)
@@ -2926,7 +2870,7 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
     CK(cudaMemsetAsync(h->d_scal + 2, 0, 2 * sizeof(unsigned long long), h->stream));
     CK(cudaMemsetAsync(h->d_counts, 0, kMaxQE * sizeof(unsigned long long), h->stream));
     CK(cudaMemsetAsync(h->d_stats, 0, 8 * sizeof(unsigned long long), h->stream));
-    CK(cudaMemsetAsync(h->d_qctr, 0, 8 * sizeof(unsigned int), h->stream));
+    CK(cudaMemsetAsync(h->d_qctr, 0, kQWords * sizeof(unsigned int), h->stream));
     CK(cudaEventRecord(h->ev[0], h->stream));
 
     // 1. index update: pending delta (add) + ins (add) + del (remove)
@@ -3056,8 +3000,7 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
         if ((s = lsum_clear(h, da)) != CGB_OK) return s;
         bool uses_sums = false;
         for (uint32_t e = 0; e < h->q.qe; ++e)
-            uses_sums |= h->plans[e].sum_from != 0 || h->plans[e].tail_lane == 2 || h->plans[e].memo_from != 0 ||
-                         h->plans[e].pair_last != 0;
+            uses_sums |= h->plans[e].sum_from != 0 || h->plans[e].memo_from != 0 || h->plans[e].pair_last != 0;
         const dim3 grid(h->num_sms * bps), block(kDfsWarps * 32);
         if (footprint && uses_sums) k_dfs_count<false, true, true><<<grid, block, 0, h->stream>>>(da);
         else if (footprint) k_dfs_count<false, true, false><<<grid, block, 0, h->stream>>>(da);

@@ -277,8 +277,8 @@ cgb_status mq_fail(cgb_mq* m, cgb_status s, const char* fmt, ...) {
     } while (0)
 
 // Plan variants the autotuner times per query (bit mask over the planner's options).
-enum : uint32_t { kVarPlainCore = 1, kVarNoTailCache = 2, kVarNoSeedGroups = 4 };
-constexpr uint32_t kVariants[] = {0, kVarPlainCore, kVarNoTailCache, kVarNoSeedGroups};
+enum : uint32_t { kVarPlainCore = 1, kVarNoTailCache = 2, kVarNoSeedGroups = 4, kVarNoFold = 8 };
+constexpr uint32_t kVariants[] = {0, kVarPlainCore, kVarNoTailCache, kVarNoSeedGroups, kVarNoFold};
 
 // Plans of one query under a variant, remapped to the label-keyed index: a
 // backward list (w -> u) is the list of label(u); the seed direction is
@@ -287,12 +287,14 @@ void mq_plan(const cgb_mq* m, cgb_mq::Query& Q, uint32_t variant) {
     const cgb::QueryMeta& q = Q.q;
     float avg[kMaxDir];
     for (uint32_t d = 0; d < q.nd; ++d) avg[d] = m->avg[q.labels[q.dir_src[d]] * m->L + q.labels[q.dir_dst[d]]];
-    cgb::plan_edges(q, avg, Q.plans, true, !(variant & kVarPlainCore), !(variant & kVarNoSeedGroups));
+    cgb::plan_edges(q, avg, Q.plans, true, !(variant & kVarPlainCore), !(variant & kVarNoSeedGroups), true, true, false,
+                    (variant & kVarNoFold) ? 0u : kMaxQV);
     for (uint32_t ei = 0; ei < q.qe; ++ei) {
         EdgePlan& P = Q.plans[ei];
         for (uint32_t j = 2; j < P.n; ++j)
             for (uint32_t k = P.bn_off[j]; k < P.bn_off[j + 1]; ++k) P.bn_dir[k] = (uint8_t)q.labels[P.vs[j]];
         P.seed_dir = (uint8_t)q.labels[P.vs[1]];
+        cgb::plan_subsets(P);
         P.flags = (variant & kVarNoTailCache) ? cgb::kPlanNoTailCache : 0;
         Q.pair[ei] = (uint16_t)((q.labels[P.vs[1]] << m->h->lb) | q.labels[P.vs[0]]);
     }
@@ -448,7 +450,7 @@ cgb_status mq_match_enqueue(cgb_mq* m, const EdgePlan* plans, const uint16_t* pa
     const uint32_t B = bits_for(h->dv);
     MCK(cudaMemsetAsync(h->d_scal + 3, 0, sizeof(unsigned long long), h->stream));
     MCK(cudaMemsetAsync(m->d_counts, 0, std::max<uint32_t>(G, 1) * sizeof(unsigned long long), h->stream));
-    MCK(cudaMemsetAsync(h->d_qctr, 0, 8 * sizeof(unsigned int), h->stream));
+    MCK(cudaMemsetAsync(h->d_qctr, 0, kQWords * sizeof(unsigned int), h->stream));
     k_mq_seed_ranges<<<1, kMqSeedThreads, 0, h->stream>>>(m->d_sel, m->d_nsel, B, pair, G, m->d_seed,
                                                           m->d_seed + m->plan_cap);
     LAUNCHED();
@@ -545,11 +547,12 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
     if (m->bps == 0) m->bps = m->cfg.dfs_blocks_per_sm ? std::min<int>(occ, m->cfg.dfs_blocks_per_sm) : occ;
     float ms = 0;
     bool any_new = false;
+    const size_t live = std::count_if(m->queries.begin(), m->queries.end(), [](const cgb_mq::Query& q) { return q.live; });
     for (uint32_t id = 0; id < m->queries.size(); ++id) {
         cgb_mq::Query& Q = m->queries[id];
         if (!Q.live || Q.tuned) continue;
         any_new = true;
-        float best = 3.4e38f;
+        float best = 3.4e38f, best_cost = 3.4e38f;
         uint32_t best_v = 0;
         std::vector<unsigned long long> ref;
         for (uint32_t v : kVariants) {
@@ -578,7 +581,16 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
                 return mq_fail(m, CGB_ERR_STATE, "autotune: query %u variant %u counts %llu, variant 0 %llu", id, v,
                                tot, rtot);
             if (ref.empty()) ref = c;
-            if (ms < best) { best = ms; best_v = v; }
+            // Alone, a variant ends with its longest chain of dependent steps while
+            // most warps wait; beside other queries their work fills that time, so
+            // of the part of its time that is not work only its share counts.  (By
+            // the time alone, the 64-query set took plans with 1.4 times the work:
+            // 37 against 31 ms a batch.)
+            unsigned long long busy = 0;
+            MCK(cudaMemcpy(&busy, h->d_qctr + kQBusy, sizeof(busy), cudaMemcpyDeviceToHost));
+            const float work = std::min(ms, (float)((double)busy / ((double)h->clock_khz * h->num_sms * m->bps * kDfsWarps)));
+            const float cost = work + (ms - work) / (float)live;
+            if (cost < best_cost) { best = ms; best_cost = cost; best_v = v; }
         }
         if (best >= 3e38f) return mq_fail(m, CGB_ERR_TIMEOUT, "autotune: query %u exceeded the matching budget", id);
         mq_plan(m, Q, best_v);

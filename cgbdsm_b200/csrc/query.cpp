@@ -117,7 +117,7 @@ std::string build_query_meta(uint32_t qv, uint32_t qe, const uint32_t* edges, co
 // same-label vertices can collide); groups are limited to 3 members, extra
 // members go back to the core.
 void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool analytic_tail, bool pick_last,
-                bool group_pendant, bool lane_tail, bool level_sum, bool dense_sums) {
+                bool group_pendant, bool lane_tail, bool level_sum, bool dense_sums, uint32_t fold_lists) {
     for (uint32_t ei = 0; ei < q.qe; ++ei) {
         EdgePlan& p = plans[ei];
         std::memset(&p, 0, sizeof(p));
@@ -135,11 +135,10 @@ void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool 
         pos[b] = 1;
         auto lab = [&](uint32_t u) { return q.labels.empty() ? 0u : q.labels[u]; };
         // A tail vertex with several lists that hangs off the last core
-        // vertex would be counted by one intersection per last-level
-        // candidate, and would keep the rest of the tail from being constant
-        // per prefix; enumerated as a core vertex its intersection runs
-        // chunked and narrowed.  Such vertices move to the core (`forced`)
-        // and the tail and last vertex are chosen again.
+        // vertex is counted by one intersection per last-level candidate;
+        // enumerated as a core vertex its intersection runs chunked and
+        // narrowed.  With more than fold_lists lists such vertices move to
+        // the core (`forced`) and the tail and last vertex are chosen again.
         std::vector<char> forced(q.qv, 0), is_tail;
         if (pendant)  // a tail vertex of the pendant's label would need per-member weights
             for (uint32_t u = 0; u < q.qv; ++u)
@@ -219,7 +218,7 @@ void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool 
             int move = -1;
             if (last >= 0)
                 for (uint32_t t : tail)
-                    if (q.nbrs[t].size() >= 2 && q.eidx[(uint32_t)last * kMaxQV + t] != 255) { move = (int)t; break; }
+                    if (q.nbrs[t].size() > std::max(fold_lists, 1u) && q.eidx[(uint32_t)last * kMaxQV + t] != 255) { move = (int)t; break; }
             if (move < 0) break;
             forced[move] = 1;
         }
@@ -405,13 +404,14 @@ void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool 
                 }
             }
         }
-        if (level_sum && known && analytic_tail && n_core >= 4) {
+        const uint32_t memo_min = fold_lists > 1 ? 1u : 2u;  // core positions a memo covers at least
+        if (level_sum && known && analytic_tail && n_core >= 2 + memo_min) {
             // subtree memo: the first split [s, n_core), with the latest prefix
             // position p < s that works (not a seed-group position), such that
             // every backward list of the range and every tail list hangs off p
             // or the range
             auto in_range = [&](uint32_t pos, uint32_t s0, uint32_t p0) { return pos == p0 || pos >= s0; };
-            for (uint32_t s0 = 2; s0 + 2 <= n_core && !p.memo_from; ++s0) {
+            for (uint32_t s0 = 2; s0 + memo_min <= n_core && !p.memo_from; ++s0) {
                 for (int pp = (int)s0 - 1; pp >= 0 && !p.memo_from; --pp) {
                     const uint32_t p0 = (uint32_t)pp;
                     if (p.grouped && p0 < 2) continue;  // one unit per first vertex: no reuse
@@ -430,7 +430,7 @@ void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool 
                             if (c != p0) ok &= lab(p.vs[k]) != lab(p.vs[c]);
                     if (p.grouped) ok &= (p.hit_mask >> s0) == 0;
                     // dense sums that already cover the range leave nothing to reuse
-                    if (p.sum_dense && p.sum_from <= s0) ok = false;
+                    if (p.sum_from && p.sum_from <= s0) ok = false;
                     if (ok) {
                         p.memo_from = (uint8_t)s0;
                         p.memo_pos = (uint8_t)p0;
@@ -438,6 +438,67 @@ void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool 
                 }
             }
         }
+        if (!lane_tail) p.flags |= kPlanWarpTail;
+        plan_subsets(p);
+    }
+}
+
+void plan_subsets(EdgePlan& p) {
+    const uint32_t nc = p.n_core;
+    p.n_sub = 0;
+    p.tail_reads = p.sub_any = 0;
+    p.sub_base = p.bn_off[nc - 1];
+    auto add = [&](uint32_t lists, uint16_t pos, uint16_t excl, uint32_t kind) {
+        const uint32_t i = p.n_sub++;
+        p.sub_lists[i] = lists;
+        p.sub_pos[i] = pos;
+        p.sub_excl[i] = excl;
+        p.sub_kind[i] = (uint8_t)kind;
+        p.sub_group[i] = (uint16_t)(pos | excl);
+    };
+    static const uint8_t order[3][7] = {{1}, {1, 2, 3}, {1, 2, 4, 3, 5, 6, 7}};
+    for (uint32_t t = nc; t < p.n;) {
+        uint32_t e = t;
+        while (e < p.n && p.tail_gid[e] == p.tail_gid[t]) ++e;
+        const uint32_t k = e - t, ns = (1u << k) - 1u, first = p.n_sub;
+        uint16_t reads = 0;
+        for (uint32_t i = 0; i < ns; ++i) {
+            const uint32_t mask = order[k - 1][i];
+            uint32_t lists = 0;
+            uint16_t pos = 0;
+            for (uint32_t mem = 0; mem < k; ++mem)
+                if ((mask >> mem) & 1u)
+                    for (uint32_t b = p.bn_off[t + mem]; b < p.bn_off[t + mem + 1]; ++b) {
+                        // of two lists of one direction and owner the one without the delta is in the other
+                        bool skip = false;
+                        for (uint32_t c = p.sub_base; c < p.bn_off[p.n]; ++c)
+                            if (((lists >> (c - p.sub_base)) & 1u) && p.bn_dir[c] == p.bn_dir[b] &&
+                                p.bn_pos[c] == p.bn_pos[b]) {
+                                if (p.bn_dvis[c] && !p.bn_dvis[b]) lists &= ~(1u << (c - p.sub_base));
+                                else skip = true;
+                            }
+                        if (!skip) lists |= 1u << (b - p.sub_base);
+                        pos |= (uint16_t)(1u << p.bn_pos[b]);
+                    }
+            add(lists, pos, p.excl[t],
+                mask | (k == 3 ? kSubThree : 0u) | (i + 1 == ns ? kSubLast : 0u) |
+                    ((p.sum_tails >> t) & 1u ? kSubPend : 0u));
+            reads |= p.sub_group[p.n_sub - 1];
+        }
+        for (uint32_t i = first; i < p.n_sub; ++i) p.sub_group[i] = reads;
+        p.tail_reads |= reads;
+        p.sub_any |= reads;
+        t = e;
+    }
+    if (p.pair_last) {
+        const uint16_t pos = (uint16_t)(1u << p.bn_pos[p.pair_a] | 1u << p.bn_pos[p.pair_b]);
+        add(1u << (p.pair_a - p.sub_base) | 1u << (p.pair_b - p.sub_base), pos, p.pair_excl, 1u | kSubLast | kSubPair);
+        p.tail_reads |= pos;
+        p.sub_any |= pos;
+    }
+    if (p.sum_from && !p.sum_dense) {
+        add(1u, (uint16_t)(1u << p.bn_pos[p.sub_base]), 0, 1u | kSubLast | kSubSum);
+        p.sub_any |= (uint16_t)(1u << (nc - 1));
     }
 }
 

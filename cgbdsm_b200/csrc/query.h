@@ -15,6 +15,7 @@ constexpr int kMaxQE = 32;
 constexpr int kMaxQEKeyed = 16;
 constexpr int kMaxDir = 2 * kMaxQE;
 constexpr int kMaxBN = 48;
+constexpr int kMaxSub = 24;  // tail groups of 3, 3, 3 and 1 members (22 subsets) and the pair or the level sum
 
 // Query graph metadata, numbered exactly as the reference numbers it:
 //   dir index  graph.cpp:137-148  (vertex ascending, neighbour ascending)
@@ -126,11 +127,28 @@ struct EdgePlan {
     // prefix-only tail count, instead of the warp descending into it.
     uint8_t pair_last;
     uint8_t pair_a, pair_b;
-    uint8_t pad_;
+    // Subsets the matcher evaluates in order (plan_subsets): for every tail
+    // label group of k members its 2^k - 1 member subsets, single members
+    // first, then the pair and the one-position level sum.
+    uint8_t n_sub;
     uint16_t pair_excl;
-    uint16_t pad2_;
+    uint8_t sub_base;            // bn index of bit 0 of sub_lists (the last core position's first list)
+    uint8_t pad_;
+    uint16_t tail_reads;         // positions whose vertices the tail subsets and the pair read
+    uint16_t sub_any;            // positions that make some subset depend on the candidate there
+    uint32_t sub_lists[kMaxSub]; // lists intersected
+    uint16_t sub_pos[kMaxSub];   // positions owning them
+    uint16_t sub_excl[kMaxSub];  // positions whose vertices are excluded from the count
+    uint16_t sub_group[kMaxSub]; // positions the whole group reads
+    uint8_t sub_kind[kMaxSub];   // kSub* and the member mask (bits 0-2)
 };
+constexpr uint8_t kSubLast = 0x8;    // last subset of its group
+constexpr uint8_t kSubThree = 0x10;  // group of three members
+constexpr uint8_t kSubPend = 0x20;   // pendant of a level-sum position (sum_tails)
+constexpr uint8_t kSubPair = 0x40;   // the last core position's two lists (pair counting)
+constexpr uint8_t kSubSum = 0x80;    // the last core position's list (one-position level sum)
 constexpr uint8_t kPlanNoTailCache = 0x1;  // recount every tail subset per core embedding
+constexpr uint8_t kPlanWarpTail = 0x2;     // count the tails of one embedding at a time
 constexpr uint32_t kMaxSumTails = 4;     // pendant tails per dense level-sum position
 constexpr uint32_t kMaxSumChildren = 4;  // level-sum positions owned by one dense level-sum position
 
@@ -171,8 +189,14 @@ std::string parse_query_file(const std::string& path, std::vector<uint32_t>& lab
 // (EdgePlan::grouped; needs labels).  lane_tail = false leaves tail_lane 0;
 // level_sum = false leaves sum_from 0; dense_sums = false allows only the
 // one-position (table) level sums.  wslot is left 0 (the engine assigns it).
+// fold_lists: a tail vertex with two to fold_lists lists stays in the tail even
+// where it hangs off the last core vertex (its intersections are then counted
+// per candidate of that vertex); below 2: none does.
 void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool analytic_tail = true,
                 bool pick_last = true, bool group_pendant = true, bool lane_tail = true, bool level_sum = true,
-                bool dense_sums = false);
+                bool dense_sums = false, uint32_t fold_lists = 0);
+// Fills the plan's subsets from its lists, tail groups, pair and level sum
+// (done by plan_edges; again after the directions are rewritten).
+void plan_subsets(EdgePlan& p);
 
 }  // namespace cgb

@@ -395,7 +395,8 @@ cgb_status cgb_mq_last_timings(const cgb_mq* m, float* t4);
 /* Work counters of the last batch (as cgb_last_stats). */
 cgb_status cgb_mq_last_stats(const cgb_mq* m, uint64_t* out8);
 /* Autotuned plan variant of a query (bit 0 plain core order, bit 1 no tail
- * cache, bit 2 no seed groups) and its matching time alone on the tuning
+ * cache, bit 2 no seed groups, bit 3 vertices with several lists kept out of
+ * the counted tail where they hang off the last core vertex) and its matching time alone on the tuning
  * batch (ms; < 0 if not tuned). */
 cgb_status cgb_mq_query_info(const cgb_mq* m, uint32_t query_id, uint32_t* variant, float* tuned_ms);
 /* The DFS schedule in use: blocks per SM and whether work stealing is on. */
