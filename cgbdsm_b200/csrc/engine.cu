@@ -79,21 +79,44 @@ __device__ __forceinline__ uint64_t pack_duv(uint32_t d, uint32_t u, uint32_t v,
     return ((uint64_t)d << (2 * B)) | ((uint64_t)u << B) | (uint64_t)v;
 }
 
+// Edits of one merge, in up to three pieces: keys already packed as (d,u,v)
+// with B0 bits per vertex (the delta kept for the merge-back, or selected
+// deletions), and external keys to add and to remove.
+struct EditSrc {
+    const uint64_t* packed = nullptr;
+    uint64_t n_packed = 0;
+    uint32_t B0 = 0, packed_op = 0;
+    const uint64_t* add = nullptr;
+    uint64_t n_add = 0;
+    const uint64_t* rem = nullptr;
+    uint64_t n_rem = 0;
+};
+
 // Edits: ((d,u,v) << 1) | op, op 0 = add, 1 = remove.  Keys whose direction
 // or vertex ids are out of range raise error bit 1 and become the all-ones
 // marker, which sorts last and is skipped by the merge.
 // Added keys with u == v (a self-loop in the data graph) set the sticky
 // self_seen flag: until one appears no vertex lies in its own lists, which
-// lets the matcher skip those exclusion tests.
-__global__ void k_pack_edits(const uint64_t* __restrict__ in, uint64_t n, uint32_t op, PackInfo pi,
-                             uint64_t* __restrict__ out, unsigned int* err, unsigned int* self_seen) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (; i < n; i += stride) {
+// lets the matcher skip those exclusion tests (packed keys were checked when
+// they were packed).
+__global__ void k_pack_edits(EditSrc src, PackInfo pi, uint64_t* __restrict__ out, unsigned int* err,
+                             unsigned int* self_seen) {
+    const uint64_t n = src.n_packed + src.n_add + src.n_rem;
+    const uint64_t m0 = (1ull << src.B0) - 1ull;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        if (i < src.n_packed) {
+            const uint64_t k = src.packed[i];
+            out[i] = k == ~0ull ? ~0ull
+                                : (pack_duv((uint32_t)(k >> (2 * src.B0)), (uint32_t)((k >> src.B0) & m0),
+                                            (uint32_t)(k & m0), pi.B) << 1) | src.packed_op;
+            continue;
+        }
+        const uint32_t op = i < src.n_packed + src.n_add ? 0u : 1u;
+        const uint64_t k = op ? src.rem[i - src.n_packed - src.n_add] : src.add[i - src.n_packed];
         uint32_t d, u, v;
-        if (pi.pad_ok && in[i] == ~0ull) {
+        if (pi.pad_ok && k == ~0ull) {
             out[i] = ~0ull;
-        } else if (decode_ext(in[i], pi, d, u, v)) {
+        } else if (decode_ext(k, pi, d, u, v)) {
             if (op == 0 && u == v) atomicOr(self_seen, 1u);
             out[i] = (pack_duv(d, u, v, pi.B) << 1) | op;
         } else {
@@ -119,18 +142,6 @@ __global__ void k_pack_delta(const uint64_t* __restrict__ in, uint64_t n, PackIn
     }
 }
 
-// du = (d << B) | u of a sorted packed array (shift = B or B+1 for edits);
-// invalid (all-ones) entries map to 0xffffffff.
-__global__ void k_extract_du(const uint64_t* __restrict__ in, uint64_t n, uint32_t shift,
-                             uint32_t* __restrict__ du) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (; i < n; i += stride) {
-        uint64_t k = in[i];
-        du[i] = (k == ~0ull) ? 0xffffffffu : (uint32_t)(k >> shift);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // fused edit merge of every touched (d, u): warp per run below kBigRun merged
 // entries, CTA per longer (hub) run
@@ -148,15 +159,10 @@ struct MergeArgs {
     unsigned long long* pool_top;
     unsigned long long pool_cap;
     long long* live_words;       // sum of round4(len) over runs
-    const uint64_t* edits;       // sorted ((d,u,v)<<1|op)
-    const uint32_t* run_du;
-    const uint32_t* run_len;
-    const uint32_t* run_off;
-    const int* num_runs;
-    uint32_t* small_runs;        // run ids merged by a warp / by a CTA / by a lane (k_merge_classify)
-    uint32_t* big_runs;
-    uint32_t* tiny_runs;
-    unsigned int* list_ctr;      // [0] small, [1] big, [2] tiny
+    const uint64_t* edits;       // ((d,u,v)<<1|op), each run's edits together and sorted
+    uint64_t n;
+    uint2* runs[3];              // {first edit, edits} of the runs merged by a warp / by a CTA / by a lane (k_edit_runs)
+    unsigned int* list_ctr;      // [0] warp, [1] CTA, [2] lane
     uint32_t B;
     unsigned int* err;
     unsigned long long* stats;   // [5] merge bytes (edits 8 B, old run 4 B/word, new run 4 B/word, record 32 B), [6] runs
@@ -164,7 +170,8 @@ struct MergeArgs {
     // (slot table [d][dvcap], slot owners, claim counter, new-slot list)
     uint32_t* rb_slot;           // nullptr: not maintained by this merge
     uint32_t* rb_sel;
-    unsigned int* rb_ctr;        // [0] slots claimed, [1] new slots this merge
+    unsigned int* rb_ctr;        // slots claimed
+    unsigned int* rb_newc;       // of them by this merge
     uint32_t* rb_new;
     uint32_t rb_cap;
     uint32_t rb_min_len;
@@ -244,18 +251,44 @@ __device__ __forceinline__ bool merge_window(const uint32_t* __restrict__ X, uin
     return emit;
 }
 
-// Splits the runs into warp-merged and CTA-merged lists by merged length.
-__global__ void k_merge_classify(MergeArgs a) {
-    const int n = *a.num_runs;
-    const uint32_t vmask = (1u << a.B) - 1u;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const uint32_t du = a.run_du[r];
-        if (du == 0xffffffffu) continue;  // invalid keys
-        const uint32_t xl = a.rec[(size_t)(du >> a.B) * a.dvcap + (du & vmask)].y;
-        const uint32_t total = xl + a.run_len[r];
-        if (total >= kBigRun) a.big_runs[atomicAdd(a.list_ctr + 1, 1u)] = (uint32_t)r;
-        else if (total > kTinyRun) a.small_runs[atomicAdd(a.list_ctr + 0, 1u)] = (uint32_t)r;
-        else a.tiny_runs[atomicAdd(a.list_ctr + 2, 1u)] = (uint32_t)r;
+// Finds the runs of the edits (an edit whose (d,u) differs from the one before
+// starts one; its end is searched by doubling steps) and lists them by merged
+// length: one pass over the edits where a run-length encoding, a scan of the
+// lengths and a classification took seven launches.  A run's place in its
+// list is arbitrary; appends are one atomic per warp and list.
+__global__ void k_edit_runs(MergeArgs a) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t vmask = (1ull << a.B) - 1ull;
+    const uint32_t sh = a.B + 1;
+    for (uint64_t base = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; base < a.n;
+         base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = base + lane;
+        uint32_t cls = 3, len = 0;
+        if (i < a.n) {
+            const uint64_t e = a.edits[i];
+            const uint64_t du = e >> sh;
+            if (e != ~0ull && (i == 0 || a.edits[i - 1] >> sh != du)) {
+                uint64_t step = 1;
+                while (i + step < a.n && a.edits[i + step] >> sh == du) step <<= 1;
+                uint64_t lo = i + (step >> 1), hi = min(i + step, a.n);  // in the run / past it
+                while (hi - lo > 1) {
+                    const uint64_t mid = (lo + hi) >> 1;
+                    if (a.edits[mid] >> sh == du) lo = mid; else hi = mid;
+                }
+                len = (uint32_t)(lo + 1 - i);
+                const uint32_t total = a.rec[(size_t)(du >> a.B) * a.dvcap + (du & vmask)].y + len;
+                cls = total >= kBigRun ? 1u : total > kTinyRun ? 0u : 2u;
+            }
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 3; ++k) {
+            const uint32_t bal = __ballot_sync(kFull, cls == k);
+            if (!bal) continue;
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(a.list_ctr + k, (uint32_t)__popc(bal));
+            at = __shfl_sync(kFull, at, 0);
+            if (cls == k) a.runs[k][at + __popc(bal & ((1u << lane) - 1u))] = make_uint2((uint32_t)i, len);
+        }
     }
 }
 
@@ -307,7 +340,7 @@ __device__ __forceinline__ void merge_record(const MergeArgs& a, uint4* recp, ui
             if (c < a.rb_cap) {
                 *sp = c;
                 a.rb_sel[c] = d << 27 | u;
-                a.rb_new[atomicAdd(a.rb_ctr + 1, 1u)] = c;
+                a.rb_new[atomicAdd(a.rb_newc, 1u)] = c;
             }
         }
     }
@@ -316,26 +349,25 @@ __device__ __forceinline__ void merge_record(const MergeArgs& a, uint4* recp, ui
 // Lane per run for runs of at most kTinyRun merged entries (most runs of a
 // batch touch a handful of entries): a serial merge per lane, one pool
 // allocation per warp step (a warp prefix over the lanes' bounds).
-__global__ void k_merge_tiny(MergeArgs a) {
+__device__ __forceinline__ void merge_tiny(const MergeArgs& a, MergeAcc& acc) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t n = a.list_ctr[2];
-    const uint32_t vmask = (1u << a.B) - 1u;
     const uint64_t emask = (1ull << a.B) - 1ull;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    MergeAcc acc;
     for (uint32_t base = gw * 32; base < n; base += nw * 32) {
         const uint32_t q = base + lane;
         const bool on = q < n;
-        uint32_t r = 0, d = 0, u = 0, yl = 0;
+        uint32_t d = 0, u = 0, yl = 0, y0 = 0;
         uint4 old = make_uint4(0, 0, 0, 0);
         uint4* recp = nullptr;
         if (on) {
-            r = a.tiny_runs[q];
-            const uint32_t du = a.run_du[r];
-            d = du >> a.B;
-            u = du & vmask;
-            yl = a.run_len[r];
+            const uint2 r = a.runs[2][q];
+            const uint64_t du = a.edits[r.x] >> (a.B + 1);
+            d = (uint32_t)(du >> a.B);
+            u = (uint32_t)(du & emask);
+            y0 = r.x;
+            yl = r.y;
             recp = a.rec + (size_t)d * a.dvcap + u;
             old = *recp;
         }
@@ -358,7 +390,7 @@ __global__ void k_merge_tiny(MergeArgs a) {
         if (!on || wbase == ~0ull) continue;  // pool exhausted: runs left unchanged, error raised
         const unsigned long long off = wbase + pre - bound;
         const uint32_t* X = a.pool + old.x;
-        const uint64_t* Y = a.edits + a.run_off[r];
+        const uint64_t* Y = a.edits + y0;
         uint32_t* C = a.pool + off;
         uint32_t i = 0, j = 0, outn = 0;
         while (i < old.y || j < yl) {
@@ -374,25 +406,21 @@ __global__ void k_merge_tiny(MergeArgs a) {
         merge_record(a, recp, old, off, outn, d, u);
         acc.add(old.y, yl, outn);
     }
-    acc.flush(a, lane);
 }
 
 // Warp per run: 32 merged entries per step from two coalesced windows.
-__global__ void k_merge_runs(MergeArgs a) {
-    __shared__ uint32_t s_win[8][32];
+__device__ __forceinline__ void merge_small(const MergeArgs& a, MergeAcc& acc, uint32_t* sbuf) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nruns = a.list_ctr[0];
     const uint64_t vmask = (1ull << a.B) - 1ull;
-    uint32_t* sbuf = s_win[(threadIdx.x >> 5) & 7];
-    MergeAcc acc;
     for (uint32_t q = gw; q < nruns; q += nw) {
-        const uint32_t r = a.small_runs[q];
-        const uint32_t du = a.run_du[r];
-        const uint32_t d = du >> a.B, u = du & (uint32_t)vmask;
-        const uint64_t* Y = a.edits + a.run_off[r];
-        const uint32_t yl = a.run_len[r];
+        const uint2 r = a.runs[0][q];
+        const uint64_t* Y = a.edits + r.x;
+        const uint32_t yl = r.y;
+        const uint64_t du = *Y >> (a.B + 1);
+        const uint32_t d = (uint32_t)(du >> a.B), u = (uint32_t)(du & vmask);
         uint4* recp = a.rec + (size_t)d * a.dvcap + u;
         const uint4 old = *recp;
         const uint32_t* X = a.pool + old.x;
@@ -417,28 +445,25 @@ __global__ void k_merge_runs(MergeArgs a) {
             acc.add(xl, yl, outn);
         }
     }
-    acc.flush(a, lane);
 }
 
 // CTA per long run: each round, warp w merges the 256 entries from diagonal
 // k0 + 256 w (one merge-path split per warp and round), stages what it emits
 // in shared memory, and the CTA writes the round's output contiguously.
-__global__ void __launch_bounds__(kMergeWarps * 32) k_merge_big(MergeArgs a) {
-    constexpr uint32_t kSeg = 32 * kSegWindows;
-    __shared__ uint32_t s_win[kMergeWarps][32];
+constexpr uint32_t kSeg = 32 * kSegWindows;
+__device__ __forceinline__ void merge_big(const MergeArgs& a, MergeAcc& acc, uint32_t (*s_win)[32]) {
     __shared__ uint32_t s_out[kMergeWarps][kSeg];
     __shared__ uint32_t s_cnt[kMergeWarps];
     __shared__ unsigned long long s_off;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t nruns = a.list_ctr[1];
     const uint64_t vmask = (1ull << a.B) - 1ull;
-    MergeAcc acc;
     for (uint32_t q = blockIdx.x; q < nruns; q += gridDim.x) {
-        const uint32_t r = a.big_runs[q];
-        const uint32_t du = a.run_du[r];
-        const uint32_t d = du >> a.B, u = du & (uint32_t)vmask;
-        const uint64_t* Y = a.edits + a.run_off[r];
-        const uint32_t yl = a.run_len[r];
+        const uint2 r = a.runs[1][q];
+        const uint64_t* Y = a.edits + r.x;
+        const uint32_t yl = r.y;
+        const uint64_t du = *Y >> (a.B + 1);
+        const uint32_t d = (uint32_t)(du >> a.B), u = (uint32_t)(du & vmask);
         uint4* recp = a.rec + (size_t)d * a.dvcap + u;
         const uint4 old = *recp;
         const uint32_t* X = a.pool + old.x;
@@ -485,65 +510,99 @@ __global__ void __launch_bounds__(kMergeWarps * 32) k_merge_big(MergeArgs a) {
         }
         __syncthreads();
     }
-    if (threadIdx.x < 32) acc.flush(a, lane);
+}
+
+// Every listed run in one launch: each block takes its share of the hub runs
+// first (they take longest), then of the warp's and the lane's runs.
+__global__ void __launch_bounds__(kMergeWarps * 32) k_merge(MergeArgs a) {
+    __shared__ uint32_t s_win[kMergeWarps][32];
+    MergeAcc acc;
+    merge_big(a, acc, s_win);
+    merge_small(a, acc, s_win[threadIdx.x >> 5]);
+    merge_tiny(a, acc);
+    acc.flush(a, threadIdx.x & 31);
 }
 
 // ---------------------------------------------------------------------------
 // delta lists
 // ---------------------------------------------------------------------------
-__global__ void k_delta_values(const uint64_t* __restrict__ keys, uint64_t n, uint64_t vmask,
-                               uint32_t* __restrict__ dval) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (; i < n; i += stride) dval[i] = (uint32_t)(keys[i] & vmask);
-}
-
-// du = (d << lb | label bits) << B | u (lb = 0: no label bits).
-__global__ void k_delta_recs(uint4* rec, uint32_t dvcap, const uint32_t* run_du, const uint32_t* run_len,
-                             const uint32_t* run_off, const int* num_runs, uint32_t B, int clear, uint32_t lb = 0) {
-    const int n = *num_runs;
-    const uint32_t umask = (1u << B) - 1u;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        uint32_t du = run_du[r];
-        if (du == 0xffffffffu) continue;
-        uint4* p = rec + (size_t)(du >> (B + lb)) * dvcap + (du & umask);
-        uint4 v = *p;
-        if (clear) { v.z = 0; v.w = 0; }
-        else { v.z = run_off[r]; v.w = run_len[r]; }
-        *p = v;
+// From the sorted packed keys ((d << lb | label bits) << 2B | u << B | v; lb =
+// 0: no label bits): the delta values, and {offset, length} of every (d,u)'s
+// stretch in its record, found as in k_edit_runs.  n keys, of which *nsel are
+// real when given (the others become all-ones padding).
+// clear: only takes the records' delta fields back to empty.
+__device__ __forceinline__ void delta_lists(uint64_t* keys, uint64_t n, const int* nsel, uint32_t B, uint32_t lb,
+                                            uint4* rec, uint32_t dvcap, uint32_t* __restrict__ dval, bool clear,
+                                            uint32_t block, uint32_t blocks) {
+    const uint64_t real = nsel ? (uint64_t)*nsel : n;
+    const uint64_t vmask = (1ull << B) - 1ull;
+    for (uint64_t i = (uint64_t)block * blockDim.x + threadIdx.x; i < (clear ? real : n);
+         i += (uint64_t)blocks * blockDim.x) {
+        if (i >= real) {
+            keys[i] = ~0ull;
+            continue;
+        }
+        const uint64_t k = keys[i];
+        if (!clear) dval[i] = (uint32_t)(k & vmask);
+        if (k == ~0ull) continue;
+        const uint64_t du = k >> B;
+        if (i > 0 && keys[i - 1] >> B == du) continue;
+        uint2 f = make_uint2(0, 0);
+        if (!clear) {
+            uint64_t step = 1;
+            while (i + step < real && keys[i + step] >> B == du) step <<= 1;
+            uint64_t lo = i + (step >> 1), hi = min(i + step, real);
+            while (hi - lo > 1) {
+                const uint64_t mid = (lo + hi) >> 1;
+                if (keys[mid] >> B == du) lo = mid; else hi = mid;
+            }
+            f = make_uint2((uint32_t)i, (uint32_t)(lo + 1 - i));
+        }
+        reinterpret_cast<uint2*>(rec + (size_t)(k >> (2 * B + lb)) * dvcap + (du & vmask))[1] = f;
     }
 }
+__global__ void k_delta_lists(uint64_t* keys, uint64_t n, const int* nsel, uint32_t B, uint32_t lb, uint4* rec,
+                              uint32_t dvcap, uint32_t* dval, int clear) {
+    delta_lists(keys, n, nsel, B, lb, rec, dvcap, dval, clear != 0, blockIdx.x, gridDim.x);
+}
 
-// Seed ranges: delta entries of direction seed_dir(ei) form one contiguous
-// range of the sorted packed delta array.
-__global__ void k_seed_ranges(const uint64_t* __restrict__ dkeys, uint64_t n, uint32_t B, uint32_t qe,
-                              const EdgePlan* __restrict__ plans, const uint8_t* qe_dirs /*[qe][2]*/,
-                              const uint8_t* edge_ok, int have_ok, uint32_t* seed_lo, uint32_t* seed_pre) {
-    __shared__ uint32_t cnt[kMaxQE];
-    const uint32_t t = threadIdx.x;
-    auto lower = [&](uint64_t key) {
+// Delta lists of the single-query engine and, in the last block, its seed
+// ranges: the delta entries of direction seed_dir(ei) form one contiguous
+// range of the sorted packed delta array.  One thread per range end (six per
+// query edge: the searches are chains of dependent loads).
+__global__ void __launch_bounds__(256) k_delta(uint64_t* dkeys, uint64_t n, uint32_t B, uint4* rec, uint32_t dvcap,
+                                               uint32_t* dval, uint32_t qe, const EdgePlan* __restrict__ plans,
+                                               const uint8_t* qe_dirs /*[qe][2]*/, const uint8_t* edge_ok, int have_ok,
+                                               uint32_t* seed_lo, uint32_t* seed_pre) {
+    if (blockIdx.x + 1 < gridDim.x) {
+        delta_lists(dkeys, n, nullptr, B, 0, rec, dvcap, dval, false, blockIdx.x, gridDim.x - 1);
+        return;
+    }
+    static_assert(cgb::kMaxQEKeyed * 6 <= 256, "one thread per range end");
+    __shared__ uint32_t s_at[cgb::kMaxQEKeyed][6];
+    __shared__ uint32_t s_cnt[cgb::kMaxQEKeyed];
+    const uint32_t t = threadIdx.x / 6, w = threadIdx.x % 6;
+    if (t < qe) {
+        const uint32_t d = w < 2 ? plans[t].seed_dir : qe_dirs[2 * t + (w < 4 ? 0 : 1)];
+        const uint64_t key = (uint64_t)(d + (w & 1u)) << (2 * B);
         uint64_t lo = 0, hi = n;
         while (lo < hi) {
-            uint64_t mid = (lo + hi) >> 1;
+            const uint64_t mid = (lo + hi) >> 1;
             if (dkeys[mid] < key) lo = mid + 1; else hi = mid;
         }
-        return (uint32_t)lo;
-    };
-    if (t < qe) {
-        uint32_t s = plans[t].seed_dir;
-        uint32_t lo = lower((uint64_t)s << (2 * B));
-        uint32_t hi = lower((uint64_t)(s + 1) << (2 * B));
-        uint32_t d0 = qe_dirs[2 * t], d1 = qe_dirs[2 * t + 1];
-        uint32_t c0 = lower((uint64_t)(d0 + 1) << (2 * B)) - lower((uint64_t)d0 << (2 * B));
-        uint32_t c1 = lower((uint64_t)(d1 + 1) << (2 * B)) - lower((uint64_t)d1 << (2 * B));
-        bool ok = have_ok ? (edge_ok[t] != 0) : (c0 > 0 && c1 > 0);
-        seed_lo[t] = lo;
-        cnt[t] = ok ? hi - lo : 0;
+        s_at[t][w] = (uint32_t)lo;
     }
     __syncthreads();
-    if (t == 0) {
+    if (threadIdx.x < qe) {
+        const uint32_t* p = s_at[threadIdx.x];
+        const bool ok = have_ok ? edge_ok[threadIdx.x] != 0 : p[3] > p[2] && p[5] > p[4];
+        seed_lo[threadIdx.x] = p[0];
+        s_cnt[threadIdx.x] = ok ? p[1] - p[0] : 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
         uint32_t acc = 0;
-        for (uint32_t e = 0; e < qe; ++e) { seed_pre[e] = acc; acc += cnt[e]; }
+        for (uint32_t e = 0; e < qe; ++e) { seed_pre[e] = acc; acc += s_cnt[e]; }
         seed_pre[qe] = acc;
     }
 }
@@ -561,7 +620,7 @@ constexpr size_t kRunBitsBytes = 512ull << 20;  // runs beyond this budget are s
 // Full rebuild: the slot of every (direction, vertex) of the table (all
 // dvcap rows) whose run is long enough, in claim order while slots last
 // (ctr[0] counts claims), else kNoSlot; sel[slot] = dir << 27 | vertex.
-// Afterwards each merge keeps the sets current (k_rb_fill_new, k_rb_edits).
+// Afterwards each merge keeps the sets current (k_rb_update).
 __global__ void k_rb_select(const uint4* __restrict__ rec, uint32_t dvcap, uint32_t nd, uint32_t min_len,
                             uint32_t cap, uint32_t* slot, uint32_t* sel, unsigned int* ctr) {
     const size_t n = (size_t)nd * dvcap;
@@ -603,33 +662,34 @@ __global__ void k_rb_fill(const uint4* __restrict__ rec, uint32_t dvcap, const u
     }
 }
 
-// Slots claimed by runs that grew past the length threshold in this merge
-// (ctr[1] of them, listed in fresh): zeroed, then filled from the merged run.
-__global__ void k_rb_fill_new(const uint4* __restrict__ rec, uint32_t dvcap, const uint32_t* __restrict__ pool,
-                              const uint32_t* __restrict__ sel, const uint32_t* __restrict__ fresh,
-                              const unsigned int* ctr, uint32_t* bits, uint32_t words) {
+// After a merge: slots claimed by runs that grew past the length threshold
+// (*newc of them, listed in fresh) are zeroed and filled from the merged run,
+// a warp each; and the merge's edits ((d,u,v) << 1 | op, each run's sorted) are
+// applied to every bit set: the last edit of each (d,u,v) decides, as in the
+// merge (an add sets the bit, a remove clears it).  Both may meet in a fresh
+// set in any order: the fill sets exactly the merged run's bits, an added value
+// is in it and a removed one is not.
+__global__ void k_rb_update(const uint4* __restrict__ rec, uint32_t dvcap, const uint32_t* __restrict__ pool,
+                            const uint32_t* __restrict__ sel, const uint32_t* __restrict__ fresh,
+                            const unsigned int* newc, uint32_t* bits, uint32_t words,
+                            const uint64_t* __restrict__ edits, uint64_t n, uint32_t B,
+                            const uint32_t* __restrict__ slot) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t n = ctr[1];
+    const uint32_t nnew = *newc;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n; q += nw) {
+    for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < nnew; q += nw) {
         const uint32_t c = fresh[q];
         const uint32_t du = sel[c];
         const uint4 r = rec[(size_t)(du >> 27) * dvcap + (du & ((1u << 27) - 1u))];
         uint32_t* b = bits + (size_t)c * words;
-        for (uint32_t t = lane; t < words; t += 32) b[t] = 0;
+        for (uint32_t t = lane; t < words; t += 32) atomicExch(b + t, 0u);
+        __threadfence();
         __syncwarp();
         for (uint32_t t = lane; t < r.y; t += 32) {
             const uint32_t v = __ldg(pool + r.x + t);
             atomicOr(b + (v >> 5), 1u << (v & 31));
         }
     }
-}
-
-// Applies a merge's sorted edits ((d,u,v) << 1 | op) to the bit sets of
-// runs that have one: the last edit of each (d,u,v) decides, as in the merge
-// (an add sets the bit, a remove clears it).
-__global__ void k_rb_edits(const uint64_t* __restrict__ edits, uint64_t n, uint32_t B, uint32_t dvcap,
-                           const uint32_t* __restrict__ slot, uint32_t* bits, uint32_t words) {
     const uint64_t vmask = (1ull << B) - 1ull;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t e = edits[i];
@@ -2175,28 +2235,23 @@ struct cgb_handle {
     uint32_t* pool = nullptr;
     uint32_t* pool_alt = nullptr;
     unsigned long long pool_cap = 0;
-    // device scalars: [0] pool_top, [1] live_words, [2] err, [3] work_next
+    // device scalars, one block (kCtl*): cleared by one memset from kCtlErr on
+    // at every batch, read back by one copy
     unsigned long long* d_scal = nullptr;
     unsigned int* d_self = nullptr;  // sticky: some added key was a self-loop (u == v)
-    unsigned long long* h_scal = nullptr;  // pinned mirror (4 scalars + counts)
+    unsigned long long* h_scal = nullptr;  // pinned mirror of d_scal
     unsigned long long h_pool_top = 0;
     long long h_live = 0;
 
     // per-batch buffers (grown on demand)
     uint64_t* d_keys_in = nullptr; size_t keys_in_cap = 0;       // uploaded ext keys (ins|del|delta)
-    uint64_t* d_pending = nullptr; size_t pending_cap = 0; uint64_t n_pending = 0;  // ext delta keys
+    uint64_t* d_pending = nullptr; size_t pending_cap = 0; uint64_t n_pending = 0;  // delta keys to merge back, packed (d,u,v) and sorted by run
+    uint32_t pending_B = 0;
     uint64_t* d_edits = nullptr; uint64_t* d_edits_alt = nullptr; size_t edits_cap = 0;
-    uint32_t* d_du = nullptr; uint32_t* d_run_du = nullptr; uint32_t* d_run_len = nullptr;
-    uint32_t* d_run_off = nullptr; size_t runs_cap = 0;
-    uint32_t* d_small_runs = nullptr; uint32_t* d_big_runs = nullptr;  // merge lists (k_merge_classify)
-    uint32_t* d_tiny_runs = nullptr;
-    unsigned int* d_list_ctr = nullptr;  // [0] small, [1] big, [2] tiny
-    int* d_num_runs = nullptr;
+    uint2* d_runs[3] = {nullptr, nullptr, nullptr};  // merge lists (k_edit_runs)
+    unsigned int* d_list_ctr = nullptr;  // [0] warp, [1] CTA, [2] lane, [3] bit-set slots claimed by the last merge
     uint64_t* d_dkeys = nullptr; uint64_t* d_dkeys_alt = nullptr; size_t dkeys_cap = 0;
     uint32_t* d_dval = nullptr;
-    uint32_t* d_ddu = nullptr;
-    uint32_t* d_drun_du = nullptr; uint32_t* d_drun_len = nullptr; uint32_t* d_drun_off = nullptr;
-    size_t druns_cap = 0;
     uint32_t* d_seed = nullptr;  // [0..kMaxQE) lo, [kMaxQE..2kMaxQE+1) pre
     unsigned long long* d_counts = nullptr;  // [kMaxQE]
     unsigned long long* d_stats = nullptr;   // [8]
@@ -2211,11 +2266,12 @@ struct cgb_handle {
     uint32_t* d_rb_sel = nullptr; size_t rb_sel_cap = 0;
     uint32_t* d_rb_bits = nullptr; size_t rb_bits_cap = 0;
     uint32_t* d_rb_new = nullptr; size_t rb_new_cap = 0;    // slots claimed by the last merge
-    unsigned int* d_rb_ctr = nullptr;  // [0] slots claimed, [1] claimed by the last merge
+    unsigned int* d_rb_ctr = nullptr;  // slots claimed
     uint32_t rb_words = 0;             // words per bit set: (dvcap + 31) / 32
     uint32_t rb_cap = 0;               // bit sets the budget holds
     bool rb_valid = false;             // slot table and bit sets match the index
     uint32_t rb_min_len = kRunBitsMinLen;
+    uint32_t rb_len_now = kRunBitsMinLen;  // doubled while the budget holds too few slots
     uint32_t pair_lane_max = kPairLaneMax;
     uint8_t* d_rev = nullptr;          // reverse direction of each direction
     uint32_t* d_touched = nullptr; size_t touched_cap = 0;  // footprint runs: record bit set
@@ -2248,6 +2304,11 @@ struct cgb_handle {
 };
 
 namespace {
+
+// Words of cgb_handle::d_scal.  The first three live as long as the handle.
+constexpr uint32_t kCtlPoolTop = 0, kCtlLive = 1, kCtlRbClaimed = 2, kCtlErr = 3, kCtlWork = 4, kCtlList = 5,
+                   kCtlStats = 8, kCtlCounts = 16, kCtlQueue = kCtlCounts + kMaxQE, kCtlWords = kCtlQueue + kQWords / 2;
+static_assert(kCtlQueue % 16 == 0, "the polled queue counters start a 128-byte line");
 
 cgb_status fail(cgb_handle* h, cgb_status s, const char* fmt, ...) {
     char buf[512];
@@ -2316,6 +2377,7 @@ cgb_status ensure_dvcap(cgb_handle* h, uint32_t dv) {
     h->rec = nr;
     h->dvcap = nc;
     h->rb_valid = false;  // the slot table and the bit sets follow the record layout
+    h->rb_len_now = h->rb_min_len;
     // level-sum table: about two slots per vertex, 2^12 to 2^24 slots (16 B each)
     uint32_t slots = 1u << 12;
     while (slots < (1u << 24) && slots < 2ull * nc) slots <<= 1;
@@ -2454,7 +2516,7 @@ cgb_status compact_pool(cgb_handle* h, unsigned long long new_cap) {
     }
     h->h_pool_top = live;
     h->h_live = (long long)live;
-    unsigned long long sc[2] = {live, live};
+    unsigned long long sc[2] = {live, live};  // kCtlPoolTop, kCtlLive
     CK(cudaMemcpyAsync(h->d_scal, sc, sizeof(sc), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     return CGB_OK;
@@ -2482,131 +2544,93 @@ cgb_status radix_sort(cgb_handle* h, uint64_t*& keys, uint64_t*& alt, uint64_t n
     return CGB_OK;
 }
 
-// Run-length segments of du over n sorted entries; offsets by exclusive scan.
-cgb_status segment(cgb_handle* h, const uint32_t* du, uint64_t n, uint32_t* run_du, uint32_t* run_len,
-                   uint32_t* run_off, int* num_runs) {
-    size_t tb = 0;
-    CK(cub::DeviceRunLengthEncode::Encode(nullptr, tb, du, run_du, run_len, num_runs, (int64_t)n, h->stream));
-    size_t tb2 = 0;
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, tb2, run_len, run_off, (int64_t)n, h->stream));
-    if (grow_temp(h, std::max(tb, tb2)) != CGB_OK) return CGB_ERR_OOM;
-    CK(cub::DeviceRunLengthEncode::Encode(h->d_temp, tb, du, run_du, run_len, num_runs, (int64_t)n, h->stream));
-    LAUNCHED();
-    // scanning n entries (runs beyond num_runs hold garbage but are never read)
-    CK(cub::DeviceScan::ExclusiveSum(h->d_temp, tb2, run_len, run_off, (int64_t)n, h->stream));
-    LAUNCHED();
-    return CGB_OK;
-}
-
 // Grow-only per-batch buffers (reallocated only when a batch is larger than any before).
 cgb_status ensure_edit_buffers(cgb_handle* h, uint64_t n) {
     if (n <= h->edits_cap && h->d_edits) return CGB_OK;
     size_t nc = std::max<size_t>(n + n / 2, 1 << 16);
     CK(cudaStreamSynchronize(h->stream));
-    void* olds[] = {h->d_edits, h->d_edits_alt, h->d_du, h->d_run_du, h->d_run_len, h->d_run_off,
-                    h->d_small_runs, h->d_big_runs, h->d_tiny_runs};
+    void* olds[] = {h->d_edits, h->d_edits_alt, h->d_runs[0], h->d_runs[1], h->d_runs[2]};
     for (void* p : olds) if (p) CK(cudaFree(p));
-    CK(cudaMalloc(&h->d_tiny_runs, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_small_runs, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_big_runs, nc * sizeof(uint32_t)));
+    for (auto& p : h->d_runs) p = nullptr;
+    h->d_edits = h->d_edits_alt = nullptr;
+    h->edits_cap = 0;
     CK(cudaMalloc(&h->d_edits, nc * sizeof(uint64_t)));
     CK(cudaMalloc(&h->d_edits_alt, nc * sizeof(uint64_t)));
-    CK(cudaMalloc(&h->d_du, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_run_du, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_run_len, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_run_off, nc * sizeof(uint32_t)));
+    for (auto& p : h->d_runs) CK(cudaMalloc(&p, nc * sizeof(uint2)));
     h->edits_cap = nc;
-    h->runs_cap = nc;
     return CGB_OK;
 }
 
+// The kept delta's buffer is one of them (same size: it changes places with
+// the sorted keys after a batch); it is free here, merged back before.
 cgb_status ensure_delta_buffers(cgb_handle* h, uint64_t n) {
     if (n <= h->dkeys_cap && h->d_dkeys) return CGB_OK;
     size_t nc = std::max<size_t>(n + n / 2, 1 << 16);
     CK(cudaStreamSynchronize(h->stream));
-    void* olds[] = {h->d_dkeys, h->d_dkeys_alt, h->d_dval, h->d_ddu, h->d_drun_du, h->d_drun_len, h->d_drun_off};
+    void* olds[] = {h->d_dkeys, h->d_dkeys_alt, h->d_pending, h->d_dval};
     for (void* p : olds) if (p) CK(cudaFree(p));
+    h->d_dkeys = h->d_dkeys_alt = h->d_pending = nullptr;
+    h->d_dval = nullptr;
+    h->dkeys_cap = h->pending_cap = 0;
+    CK(cudaMalloc(&h->d_pending, nc * sizeof(uint64_t)));
     CK(cudaMalloc(&h->d_dkeys, nc * sizeof(uint64_t)));
     CK(cudaMalloc(&h->d_dkeys_alt, nc * sizeof(uint64_t)));
     CK(cudaMalloc(&h->d_dval, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_ddu, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_drun_du, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_drun_len, nc * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_drun_off, nc * sizeof(uint32_t)));
-    h->dkeys_cap = nc;
-    h->druns_cap = nc;
+    h->dkeys_cap = h->pending_cap = nc;
     return CGB_OK;
 }
 
-// Applies edits = adds0 (ext keys, device) + adds1 + removes to the index.
-cgb_status apply_edits(cgb_handle* h, const uint64_t* adds0, uint64_t n0, const uint64_t* adds1, uint64_t n1,
-                       const uint64_t* rems, uint64_t n2) {
-    const uint64_t n = n0 + n1 + n2;
+// Applies the edits to the index.  Packed edits alone are in run order already
+// (they were sorted as a delta) and are not sorted again.
+cgb_status apply_edits(cgb_handle* h, const EditSrc& src) {
+    const uint64_t n = src.n_packed + src.n_add + src.n_rem;
     if (n == 0) return CGB_OK;
     cgb_status s;
     if ((s = reserve_pool(h, n)) != CGB_OK) return s;
     if ((s = ensure_edit_buffers(h, n)) != CGB_OK) return s;
     PackInfo pi{bits_for(h->dv), h->nd, h->dv, h->mq ? 1u : 0u};
-    unsigned int* d_err = (unsigned int*)(h->d_scal + 2);
-    if (n0) { k_pack_edits<<<grid_for(h, n0), 256, 0, h->stream>>>(adds0, n0, 0, pi, h->d_edits, d_err, h->d_self); LAUNCHED(); }
-    if (n1) { k_pack_edits<<<grid_for(h, n1), 256, 0, h->stream>>>(adds1, n1, 0, pi, h->d_edits + n0, d_err, h->d_self); LAUNCHED(); }
-    if (n2) { k_pack_edits<<<grid_for(h, n2), 256, 0, h->stream>>>(rems, n2, 1, pi, h->d_edits + n0 + n1, d_err, h->d_self); LAUNCHED(); }
+    unsigned int* d_err = (unsigned int*)(h->d_scal + kCtlErr);
+    k_pack_edits<<<grid_for(h, n), 256, 0, h->stream>>>(src, pi, h->d_edits, d_err, h->d_self);
+    LAUNCHED();
     CK(cudaGetLastError());
     // valid keys use 2B+6 bits; one more bit makes the all-ones invalid marker sort last
-    if ((s = radix_sort(h, h->d_edits, h->d_edits_alt, n, 2 * (int)pi.B + 7)) != CGB_OK) return s;
-    k_extract_du<<<grid_for(h, n), 256, 0, h->stream>>>(h->d_edits, n, pi.B + 1, h->d_du);
-    LAUNCHED();
-    if ((s = segment(h, h->d_du, n, h->d_run_du, h->d_run_len, h->d_run_off, h->d_num_runs)) != CGB_OK) return s;
+    if (src.n_add + src.n_rem)
+        if ((s = radix_sort(h, h->d_edits, h->d_edits_alt, n, 2 * (int)pi.B + 7)) != CGB_OK) return s;
     MergeArgs ma;
     ma.rec = h->rec;
     ma.dvcap = h->dvcap;
     ma.pool = h->pool;
-    ma.pool_top = h->d_scal + 0;
+    ma.pool_top = h->d_scal + kCtlPoolTop;
     ma.pool_cap = h->pool_cap;
-    ma.live_words = (long long*)(h->d_scal + 1);
+    ma.live_words = (long long*)(h->d_scal + kCtlLive);
     ma.edits = h->d_edits;
-    ma.run_du = h->d_run_du;
-    ma.run_len = h->d_run_len;
-    ma.run_off = h->d_run_off;
-    ma.num_runs = h->d_num_runs;
-    ma.small_runs = h->d_small_runs;
-    ma.big_runs = h->d_big_runs;
-    ma.tiny_runs = h->d_tiny_runs;
+    ma.n = n;
+    for (int k = 0; k < 3; ++k) ma.runs[k] = h->d_runs[k];
     ma.list_ctr = h->d_list_ctr;
     ma.B = pi.B;
     ma.err = d_err;
     ma.stats = h->d_stats;
-    // bit sets are kept current by the merge once built (k_rb_fill_new, k_rb_edits)
+    // bit sets are kept current by the merge once built (k_rb_update)
     const bool rb = h->rb_valid && !(h->cfg.flags & CGB_FLAG_NO_RUN_BITS);
     ma.rb_slot = rb ? h->d_rb_slot : nullptr;
     ma.rb_sel = h->d_rb_sel;
     ma.rb_ctr = h->d_rb_ctr;
-    ma.rb_new = h->d_rb_new;
+    ma.rb_newc = h->d_list_ctr + 3;
     ma.rb_cap = h->rb_cap;
-    ma.rb_min_len = h->rb_min_len;
-    if (rb) {
-        if ((s = grow(h, h->d_rb_new, h->rb_new_cap, std::max<size_t>(h->rb_cap, 1))) != CGB_OK) return s;
-        ma.rb_new = h->d_rb_new;
-        CK(cudaMemsetAsync(h->d_rb_ctr + 1, 0, sizeof(unsigned int), h->stream));
-    }
-    CK(cudaMemsetAsync(h->d_list_ctr, 0, 3 * sizeof(unsigned int), h->stream));
-    k_merge_classify<<<grid_for(h, n), 256, 0, h->stream>>>(ma);
+    ma.rb_min_len = h->rb_len_now;
+    if (rb && (s = grow(h, h->d_rb_new, h->rb_new_cap, std::max<size_t>(h->rb_cap, 1))) != CGB_OK) return s;
+    ma.rb_new = h->d_rb_new;
+    CK(cudaMemsetAsync(h->d_list_ctr, 0, 4 * sizeof(unsigned int), h->stream));
+    k_edit_runs<<<grid_for(h, n), 256, 0, h->stream>>>(ma);
     LAUNCHED();
-    k_merge_tiny<<<grid_for(h, n), 256, 0, h->stream>>>(ma);
-    LAUNCHED();
-    const int mg = std::max(1, std::min<int>((int)((n * 32 + 255) / 256), h->num_sms * 16));
-    k_merge_runs<<<mg, 256, 0, h->stream>>>(ma);
-    LAUNCHED();
-    // hub runs: one CTA each (at most n / kBigRun of them)
-    const int bg = (int)std::max<uint64_t>(1, std::min<uint64_t>(n / kBigRun + 1, (uint64_t)h->num_sms * 2));
-    k_merge_big<<<bg, kMergeWarps * 32, 0, h->stream>>>(ma);
+    // a warp per run at most, up to the blocks that can be resident
+    const int mg = std::max(1, (int)std::min<uint64_t>((n * 32 + 255) / 256, (uint64_t)h->num_sms * 8));
+    k_merge<<<mg, kMergeWarps * 32, 0, h->stream>>>(ma);
     LAUNCHED();
     if (rb) {
-        k_rb_fill_new<<<h->num_sms * 4, 256, 0, h->stream>>>(h->rec, h->dvcap, h->pool, h->d_rb_sel, h->d_rb_new,
-                                                           h->d_rb_ctr, h->d_rb_bits, h->rb_words);
-        LAUNCHED();
-        k_rb_edits<<<grid_for(h, n), 256, 0, h->stream>>>(h->d_edits, n, pi.B, h->dvcap, h->d_rb_slot,
-                                                           h->d_rb_bits, h->rb_words);
+        k_rb_update<<<std::max(grid_for(h, n), h->num_sms), 256, 0, h->stream>>>(
+            h->rec, h->dvcap, h->pool, h->d_rb_sel, h->d_rb_new, h->d_list_ctr + 3, h->d_rb_bits, h->rb_words,
+            h->d_edits, n, pi.B, h->d_rb_slot);
         LAUNCHED();
     }
     CK(cudaGetLastError());
@@ -2625,9 +2649,9 @@ cgb_status rebuild_run_bits(cgb_handle* h) {
     if ((s = grow(h, h->d_rb_slot, h->rb_slot_cap, (size_t)h->nd * h->dvcap)) != CGB_OK) return s;
     if ((s = grow(h, h->d_rb_sel, h->rb_sel_cap, (size_t)cap)) != CGB_OK) return s;
     if ((s = grow(h, h->d_rb_bits, h->rb_bits_cap, (size_t)cap * h->rb_words)) != CGB_OK) return s;
-    CK(cudaMemsetAsync(h->d_rb_ctr, 0, 2 * sizeof(unsigned int), h->stream));
+    CK(cudaMemsetAsync(h->d_rb_ctr, 0, sizeof(unsigned int), h->stream));
     k_rb_select<<<grid_for(h, (uint64_t)h->nd * h->dvcap), 256, 0, h->stream>>>(
-        h->rec, h->dvcap, h->nd, h->rb_min_len, cap, h->d_rb_slot, h->d_rb_sel, h->d_rb_ctr);
+        h->rec, h->dvcap, h->nd, h->rb_len_now, cap, h->d_rb_slot, h->d_rb_sel, h->d_rb_ctr);
     LAUNCHED();
     k_rb_zero<<<h->num_sms * 8, 256, 0, h->stream>>>(h->d_rb_bits, h->rb_words, cap, h->d_rb_ctr);
     LAUNCHED();
@@ -2640,23 +2664,28 @@ cgb_status rebuild_run_bits(cgb_handle* h) {
 }
 
 cgb_status sync_scalars(cgb_handle* h) {
-    CK(cudaMemcpyAsync(h->h_scal, h->d_scal, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(h->h_scal + 4, h->d_counts, kMaxQE * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                       h->stream));
-    CK(cudaMemcpyAsync(h->h_scal + 4 + kMaxQE, h->d_stats, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                       h->stream));
-    CK(cudaMemcpyAsync(h->h_scal + 12 + kMaxQE, h->d_rb_ctr, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(h->h_scal, h->d_scal, kCtlQueue * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    // every slot claimed: rebuild on the next batch, so today's long runs get them
-    if (h->rb_valid && (uint32_t)h->h_scal[12 + kMaxQE] >= h->rb_cap) h->rb_valid = false;
-    h->h_pool_top = h->h_scal[0];
-    h->h_live = (long long)h->h_scal[1];
+    // every slot claimed: rebuild on the next batch with runs of twice the
+    // length, so the longest runs of the index get them (at one length the
+    // sets were rebuilt on every batch: 0.55 ms of a 16 ms batch on R-MAT
+    // 2M/17M with 32 labels)
+    if (h->rb_valid && (uint32_t)h->h_scal[kCtlRbClaimed] >= h->rb_cap) {
+        h->rb_valid = false;
+        if (h->rb_len_now < (1u << 26)) h->rb_len_now *= 2;
+    }
+    h->h_pool_top = h->h_scal[kCtlPoolTop];
+    h->h_live = (long long)h->h_scal[kCtlLive];
     return CGB_OK;
 }
 
 cgb_status flush_pending(cgb_handle* h) {
     if (h->n_pending == 0) return CGB_OK;
-    cgb_status s = apply_edits(h, h->d_pending, h->n_pending, nullptr, 0, nullptr, 0);
+    EditSrc src;
+    src.packed = h->d_pending;
+    src.n_packed = h->n_pending;
+    src.B0 = h->pending_B;
+    cgb_status s = apply_edits(h, src);
     if (s != CGB_OK) return s;
     h->n_pending = 0;
     return sync_scalars(h);
@@ -2677,7 +2706,7 @@ cgb_status cgb_create(const cgb_config* cfg, cgb_handle** out) {
     cgb_handle* h = new cgb_handle();
     if (cfg) h->cfg = *cfg; else cgb_default_config(&h->cfg);
     h->device = h->cfg.device;
-    if (const char* e = std::getenv("CGB_RUN_BITS_MIN_LEN")) h->rb_min_len = (uint32_t)std::max(1l, std::atol(e));
+    if (const char* e = std::getenv("CGB_RUN_BITS_MIN_LEN")) h->rb_len_now = h->rb_min_len = (uint32_t)std::max(1l, std::atol(e));
     if (const char* e = std::getenv("CGB_PAIR_LANE_MAX")) h->pair_lane_max = (uint32_t)std::max(0l, std::atol(e));
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);
@@ -2693,21 +2722,19 @@ cgb_status cgb_create(const cgb_config* cfg, cgb_handle** out) {
     CKC(cudaDeviceGetAttribute(&h->clock_khz, cudaDevAttrClockRate, h->device));
     CKC(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
-    CKC(cudaMalloc(&h->d_scal, 4 * sizeof(unsigned long long)));
-    CKC(cudaMemset(h->d_scal, 0, 4 * sizeof(unsigned long long)));
+    CKC(cudaMalloc(&h->d_scal, kCtlWords * sizeof(unsigned long long)));
+    CKC(cudaMemset(h->d_scal, 0, kCtlWords * sizeof(unsigned long long)));
+    h->d_rb_ctr = (unsigned int*)(h->d_scal + kCtlRbClaimed);
+    h->d_list_ctr = (unsigned int*)(h->d_scal + kCtlList);
+    h->d_stats = h->d_scal + kCtlStats;
+    h->d_counts = h->d_scal + kCtlCounts;
+    h->d_qctr = (unsigned int*)(h->d_scal + kCtlQueue);
     CKC(cudaMalloc(&h->d_self, sizeof(unsigned int)));
     CKC(cudaMemset(h->d_self, 0, sizeof(unsigned int)));
-    CKC(cudaMallocHost(&h->h_scal, (16 + kMaxQE) * sizeof(unsigned long long)));
-    CKC(cudaMalloc(&h->d_num_runs, 2 * sizeof(int)));
-    CKC(cudaMalloc(&h->d_list_ctr, 3 * sizeof(unsigned int)));
-    CKC(cudaMalloc(&h->d_rb_ctr, 2 * sizeof(unsigned int)));
-    CKC(cudaMemset(h->d_rb_ctr, 0, 2 * sizeof(unsigned int)));
+    CKC(cudaMallocHost(&h->h_scal, kCtlWords * sizeof(unsigned long long)));
     CKC(cudaMalloc(&h->d_rev, kMaxDir));
     CKC(cudaMalloc(&h->d_seed, (3 * kMaxQE + 2) * sizeof(uint32_t)));
-    CKC(cudaMalloc(&h->d_counts, kMaxQE * sizeof(unsigned long long)));
-    CKC(cudaMalloc(&h->d_stats, 8 * sizeof(unsigned long long)));
     CKC(cudaMalloc(&h->d_tasks, (size_t)kTaskCap * kTaskWords * sizeof(uint32_t)));
-    CKC(cudaMalloc(&h->d_qctr, kQWords * sizeof(unsigned int)));
     CKC(cudaMemset(h->d_tasks, 0, (size_t)kTaskCap * kTaskWords * sizeof(uint32_t)));
     CKC(cudaMalloc(&h->d_qe_dirs, 2 * kMaxQE));
     CKC(cudaMalloc(&h->d_edge_ok, kMaxQE));
@@ -2725,11 +2752,10 @@ void cgb_destroy(cgb_handle* h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     void* ptrs[] = {h->rec, h->pool, h->pool_alt, h->d_scal, h->d_self, h->d_keys_in, h->d_pending, h->d_edits,
-                    h->d_edits_alt, h->d_du, h->d_run_du, h->d_run_len, h->d_run_off, h->d_num_runs,
-                    h->d_dkeys, h->d_dkeys_alt, h->d_dval, h->d_ddu, h->d_drun_du, h->d_drun_len, h->d_drun_off,
-                    h->d_seed, h->d_counts, h->d_stats, h->d_tasks, h->d_qctr, h->d_temp, h->d_qe_dirs, h->d_edge_ok,
-                    h->d_vb, h->d_rb_slot, h->d_rb_sel, h->d_rb_bits, h->d_rb_ctr, h->d_rb_new, h->d_small_runs,
-                    h->d_big_runs, h->d_tiny_runs, h->d_list_ctr, h->d_rev, h->d_touched, h->d_plans,
+                    h->d_edits_alt, h->d_runs[0], h->d_runs[1], h->d_runs[2],
+                    h->d_dkeys, h->d_dkeys_alt, h->d_dval,
+                    h->d_seed, h->d_tasks, h->d_temp, h->d_qe_dirs, h->d_edge_ok,
+                    h->d_vb, h->d_rb_slot, h->d_rb_sel, h->d_rb_bits, h->d_rb_new, h->d_rev, h->d_touched, h->d_plans,
                     h->d_vbplans, h->d_dir_edge, h->d_lsum, h->d_wsum, h->d_wjobs};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -2833,12 +2859,15 @@ cgb_status cgb_build_index(cgb_handle* h, const uint64_t* keys, uint64_t n, uint
     h->pool_cap = cap;
     h->h_pool_top = 0;
     h->h_live = 0;
-    CK(cudaMemsetAsync(h->d_scal, 0, 4 * sizeof(unsigned long long), h->stream));
+    CK(cudaMemsetAsync(h->d_scal, 0, kCtlWords * sizeof(unsigned long long), h->stream));
     if ((s = grow(h, h->d_keys_in, h->keys_in_cap, std::max<uint64_t>(n, 1))) != CGB_OK) return s;
     if (n) CK(cudaMemcpyAsync(h->d_keys_in, keys, n * sizeof(uint64_t), cudaMemcpyHostToDevice, h->stream));
-    if ((s = apply_edits(h, h->d_keys_in, n, nullptr, 0, nullptr, 0)) != CGB_OK) return s;
+    EditSrc src;
+    src.add = h->d_keys_in;
+    src.n_add = n;
+    if ((s = apply_edits(h, src)) != CGB_OK) return s;
     if ((s = sync_scalars(h)) != CGB_OK) return s;
-    if (h->h_scal[2]) return fail(h, CGB_ERR_ARG, "invalid keys (error bits %llu)", h->h_scal[2]);
+    if (h->h_scal[kCtlErr]) return fail(h, CGB_ERR_ARG, "invalid keys (error bits %llu)", h->h_scal[kCtlErr]);
     h->have_index = true;
     return CGB_OK;
 }
@@ -2866,15 +2895,20 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
     h->dv = dv_count;
     const uint32_t B = bits_for(dv_count);
     PackInfo pi{B, h->nd, dv_count};
-    unsigned int* d_err = (unsigned int*)(h->d_scal + 2);
-    CK(cudaMemsetAsync(h->d_scal + 2, 0, 2 * sizeof(unsigned long long), h->stream));
-    CK(cudaMemsetAsync(h->d_counts, 0, kMaxQE * sizeof(unsigned long long), h->stream));
-    CK(cudaMemsetAsync(h->d_stats, 0, 8 * sizeof(unsigned long long), h->stream));
-    CK(cudaMemsetAsync(h->d_qctr, 0, kQWords * sizeof(unsigned int), h->stream));
+    unsigned int* d_err = (unsigned int*)(h->d_scal + kCtlErr);
+    CK(cudaMemsetAsync(h->d_scal + kCtlErr, 0, (kCtlWords - kCtlErr) * sizeof(unsigned long long), h->stream));
     CK(cudaEventRecord(h->ev[0], h->stream));
 
     // 1. index update: pending delta (add) + ins (add) + del (remove)
-    if ((s = apply_edits(h, h->d_pending, h->n_pending, ins, n_ins, del, n_del)) != CGB_OK) return s;
+    EditSrc src;
+    src.packed = h->d_pending;
+    src.n_packed = h->n_pending;
+    src.B0 = h->pending_B;
+    src.add = ins;
+    src.n_add = n_ins;
+    src.rem = del;
+    src.n_rem = n_del;
+    if ((s = apply_edits(h, src)) != CGB_OK) return s;
     h->n_pending = 0;
     CK(cudaEventRecord(h->ev[1], h->stream));
 
@@ -2882,22 +2916,13 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
     const bool match = n_delta > 0;
     if (match) {
         if ((s = ensure_delta_buffers(h, n_delta)) != CGB_OK) return s;
-        uint32_t* du = h->d_ddu;
         k_pack_delta<<<grid_for(h, n_delta), 256, 0, h->stream>>>(delta, n_delta, pi, h->d_dkeys, d_err, h->d_self);
         LAUNCHED();
         if ((s = radix_sort(h, h->d_dkeys, h->d_dkeys_alt, n_delta, 2 * (int)B + 6)) != CGB_OK) return s;
-        k_delta_values<<<grid_for(h, n_delta), 256, 0, h->stream>>>(h->d_dkeys, n_delta, (1ull << B) - 1, h->d_dval);
-        LAUNCHED();
-        k_extract_du<<<grid_for(h, n_delta), 256, 0, h->stream>>>(h->d_dkeys, n_delta, B, du);
-        LAUNCHED();
-        if ((s = segment(h, du, n_delta, h->d_drun_du, h->d_drun_len, h->d_drun_off, h->d_num_runs + 1)) != CGB_OK)
-            return s;
-        k_delta_recs<<<grid_for(h, n_delta), 256, 0, h->stream>>>(h->rec, h->dvcap, h->d_drun_du, h->d_drun_len,
-                                                                   h->d_drun_off, h->d_num_runs + 1, B, 0);
-        LAUNCHED();
         if (edge_ok) CK(cudaMemcpyAsync(h->d_edge_ok, edge_ok, h->q.qe, cudaMemcpyHostToDevice, h->stream));
-        k_seed_ranges<<<1, 32, 0, h->stream>>>(h->d_dkeys, n_delta, B, h->q.qe, h->d_plans, h->d_qe_dirs, h->d_edge_ok,
-                                               edge_ok ? 1 : 0, h->d_seed, h->d_seed + kMaxQE);
+        k_delta<<<grid_for(h, n_delta) + 1, 256, 0, h->stream>>>(h->d_dkeys, n_delta, B, h->rec, h->dvcap, h->d_dval,
+                                                                 h->q.qe, h->d_plans, h->d_qe_dirs, h->d_edge_ok,
+                                                                 edge_ok ? 1 : 0, h->d_seed, h->d_seed + kMaxQE);
         LAUNCHED();
         CK(cudaGetLastError());
         const bool vb_on = (h->cfg.flags & (CGB_FLAG_VALID_BITS | CGB_FLAG_MASK_PRUNE)) != 0;
@@ -2945,7 +2970,7 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
         da.seed_lo = h->d_seed;
         da.seed_pre = h->d_seed + kMaxQE;
         da.counts = h->d_counts;
-        da.work_next = (unsigned int*)(h->d_scal + 3);
+        da.work_next = (unsigned int*)(h->d_scal + kCtlWork);
         da.err = d_err;
         da.stats = h->d_stats;
         da.tasks = h->d_tasks;
@@ -3016,11 +3041,11 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
         }
 
         // 4. clear delta records; this delta becomes the pending merge-back
-        k_delta_recs<<<grid_for(h, n_delta), 256, 0, h->stream>>>(h->rec, h->dvcap, h->d_drun_du, h->d_drun_len,
-                                                                   h->d_drun_off, h->d_num_runs + 1, B, 1);
+        k_delta_lists<<<grid_for(h, n_delta), 256, 0, h->stream>>>(h->d_dkeys, n_delta, nullptr, B, 0, h->rec,
+                                                                   h->dvcap, nullptr, 1);
         LAUNCHED();
-        if ((s = grow(h, h->d_pending, h->pending_cap, n_delta)) != CGB_OK) return s;
-        CK(cudaMemcpyAsync(h->d_pending, delta, n_delta * sizeof(uint64_t), cudaMemcpyDeviceToDevice, h->stream));
+        std::swap(h->d_pending, h->d_dkeys);  // the sorted delta itself: nothing is copied
+        h->pending_B = B;
         h->n_pending = n_delta;
     } else {
         CK(cudaEventRecord(h->ev[2], h->stream));
@@ -3036,19 +3061,19 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
     h->last_vb_ms = 0;
     if (h->vb_stride) cudaEventElapsedTime(&h->last_vb_ms, h->ev[6], h->ev[2]);
     h->last_t[0] = t01; h->last_t[1] = t12; h->last_t[2] = t23; h->last_t[3] = t03;
-    for (int i = 0; i < 8; ++i) h->last_stats[i] = h->h_scal[4 + kMaxQE + i];
-    if (h->h_scal[2]) {
+    for (int i = 0; i < 8; ++i) h->last_stats[i] = h->h_scal[kCtlStats + i];
+    if (h->h_scal[kCtlErr]) {
         h->n_pending = 0;
         h->rb_valid = false;  // a rejected batch may have left runs and bit sets apart
-        cgb_status st = (h->h_scal[2] & 24u) ? CGB_ERR_TIMEOUT : (h->h_scal[2] & 4u) ? CGB_ERR_OOM : CGB_ERR_ARG;
+        cgb_status st = (h->h_scal[kCtlErr] & 24u) ? CGB_ERR_TIMEOUT : (h->h_scal[kCtlErr] & 4u) ? CGB_ERR_OOM : CGB_ERR_ARG;
         return fail(h, st,
                     "batch rejected: error bits %llu (1/2 = key out of range, 4 = pool exhausted, "
                     "8 = matching exceeded its time budget, 16 = a queued task was never published)",
-                    h->h_scal[2]);
+                    h->h_scal[kCtlErr]);
     }
     uint64_t total = 0;
-    for (uint32_t e = 0; e < h->q.qe; ++e) { h->last_counts[e] = h->h_scal[4 + e]; total += h->h_scal[4 + e]; }
-    for (int i = 0; i < 8; ++i) h->last_stats[i] = h->h_scal[4 + kMaxQE + i];
+    for (uint32_t e = 0; e < h->q.qe; ++e) { h->last_counts[e] = h->h_scal[kCtlCounts + e]; total += h->h_scal[kCtlCounts + e]; }
+    for (int i = 0; i < 8; ++i) h->last_stats[i] = h->h_scal[kCtlStats + i];
     *out_count = total;
     if (h->cfg.flags & CGB_FLAG_NO_MERGE_BACK_DEFER) {
         if ((s = flush_pending(h)) != CGB_OK) return s;

@@ -94,33 +94,14 @@ __global__ void k_mq_mark(const uint64_t* __restrict__ P, uint64_t n, const uint
     }
 }
 
-// Run key (label(y) << B | x) of every packed delta key (all ones for
-// padding): the delta runs are the runs of equal keys, since the source label
-// between them is a function of x.
-__global__ void k_mq_extract_du(const uint64_t* __restrict__ P, uint64_t n, uint32_t B, uint32_t lb,
-                                uint32_t* __restrict__ du) {
-    const uint64_t vmask = (1ull << B) - 1ull;
+// (d,u,v) keys of packed delta keys (the label bits between d and u dropped):
+// the order of the runs changes nothing for the merge; padding stays all ones.
+__global__ void k_mq_strip(const uint64_t* __restrict__ P, uint64_t n, uint32_t B, uint32_t lb,
+                           uint64_t* __restrict__ out) {
+    const uint64_t m = (1ull << (2 * B)) - 1ull;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t k = P[i];
-        du[i] = k == ~0ull ? 0xffffffffu : (uint32_t)(((k >> (2 * B + lb)) << B) | ((k >> B) & vmask));
-    }
-}
-
-// Entries [*nsel, n) of the selected keys become padding (all ones, sorted last).
-__global__ void k_mq_pad(uint64_t* P, uint64_t n, const int* nsel) {
-    for (uint64_t i = (uint64_t)*nsel + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        P[i] = ~0ull;
-}
-
-// Index keys (dir << 59 | u << 32 | v) of packed delta keys; padding stays all ones.
-__global__ void k_mq_unpack(const uint64_t* __restrict__ P, uint64_t n, uint32_t B, uint32_t lb,
-                            uint64_t* __restrict__ ext) {
-    const uint64_t vmask = (1ull << B) - 1ull;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = P[i];
-        ext[i] = k == ~0ull ? ~0ull
-                            : ((k >> (2 * B + lb)) << 59) | (((k >> B) & vmask) << 32) | (k & vmask);
+        out[i] = k == ~0ull ? ~0ull : ((k >> (2 * B + lb)) << (2 * B)) | (k & m);
     }
 }
 
@@ -360,7 +341,7 @@ cgb_status mq_prepare_delta(cgb_mq* m, const uint32_t* pairs, uint64_t mpairs, b
     const uint64_t n = 2 * mpairs;
     *n2 = n;
     const uint32_t B = bits_for(h->dv);
-    unsigned int* d_err = (unsigned int*)(h->d_scal + 2);
+    unsigned int* d_err = (unsigned int*)(h->d_scal + kCtlErr);
     MQ_TRY(ensure_delta_buffers(h, n));
     if (n > m->sel_cap || !m->d_sel) {
         if (m->d_sel) MCK(cudaFree(m->d_sel));
@@ -382,15 +363,8 @@ cgb_status mq_prepare_delta(cgb_mq* m, const uint32_t* pairs, uint64_t mpairs, b
     MCK(cub::DeviceSelect::Flagged(h->d_temp, tb, h->d_dkeys, m->d_keep, m->d_sel, m->d_nsel, (int64_t)n,
                                    h->stream));
     LAUNCHED();
-    k_mq_pad<<<grid_for(h, n), 256, 0, h->stream>>>(m->d_sel, n, m->d_nsel);
-    LAUNCHED();
-    k_delta_values<<<grid_for(h, n), 256, 0, h->stream>>>(m->d_sel, n, (1ull << B) - 1, h->d_dval);
-    LAUNCHED();
-    k_mq_extract_du<<<grid_for(h, n), 256, 0, h->stream>>>(m->d_sel, n, B, h->lb, h->d_ddu);
-    LAUNCHED();
-    MQ_TRY(segment(h, h->d_ddu, n, h->d_drun_du, h->d_drun_len, h->d_drun_off, h->d_num_runs + 1));
-    k_delta_recs<<<grid_for(h, n), 256, 0, h->stream>>>(h->rec, h->dvcap, h->d_drun_du, h->d_drun_len,
-                                                        h->d_drun_off, h->d_num_runs + 1, B, 0);
+    k_delta_lists<<<grid_for(h, n), 256, 0, h->stream>>>(m->d_sel, n, m->d_nsel, B, h->lb, h->rec, h->dvcap, h->d_dval,
+                                                         0);
     LAUNCHED();
     MCK(cudaGetLastError());
     return CGB_OK;
@@ -410,8 +384,8 @@ DfsArgs mq_dfs_args(cgb_mq* m, const EdgePlan* plans, uint32_t G, uint64_t budge
     da.seed_lo = m->d_seed;
     da.seed_pre = m->d_seed + m->plan_cap;
     da.counts = m->d_counts;
-    da.work_next = (unsigned int*)(h->d_scal + 3);
-    da.err = (unsigned int*)(h->d_scal + 2);
+    da.work_next = (unsigned int*)(h->d_scal + kCtlWork);
+    da.err = (unsigned int*)(h->d_scal + kCtlErr);
     da.stats = h->d_stats;
     da.tasks = h->d_tasks;
     da.task_cap = kTaskCap;
@@ -448,7 +422,7 @@ cgb_status mq_match_enqueue(cgb_mq* m, const EdgePlan* plans, const uint16_t* pa
                             int bps, bool steal, uint64_t budget_ms, bool clear = true) {
     cgb_handle* h = m->h;
     const uint32_t B = bits_for(h->dv);
-    MCK(cudaMemsetAsync(h->d_scal + 3, 0, sizeof(unsigned long long), h->stream));
+    MCK(cudaMemsetAsync(h->d_scal + kCtlWork, 0, sizeof(unsigned long long), h->stream));
     MCK(cudaMemsetAsync(m->d_counts, 0, std::max<uint32_t>(G, 1) * sizeof(unsigned long long), h->stream));
     MCK(cudaMemsetAsync(h->d_qctr, 0, kQWords * sizeof(unsigned int), h->stream));
     k_mq_seed_ranges<<<1, kMqSeedThreads, 0, h->stream>>>(m->d_sel, m->d_nsel, B, pair, G, m->d_seed,
@@ -463,8 +437,8 @@ cgb_status mq_match_enqueue(cgb_mq* m, const EdgePlan* plans, const uint16_t* pa
     // fixed grid (grid-stride over the runs counted on the device): the step's
     // launch arguments do not depend on the batch size
     if (clear) {
-        k_delta_recs<<<h->num_sms * 8, 256, 0, h->stream>>>(h->rec, h->dvcap, h->d_drun_du, h->d_drun_len,
-                                                            h->d_drun_off, h->d_num_runs + 1, B, 1);
+        k_delta_lists<<<h->num_sms * 8, 256, 0, h->stream>>>(m->d_sel, 0, m->d_nsel, B, h->lb, h->rec, h->dvcap,
+                                                             nullptr, 1);
         LAUNCHED();
     }
     MCK(cudaGetLastError());
@@ -498,7 +472,6 @@ cgb_status mq_match_all(cgb_mq* m, uint64_t n2) {
     put(&da, sizeof(da));
     const int bps = m->bps;
     put(&bps, sizeof(bps));
-    put(&h->d_drun_du, sizeof(void*));
     put(&m->d_pair, sizeof(void*));
     if (m->gexec && kl == m->gkey_len && std::memcmp(key, m->gkey, kl) == 0) {
         MCK(cudaGraphLaunch(m->gexec, h->stream));
@@ -531,7 +504,7 @@ cgb_status mq_match_all(cgb_mq* m, uint64_t n2) {
 cgb_status mq_sync(cgb_mq* m) {
     cgb_handle* h = m->h;
     MQ_TRY(sync_scalars(h));
-    for (int i = 0; i < 8; ++i) m->last_stats[i] = h->h_scal[4 + kMaxQE + i];
+    for (int i = 0; i < 8; ++i) m->last_stats[i] = h->h_scal[kCtlStats + i];
     return CGB_OK;
 }
 
@@ -560,7 +533,7 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
             mq_plan(m, T, v);
             MCK(cudaMemcpyAsync(m->d_tplans, T.plans, Q.q.qe * sizeof(EdgePlan), cudaMemcpyHostToDevice, h->stream));
             MCK(cudaMemcpyAsync(m->d_tpair, T.pair, Q.q.qe * sizeof(uint16_t), cudaMemcpyHostToDevice, h->stream));
-            MCK(cudaMemsetAsync(h->d_scal + 2, 0, sizeof(unsigned long long), h->stream));
+            MCK(cudaMemsetAsync(h->d_scal + kCtlErr, 0, sizeof(unsigned long long), h->stream));
             // later variants stop once they are clearly slower than the best so far
             const uint64_t budget = best < 3e38f ? (uint64_t)std::max(2.0f * best + 20.0f, 50.0f)
                                                  : (m->cfg.dfs_budget_ms ? m->cfg.dfs_budget_ms : 600000ull);
@@ -570,8 +543,8 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
             MCK(cudaEventRecord(m->ev[5], h->stream));
             MQ_TRY(sync_scalars(h));
             MCK(cudaEventElapsedTime(&ms, m->ev[4], m->ev[5]));
-            if (h->h_scal[2] & 8u) continue;  // over budget
-            if (h->h_scal[2]) return mq_fail(m, CGB_ERR_ARG, "autotune: error bits %llu", h->h_scal[2]);
+            if (h->h_scal[kCtlErr] & 8u) continue;  // over budget
+            if (h->h_scal[kCtlErr]) return mq_fail(m, CGB_ERR_ARG, "autotune: error bits %llu", h->h_scal[kCtlErr]);
             std::vector<unsigned long long> c(Q.q.qe);
             MCK(cudaMemcpy(c.data(), m->d_counts, Q.q.qe * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
             unsigned long long tot = 0, rtot = 0;
@@ -613,7 +586,7 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
     float best = 3.4e38f;
     Cfg best_c = cfgs.front();
     for (const Cfg& c : cfgs) {
-        MCK(cudaMemsetAsync(h->d_scal + 2, 0, sizeof(unsigned long long), h->stream));
+        MCK(cudaMemsetAsync(h->d_scal + kCtlErr, 0, sizeof(unsigned long long), h->stream));
         const uint64_t budget = best < 3e38f ? (uint64_t)std::max(2.0f * best + 20.0f, 50.0f)
                                              : (m->cfg.dfs_budget_ms ? m->cfg.dfs_budget_ms : 600000ull);
         MCK(cudaEventRecord(m->ev[4], h->stream));
@@ -622,15 +595,15 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
         MCK(cudaEventRecord(m->ev[5], h->stream));
         MQ_TRY(sync_scalars(h));
         MCK(cudaEventElapsedTime(&ms, m->ev[4], m->ev[5]));
-        if (h->h_scal[2] & 8u) continue;
-        if (h->h_scal[2]) return mq_fail(m, CGB_ERR_ARG, "autotune: error bits %llu", h->h_scal[2]);
+        if (h->h_scal[kCtlErr] & 8u) continue;
+        if (h->h_scal[kCtlErr]) return mq_fail(m, CGB_ERR_ARG, "autotune: error bits %llu", h->h_scal[kCtlErr]);
         if (ms < best) { best = ms; best_c = c; }
     }
     m->bps = best_c.bps;
     m->steal = best_c.steal;
     m->tuned_global = true;
     m->tuned_plans = m->G;
-    MCK(cudaMemsetAsync(h->d_scal + 2, 0, sizeof(unsigned long long), h->stream));
+    MCK(cudaMemsetAsync(h->d_scal + kCtlErr, 0, sizeof(unsigned long long), h->stream));
     MCK(cudaMemsetAsync(h->d_stats, 0, 8 * sizeof(unsigned long long), h->stream));
     return CGB_OK;
 }
@@ -649,8 +622,8 @@ cgb_status mq_collect(cgb_mq* m, uint64_t* out, uint32_t cap) {
 
 cgb_status mq_check_err(cgb_mq* m) {
     cgb_handle* h = m->h;
-    if (h->h_scal[2]) {
-        const unsigned long long e = h->h_scal[2];
+    if (h->h_scal[kCtlErr]) {
+        const unsigned long long e = h->h_scal[kCtlErr];
         h->rb_valid = false;
         cgb_status st = (e & 24u) ? CGB_ERR_TIMEOUT : (e & 4u) ? CGB_ERR_OOM : CGB_ERR_ARG;
         return mq_fail(m, st,
@@ -749,7 +722,7 @@ cgb_status cgb_mq_load_graph(cgb_mq* m, uint32_t n, const uint32_t* labels, uint
     h->pool_cap = cap;
     h->h_pool_top = 0;
     h->h_live = 0;
-    MCK(cudaMemsetAsync(h->d_scal, 0, 4 * sizeof(unsigned long long), h->stream));
+    MCK(cudaMemsetAsync(h->d_scal, 0, kCtlWords * sizeof(unsigned long long), h->stream));
     uint32_t* d_edges = nullptr;
     MCK(cudaMalloc(&d_edges, std::max<uint64_t>(num_edges, 1) * 2 * sizeof(uint32_t)));
     if (num_edges) MCK(cudaMemcpyAsync(d_edges, edges, num_edges * 8, cudaMemcpyHostToDevice, h->stream));
@@ -758,10 +731,13 @@ cgb_status cgb_mq_load_graph(cgb_mq* m, uint32_t n, const uint32_t* labels, uint
         if (num_edges) {
             k_mq_edge_keys<<<grid_for(h, num_edges), 256, 0, h->stream>>>(d_edges, num_edges, h->d_vlabel, n,
                                                                            h->d_keys_in,
-                                                                           (unsigned int*)(h->d_scal + 2));
+                                                                           (unsigned int*)(h->d_scal + kCtlErr));
             LAUNCHED();
         }
-        s = apply_edits(h, h->d_keys_in, nk, nullptr, 0, nullptr, 0);
+        EditSrc src;
+        src.add = h->d_keys_in;
+        src.n_add = nk;
+        s = apply_edits(h, src);
     }
     // planner statistics: directed edges and vertices with such an edge per label pair
     unsigned long long* d_st = nullptr;
@@ -787,8 +763,8 @@ cgb_status cgb_mq_load_graph(cgb_mq* m, uint32_t n, const uint32_t* labels, uint
         return s;
     }
     MQ_TRY(sync_scalars(h));
-    if (h->h_scal[2]) return mq_fail(m, CGB_ERR_ARG, "edges out of range or self-loops (error bits %llu)",
-                                     h->h_scal[2]);
+    if (h->h_scal[kCtlErr]) return mq_fail(m, CGB_ERR_ARG, "edges out of range or self-loops (error bits %llu)",
+                                     h->h_scal[kCtlErr]);
     m->avg.assign((size_t)L * L, 0.f);
     for (size_t i = 0; i < cnt.size(); ++i) m->avg[i] = nodes[i] ? (float)cnt[i] / (float)nodes[i] : 0.f;
     h->have_index = true;
@@ -846,11 +822,14 @@ cgb_status cgb_mq_apply_batch_device(cgb_mq* m, const uint32_t* ins_device, uint
     }
     cgb_status s;
     if ((s = mq_upload_plans(m)) != CGB_OK) return s;
-    MCK(cudaMemsetAsync(h->d_scal + 2, 0, 2 * sizeof(unsigned long long), h->stream));
-    MCK(cudaMemsetAsync(h->d_stats, 0, 8 * sizeof(unsigned long long), h->stream));
+    MCK(cudaMemsetAsync(h->d_scal + kCtlErr, 0, (kCtlCounts - kCtlErr) * sizeof(unsigned long long), h->stream));
     MCK(cudaEventRecord(m->ev[0], h->stream));
     // 1. the previous batch's insertions join the index
-    MQ_TRY(apply_edits(h, h->d_pending, h->n_pending, nullptr, 0, nullptr, 0));
+    EditSrc pend;
+    pend.packed = h->d_pending;
+    pend.n_packed = h->n_pending;
+    pend.B0 = h->pending_B;
+    MQ_TRY(apply_edits(h, pend));
     h->n_pending = 0;
     const bool rb_on = !(h->cfg.flags & CGB_FLAG_NO_RUN_BITS);
     if (rb_on && !h->rb_valid) MQ_TRY(rebuild_run_bits(h));
@@ -863,18 +842,22 @@ cgb_status cgb_mq_apply_batch_device(cgb_mq* m, const uint32_t* ins_device, uint
         MCK(cudaEventRecord(m->ev[2], h->stream));
         if ((s = mq_prepare_delta(m, del_device, n_del, true, &n2)) != CGB_OK) return s;
         MQ_TRY(grow(h, h->d_keys_in, h->keys_in_cap, n2));
-        k_mq_unpack<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, n2, bits_for(h->dv), h->lb, h->d_keys_in);
+        EditSrc gone;
+        gone.B0 = bits_for(h->dv);
+        k_mq_strip<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, n2, gone.B0, h->lb, h->d_keys_in);
         LAUNCHED();
-        MQ_TRY(apply_edits(h, nullptr, 0, nullptr, 0, h->d_keys_in, n2));
+        gone.packed = h->d_keys_in;
+        gone.n_packed = n2;
+        gone.packed_op = 1;
+        MQ_TRY(apply_edits(h, gone));
         MCK(cudaEventRecord(m->ev[3], h->stream));
         if (m->G) {
             if ((s = mq_match_enqueue(m, m->d_plans, m->d_pair, m->G, n2, m->bps ? m->bps : mq_occupancy(m),
                                       m->steal, m->cfg.dfs_budget_ms ? m->cfg.dfs_budget_ms : 600000ull)) != CGB_OK)
                 return s;
         } else {
-            k_delta_recs<<<grid_for(h, n2), 256, 0, h->stream>>>(h->rec, h->dvcap, h->d_drun_du, h->d_drun_len,
-                                                                 h->d_drun_off, h->d_num_runs + 1,
-                                                                 bits_for(h->dv), 1);
+            k_delta_lists<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, 0, m->d_nsel, bits_for(h->dv), h->lb,
+                                                                  h->rec, h->dvcap, nullptr, 1);
             LAUNCHED();
         }
         MCK(cudaEventRecord(m->ev[4], h->stream));
@@ -906,15 +889,15 @@ cgb_status cgb_mq_apply_batch_device(cgb_mq* m, const uint32_t* ins_device, uint
             }
             if ((s = mq_match_all(m, n2)) != CGB_OK) return s;
         } else {
-            k_delta_recs<<<grid_for(h, n2), 256, 0, h->stream>>>(h->rec, h->dvcap, h->d_drun_du, h->d_drun_len,
-                                                                 h->d_drun_off, h->d_num_runs + 1,
-                                                                 bits_for(h->dv), 1);
+            k_delta_lists<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, 0, m->d_nsel, bits_for(h->dv), h->lb,
+                                                                  h->rec, h->dvcap, nullptr, 1);
             LAUNCHED();
         }
         MCK(cudaEventRecord(m->ev[4], h->stream));
         // this batch's new edges, as index keys, are merged at the next batch
         MQ_TRY(grow(h, h->d_pending, h->pending_cap, n2));
-        k_mq_unpack<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, n2, bits_for(h->dv), h->lb, h->d_pending);
+        h->pending_B = bits_for(h->dv);
+        k_mq_strip<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, n2, h->pending_B, h->lb, h->d_pending);
         LAUNCHED();
         h->n_pending = n2;
         MQ_TRY(mq_sync(m));
