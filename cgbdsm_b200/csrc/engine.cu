@@ -2137,16 +2137,21 @@ __global__ void k_vb_depth(const cgb::VbPlan* __restrict__ vbp, const uint4* __r
 // ---------------------------------------------------------------------------
 // maintenance kernels
 // ---------------------------------------------------------------------------
-__global__ void k_rec_sizes(const uint4* rec, uint32_t dvcap, uint32_t dv, uint32_t nd, uint32_t* out_round4,
-                            uint32_t* out_len) {
+__global__ void k_rec_sizes(const uint4* rec, uint32_t dvcap, uint32_t dv, uint32_t nd, uint32_t* out_round4) {
     uint64_t total = (uint64_t)nd * dv;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t d = (uint32_t)(i / dv), u = (uint32_t)(i % dv);
         uint32_t len = rec[(size_t)d * dvcap + u].y;
-        if (out_round4) out_round4[i] = round4(len);
-        if (out_len) out_len[i] = len;
+        out_round4[i] = round4(len);
     }
+}
+
+// Run lengths in (d, u) order, and a 0 after the last (scanned in place to offsets).
+__global__ void k_rec_lens(const uint4* rec, uint32_t dvcap, uint32_t dv, uint32_t nd, unsigned long long* out) {
+    const uint64_t total = (uint64_t)nd * dv;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= total; i += (uint64_t)gridDim.x * blockDim.x)
+        out[i] = i < total ? rec[(size_t)(i / dv) * dvcap + i % dv].y : 0;
 }
 
 // Copies every run to its compacted offset (warp per (d,u)).
@@ -2259,6 +2264,8 @@ struct cgb_handle {
     unsigned int* d_qctr = nullptr;          // DFS queue counters [kQWords]
     unsigned long long last_stats[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     void* d_temp = nullptr; size_t temp_cap = 0;
+    unsigned long long* d_read_off = nullptr; size_t read_off_cap = 0;  // cgb_read_index
+    uint64_t* d_read = nullptr; size_t read_cap = 0;
 
     // run bit sets: built in full on the first matched batch (and after the
     // record table grows), then kept current by every merge
@@ -2475,7 +2482,7 @@ cgb_status compact_pool(cgb_handle* h, unsigned long long new_cap) {
     CK(cudaMalloc(&offs, (n + 1) * sizeof(unsigned long long)));
     CK(cudaMemsetAsync(offs, 0, (n + 1) * sizeof(unsigned long long), h->stream));
     if (n > 0) {
-        k_rec_sizes<<<grid_for(h, n), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, sizes, nullptr);
+        k_rec_sizes<<<grid_for(h, n), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, sizes);
         LAUNCHED();
         k_u32_to_u64<<<grid_for(h, n), 256, 0, h->stream>>>(sizes, offs, n);
         LAUNCHED();
@@ -2754,7 +2761,7 @@ void cgb_destroy(cgb_handle* h) {
     void* ptrs[] = {h->rec, h->pool, h->pool_alt, h->d_scal, h->d_self, h->d_keys_in, h->d_pending, h->d_edits,
                     h->d_edits_alt, h->d_runs[0], h->d_runs[1], h->d_runs[2],
                     h->d_dkeys, h->d_dkeys_alt, h->d_dval,
-                    h->d_seed, h->d_tasks, h->d_temp, h->d_qe_dirs, h->d_edge_ok,
+                    h->d_seed, h->d_tasks, h->d_temp, h->d_read_off, h->d_read, h->d_qe_dirs, h->d_edge_ok,
                     h->d_vb, h->d_rb_slot, h->d_rb_sel, h->d_rb_bits, h->d_rb_new, h->d_rev, h->d_touched, h->d_plans,
                     h->d_vbplans, h->d_dir_edge, h->d_lsum, h->d_wsum, h->d_wjobs};
     for (void* p : ptrs)
@@ -3199,17 +3206,12 @@ cgb_status cgb_read_index(cgb_handle* h, uint64_t* out, uint64_t cap, uint64_t* 
     cgb_status s;
     if ((s = flush_pending(h)) != CGB_OK) return s;
     const uint64_t n = (uint64_t)h->nd * h->dv;
-    uint32_t* lens = nullptr;
-    unsigned long long* offs = nullptr;
-    CK(cudaMalloc(&lens, std::max<uint64_t>(n, 1) * sizeof(uint32_t)));
-    CK(cudaMalloc(&offs, (n + 1) * sizeof(unsigned long long)));
-    CK(cudaMemsetAsync(offs, 0, (n + 1) * sizeof(unsigned long long), h->stream));
-    if (n) {
-        k_rec_sizes<<<grid_for(h, n), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, nullptr, lens);
-        LAUNCHED();
-        k_u32_to_u64<<<grid_for(h, n), 256, 0, h->stream>>>(lens, offs, n);
-        LAUNCHED();
-    }
+    // offsets of the runs and the key buffer stay with the handle (the key
+    // buffer up to kReadKeep): allocating them took 1 of a small index's 1.2 ms
+    if ((s = grow(h, h->d_read_off, h->read_off_cap, n + 1)) != CGB_OK) return s;
+    unsigned long long* offs = h->d_read_off;
+    k_rec_lens<<<grid_for(h, n + 1), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, offs);
+    LAUNCHED();
     size_t tb = 0;
     CK(cub::DeviceScan::ExclusiveSum(nullptr, tb, offs, offs, (int64_t)n + 1, h->stream));
     if ((s = grow_temp(h, tb)) != CGB_OK) return s;
@@ -3219,21 +3221,26 @@ cgb_status cgb_read_index(cgb_handle* h, uint64_t* out, uint64_t cap, uint64_t* 
     CK(cudaMemcpyAsync(&total, offs + n, sizeof(total), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     *n_out = total;
-    if (out && cap >= total && total > 0) {
-        uint64_t* d_out = nullptr;
-        CK(cudaMalloc(&d_out, total * sizeof(uint64_t)));
-        k_dump<<<grid_for(h, n * 32), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, h->pool, offs, d_out);
-        LAUNCHED();
-        CK(cudaMemcpyAsync(out, d_out, total * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        CK(cudaFree(d_out));
-    } else if (out && cap < total) {
-        CK(cudaFree(lens));
-        CK(cudaFree(offs));
-        return fail(h, CGB_ERR_ARG, "output capacity %llu < %llu", (unsigned long long)cap, total);
+    if (out && cap < total) return fail(h, CGB_ERR_ARG, "output capacity %llu < %llu", (unsigned long long)cap, total);
+    if (out && total > 0) {
+        constexpr size_t kReadKeep = (64u << 20) / sizeof(uint64_t);
+        if (total > kReadKeep) {
+            uint64_t* d_out = nullptr;
+            CK(cudaMalloc(&d_out, total * sizeof(uint64_t)));
+            k_dump<<<grid_for(h, n * 32), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, h->pool, offs, d_out);
+            LAUNCHED();
+            cudaError_t e = cudaMemcpyAsync(out, d_out, total * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+            cudaFree(d_out);
+            CK(e);
+        } else {
+            if ((s = grow(h, h->d_read, h->read_cap, (size_t)total)) != CGB_OK) return s;
+            k_dump<<<grid_for(h, n * 32), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, h->pool, offs, h->d_read);
+            LAUNCHED();
+            CK(cudaMemcpyAsync(out, h->d_read, total * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaStreamSynchronize(h->stream));
+        }
     }
-    CK(cudaFree(lens));
-    CK(cudaFree(offs));
     return CGB_OK;
 }
 

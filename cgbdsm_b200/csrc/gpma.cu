@@ -334,7 +334,11 @@ struct cgb_gpma {
     uint64_t* d_off = nullptr; uint64_t* d_cap = nullptr; uint32_t* d_h = nullptr; uint64_t* d_leaf0 = nullptr;
     unsigned long long* d_scal = nullptr;  // [0] n_ins, [1] n_win, [2] resize|err<<1 (u32 pair), [3..] hist
     void* temp = nullptr; size_t temp_cap = 0;
-    std::vector<void*> bufs;  // per-batch buffers, freed on growth / destroy
+    // per-call buffers, kept between calls (galloc, reclaim): a call's 16
+    // cudaMalloc and cudaFree took 14 of a 100k + 100k update's 17 ms
+    struct Buf { void* p; size_t bytes; bool used; };
+    std::vector<Buf> bufs;
+    size_t call_bytes = 0;    // handed out since the last reclaim
     uint64_t stats[6] = {0, 0, 0, 0, 0, 0};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
 };
@@ -360,22 +364,35 @@ cgb_status gfail(cgb_gpma* g, cgb_status s, const char* fmt, ...) {
 
 unsigned grid_of(uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, 148ull * 16)); }
 
+// A buffer of n T for the current call: the smallest kept one that holds it
+// without wasting more than three quarters, else a new one.
 template <typename T>
 cgb_status galloc(cgb_gpma* g, T*& p, uint64_t n) {
-    void* q = nullptr;
-    GCK(cudaMalloc(&q, std::max<uint64_t>(n, 1) * sizeof(T)));
-    g->bufs.push_back(q);
-    p = (T*)q;
+    const size_t need = std::max<uint64_t>(n, 1) * sizeof(T);
+    cgb_gpma::Buf* best = nullptr;
+    for (auto& b : g->bufs)
+        if (!b.used && b.bytes >= need && b.bytes <= 4 * need + (1u << 20) && (!best || b.bytes < best->bytes)) best = &b;
+    if (!best) {
+        const size_t bytes = need + need / 4;
+        void* q = nullptr;
+        GCK(cudaMalloc(&q, bytes));
+        g->bufs.push_back({q, bytes, false});
+        best = &g->bufs.back();
+    }
+    best->used = true;
+    g->call_bytes += best->bytes;
+    p = (T*)best->p;
     return CGB_OK;
 }
 
 cgb_status gtemp(cgb_gpma* g, size_t need) {
-    if (need <= g->temp_cap) return CGB_OK;
+    if (need <= g->temp_cap && g->temp) return CGB_OK;
+    const size_t bytes = need + need / 2;
     if (g->temp) cudaFree(g->temp);
     g->temp = nullptr;
     g->temp_cap = 0;
-    GCK(cudaMalloc(&g->temp, need));
-    g->temp_cap = need;
+    GCK(cudaMalloc(&g->temp, bytes));
+    g->temp_cap = bytes;
     return CGB_OK;
 }
 
@@ -387,9 +404,30 @@ void free_structure(cgb_gpma* g) {
     g->leaf_ins = nullptr; g->leaf_dir = nullptr;
 }
 
-void free_bufs(cgb_gpma* g) {
-    for (void* p : g->bufs) cudaFree(p);
-    g->bufs.clear();
+// Returns the call's buffers to the handle.  What is kept is bounded by twice
+// what the call used (at least 64 MiB): the largest go first.  all: frees all.
+void reclaim(cgb_gpma* g, bool all = false) {
+    size_t total = 0;
+    for (auto& b : g->bufs) {
+        b.used = false;
+        total += b.bytes;
+    }
+    const size_t keep = all ? 0 : std::max<size_t>(2 * g->call_bytes, 64u << 20);
+    g->call_bytes = 0;
+    if (total <= keep) return;
+    std::sort(g->bufs.begin(), g->bufs.end(), [](const cgb_gpma::Buf& x, const cgb_gpma::Buf& y) { return x.bytes < y.bytes; });
+    while (!g->bufs.empty() && total > keep) {
+        total -= g->bufs.back().bytes;
+        cudaFree(g->bufs.back().p);
+        g->bufs.pop_back();
+    }
+}
+
+// The caller's key arrays may come from work queued on the default stream.
+cgb_status after_default_stream(cgb_gpma* g) {
+    GCK(cudaEventRecord(g->e0, cudaStreamLegacy));
+    GCK(cudaStreamWaitEvent(g->stream, g->e0, 0));
+    return CGB_OK;
 }
 
 // Rebuilds the structure from n sorted unique keys (device).
@@ -446,7 +484,7 @@ cgb_status rebuild(cgb_gpma* g, const uint64_t* keys, uint64_t n) {
     k_gp_leafdir<<<grid_of(leaf), 256, 0, g->stream>>>(g->leaf_dir, g->d_leaf0, g->nd, leaf);
     GCK(cudaGetLastError());
     GCK(cudaStreamSynchronize(g->stream));
-    free_bufs(g);
+    reclaim(g);
     return CGB_OK;
 }
 
@@ -501,7 +539,7 @@ void cgb_gpma_destroy(cgb_gpma* g) {
     cudaSetDevice(g->device);
     if (g->stream) cudaStreamSynchronize(g->stream);
     free_structure(g);
-    free_bufs(g);
+    reclaim(g, true);
     for (void* p : {(void*)g->d_off, (void*)g->d_cap, (void*)g->d_h, (void*)g->d_leaf0, (void*)g->d_scal, g->temp})
         if (p) cudaFree(p);
     if (g->e0) cudaEventDestroy(g->e0);
@@ -518,6 +556,8 @@ cgb_status cgb_gpma_bulk_load(cgb_gpma* g, const uint64_t* keys_device, uint64_t
     uint64_t* u = nullptr;
     uint64_t m = 0;
     cgb_status s;
+    reclaim(g);  // a call that failed left its buffers out
+    if ((s = after_default_stream(g)) != CGB_OK) return s;
     if (n) {
         if ((s = sort_unique(g, keys_device, n, u, m)) != CGB_OK) return s;
     }
@@ -535,8 +575,10 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
     for (auto& x : g->stats) x = 0;
     const uint64_t n = n_ins + n_del;
     if (n == 0) return CGB_OK;
-    GCK(cudaEventRecord(g->e0, g->stream));
     cgb_status s;
+    reclaim(g);
+    if ((s = after_default_stream(g)) != CGB_OK) return s;
+    GCK(cudaEventRecord(g->e0, g->stream));
     // 1. edits sorted by key with their op (0 insert, 1 delete)
     uint64_t *k_in = nullptr, *k_out = nullptr;
     uint8_t *o_in = nullptr, *o_out = nullptr;
@@ -704,7 +746,7 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
     g->stats[3] = 0;
     g->stats[4] = (uint64_t)(ms * 1000.0f);
     g->stats[5] = g->n_keys;
-    free_bufs(g);
+    reclaim(g);
     return CGB_OK;
 }
 
@@ -713,6 +755,8 @@ cgb_status cgb_gpma_extract(cgb_gpma* g, uint32_t dir, uint64_t* out_device, uin
     GCK(cudaSetDevice(g->device));
     const GpmaDir& D = g->dirs[dir];
     cgb_status s;
+    reclaim(g);
+    if ((s = after_default_stream(g)) != CGB_OK) return s;
     uint64_t* tmp = nullptr;
     if ((s = galloc(g, tmp, D.cap)) != CGB_OK) return s;
     size_t bytes = 0;
@@ -726,11 +770,11 @@ cgb_status cgb_gpma_extract(cgb_gpma* g, uint32_t dir, uint64_t* out_device, uin
     GCK(cudaStreamSynchronize(g->stream));
     *n_out = m;
     if (out_device) {
-        if (cap < m) { free_bufs(g); return gfail(g, CGB_ERR_ARG, "buffer holds %llu of %llu keys", (unsigned long long)cap, m); }
+        if (cap < m) { reclaim(g); return gfail(g, CGB_ERR_ARG, "buffer holds %llu of %llu keys", (unsigned long long)cap, m); }
         if (m) k_gp_strip_dir<<<grid_of(m), 256, 0, g->stream>>>(tmp, m, out_device);
         GCK(cudaStreamSynchronize(g->stream));
     }
-    free_bufs(g);
+    reclaim(g);
     return CGB_OK;
 }
 

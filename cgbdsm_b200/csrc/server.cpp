@@ -95,6 +95,8 @@ struct cgb_server {
     bool stop = false;
     std::thread sched, stager;
     uint32_t live = 0;
+    uint64_t used_seen = 0;   // device memory in use when last asked (scheduler thread)
+    double used_at = -1;      // and when
     // stats
     uint64_t batches_done = 0, edges_done = 0, rejected = 0;
     double busy_ms = 0;
@@ -153,6 +155,23 @@ void complete(cgb_server* s, const std::shared_ptr<Req>& r) {
     s->cv_done.notify_all();
 }
 
+// Device memory in use, for the admission of a batch that needs `need` bytes
+// (scheduler thread).  The driver's answer takes about half a millisecond, as
+// long as a small batch, so the last one stands for kMemoryCheckMs while the
+// budget is a quarter away; near the limit every batch asks.
+constexpr double kMemoryCheckMs = 20.0;
+uint64_t memory_used(cgb_server* s, uint64_t need) {
+    const double now = s->now_ms();
+    if (s->used_at >= 0 && now - s->used_at < kMemoryCheckMs &&
+        s->used_seen + need <= s->base_used + s->budget - s->budget / 4)
+        return s->used_seen;
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    s->used_seen = (uint64_t)(total_b - free_b);
+    s->used_at = now;
+    return s->used_seen;
+}
+
 void scheduler_loop(cgb_server* s) {
     cudaSetDevice(s->device);
     std::unique_lock<std::mutex> lk(s->mu);
@@ -193,10 +212,8 @@ void scheduler_loop(cgb_server* s) {
             continue;
         }
         // the batch's device working set must fit the budget
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        const uint64_t used = (uint64_t)(total_b - free_b);
         const uint64_t need = (r->n_ins + r->n_del) * kWorkBytesPerEdge;
+        const uint64_t used = memory_used(s, need);
         r->live_queries = s->live;
         r->t_start = s->now_ms();
         lk.unlock();
