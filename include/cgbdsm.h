@@ -260,7 +260,7 @@ cgb_status cgb_producer_vertex_map(const cgb_producer* p, const uint32_t** new2o
  * out (capacity >= n_old + n_ins), out_n (one u64: the output length, or
  * UINT64_MAX if an edit key has u or v >= dv_count).  Work is enqueued on
  * `stream` (a cudaStream_t; NULL = legacy default stream); nothing is
- * synchronized.  All temporaries live in one static device array of 11.5 MiB
+ * synchronized.  All temporaries live in one static device array of 10.5 MiB
  * that every GPU loading this library holds until the process exits; calls
  * keep their contents in it, so calls whose work overlaps on one GPU race and
  * must be ordered by the caller.  The first call on a device looks up the
