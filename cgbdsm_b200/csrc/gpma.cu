@@ -71,6 +71,16 @@ struct DirTab {
     const uint64_t* leaf0;
 };
 
+// The batch's keys with their op (0 insert, 1 delete).
+__global__ void k_gp_edits(const uint64_t* __restrict__ ins, uint64_t n_ins, const uint64_t* __restrict__ del, uint64_t n_del,
+                           uint64_t* __restrict__ key, uint8_t* __restrict__ op) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_ins + n_del;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        key[i] = i < n_ins ? ins[i] : del[i - n_ins];
+        op[i] = i < n_ins ? 0 : 1;
+    }
+}
+
 // One thread per sorted edit; the first of each run of equal keys applies
 // the run's effect (any delete wins: (S + ins) - del).
 __global__ void k_gp_effect(const uint64_t* __restrict__ key, const uint8_t* __restrict__ op, uint64_t n,
@@ -106,28 +116,44 @@ __global__ void k_gp_effect(const uint64_t* __restrict__ key, const uint8_t* __r
     }
 }
 
-// Valid keys per leaf (one warp per leaf).
-__global__ void k_gp_leafcount(const uint8_t* __restrict__ valid, uint64_t n_leaves, uint32_t* cnt) {
+// Valid keys per leaf (one warp per leaf) and per direction (added to dir_n).
+__global__ void k_gp_leafcount(const uint8_t* valid, uint64_t n_leaves, const uint32_t* __restrict__ leaf_dir,
+                               uint32_t* cnt, unsigned long long* dir_n) {
+    __shared__ unsigned int s_n[CGB_MAX_DIR];
+    for (uint32_t t = threadIdx.x; t < CGB_MAX_DIR; t += blockDim.x) s_n[t] = 0;
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t l = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < n_leaves; l += nw) {
         const uint32_t b = __ballot_sync(0xffffffffu, valid[l * kSeg + lane] != 0);
-        if (lane == 0) cnt[l] = __popc(b);
+        if (lane == 0) {
+            cnt[l] = __popc(b);
+            if (b) atomicAdd(s_n + leaf_dir[l], (unsigned int)__popc(b));
+        }
+    }
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < CGB_MAX_DIR; t += blockDim.x)
+        if (s_n[t]) atomicAdd(dir_n + t, (unsigned long long)s_n[t]);
+}
+
+// Per leaf, the keys after the batch (newc) and the keys kept in place
+// (without the queued inserts); both are prefix-summed next.
+__global__ void k_gp_newcount(const uint32_t* cnt, const int* delta, const uint32_t* leaf_ins, uint64_t n,
+                              uint64_t* newc, uint64_t* kept) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t c = (uint64_t)((int64_t)cnt[i] + delta[i]);
+        newc[i] = c;
+        kept[i] = c - leaf_ins[i];
     }
 }
 
-__global__ void k_gp_newcount(const uint32_t* cnt, const int* delta, uint64_t n, uint64_t* out) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = (uint64_t)((int64_t)cnt[i] + delta[i]);
-}
-
 // Window of each leaf with queued inserts: smallest node within its level's
-// upper density bound; encoded (first leaf << 32 | ~end leaf) so that an
-// ascending sort lists windows by start, larger first.  P = inclusive prefix
+// upper density bound, entered at its first leaf as the largest level there
+// (wlv: level + 1; 0: no window starts at the leaf).  P = inclusive prefix
 // sums of the new per-leaf counts (P[l] = sum over leaves <= l).
 __global__ void k_gp_window(const uint32_t* __restrict__ leaf_ins, const uint64_t* __restrict__ P,
-                            const uint32_t* __restrict__ leaf_dir, DirTab dt, uint64_t n_leaves, uint64_t* win,
-                            unsigned long long* n_win, unsigned int* resize) {
+                            const uint32_t* __restrict__ leaf_dir, DirTab dt, uint64_t n_leaves, uint32_t* wlv,
+                            unsigned int* resize) {
     for (uint64_t l = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; l < n_leaves;
          l += (uint64_t)gridDim.x * blockDim.x) {
         if (!leaf_ins[l]) continue;
@@ -140,8 +166,7 @@ __global__ void k_gp_window(const uint32_t* __restrict__ leaf_ins, const uint64_
             const uint64_t c = P[b - 1] - (a > 0 ? P[a - 1] : 0);
             const double up = h ? kUpLeaf - (kUpLeaf - kUpRoot) * (double)lv / (double)h : kUpRoot;
             if ((double)c <= up * (double)((uint64_t)kSeg << lv)) {
-                const unsigned long long q = atomicAdd(n_win, 1ull);
-                win[q] = (a << 32) | (0xffffffffull - b);
+                atomicMax(wlv + a, lv + 1);
                 found = true;
                 break;
             }
@@ -150,105 +175,111 @@ __global__ void k_gp_window(const uint32_t* __restrict__ leaf_ins, const uint64_
     }
 }
 
-// Windows are maximal when their end exceeds every end before them.
-__global__ void k_gp_maximal(const uint64_t* __restrict__ win, const uint64_t* __restrict__ prefmax_end, uint64_t n,
-                             uint8_t* flag) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b = 0xffffffffull - (win[i] & 0xffffffffull);
-        flag[i] = (i == 0 || b > prefmax_end[i - 1]) ? 1 : 0;
+// End (first leaf past it) of the window starting at each leaf, 0 if none.
+__global__ void k_gp_end(const uint32_t* __restrict__ wlv, uint64_t n, uint64_t* end) {
+    for (uint64_t l = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; l < n; l += (uint64_t)gridDim.x * blockDim.x)
+        end[l] = wlv[l] ? l + (1ull << (wlv[l] - 1)) : 0;
+}
+
+// A window is maximal when its end exceeds every end before it (pmax: running
+// maximum): 1 at its first leaf.  The running sum of these numbers the windows
+// and, with pmax, says which leaves lie in one: nothing is sorted or searched.
+__global__ void k_gp_maximal(const uint32_t* __restrict__ wlv, const uint64_t* __restrict__ pmax, uint64_t n,
+                             uint32_t* flag) {
+    for (uint64_t l = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; l < n; l += (uint64_t)gridDim.x * blockDim.x)
+        flag[l] = wlv[l] && pmax[l] > (l ? pmax[l - 1] : 0ull) ? 1u : 0u;
+}
+
+// Window w (flag at leaf l, widx[l] = w + 1): first leaf and level, new key
+// count, the keys kept in place (the inserts go behind them), and the value
+// before it (read before any rewrite).  The last leaf writes the counts.
+struct GpWin {
+    uint64_t a, b, count, pred;
+};
+__global__ void k_gp_wininfo(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ widx,
+                             const uint64_t* __restrict__ pmax, uint64_t n_leaves, const uint64_t* __restrict__ P,
+                             const uint64_t* __restrict__ Q, const uint64_t* __restrict__ slots, GpWin* win,
+                             uint64_t* wcount, unsigned long long* wfill, unsigned long long* n_win) {
+    for (uint64_t l = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; l < n_leaves;
+         l += (uint64_t)gridDim.x * blockDim.x) {
+        if (l == n_leaves - 1) *n_win = widx[l];
+        if (!flag[l]) continue;
+        const uint32_t w = widx[l] - 1;
+        const uint64_t b = pmax[l];
+        const uint64_t c = P[b - 1] - (l > 0 ? P[l - 1] : 0);
+        win[w] = {l, b, c, l > 0 ? slots[l * kSeg - 1] : 0ull};
+        wcount[w] = c;
+        wfill[w] = Q[b - 1] - (l > 0 ? Q[l - 1] : 0);
     }
 }
 
-__global__ void k_gp_end(const uint64_t* win, uint64_t n, uint64_t* end) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        end[i] = 0xffffffffull - (win[i] & 0xffffffffull);
-}
-
-// New key count of each window and the value before it (read before any rewrite).
-__global__ void k_gp_wininfo(const uint64_t* __restrict__ win, uint64_t n, const uint64_t* __restrict__ P,
-                             const uint64_t* __restrict__ slots, uint64_t* wcount, uint64_t* wpred) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t a = win[i] >> 32, b = 0xffffffffull - (win[i] & 0xffffffffull);
-        wcount[i] = P[b - 1] - (a > 0 ? P[a - 1] : 0);
-        wpred[i] = a > 0 ? slots[a * kSeg - 1] : 0ull;
-    }
-}
-
-// Gather a window's valid keys (block per window, in slot order) to tmp[off..).
-__global__ void k_gp_gather(const uint64_t* __restrict__ win, uint64_t n_win, const uint64_t* __restrict__ woff,
-                            const uint64_t* __restrict__ wcount, const uint64_t* __restrict__ slots,
-                            const uint8_t* __restrict__ valid, uint64_t* tmp, uint64_t* wfill, unsigned int* bad) {
-    typedef cub::BlockScan<uint32_t, 256> Scan;
-    __shared__ typename Scan::TempStorage ts;
-    __shared__ uint64_t s_base;
-    for (uint64_t w = blockIdx.x; w < n_win; w += gridDim.x) {
-        const uint64_t a = win[w] >> 32, b = 0xffffffffull - (win[w] & 0xffffffffull);
-        const uint64_t s0 = a * kSeg, s1 = b * kSeg;
-        if (threadIdx.x == 0) s_base = 0;
-        __syncthreads();
-        for (uint64_t t = s0; t < s1; t += 256) {
-            const uint64_t s = t + threadIdx.x;
-            const uint32_t f = (s < s1 && valid[s]) ? 1u : 0u;
-            uint32_t pos, tot;
-            Scan(ts).ExclusiveSum(f, pos, tot);
-            if (f && s_base + pos < wcount[w]) tmp[woff[w] + s_base + pos] = slots[s];
-            __syncthreads();
-            if (threadIdx.x == 0) s_base += tot;
-            __syncthreads();
+// The windows' valid keys to tmp, in slot order: a warp per leaf that lies in
+// a window (a block per window left most threads idle: nearly every window
+// is one leaf; 98 -> 12 us for 100 k inserts into 2 M keys).
+__global__ void k_gp_gather(const GpWin* __restrict__ win, const uint32_t* __restrict__ widx,
+                            const uint64_t* __restrict__ pmax, uint64_t n_leaves, const uint64_t* __restrict__ woff,
+                            const uint64_t* __restrict__ Q, const uint64_t* __restrict__ slots,
+                            const uint8_t* __restrict__ valid, uint64_t* tmp, unsigned int* bad) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t l = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < n_leaves; l += nw) {
+        if (pmax[l] <= l) continue;
+        const uint32_t w = widx[l] - 1;
+        const uint64_t a = win[w].a, n = win[w].count;
+        const uint64_t at = (l > 0 ? Q[l - 1] : 0) - (a > 0 ? Q[a - 1] : 0);
+        const bool f = valid[l * kSeg + lane] != 0;
+        const uint32_t b = __ballot_sync(0xffffffffu, f);
+        const uint64_t p = at + __popc(b & ((1u << lane) - 1u));
+        if (f) {
+            if (p < n) tmp[woff[w] + p] = slots[l * kSeg + lane];
+            else atomicOr(bad, 1u);
         }
-        if (threadIdx.x == 0) {
-            if (s_base > wcount[w]) atomicOr(bad, 1u);
-            wfill[w] = min(s_base, wcount[w]);
-        }
-        __syncthreads();
     }
 }
 
-// Queued inserts join their window (the maximal window holding their leaf).
-// Every such leaf lies in a window and every window's slots in tmp number
-// its new count; a violation of either sets `bad` and writes nothing.
+// Queued inserts join their window, behind the keys kept in place.  Every
+// such leaf lies in a window and every window's slots in tmp number its new
+// count; a violation of either sets `bad` and writes nothing.
 __global__ void k_gp_place_ins(const uint64_t* __restrict__ ins_key, const uint64_t* __restrict__ ins_leaf,
-                               uint64_t n, const uint64_t* __restrict__ win, uint64_t n_win,
-                               const uint64_t* __restrict__ woff, const uint64_t* __restrict__ wcount,
+                               uint64_t n, const uint32_t* __restrict__ widx, const uint64_t* __restrict__ pmax,
+                               const uint64_t* __restrict__ woff, const GpWin* __restrict__ win,
                                unsigned long long* wfill, uint64_t* tmp, unsigned int* bad) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t leaf = ins_leaf[i];
-        // last window whose first leaf <= leaf
-        uint64_t lo = 0, len = n_win;
-        while (len > 0) {
-            const uint64_t half = len >> 1;
-            if ((win[lo + half] >> 32) <= leaf) { lo += half + 1; len -= half + 1; }
-            else len = half;
-        }
-        if (lo == 0) { atomicOr(bad, 1u); continue; }
-        const uint64_t w = lo - 1;
-        if (leaf >= 0xffffffffull - (win[w] & 0xffffffffull)) { atomicOr(bad, 1u); continue; }
+        if (pmax[leaf] <= leaf) { atomicOr(bad, 1u); continue; }
+        const uint32_t w = widx[leaf] - 1;
         const unsigned long long q = atomicAdd(wfill + w, 1ull);
-        if (q >= wcount[w]) { atomicOr(bad, 1u); continue; }
+        if (q >= win[w].count) { atomicOr(bad, 1u); continue; }
         tmp[woff[w] + q] = ins_key[i];
     }
 }
 
 // Spread each window's sorted keys evenly: key i to slot s0 + floor(i W / n);
-// every other slot copies the last key before it (or the value before the window).
-__global__ void k_gp_scatter(const uint64_t* __restrict__ win, uint64_t n_win, const uint64_t* __restrict__ woff,
-                             const uint64_t* __restrict__ wcount, const uint64_t* __restrict__ wpred,
+// every other slot copies the last key before it (or the value before the
+// window).  A warp per leaf in a window; W is a power of two, and whether slot
+// r holds key i needs no division (r n <= i W < (r + 1) n).
+__global__ void k_gp_scatter(const GpWin* __restrict__ win, const uint32_t* __restrict__ widx,
+                             const uint64_t* __restrict__ pmax, uint64_t n_leaves, const uint64_t* __restrict__ woff,
                              const uint64_t* __restrict__ sorted, uint64_t* slots, uint8_t* valid) {
-    for (uint64_t w = blockIdx.x; w < n_win; w += gridDim.x) {
-        const uint64_t a = win[w] >> 32, b = 0xffffffffull - (win[w] & 0xffffffffull);
-        const uint64_t s0 = a * kSeg, W = (b - a) * kSeg, n = wcount[w];
-        const uint64_t* src = sorted + woff[w];
-        for (uint64_t r = threadIdx.x; r < W; r += blockDim.x) {
-            // last key index placed at or before slot r: ceil((r + 1) n / W) - 1
-            const uint64_t im = n ? ((r + 1) * n + W - 1) / W : 0;
-            if (im == 0) {
-                slots[s0 + r] = wpred[w];
-                valid[s0 + r] = 0;
-            } else {
-                const uint64_t i = im - 1;
-                slots[s0 + r] = src[i];
-                valid[s0 + r] = (i * W / n == r) ? 1 : 0;
-            }
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t l = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < n_leaves; l += nw) {
+        if (pmax[l] <= l) continue;
+        const uint32_t w = widx[l] - 1;
+        const GpWin W = win[w];
+        const uint32_t sh = 31 - __clz((uint32_t)(W.b - W.a)) + 5;  // log2 of its slots
+        static_assert(kSeg == 32, "a lane per slot of a leaf");
+        const uint64_t r = (l - W.a) * kSeg + lane, n = W.count;
+        // last key index placed at or before slot r: ceil((r + 1) n / W) - 1
+        const uint64_t im = n ? ((r + 1) * n + (1ull << sh) - 1) >> sh : 0;
+        const uint64_t at = l * kSeg + lane;
+        if (im == 0) {
+            slots[at] = W.pred;
+            valid[at] = 0;
+        } else {
+            const uint64_t i = im - 1;
+            slots[at] = sorted[woff[w] + i];
+            valid[at] = (i << sh) >= r * n && (i << sh) < (r + 1) * n ? 1 : 0;
         }
     }
 }
@@ -307,9 +338,17 @@ __global__ void k_gp_valid_flags(const uint8_t* valid, uint64_t n, uint8_t* out)
         out[i] = valid[i];
 }
 
-__global__ void k_gp_strip_dir(const uint64_t* in, uint64_t n, uint64_t* out) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = in[i] & ((1ull << 59) - 1ull);
+// The keys of a direction's leaves, ascending, without their direction: a
+// warp per leaf, at the scanned leaf counts.
+__global__ void k_gp_extract(const uint64_t* __restrict__ slots, const uint8_t* __restrict__ valid, uint64_t n_leaves,
+                             const uint64_t* __restrict__ off, uint64_t* __restrict__ out) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t l = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < n_leaves; l += nw) {
+        const bool f = valid[l * kSeg + lane] != 0;
+        const uint32_t b = __ballot_sync(0xffffffffu, f);
+        if (f) out[off[l] + __popc(b & ((1u << lane) - 1u))] = slots[l * kSeg + lane] & ((1ull << 59) - 1ull);
+    }
 }
 
 struct MaxOp {
@@ -325,6 +364,8 @@ struct cgb_gpma {
     std::string err;
     std::vector<GpmaDir> dirs;
     uint64_t total_slots = 0, n_leaves = 0, n_keys = 0;
+    uint64_t dir_n[CGB_MAX_DIR] = {0};  // keys per direction
+    bool counts_stale = false;  // an update failed after its deletes: leaf and direction counts are behind
     uint64_t* slots = nullptr;
     uint8_t* valid = nullptr;
     uint32_t* leaf_cnt = nullptr;
@@ -447,7 +488,7 @@ cgb_status rebuild(cgb_gpma* g, const uint64_t* keys, uint64_t n) {
     std::vector<uint64_t> start(g->nd), cnt(g->nd);
     uint64_t acc = 0;
     for (uint32_t d = 0; d < g->nd; ++d) {
-        cnt[d] = h[1 + d];
+        cnt[d] = g->dir_n[d] = h[1 + d];
         start[d] = acc;
         acc += cnt[d];
         uint32_t hh = 0;
@@ -480,11 +521,27 @@ cgb_status rebuild(cgb_gpma* g, const uint64_t* keys, uint64_t n) {
     GCK(cudaMemcpyAsync(d_cnt, cnt.data(), g->nd * 8, cudaMemcpyHostToDevice, g->stream));
     DirTab dt{g->d_off, g->d_cap, g->d_h, g->d_leaf0};
     k_gp_spread<<<grid_of(off), 256, 0, g->stream>>>(keys, n, d_start, d_cnt, dt, g->nd, g->slots, g->valid, off);
-    k_gp_leafcount<<<grid_of(leaf * 32), 256, 0, g->stream>>>(g->valid, leaf, g->leaf_cnt);
     k_gp_leafdir<<<grid_of(leaf), 256, 0, g->stream>>>(g->leaf_dir, g->d_leaf0, g->nd, leaf);
+    k_gp_leafcount<<<grid_of(leaf * 32), 256, 0, g->stream>>>(g->valid, leaf, g->leaf_dir, g->leaf_cnt, hist);
     GCK(cudaGetLastError());
     GCK(cudaStreamSynchronize(g->stream));
+    g->counts_stale = false;
     reclaim(g);
+    return CGB_OK;
+}
+
+// Leaf counts and direction counts from the valid flags.
+cgb_status recount(cgb_gpma* g) {
+    GCK(cudaMemsetAsync(g->d_scal + 3, 0, CGB_MAX_DIR * sizeof(unsigned long long), g->stream));
+    k_gp_leafcount<<<grid_of(g->n_leaves * 32), 256, 0, g->stream>>>(g->valid, g->n_leaves, g->leaf_dir, g->leaf_cnt,
+                                                                     g->d_scal + 3);
+    GCK(cudaGetLastError());
+    unsigned long long dn[CGB_MAX_DIR];
+    GCK(cudaMemcpyAsync(dn, g->d_scal + 3, sizeof(dn), cudaMemcpyDeviceToHost, g->stream));
+    GCK(cudaStreamSynchronize(g->stream));
+    g->n_keys = 0;
+    for (uint32_t d = 0; d < g->nd; ++d) g->n_keys += g->dir_n[d] = dn[d];
+    g->counts_stale = false;
     return CGB_OK;
 }
 
@@ -576,6 +633,7 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
     const uint64_t n = n_ins + n_del;
     if (n == 0) return CGB_OK;
     cgb_status s;
+    if (g->counts_stale && (s = recount(g)) != CGB_OK) return s;
     reclaim(g);
     if ((s = after_default_stream(g)) != CGB_OK) return s;
     GCK(cudaEventRecord(g->e0, g->stream));
@@ -586,10 +644,7 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
     if ((s = galloc(g, k_out, n)) != CGB_OK) return s;
     if ((s = galloc(g, o_in, n)) != CGB_OK) return s;
     if ((s = galloc(g, o_out, n)) != CGB_OK) return s;
-    if (n_ins) GCK(cudaMemcpyAsync(k_in, ins_device, n_ins * 8, cudaMemcpyDeviceToDevice, g->stream));
-    if (n_del) GCK(cudaMemcpyAsync(k_in + n_ins, del_device, n_del * 8, cudaMemcpyDeviceToDevice, g->stream));
-    GCK(cudaMemsetAsync(o_in, 0, n_ins, g->stream));
-    GCK(cudaMemsetAsync(o_in + n_ins, 1, n_del, g->stream));
+    k_gp_edits<<<grid_of(n), 256, 0, g->stream>>>(ins_device, n_ins, del_device, n_del, k_in, o_in);
     size_t bytes = 0;
     GCK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, k_in, k_out, o_in, o_out, n, 0, 64, g->stream));
     if ((s = gtemp(g, bytes)) != CGB_OK) return s;
@@ -598,29 +653,54 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
     uint64_t *ins_key = nullptr, *ins_leaf = nullptr;
     if ((s = galloc(g, ins_key, n)) != CGB_OK) return s;
     if ((s = galloc(g, ins_leaf, n)) != CGB_OK) return s;
-    GCK(cudaMemsetAsync(g->d_scal, 0, 3 * sizeof(unsigned long long), g->stream));
+    GCK(cudaMemsetAsync(g->d_scal, 0, (3 + CGB_MAX_DIR) * sizeof(unsigned long long), g->stream));
     GCK(cudaMemsetAsync(g->leaf_delta, 0, g->n_leaves * sizeof(int), g->stream));
     GCK(cudaMemsetAsync(g->leaf_ins, 0, g->n_leaves * sizeof(uint32_t), g->stream));
     DirTab dt{g->d_off, g->d_cap, g->d_h, g->d_leaf0};
+    g->counts_stale = true;
     unsigned int* d_flags = (unsigned int*)(g->d_scal + 2);  // [0] resize, [1] error
     k_gp_effect<<<grid_of(n), 256, 0, g->stream>>>(k_out, o_out, n, g->slots, g->valid, dt, g->nd, ins_key, ins_leaf,
                                                    g->d_scal + 0, g->leaf_delta, g->leaf_ins, d_flags + 1);
-    // 3. windows
-    uint64_t *newc = nullptr, *P = nullptr, *win = nullptr;
-    if ((s = galloc(g, newc, g->n_leaves)) != CGB_OK) return s;
-    if ((s = galloc(g, P, g->n_leaves)) != CGB_OK) return s;
-    if ((s = galloc(g, win, n)) != CGB_OK) return s;
-    k_gp_newcount<<<grid_of(g->n_leaves), 256, 0, g->stream>>>(g->leaf_cnt, g->leaf_delta, g->n_leaves, newc);
-    bytes = 0;
-    GCK(cub::DeviceScan::InclusiveSum(nullptr, bytes, newc, P, g->n_leaves, g->stream));
-    if ((s = gtemp(g, bytes)) != CGB_OK) return s;
-    GCK(cub::DeviceScan::InclusiveSum(g->temp, bytes, newc, P, g->n_leaves, g->stream));
-    k_gp_window<<<grid_of(g->n_leaves), 256, 0, g->stream>>>(g->leaf_ins, P, g->leaf_dir, dt, g->n_leaves, win,
-                                                             g->d_scal + 1, d_flags);
+    // 3. windows: per leaf, the level of the window starting there; the maximal
+    // ones numbered by a running sum
+    uint64_t *newc = nullptr, *kept = nullptr, *P = nullptr, *Q = nullptr, *wend = nullptr, *pmax = nullptr;
+    uint32_t *wlv = nullptr, *flag = nullptr, *widx = nullptr;
+    GpWin* win = nullptr;
+    uint64_t* wcount = nullptr;
+    unsigned long long* wfill = nullptr;
+    const uint64_t L = g->n_leaves, maxwin = std::min(L, n);
+    if ((s = galloc(g, newc, L)) != CGB_OK) return s;
+    if ((s = galloc(g, kept, L)) != CGB_OK) return s;
+    if ((s = galloc(g, P, L)) != CGB_OK) return s;
+    if ((s = galloc(g, Q, L)) != CGB_OK) return s;
+    if ((s = galloc(g, wend, L)) != CGB_OK) return s;
+    if ((s = galloc(g, pmax, L)) != CGB_OK) return s;
+    if ((s = galloc(g, wlv, L)) != CGB_OK) return s;
+    if ((s = galloc(g, flag, L)) != CGB_OK) return s;
+    if ((s = galloc(g, widx, L)) != CGB_OK) return s;
+    if ((s = galloc(g, win, maxwin)) != CGB_OK) return s;
+    if ((s = galloc(g, wcount, maxwin)) != CGB_OK) return s;
+    if ((s = galloc(g, wfill, maxwin)) != CGB_OK) return s;
+    GCK(cudaMemsetAsync(wlv, 0, L * sizeof(uint32_t), g->stream));
+    k_gp_newcount<<<grid_of(L), 256, 0, g->stream>>>(g->leaf_cnt, g->leaf_delta, g->leaf_ins, L, newc, kept);
+    size_t b1 = 0, b2 = 0, b3 = 0;
+    GCK(cub::DeviceScan::InclusiveSum(nullptr, b1, newc, P, L, g->stream));
+    GCK(cub::DeviceScan::InclusiveScan(nullptr, b2, wend, pmax, MaxOp(), L, g->stream));
+    GCK(cub::DeviceScan::InclusiveSum(nullptr, b3, flag, widx, L, g->stream));
+    if ((s = gtemp(g, std::max(b1, std::max(b2, b3)))) != CGB_OK) return s;
+    GCK(cub::DeviceScan::InclusiveSum(g->temp, b1, newc, P, L, g->stream));
+    GCK(cub::DeviceScan::InclusiveSum(g->temp, b1, kept, Q, L, g->stream));
+    k_gp_window<<<grid_of(L), 256, 0, g->stream>>>(g->leaf_ins, P, g->leaf_dir, dt, L, wlv, d_flags);
+    k_gp_end<<<grid_of(L), 256, 0, g->stream>>>(wlv, L, wend);
+    GCK(cub::DeviceScan::InclusiveScan(g->temp, b2, wend, pmax, MaxOp(), L, g->stream));
+    k_gp_maximal<<<grid_of(L), 256, 0, g->stream>>>(wlv, pmax, L, flag);
+    GCK(cub::DeviceScan::InclusiveSum(g->temp, b3, flag, widx, L, g->stream));
+    k_gp_wininfo<<<grid_of(L), 256, 0, g->stream>>>(flag, widx, pmax, L, P, Q, g->slots, win, wcount, wfill,
+                                                    g->d_scal + 1);
     unsigned long long h3[3];
     GCK(cudaMemcpyAsync(h3, g->d_scal, sizeof(h3), cudaMemcpyDeviceToHost, g->stream));
     GCK(cudaStreamSynchronize(g->stream));
-    const uint64_t nins = h3[0], nwin_all = h3[1];
+    const uint64_t nins = h3[0], nwin = h3[1];
     const unsigned int resize = (unsigned int)(h3[2] & 0xffffffffull), kerr = (unsigned int)(h3[2] >> 32);
     if (kerr) return gfail(g, CGB_ERR_ARG, "key direction out of range (>= %u)", g->nd);
     if (resize) {
@@ -653,44 +733,13 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
         g->stats[5] = g->n_keys;
         return s;
     }
-    uint64_t nwin = 0;
-    uint64_t *wsorted = nullptr, *wmax = nullptr, *wend = nullptr;
-    if (nwin_all) {
-        if ((s = galloc(g, wsorted, nwin_all)) != CGB_OK) return s;
-        if ((s = galloc(g, wend, nwin_all)) != CGB_OK) return s;
-        if ((s = galloc(g, wmax, nwin_all)) != CGB_OK) return s;
-        bytes = 0;
-        GCK(cub::DeviceRadixSort::SortKeys(nullptr, bytes, win, wsorted, nwin_all, 0, 64, g->stream));
-        if ((s = gtemp(g, bytes)) != CGB_OK) return s;
-        GCK(cub::DeviceRadixSort::SortKeys(g->temp, bytes, win, wsorted, nwin_all, 0, 64, g->stream));
-        k_gp_end<<<grid_of(nwin_all), 256, 0, g->stream>>>(wsorted, nwin_all, wend);
-        bytes = 0;
-        GCK(cub::DeviceScan::InclusiveScan(nullptr, bytes, wend, wmax, MaxOp(), nwin_all, g->stream));
-        if ((s = gtemp(g, bytes)) != CGB_OK) return s;
-        GCK(cub::DeviceScan::InclusiveScan(g->temp, bytes, wend, wmax, MaxOp(), nwin_all, g->stream));
-        uint8_t* flag = nullptr;
-        if ((s = galloc(g, flag, nwin_all)) != CGB_OK) return s;
-        k_gp_maximal<<<grid_of(nwin_all), 256, 0, g->stream>>>(wsorted, wmax, nwin_all, flag);
-        bytes = 0;
-        GCK(cub::DeviceSelect::Flagged(nullptr, bytes, wsorted, flag, win, g->d_scal + 1, nwin_all, g->stream));
-        if ((s = gtemp(g, bytes)) != CGB_OK) return s;
-        GCK(cub::DeviceSelect::Flagged(g->temp, bytes, wsorted, flag, win, g->d_scal + 1, nwin_all, g->stream));
-        unsigned long long hw = 0;
-        GCK(cudaMemcpyAsync(&hw, g->d_scal + 1, 8, cudaMemcpyDeviceToHost, g->stream));
-        GCK(cudaStreamSynchronize(g->stream));
-        nwin = hw;
-    }
     uint64_t rewritten = 0;
     if (nwin) {
         // 5. rewrite the windows: gather, sort, spread
-        uint64_t *wcount = nullptr, *wpred = nullptr, *woff = nullptr, *wfill = nullptr;
-        if ((s = galloc(g, wcount, nwin)) != CGB_OK) return s;
-        if ((s = galloc(g, wpred, nwin)) != CGB_OK) return s;
+        uint64_t* woff = nullptr;
         if ((s = galloc(g, woff, nwin + 1)) != CGB_OK) return s;
-        if ((s = galloc(g, wfill, nwin)) != CGB_OK) return s;
-        k_gp_wininfo<<<grid_of(nwin), 256, 0, g->stream>>>(win, nwin, P, g->slots, wcount, wpred);
         bytes = 0;
-        GCK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, wcount, woff, nwin + 0, g->stream));
+        GCK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, wcount, woff, nwin, g->stream));
         if ((s = gtemp(g, bytes)) != CGB_OK) return s;
         GCK(cub::DeviceScan::ExclusiveSum(g->temp, bytes, wcount, woff, nwin, g->stream));
         unsigned long long tail[2];
@@ -703,11 +752,10 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
         if ((s = galloc(g, srt, total)) != CGB_OK) return s;
         GCK(cudaMemcpyAsync(woff + nwin, &total, 8, cudaMemcpyHostToDevice, g->stream));
         unsigned int* d_bad = d_flags + 1;  // cleared at the start of the batch
-        k_gp_gather<<<(unsigned)std::min<uint64_t>(nwin, 148ull * 8), 256, 0, g->stream>>>(
-            win, nwin, woff, wcount, g->slots, g->valid, tmp, wfill, d_bad);
+        k_gp_gather<<<grid_of(L * 32), 256, 0, g->stream>>>(win, widx, pmax, L, woff, Q, g->slots, g->valid, tmp, d_bad);
         if (nins)
-            k_gp_place_ins<<<grid_of(nins), 256, 0, g->stream>>>(ins_key, ins_leaf, nins, win, nwin, woff, wcount,
-                                                                 (unsigned long long*)wfill, tmp, d_bad);
+            k_gp_place_ins<<<grid_of(nins), 256, 0, g->stream>>>(ins_key, ins_leaf, nins, widx, pmax, woff, win, wfill,
+                                                                 tmp, d_bad);
         unsigned int hb = 0;
         GCK(cudaMemcpyAsync(&hb, d_bad, 4, cudaMemcpyDeviceToHost, g->stream));
         GCK(cudaStreamSynchronize(g->stream));
@@ -716,30 +764,14 @@ cgb_status cgb_gpma_batch_update(cgb_gpma* g, const uint64_t* ins_device, uint64
         GCK(cub::DeviceSegmentedSort::SortKeys(nullptr, bytes, tmp, srt, total, nwin, woff, woff + 1, g->stream));
         if ((s = gtemp(g, bytes)) != CGB_OK) return s;
         GCK(cub::DeviceSegmentedSort::SortKeys(g->temp, bytes, tmp, srt, total, nwin, woff, woff + 1, g->stream));
-        k_gp_scatter<<<(unsigned)std::min<uint64_t>(nwin, 148ull * 8), 256, 0, g->stream>>>(win, nwin, woff, wcount,
-                                                                                             wpred, srt, g->slots,
-                                                                                             g->valid);
+        k_gp_scatter<<<grid_of(L * 32), 256, 0, g->stream>>>(win, widx, pmax, L, woff, srt, g->slots, g->valid);
         rewritten = total;
     }
-    k_gp_leafcount<<<grid_of(g->n_leaves * 32), 256, 0, g->stream>>>(g->valid, g->n_leaves, g->leaf_cnt);
     GCK(cudaGetLastError());
     GCK(cudaEventRecord(g->e1, g->stream));
-    GCK(cudaEventSynchronize(g->e1));
+    if ((s = recount(g)) != CGB_OK) return s;
     float ms = 0;
     cudaEventElapsedTime(&ms, g->e0, g->e1);
-    // key count: sum of leaf counts
-    {
-        uint64_t* tot = nullptr;
-        if ((s = galloc(g, tot, 1)) != CGB_OK) return s;
-        bytes = 0;
-        GCK(cub::DeviceReduce::Sum(nullptr, bytes, g->leaf_cnt, tot, g->n_leaves, g->stream));
-        if ((s = gtemp(g, bytes)) != CGB_OK) return s;
-        GCK(cub::DeviceReduce::Sum(g->temp, bytes, g->leaf_cnt, tot, g->n_leaves, g->stream));
-        uint64_t ht = 0;
-        GCK(cudaMemcpyAsync(&ht, tot, 8, cudaMemcpyDeviceToHost, g->stream));
-        GCK(cudaStreamSynchronize(g->stream));
-        g->n_keys = ht;
-    }
     g->stats[0] = g->total_slots;
     g->stats[1] = nwin;
     g->stats[2] = rewritten;
@@ -755,25 +787,24 @@ cgb_status cgb_gpma_extract(cgb_gpma* g, uint32_t dir, uint64_t* out_device, uin
     GCK(cudaSetDevice(g->device));
     const GpmaDir& D = g->dirs[dir];
     cgb_status s;
+    if (g->counts_stale && (s = recount(g)) != CGB_OK) return s;
+    const uint64_t m = g->dir_n[dir];  // kept by every load and update
+    *n_out = m;
+    if (!out_device) return CGB_OK;
+    if (cap < m) return gfail(g, CGB_ERR_ARG, "buffer holds %llu of %llu keys", (unsigned long long)cap, (unsigned long long)m);
+    if (!m) return CGB_OK;
     reclaim(g);
     if ((s = after_default_stream(g)) != CGB_OK) return s;
-    uint64_t* tmp = nullptr;
-    if ((s = galloc(g, tmp, D.cap)) != CGB_OK) return s;
+    const uint64_t L = D.cap / kSeg;
+    uint64_t* off = nullptr;
+    if ((s = galloc(g, off, L)) != CGB_OK) return s;
     size_t bytes = 0;
-    GCK(cub::DeviceSelect::Flagged(nullptr, bytes, g->slots + D.off, g->valid + D.off, tmp, g->d_scal + 1, D.cap,
-                                   g->stream));
+    GCK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, g->leaf_cnt + D.leaf0, off, L, g->stream));
     if ((s = gtemp(g, bytes)) != CGB_OK) return s;
-    GCK(cub::DeviceSelect::Flagged(g->temp, bytes, g->slots + D.off, g->valid + D.off, tmp, g->d_scal + 1, D.cap,
-                                   g->stream));
-    unsigned long long m = 0;
-    GCK(cudaMemcpyAsync(&m, g->d_scal + 1, 8, cudaMemcpyDeviceToHost, g->stream));
+    GCK(cub::DeviceScan::ExclusiveSum(g->temp, bytes, g->leaf_cnt + D.leaf0, off, L, g->stream));
+    k_gp_extract<<<grid_of(L * 32), 256, 0, g->stream>>>(g->slots + D.off, g->valid + D.off, L, off, out_device);
+    GCK(cudaGetLastError());
     GCK(cudaStreamSynchronize(g->stream));
-    *n_out = m;
-    if (out_device) {
-        if (cap < m) { reclaim(g); return gfail(g, CGB_ERR_ARG, "buffer holds %llu of %llu keys", (unsigned long long)cap, m); }
-        if (m) k_gp_strip_dir<<<grid_of(m), 256, 0, g->stream>>>(tmp, m, out_device);
-        GCK(cudaStreamSynchronize(g->stream));
-    }
     reclaim(g);
     return CGB_OK;
 }
