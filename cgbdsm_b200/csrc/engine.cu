@@ -2539,13 +2539,13 @@ cgb_status reserve_pool(cgb_handle* h, uint64_t n_edits) {
 }
 
 // Sorts packed keys in place (alt buffer used as ping-pong); returns sorted pointer.
-cgb_status radix_sort(cgb_handle* h, uint64_t*& keys, uint64_t*& alt, uint64_t n, int end_bit) {
+cgb_status radix_sort(cgb_handle* h, uint64_t*& keys, uint64_t*& alt, uint64_t n, int begin_bit, int end_bit) {
     if (n == 0) return CGB_OK;
     cub::DoubleBuffer<uint64_t> db(keys, alt);
     size_t tb = 0;
-    CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (int64_t)n, 0, end_bit, h->stream));
+    CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (int64_t)n, begin_bit, end_bit, h->stream));
     if (grow_temp(h, tb) != CGB_OK) return CGB_ERR_OOM;
-    CK(cub::DeviceRadixSort::SortKeys(h->d_temp, tb, db, (int64_t)n, 0, end_bit, h->stream));
+    CK(cub::DeviceRadixSort::SortKeys(h->d_temp, tb, db, (int64_t)n, begin_bit, end_bit, h->stream));
     LAUNCHED();
     if (db.Current() != keys) std::swap(keys, alt);
     return CGB_OK;
@@ -2600,9 +2600,11 @@ cgb_status apply_edits(cgb_handle* h, const EditSrc& src) {
     k_pack_edits<<<grid_for(h, n), 256, 0, h->stream>>>(src, pi, h->d_edits, d_err, h->d_self);
     LAUNCHED();
     CK(cudaGetLastError());
-    // valid keys use 2B+6 bits; one more bit makes the all-ones invalid marker sort last
+    // by (d,u,v), and one bit more that makes the all-ones invalid marker sort
+    // last; the op bit is left out: the sort is stable and adds come first
     if (src.n_add + src.n_rem)
-        if ((s = radix_sort(h, h->d_edits, h->d_edits_alt, n, 2 * (int)pi.B + 7)) != CGB_OK) return s;
+        if ((s = radix_sort(h, h->d_edits, h->d_edits_alt, n, 1, 2 * (int)pi.B + (int)bits_for(h->nd) + 2)) != CGB_OK)
+            return s;
     MergeArgs ma;
     ma.rec = h->rec;
     ma.dvcap = h->dvcap;
@@ -2925,7 +2927,7 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
         if ((s = ensure_delta_buffers(h, n_delta)) != CGB_OK) return s;
         k_pack_delta<<<grid_for(h, n_delta), 256, 0, h->stream>>>(delta, n_delta, pi, h->d_dkeys, d_err, h->d_self);
         LAUNCHED();
-        if ((s = radix_sort(h, h->d_dkeys, h->d_dkeys_alt, n_delta, 2 * (int)B + 6)) != CGB_OK) return s;
+        if ((s = radix_sort(h, h->d_dkeys, h->d_dkeys_alt, n_delta, 0, 2 * (int)B + (int)bits_for(h->nd) + 1)) != CGB_OK) return s;
         if (edge_ok) CK(cudaMemcpyAsync(h->d_edge_ok, edge_ok, h->q.qe, cudaMemcpyHostToDevice, h->stream));
         k_delta<<<grid_for(h, n_delta) + 1, 256, 0, h->stream>>>(h->d_dkeys, n_delta, B, h->rec, h->dvcap, h->d_dval,
                                                                  h->q.qe, h->d_plans, h->d_qe_dirs, h->d_edge_ok,

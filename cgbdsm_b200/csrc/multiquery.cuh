@@ -353,7 +353,7 @@ cgb_status mq_prepare_delta(cgb_mq* m, const uint32_t* pairs, uint64_t mpairs, b
     k_mq_pack<<<grid_for(h, mpairs), 256, 0, h->stream>>>(pairs, mpairs, h->d_vlabel, h->dv, B, h->lb, h->d_dkeys,
                                                           d_err);
     LAUNCHED();
-    MQ_TRY(radix_sort(h, h->d_dkeys, h->d_dkeys_alt, n, 2 * (int)B + 5 + (int)h->lb));
+    MQ_TRY(radix_sort(h, h->d_dkeys, h->d_dkeys_alt, n, 0, std::min(64, 2 * (int)(B + h->lb) + 1)));
     k_mq_mark<<<grid_for(h, n), 256, 0, h->stream>>>(h->d_dkeys, n, h->rec, h->dvcap, h->pool, B, h->lb,
                                                      want_present ? 1 : 0, m->d_keep);
     LAUNCHED();
@@ -500,9 +500,12 @@ cgb_status mq_match_all(cgb_mq* m, uint64_t n2) {
     return CGB_OK;
 }
 
-// Reads the error word and stats of the last step (synchronizes).
+// Reads the error word, stats and counts of the last step (synchronizes).
 cgb_status mq_sync(cgb_mq* m) {
     cgb_handle* h = m->h;
+    if (m->G)
+        MCK(cudaMemcpyAsync(m->h_counts, m->d_counts, m->G * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                            h->stream));
     MQ_TRY(sync_scalars(h));
     for (int i = 0; i < 8; ++i) m->last_stats[i] = h->h_scal[kCtlStats + i];
     return CGB_OK;
@@ -608,13 +611,8 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
     return CGB_OK;
 }
 
-// Adds the counts of the last matching step (plans) into out[query id].
+// Adds the counts of the last matching step (plans, read by mq_sync) into out[query id].
 cgb_status mq_collect(cgb_mq* m, uint64_t* out, uint32_t cap) {
-    if (m->G) {
-        MCK(cudaMemcpyAsync(m->h_counts, m->d_counts, m->G * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                            m->h->stream));
-        MCK(cudaStreamSynchronize(m->h->stream));
-    }
     for (uint32_t g = 0; g < m->G; ++g)
         if (out && m->plan_query[g] < cap) out[m->plan_query[g]] += m->h_counts[g];
     return CGB_OK;
@@ -852,15 +850,17 @@ cgb_status cgb_mq_apply_batch_device(cgb_mq* m, const uint32_t* ins_device, uint
         MQ_TRY(apply_edits(h, gone));
         MCK(cudaEventRecord(m->ev[3], h->stream));
         if (m->G) {
-            if ((s = mq_match_enqueue(m, m->d_plans, m->d_pair, m->G, n2, m->bps ? m->bps : mq_occupancy(m),
-                                      m->steal, m->cfg.dfs_budget_ms ? m->cfg.dfs_budget_ms : 600000ull)) != CGB_OK)
-                return s;
+            if (m->bps == 0)
+                m->bps = m->cfg.dfs_blocks_per_sm ? std::min<int>(mq_occupancy(m), m->cfg.dfs_blocks_per_sm)
+                                                  : mq_occupancy(m);
+            if ((s = mq_match_all(m, n2)) != CGB_OK) return s;
         } else {
             k_delta_lists<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, 0, m->d_nsel, bits_for(h->dv), h->lb,
                                                                   h->rec, h->dvcap, nullptr, 1);
             LAUNCHED();
         }
         MCK(cudaEventRecord(m->ev[4], h->stream));
+        if (!n_ins) MCK(cudaEventRecord(m->ev[5], h->stream));
         MQ_TRY(mq_sync(m));
         if ((s = mq_check_err(m)) != CGB_OK) return s;
         if ((s = mq_collect(m, neg_counts, cap)) != CGB_OK) return s;
@@ -900,6 +900,7 @@ cgb_status cgb_mq_apply_batch_device(cgb_mq* m, const uint32_t* ins_device, uint
         k_mq_strip<<<grid_for(h, n2), 256, 0, h->stream>>>(m->d_sel, n2, h->pending_B, h->lb, h->d_pending);
         LAUNCHED();
         h->n_pending = n2;
+        MCK(cudaEventRecord(m->ev[5], h->stream));
         MQ_TRY(mq_sync(m));
         if ((s = mq_check_err(m)) != CGB_OK) {
             h->n_pending = 0;
@@ -910,12 +911,11 @@ cgb_status cgb_mq_apply_batch_device(cgb_mq* m, const uint32_t* ins_device, uint
         t_delta += ms;
         MCK(cudaEventElapsedTime(&ms, m->ev[3], m->ev[4]));
         t_match += ms;
-    } else {
+    } else if (!n_del) {
+        MCK(cudaEventRecord(m->ev[5], h->stream));
         MQ_TRY(mq_sync(m));
         if ((s = mq_check_err(m)) != CGB_OK) return s;
     }
-    MCK(cudaEventRecord(m->ev[5], h->stream));
-    MCK(cudaEventSynchronize(m->ev[5]));
     float t_upd = 0, t_all = 0;
     MCK(cudaEventElapsedTime(&t_upd, m->ev[0], m->ev[1]));
     MCK(cudaEventElapsedTime(&t_all, m->ev[0], m->ev[5]));
