@@ -143,13 +143,19 @@ __global__ void k_pack_delta(const uint64_t* __restrict__ in, uint64_t n, PackIn
 }
 
 // ---------------------------------------------------------------------------
-// fused edit merge of every touched (d, u): warp per run below kBigRun merged
-// entries, CTA per longer (hub) run
+// fused edit merge of every touched (d, u): lane per run up to kTinyRun merged
+// entries, warp per run below kBigRun, longer (hub) runs in tiles, a CTA each
 // ---------------------------------------------------------------------------
 constexpr uint32_t kTinyRun = 32;        // merged entries up to which one lane merges the run
-constexpr uint32_t kBigRun = 4096;       // merged entries (old run + edits) from which a CTA merges the run
-constexpr uint32_t kMergeWarps = 8;      // warps of a CTA merge
-constexpr uint32_t kSegWindows = 8;      // 32-entry windows a CTA warp merges per round
+// Merged entries (old run + edits) from which CTAs merge the run: a warp takes
+// about 0.45 us per 32 entries (a chain of two dependent loads), a CTA about
+// 3 us for a tile.
+constexpr uint32_t kBigRun = 512;
+constexpr uint32_t kMergeThreads = 256;
+constexpr uint32_t kMergeItems = 11;     // merged entries per thread of a tile; odd: no bank conflicts
+constexpr uint32_t kMergeTile = kMergeThreads * kMergeItems;
+constexpr uint64_t kTileAggregate = 1ull << 62, kTilePrefix = 2ull << 62, kTileValue = kTileAggregate - 1;  // tile states
+constexpr uint32_t kTileSpins = 1u << 24;
 constexpr uint32_t kNoVal = 0xffffffffu; // window padding: above every vertex id (< 2^27)
 
 struct MergeArgs {
@@ -161,8 +167,14 @@ struct MergeArgs {
     long long* live_words;       // sum of round4(len) over runs
     const uint64_t* edits;       // ((d,u,v)<<1|op), each run's edits together and sorted
     uint64_t n;
-    uint2* runs[3];              // {first edit, edits} of the runs merged by a warp / by a CTA / by a lane (k_edit_runs)
-    unsigned int* list_ctr;      // [0] warp, [1] CTA, [2] lane
+    uint2* runs[3];              // {first edit, edits} of the runs merged by a warp / in tiles / by a lane (k_edit_runs)
+    unsigned int* list_ctr;      // [0] warp, [1] tiled, [2] lane, [4] tiles listed, [5] tiles taken
+    unsigned long long* big_off; // tiled runs: where in the pool they go
+    uint32_t* big_tile0;         //             their first tile
+    uint32_t big_cap;
+    uint2* tiles;                // {tiled run, tile of it}, a run's tiles in order
+    unsigned long long* tile_state;  // per tile: its count, or the count up to it (zeroed before)
+    uint32_t tile_cap;
     uint32_t B;
     unsigned int* err;
     unsigned long long* stats;   // [5] merge bytes (edits 8 B, old run 4 B/word, new run 4 B/word, record 32 B), [6] runs
@@ -193,18 +205,24 @@ __device__ __forceinline__ uint32_t win_rank(uint32_t w, uint32_t x, bool le) {
     return lo + ((le ? v <= x : v < x) ? 1u : 0u);
 }
 
-// Merge-path split of diagonal k of X (old run) and Y (edits): the number of
-// X entries among the first k merged entries, X winning ties (so for equal
-// values the old entry precedes an add, and an add precedes a remove).
-__device__ __forceinline__ uint32_t merge_split(const uint32_t* X, uint32_t xl, const uint64_t* Y,
-                                                uint32_t yl, uint32_t k, uint64_t vmask) {
+// Merge-path split of diagonal k of X (old run) and Y (edits) by one warp: the
+// number of X entries among the first k merged entries, X winning ties (so
+// for equal values the old entry precedes an add, and an add precedes a
+// remove).  32 pivots a round.
+__device__ __forceinline__ uint32_t merge_split(const uint32_t* __restrict__ X, uint32_t xl,
+                                                const uint64_t* __restrict__ Y, uint32_t yl, uint32_t k,
+                                                uint64_t vmask, uint32_t lane) {
     uint32_t lo = k > yl ? k - yl : 0;
     uint32_t hi = k < xl ? k : xl;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        uint32_t yv = (uint32_t)((__ldg(Y + (k - 1 - mid)) >> 1) & vmask);
-        if (__ldg(X + mid) <= yv) lo = mid + 1;
-        else hi = mid;
+    while (hi > lo) {
+        const uint32_t n = hi - lo, step = n > 32 ? n >> 5 : 1u;
+        const uint32_t p = lo + (lane + 1) * step - 1;
+        const bool below = p < hi && __ldg(X + p) <= (uint32_t)((__ldg(Y + (k - 1 - p)) >> 1) & vmask);
+        const uint32_t c = __popc(__ballot_sync(kFull, below));
+        if (n <= 32) return lo + c;
+        const uint32_t base = lo;
+        if (c) lo = base + c * step;
+        if (c < 32) hi = base + (c + 1) * step - 1;
     }
     return lo;
 }
@@ -251,6 +269,16 @@ __device__ __forceinline__ bool merge_window(const uint32_t* __restrict__ X, uin
     return emit;
 }
 
+// Pool space for a merged run of at most `bound` entries (~0 when exhausted).
+__device__ __forceinline__ unsigned long long pool_alloc(const MergeArgs& a, uint32_t bound) {
+    unsigned long long off = atomicAdd(a.pool_top, (unsigned long long)round4(bound));
+    if (off + round4(bound) > a.pool_cap) {
+        atomicOr(a.err, 4u);
+        off = ~0ull;
+    }
+    return off;
+}
+
 // Finds the runs of the edits (an edit whose (d,u) differs from the one before
 // starts one; its end is searched by doubling steps) and lists them by merged
 // length: one pass over the edits where a run-length encoding, a scan of the
@@ -277,11 +305,30 @@ __global__ void k_edit_runs(MergeArgs a) {
                 }
                 len = (uint32_t)(lo + 1 - i);
                 const uint32_t total = a.rec[(size_t)(du >> a.B) * a.dvcap + (du & vmask)].y + len;
-                cls = total >= kBigRun ? 1u : total > kTinyRun ? 0u : 2u;
+                cls = total > kTinyRun ? 0u : 2u;
+                if (total >= kBigRun) {
+                    // its tiles follow one another in the tile list; a run for which
+                    // the lists have no room is left to a warp
+                    const uint32_t nt = (total + kMergeTile - 1) / kMergeTile;
+                    const uint32_t t0 = atomicAdd(a.list_ctr + 4, nt);
+                    uint32_t r = a.big_cap;
+                    if (t0 <= a.tile_cap && nt <= a.tile_cap - t0) r = atomicAdd(a.list_ctr + 1, 1u);
+                    const bool fits = r < a.big_cap;
+                    unsigned long long off = ~0ull;
+                    if (fits) {
+                        off = pool_alloc(a, total);
+                        a.runs[1][r] = make_uint2((uint32_t)i, len);
+                        a.big_off[r] = off;
+                        a.big_tile0[r] = t0;
+                        cls = 3;
+                    }
+                    for (uint32_t t = 0; t < nt && t0 + t < a.tile_cap; ++t)
+                        a.tiles[t0 + t] = make_uint2(off != ~0ull ? r : kNoVal, t);
+                }
             }
         }
 #pragma unroll
-        for (uint32_t k = 0; k < 3; ++k) {
+        for (uint32_t k = 0; k < 3; k += 2) {
             const uint32_t bal = __ballot_sync(kFull, cls == k);
             if (!bal) continue;
             uint32_t at = 0;
@@ -290,16 +337,6 @@ __global__ void k_edit_runs(MergeArgs a) {
             if (cls == k) a.runs[k][at + __popc(bal & ((1u << lane) - 1u))] = make_uint2((uint32_t)i, len);
         }
     }
-}
-
-// Pool space for a merged run of at most `bound` entries (~0 when exhausted).
-__device__ __forceinline__ unsigned long long pool_alloc(const MergeArgs& a, uint32_t bound) {
-    unsigned long long off = atomicAdd(a.pool_top, (unsigned long long)round4(bound));
-    if (off + round4(bound) > a.pool_cap) {
-        atomicOr(a.err, 4u);
-        off = ~0ull;
-    }
-    return off;
 }
 
 // Accounting of the runs one warp merged, added to the launch's counters
@@ -447,19 +484,36 @@ __device__ __forceinline__ void merge_small(const MergeArgs& a, MergeAcc& acc, u
     }
 }
 
-// CTA per long run: each round, warp w merges the 256 entries from diagonal
-// k0 + 256 w (one merge-path split per warp and round), stages what it emits
-// in shared memory, and the CTA writes the round's output contiguously.
-constexpr uint32_t kSeg = 32 * kSegWindows;
-__device__ __forceinline__ void merge_big(const MergeArgs& a, MergeAcc& acc, uint32_t (*s_win)[32]) {
-    __shared__ uint32_t s_out[kMergeWarps][kSeg];
-    __shared__ uint32_t s_cnt[kMergeWarps];
-    __shared__ unsigned long long s_off;
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t nruns = a.list_ctr[1];
+// Long runs, a tile of kMergeTile merged entries per CTA and step: the tile's
+// part of X and Y staged in shared memory by coalesced loads, merged serially
+// by each thread (kMergeItems entries), compacted, and written as one stretch
+// behind the run's earlier tiles (their states; tiles are taken in list order,
+// so every earlier one is done or running).  The run's last tile writes its
+// record: by then every earlier tile has read the old one.
+// One CTA per run and 2,048 entries per round (eight dependent windows a warp)
+// took 98 us for the R-MAT 4M/34M tree's batch.
+struct TileMem {
+    uint32_t e[kMergeTile];  // [0, nx): X (value << 1), [nx, nt): Y (value << 1 | op); then the output
+    uint32_t split[3];       // X entries before the tile, before its end; value after the tile
+    uint32_t take;
+    uint32_t base;
+    typename cub::BlockScan<uint32_t, kMergeThreads>::TempStorage scan;
+};
+__device__ __forceinline__ void merge_tiles(const MergeArgs& a, MergeAcc& acc, TileMem& sm) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t ntiles = min(a.list_ctr[4], a.tile_cap);
     const uint64_t vmask = (1ull << a.B) - 1ull;
-    for (uint32_t q = blockIdx.x; q < nruns; q += gridDim.x) {
-        const uint2 r = a.runs[1][q];
+    for (;;) {
+        __syncthreads();  // the previous tile's output has been written
+        if (threadIdx.x == 0) sm.take = atomicAdd(a.list_ctr + 5, 1u);
+        __syncthreads();
+        const uint32_t ti = sm.take;
+        if (ti >= ntiles) break;
+        const uint2 tl = a.tiles[ti];
+        if (tl.x == kNoVal) continue;  // no room for the run (error raised, run left unchanged) or merged by a warp
+        const uint2 r = a.runs[1][tl.x];
+        const uint32_t t0 = a.big_tile0[tl.x];
+        const unsigned long long off = a.big_off[tl.x];
         const uint64_t* Y = a.edits + r.x;
         const uint32_t yl = r.y;
         const uint64_t du = *Y >> (a.B + 1);
@@ -467,58 +521,113 @@ __device__ __forceinline__ void merge_big(const MergeArgs& a, MergeAcc& acc, uin
         uint4* recp = a.rec + (size_t)d * a.dvcap + u;
         const uint4 old = *recp;
         const uint32_t* X = a.pool + old.x;
-        const uint32_t xl = old.y;
-        const uint32_t total = xl + yl;
-        if (threadIdx.x == 0) s_off = pool_alloc(a, total);
+        const uint32_t xl = old.y, total = xl + yl;
+        const uint32_t k0 = tl.y * kMergeTile, k1 = min(k0 + kMergeTile, total), nt = k1 - k0;
+        if (threadIdx.x < 32) {
+            const uint32_t i0 = merge_split(X, xl, Y, yl, k0, vmask, lane);
+            if (lane == 0) sm.split[0] = i0;
+        } else if (threadIdx.x < 64) {
+            const uint32_t i1 = merge_split(X, xl, Y, yl, k1, vmask, lane);
+            if (lane == 0) {
+                sm.split[1] = i1;
+                uint32_t nxt = kNoVal;
+                if (i1 < xl) nxt = __ldg(X + i1);
+                if (k1 - i1 < yl) nxt = min(nxt, (uint32_t)((__ldg(Y + (k1 - i1)) >> 1) & vmask));
+                sm.split[2] = nxt;
+            }
+        }
         __syncthreads();
-        const unsigned long long off = s_off;
-        if (off == ~0ull) { __syncthreads(); continue; }
-        uint32_t* C = a.pool + off;
-        uint32_t outn = 0;
-        for (uint32_t k0 = 0; k0 < total; k0 += kMergeWarps * kSeg) {
-            const uint32_t ks = k0 + w * kSeg;
-            uint32_t cnt = 0;
-            if (ks < total) {
-                const uint32_t ke = min(ks + kSeg, total);
-                uint32_t i = 0;
-                if (lane == 0) i = merge_split(X, xl, Y, yl, ks, vmask);
-                i = __shfl_sync(kFull, i, 0);
-                uint32_t j = ks - i;
-                for (uint32_t k = ks; k < ke; k += 32) {
-                    const uint32_t nout = min(32u, ke - k);
-                    uint32_t val = 0;
-                    const bool emit = merge_window(X, xl, Y, yl, vmask, i, j, nout, lane, s_win[w], val);
-                    const uint32_t bal = __ballot_sync(kFull, emit);
-                    if (emit) s_out[w][cnt + __popc(bal & ((1u << lane) - 1u))] = val;
-                    cnt += __popc(bal);
+        const uint32_t i0 = sm.split[0], nx = sm.split[1] - i0, ny = nt - nx, j0 = k0 - i0, after = sm.split[2];
+        for (uint32_t t = threadIdx.x; t < nt; t += kMergeThreads) {
+            uint32_t e;
+            if (t < nx) {
+                e = __ldg(X + i0 + t) << 1;
+            } else {
+                const uint64_t y = __ldg(Y + j0 + (t - nx));
+                e = (uint32_t)((y >> 1) & vmask) << 1 | (uint32_t)(y & 1ull);
+            }
+            sm.e[t] = e;
+        }
+        __syncthreads();
+        const uint32_t* sx = sm.e;
+        const uint32_t* sy = sm.e + nx;
+        const uint32_t a0 = min(threadIdx.x * kMergeItems, nt), a1 = min(a0 + kMergeItems, nt);
+        uint32_t lo = a0 > ny ? a0 - ny : 0, hi = min(a0, nx);
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (sx[mid] <= (sy[a0 - 1 - mid] | 1u)) lo = mid + 1;  // by value, X first
+            else hi = mid;
+        }
+        uint32_t i = lo, j = a0 - lo;
+        uint32_t val[kMergeItems + 1];
+#pragma unroll
+        for (uint32_t q = 0; q <= kMergeItems; ++q) {
+            if (a0 + q < a1 || (a0 + q == a1 && a1 < nt && a0 < a1)) {
+                const bool fx = i < nx && (j >= ny || sx[i] <= (sy[j] | 1u));
+                val[q] = fx ? sx[i] : sy[j];
+                i += fx ? 1u : 0u;
+                j += fx ? 0u : 1u;
+            } else {
+                val[q] = a0 + q == nt ? after << 1 : kNoVal;
+            }
+        }
+        uint32_t emit = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kMergeItems; ++q)
+            if (a0 + q < a1 && (val[q] >> 1) != (val[q + 1] >> 1) && !(val[q] & 1u)) emit |= 1u << q;
+        uint32_t before = 0, all = 0;
+        cub::BlockScan<uint32_t, kMergeThreads>(sm.scan).ExclusiveSum((uint32_t)__popc(emit), before, all);
+        if (threadIdx.x < 32) {
+            unsigned long long base = 0;
+            if (tl.y) {
+                if (lane == 0) atomicExch(a.tile_state + ti, kTileAggregate | all);
+                int at = (int)(ti - 1);
+                bool gave_up = false;
+                for (;;) {
+                    unsigned long long v = kTilePrefix;  // before the run's first tile: 0
+                    if (at - (int)lane >= (int)t0) {
+                        uint32_t spins = 0;
+                        while ((v = *(volatile unsigned long long*)(a.tile_state + at - lane)) == 0 && ++spins < kTileSpins)
+                            __nanosleep(20);
+                    }
+                    if (__any_sync(kFull, v == 0)) { gave_up = true; break; }
+                    const uint32_t pre = __ballot_sync(kFull, (v & kTilePrefix) != 0);
+                    const uint32_t last = pre ? __ffs(pre) - 1 : 31;
+                    unsigned long long c = lane <= last ? (v & kTileValue) : 0ull;
+                    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
+                    base += c;
+                    if (pre) break;
+                    at -= 32;
+                }
+                if (gave_up && lane == 0) atomicOr(a.err, 16u);
+            }
+            if (lane == 0) {
+                atomicExch(a.tile_state + ti, kTilePrefix | (base + all));
+                sm.base = (uint32_t)base;
+                if (k1 == total) {
+                    merge_record(a, recp, old, off, (uint32_t)base + all, d, u);
+                    acc.add(xl, yl, (uint32_t)base + all);
                 }
             }
-            if (lane == 0) s_cnt[w] = cnt;
-            __syncthreads();
-            uint32_t before = 0, all = 0;
-            for (uint32_t t = 0; t < kMergeWarps; ++t) {
-                before += t < w ? s_cnt[t] : 0u;
-                all += s_cnt[t];
-            }
-            for (uint32_t t = lane; t < cnt; t += 32) C[outn + before + t] = s_out[w][t];
-            outn += all;
-            __syncthreads();
         }
-        if (threadIdx.x == 0) {
-            merge_record(a, recp, old, off, outn, d, u);
-            acc.add(xl, yl, outn);
-        }
+        __syncthreads();  // every entry of the tile is in registers: its memory takes the output
+#pragma unroll
+        for (uint32_t q = 0; q < kMergeItems; ++q)
+            if ((emit >> q) & 1u) sm.e[before++] = val[q] >> 1;
         __syncthreads();
+        uint32_t* C = a.pool + off + sm.base;
+        for (uint32_t t = threadIdx.x; t < all; t += kMergeThreads) C[t] = sm.e[t];
     }
 }
 
-// Every listed run in one launch: each block takes its share of the hub runs
-// first (they take longest), then of the warp's and the lane's runs.
-__global__ void __launch_bounds__(kMergeWarps * 32) k_merge(MergeArgs a) {
-    __shared__ uint32_t s_win[kMergeWarps][32];
+// Every listed run in one launch: each block takes tiles of the hub runs first
+// (they take longest), then its share of the warp's and the lane's runs.
+__global__ void __launch_bounds__(kMergeThreads) k_merge(MergeArgs a) {
+    __shared__ TileMem sm;
     MergeAcc acc;
-    merge_big(a, acc, s_win);
-    merge_small(a, acc, s_win[threadIdx.x >> 5]);
+    merge_tiles(a, acc, sm);
+    __syncthreads();
+    merge_small(a, acc, sm.e + 32 * (threadIdx.x >> 5));
     merge_tiny(a, acc);
     acc.flush(a, threadIdx.x & 31);
 }
@@ -2052,9 +2161,21 @@ __global__ void k_wsum(const uint4* __restrict__ rec, uint32_t dvcap, const uint
             big &= big - 1;
             const uint32_t rx = __shfl_sync(kFull, r.x, i), ry = __shfl_sync(kFull, r.y, i);
             const uint32_t rz = __shfl_sync(kFull, r.z, i), rw = __shfl_sync(kFull, r.w, i);
+            // four entries a lane and step: a hub's list is a chain of record
+            // reads, and their latency is all there is to hide
             unsigned long long sv = 0;
-            for (uint32_t t = lane; t < ry + rw; t += 32)
-                sv += term(t < ry ? __ldg(pool + rx + t) : __ldg(dval + rz + (t - ry)));
+            const uint32_t n = ry + rw;
+            for (uint32_t t = lane; t < n; t += 128) {
+                uint32_t c[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    const uint32_t e = t + 32 * k;
+                    c[k] = e < ry ? __ldg(pool + rx + e) : e < n ? __ldg(dval + rz + (e - ry)) : kNoVal;
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k)
+                    if (c[k] != kNoVal) sv += term(c[k]);
+            }
             for (int o = 16; o > 0; o >>= 1) sv += __shfl_xor_sync(kFull, sv, o);
             if (lane == i) acc = sv;
         }
@@ -2254,7 +2375,12 @@ struct cgb_handle {
     uint32_t pending_B = 0;
     uint64_t* d_edits = nullptr; uint64_t* d_edits_alt = nullptr; size_t edits_cap = 0;
     uint2* d_runs[3] = {nullptr, nullptr, nullptr};  // merge lists (k_edit_runs)
-    unsigned int* d_list_ctr = nullptr;  // [0] warp, [1] CTA, [2] lane, [3] bit-set slots claimed by the last merge
+    unsigned int* d_list_ctr = nullptr;  // MergeArgs::list_ctr, and [3] bit-set slots claimed by the last merge
+    unsigned long long* d_big_off = nullptr; size_t big_off_cap = 0;
+    uint32_t* d_big_tile0 = nullptr; size_t big_tile0_cap = 0;
+    uint2* d_tiles = nullptr; size_t tiles_cap = 0;
+    unsigned long long* d_tile_state = nullptr; size_t tile_state_cap = 0;
+    uint64_t unsynced_edits = 0;  // edits merged since h_live was read
     uint64_t* d_dkeys = nullptr; uint64_t* d_dkeys_alt = nullptr; size_t dkeys_cap = 0;
     uint32_t* d_dval = nullptr;
     uint32_t* d_seed = nullptr;  // [0..kMaxQE) lo, [kMaxQE..2kMaxQE+1) pre
@@ -2605,7 +2731,23 @@ cgb_status apply_edits(cgb_handle* h, const EditSrc& src) {
     if (src.n_add + src.n_rem)
         if ((s = radix_sort(h, h->d_edits, h->d_edits_alt, n, 1, 2 * (int)pi.B + (int)bits_for(h->nd) + 2)) != CGB_OK)
             return s;
+    // tiled runs and tiles this merge can list at most: every run entry in the
+    // index (and those merged since the last read-back) and every edit
+    const uint64_t entries = (uint64_t)std::max<long long>(h->h_live, 0) + 4 * h->unsynced_edits + n;
+    h->unsynced_edits += n;
+    const uint64_t big_cap = std::min<uint64_t>(entries / kBigRun, n) + 1;
+    const uint64_t tile_cap = std::min<uint64_t>(entries / kMergeTile + big_cap, 1u << 30);
+    if ((s = grow(h, h->d_big_off, h->big_off_cap, (size_t)big_cap)) != CGB_OK) return s;
+    if ((s = grow(h, h->d_big_tile0, h->big_tile0_cap, (size_t)big_cap)) != CGB_OK) return s;
+    if ((s = grow(h, h->d_tiles, h->tiles_cap, (size_t)tile_cap)) != CGB_OK) return s;
+    if ((s = grow(h, h->d_tile_state, h->tile_state_cap, (size_t)tile_cap)) != CGB_OK) return s;
     MergeArgs ma;
+    ma.big_off = h->d_big_off;
+    ma.big_tile0 = h->d_big_tile0;
+    ma.big_cap = (uint32_t)big_cap;
+    ma.tiles = h->d_tiles;
+    ma.tile_state = h->d_tile_state;
+    ma.tile_cap = (uint32_t)tile_cap;
     ma.rec = h->rec;
     ma.dvcap = h->dvcap;
     ma.pool = h->pool;
@@ -2629,12 +2771,13 @@ cgb_status apply_edits(cgb_handle* h, const EditSrc& src) {
     ma.rb_min_len = h->rb_len_now;
     if (rb && (s = grow(h, h->d_rb_new, h->rb_new_cap, std::max<size_t>(h->rb_cap, 1))) != CGB_OK) return s;
     ma.rb_new = h->d_rb_new;
-    CK(cudaMemsetAsync(h->d_list_ctr, 0, 4 * sizeof(unsigned int), h->stream));
+    CK(cudaMemsetAsync(h->d_list_ctr, 0, 6 * sizeof(unsigned int), h->stream));
+    CK(cudaMemsetAsync(h->d_tile_state, 0, tile_cap * sizeof(unsigned long long), h->stream));
     k_edit_runs<<<grid_for(h, n), 256, 0, h->stream>>>(ma);
     LAUNCHED();
-    // a warp per run at most, up to the blocks that can be resident
-    const int mg = std::max(1, (int)std::min<uint64_t>((n * 32 + 255) / 256, (uint64_t)h->num_sms * 8));
-    k_merge<<<mg, kMergeWarps * 32, 0, h->stream>>>(ma);
+    // a warp per run at most, up to the blocks that can be resident; a block per SM for the tiles
+    const int mg = std::max(h->num_sms, (int)std::min<uint64_t>((n * 32 + 255) / 256, (uint64_t)h->num_sms * 8));
+    k_merge<<<mg, kMergeThreads, 0, h->stream>>>(ma);
     LAUNCHED();
     if (rb) {
         k_rb_update<<<std::max(grid_for(h, n), h->num_sms), 256, 0, h->stream>>>(
@@ -2685,6 +2828,7 @@ cgb_status sync_scalars(cgb_handle* h) {
     }
     h->h_pool_top = h->h_scal[kCtlPoolTop];
     h->h_live = (long long)h->h_scal[kCtlLive];
+    h->unsynced_edits = 0;
     return CGB_OK;
 }
 
@@ -2763,7 +2907,8 @@ void cgb_destroy(cgb_handle* h) {
     void* ptrs[] = {h->rec, h->pool, h->pool_alt, h->d_scal, h->d_self, h->d_keys_in, h->d_pending, h->d_edits,
                     h->d_edits_alt, h->d_runs[0], h->d_runs[1], h->d_runs[2],
                     h->d_dkeys, h->d_dkeys_alt, h->d_dval,
-                    h->d_seed, h->d_tasks, h->d_temp, h->d_read_off, h->d_read, h->d_qe_dirs, h->d_edge_ok,
+                    h->d_seed, h->d_tasks, h->d_temp, h->d_read_off, h->d_read, h->d_big_off, h->d_big_tile0, h->d_tiles,
+                    h->d_tile_state, h->d_qe_dirs, h->d_edge_ok,
                     h->d_vb, h->d_rb_slot, h->d_rb_sel, h->d_rb_bits, h->d_rb_new, h->d_rev, h->d_touched, h->d_plans,
                     h->d_vbplans, h->d_dir_edge, h->d_lsum, h->d_wsum, h->d_wjobs};
     for (void* p : ptrs)
