@@ -849,6 +849,8 @@ __global__ void k_asymmetry(const uint4* __restrict__ rec, uint32_t dvcap, uint3
 // ---------------------------------------------------------------------------
 // persistent warp DFS (count only)
 // ---------------------------------------------------------------------------
+// DFS queue counters (words); the polled ones on lines of their own
+constexpr uint32_t kQReserved = 0, kQTickets = 1, kQDone = 32, kQBusy = 40, kQMemo = 44, kQWords = 64;
 struct DfsArgs {
     const uint4* rec;
     uint32_t dvcap;
@@ -884,6 +886,9 @@ struct DfsArgs {
     uint32_t* touched;           // footprint runs: bit per record resolved (nullptr: off)
     unsigned long long* lsum_tab;  // level-sum table [lsum_mask + 1][2], zeroed before the launch (nullptr: none)
     uint32_t lsum_mask;
+    unsigned long long* memo_tab;  // subtree memos [memo_mask + 1][4], empty before and after a launch (nullptr: none)
+    uint32_t memo_mask;
+    uint32_t* memo_list;           // claimed slots (their number at kQMemo)
     const unsigned long long* wsum;  // dense level sums [array][dvcap] (nullptr: none)
     uint32_t pair_lane_max;      // pair counting: longest shorter list a lane scans alone
 };
@@ -1178,24 +1183,54 @@ __device__ __forceinline__ uint32_t lsum_find(unsigned long long* tab, uint32_t 
     return kLsumNone;
 }
 
-// One thread: the published value of K, without claiming its slot.
-__device__ __forceinline__ bool lsum_peek(const unsigned long long* tab, uint32_t mask, unsigned long long K,
-                                          unsigned long long& val) {
-    uint32_t s = (uint32_t)((K * 0x9e3779b97f4a7c15ull) >> 32) & mask;
-    for (uint32_t probe = 0; probe < kLsumProbes; ++probe, s = (s + 1) & mask) {
-        unsigned long long k, v;
-        lsum_load(tab + 2 * (size_t)s, k, v);
-        if (k == ((K << 1) | 1ull)) {
-            val = v;
-            return true;
-        }
-        if (k == 0) return false;
-    }
-    return false;
-}
-// key of the subtree memo of plan ei at vertex x (level sums use the same table without the top bit)
+// Subtree memos.  The count S(x) of the subtree below a memo's level is a
+// function of x = m[memo_pos] alone, so all the launch needs of it is
+//     sum over x of S(x) * (sum of the weights of the prefixes that end in x).
+// A slot {key, S, weight, -} gathers both: every prefix adds its weight; the
+// one that claimed the slot expands the subtree, which may be handed to any
+// number of warps (a task carries the slot), each adding its part of S;
+// k_memo_finish multiplies.  Nobody waits for a value and no subtree is
+// expanded twice.  (Publishing a finished S left the heaviest subtrees
+// unpublished, their work being split among warps at once, and expanded by
+// every warp that met them meanwhile.)  Slots are empty between launches.
+constexpr uint32_t kMemoProbes = 8;
+
+// key of the memo of plan ei at vertex x (never 0)
 __device__ __forceinline__ unsigned long long memo_key(uint32_t ei, uint32_t x) {
-    return ((1ull << 42) | ((unsigned long long)ei << 27) | x) + 1ull;
+    return (1ull << 63) | ((unsigned long long)ei << 27) | x;
+}
+// One thread: the slot of K, claimed if there is none (fresh) and `create`;
+// kLsumNone when there is none or the probes are taken by other keys.
+__device__ __forceinline__ uint32_t memo_slot(const DfsArgs& a, unsigned long long K, bool create, bool& fresh) {
+    uint32_t s = (uint32_t)((K * 0x9e3779b97f4a7c15ull) >> 32) & a.memo_mask;
+    for (uint32_t probe = 0; probe < kMemoProbes; ++probe, s = (s + 1) & a.memo_mask) {
+        unsigned long long* slot = a.memo_tab + 4 * (size_t)s;
+        unsigned long long k = *(volatile unsigned long long*)slot;
+        if (k == 0) {
+            if (!create) return kLsumNone;
+            k = atomicCAS(slot, 0ull, K);
+            if (k == 0) {
+                fresh = true;
+                a.memo_list[atomicAdd(a.qctr + kQMemo, 1u)] = s;
+                return s;
+            }
+        }
+        if (k == K) return s;
+    }
+    return kLsumNone;
+}
+// Adds S * weight of every claimed slot to its plan's count and empties it.
+__global__ void k_memo_finish(unsigned long long* tab, const uint32_t* __restrict__ list, const unsigned int* n,
+                              unsigned long long* counts) {
+    const uint32_t total = *n;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        ulonglong2* slot = reinterpret_cast<ulonglong2*>(tab + 4 * (size_t)list[i]);
+        const ulonglong2 ks = slot[0], wx = slot[1];
+        const unsigned long long v = ks.y * wx.x;
+        if (v) atomicAdd(counts + ((ks.x >> 27) & 0xffffu), v);
+        slot[0] = make_ulonglong2(0, 0);
+        slot[1] = make_ulonglong2(0, 0);
+    }
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
@@ -1239,8 +1274,7 @@ __device__ __forceinline__ void add_release(unsigned int* p, unsigned int v) {
 }
 
 constexpr uint32_t kTaskWords = 16;
-// DFS queue counters (words); the polled ones on lines of their own
-constexpr uint32_t kQReserved = 0, kQTickets = 1, kQDone = 32, kQBusy = 40, kQWords = 64;
+constexpr uint32_t kTaskMemo = 15;  // word of a task: memo slot its counts go to (no prefix reaches position 11)
 // Tail vertices with up to this many lists stay in the tail where they hang off
 // the last core vertex (single-query engine).  R-MAT 1M/10M, 9-vertex dense,
 // matching per batch: none 14.4 ms, up to three lists 14.0, all 16.4 (four
@@ -1439,10 +1473,9 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     bool waiting = false;         // lane 0: this warp's bit of s_wait was set
     uint32_t ticket = kNoTicket;  // lane 0: ticket of the task ring this warp waits on
     uint32_t dirty = 0;  // shallowest position changed since the tail cache was filled (kClean: none)
-    bool mb = false;              // counting a subtree memo (EdgePlan::memo_from) to publish
-    bool mb_split = false;        // part of that subtree went to other warps: count it, publish nothing
+    bool mb = false;              // counting (a part of) a subtree memo's S, unweighted, into mb_slot
     uint32_t mb_slot = kLsumNone;
-    unsigned long long mb_base = 0;  // lane-local count when the memo's subtree was entered
+    unsigned long long mb_base = 0;  // lane-local count when it was entered
     unsigned long long tail_k = 0;  // product of the tail groups that depend on the current prefix alone
     uint32_t idle_spins = 0;
     bool first_seed = true;
@@ -1536,6 +1569,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
 
         int ei = 0;
         uint32_t jbase = 2, tgen = 0, tlo = 0, thi = 0;
+        mb_slot = kLsumNone;
         if (kind == 1) {
             if (kMulti) {
                 // last plan whose seeds start at or before item (empty plans skipped)
@@ -1577,6 +1611,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
             tgen = (w0 >> 24) & 0xffu;
             tlo = __shfl_sync(kFull, wv, 1);
             thi = __shfl_sync(kFull, wv, 2);
+            if (kSums) mb_slot = __shfl_sync(kFull, wv, kTaskMemo);
             if (lane >= 4 && lane < 4 + kMaxQV) m[lane - 4] = wv;
             ++n_tasks;
         }
@@ -1602,7 +1637,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         SeedGroup X{nullptr, 0u, kNoVertex};
         // weight of a grouped embedding with hs hits (1 inside a memo's subtree,
         // whose count is weighted once when it is complete)
-        auto gw = [&](uint32_t hs) -> unsigned long long { return mb ? 1ull : (unsigned long long)(X.n - hs); };
+        auto gw = [&](uint32_t hs) -> unsigned long long { return kSums && mb ? 1ull : (unsigned long long)(X.n - hs); };
         if (P.grouped) {
             const size_t xat = (size_t)P.seed_dir * a.dvcap + m[0];
             const uint4 xr = a.rec[xat];
@@ -1638,16 +1673,19 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
 
         dirty = 0;  // new unit: every cached tail count is stale
         const bool level_sum = kSums && P.sum_from && !a.vb && !self_loops && (!serial);
-        const bool memo_on = kSums && P.memo_from && a.lsum_tab && !a.vb && !self_loops;
+        const bool memo_on = kSums && P.memo_from && a.memo_tab && !a.vb && !self_loops;
         const bool pair_on = kSums && P.pair_last && !a.vb && !self_loops && (!serial);
         const bool sum_on = level_sum && !P.sum_dense;  // one-position sums, through the table
         const bool peek_on = memo_on && P.memo_from == P.memo_pos + 1;
         // position whose chunks are evaluated per lane besides the last one
         const uint32_t dpre = (pair_on || (sum_on && nc > 3)) ? nc - 2 : kNoPos;
         // depths where a chunk's passing candidates are partly counted at once:
-        // only what is not scanned yet is ever shared from them
+        // what is not scanned yet is shared from them, then single survivors (a
+        // unit that kept the survivors of a memo's position ran as long as the
+        // whole launch: 2.2 ms of the R-MAT 4M/34M sparse pattern's batch)
         const uint32_t counted = (dpre != kNoPos ? 1u << dpre : 0u) | (peek_on ? 1u << P.memo_pos : 0u);
-        mb = false;
+        mb = kSums && mb_slot != kLsumNone;  // a task inside a memo's subtree
+        mb_base = cnt;
         if (nc > 2) {
             setup(jbase);
             if (kind != 1 && lane == jbase) { st_gen = tgen; st_next = tlo; st_len = thi; }
@@ -1696,14 +1734,11 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                 gnext = __shfl_sync(kFull, st_next, j);
                 glen = __shfl_sync(kFull, st_len, j);
                 if (gnext >= glen) {
-                    if (mb && j == P.memo_from) {
-                        // the memo's subtree is complete: publish its count, weight it once
+                    if (kSums && mb && (j == P.memo_from || j == jbase)) {
+                        // this warp's part of the memo's subtree is complete
                         const unsigned long long S = warp_sum(cnt - mb_base);
-                        if (lane == 0 && !mb_split)
-                            lsum_publish(a.lsum_tab + 2 * (size_t)mb_slot, memo_key((uint32_t)ei, m[P.memo_pos]), S);
-                        const unsigned long long wv =
-                            P.grouped ? (unsigned long long)(X.n - __shfl_sync(kFull, st_hs, j)) : 1ull;
-                        cnt = mb_base + (lane == 0 ? S * wv : 0ull);
+                        if (lane == 0 && S) atomicAdd(a.memo_tab + 4 * (size_t)mb_slot + 1, S);
+                        cnt = mb_base;
                         mb = false;
                     }
                     if (j == jbase) break;
@@ -1714,26 +1749,26 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                     const uint4 gr = bn[P.bn_off[j] + __shfl_sync(kFull, st_gen, j)];
                     if (glen == gr.y + gr.w) {
                         if (memo_on && !mb && j == P.memo_from) {
-                            // the whole level below m[memo_pos]: its count from the table,
-                            // or counted here (unweighted) and published at the level's end
-                            uint32_t claim = kLsumNone;
-                            bool hit = false;
-                            unsigned long long hv = 0;
-                            if (lane == 0)
-                                claim = lsum_find(a.lsum_tab, a.lsum_mask, memo_key((uint32_t)ei, m[P.memo_pos]), hit, hv);
-                            if (__shfl_sync(kFull, hit ? 1u : 0u, 0)) {
-                                unsigned long long v = __shfl_sync(kFull, hv, 0);
-                                if (P.grouped) v *= gw(__shfl_sync(kFull, st_hs, j));
-                                if (lane == 0) { cnt += v; count_tails(1); }
+                            // the whole level below m[memo_pos]: this prefix's weight goes to the
+                            // memo; its subtree is expanded here if no other prefix did
+                            uint32_t slot = kLsumNone;
+                            bool fresh = false;
+                            unsigned long long wt = 1;
+                            if (P.grouped) wt = X.n - __shfl_sync(kFull, st_hs, j);
+                            if (lane == 0) {
+                                slot = memo_slot(a, memo_key((uint32_t)ei, m[P.memo_pos]), true, fresh);
+                                if (slot != kLsumNone) atomicAdd(a.memo_tab + 4 * (size_t)slot + 2, wt);
+                            }
+                            slot = __shfl_sync(kFull, slot, 0);
+                            if (slot != kLsumNone && !__shfl_sync(kFull, fresh ? 1u : 0u, 0)) {
+                                if (lane == 0) count_tails(1);
                                 if (lane == j) st_next = glen;
                                 __syncwarp();
                                 continue;
                             }
-                            claim = __shfl_sync(kFull, claim, 0);
-                            if (claim != kLsumNone) {
+                            if (slot != kLsumNone) {
                                 mb = true;
-                                mb_split = false;
-                                mb_slot = claim;
+                                mb_slot = slot;
                                 mb_base = cnt;
                             }
                         }
@@ -1779,9 +1814,6 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                         if (want) {
                             bool has = false;
                             if (lane >= jbase && lane < j) has = st_next < st_len || st_pos < st_ncand;
-                            // at a depth of `counted` a chunk's passing candidates were partly
-                            // counted already: only its unscanned range is shared
-                            if (lane >= jbase && lane < j && ((counted >> lane) & 1u)) has = st_next < st_len;
                             if (lane == j) has = glen > gnext + 32u;
                             const uint32_t hb = __ballot_sync(kFull, has);
                             uint32_t slot = 0xffffffffu;
@@ -1807,14 +1839,18 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                             slot = __shfl_sync(kFull, slot, 0);
                             if (slot != 0xffffffffu) {
                                 const uint32_t d = __ffs(hb) - 1;
-                                if (mb && d >= P.memo_from) mb_split = true;  // the memo's count is no longer all here
                                 uint32_t lo = 0, hi = 0;
                                 if (lane == d) {
                                     if (d == j) {
                                         lo = gnext + 32u;
                                         hi = glen;
+                                    } else if (((counted >> d) & 1u) && st_next >= st_len) {
+                                        // some of the chunk's candidates were counted at once, so the
+                                        // survivors are no stretch: the last one goes alone
+                                        lo = st_next - 32u + (s_cand[w][d][st_ncand - 1u] >> kCandBits);
+                                        hi = lo + 1u;
                                     } else if ((counted >> d) & 1u) {
-                                        lo = st_next;  // the buffered survivors stay with this warp
+                                        lo = st_next;  // the buffered survivors stay for now
                                         hi = st_len;
                                     } else {
                                         lo = st_pos < st_ncand ? st_next - 32u + (s_cand[w][d][st_pos] >> kCandBits)
@@ -1831,6 +1867,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                                 if (lane == 0) v = (uint32_t)ei | (d << 16) | (gd << 24);
                                 else if (lane == 1) v = lo;
                                 else if (lane == 2) v = hi;
+                                else if (lane == kTaskMemo) v = kSums && mb && d >= P.memo_from ? mb_slot : kLsumNone;
                                 else if (lane >= 4 && lane < 4 + kMaxQV) v = (lane - 4 < d) ? m[lane - 4] : 0u;
                                 if (lane < kTaskWords && lane != 3) tk[lane] = v;
                                 if (want == 2u) __threadfence_block(); else __threadfence();
@@ -1841,6 +1878,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                                 }
                                 if (lane == d) {
                                     if (d == j) st_len = gnext + 32u;
+                                    else if (((counted >> d) & 1u) && st_next >= st_len) --st_ncand;
                                     else if ((counted >> d) & 1u) st_len = st_next;
                                     else { st_len = st_next; st_ncand = st_pos; }
                                 }
@@ -1891,16 +1929,17 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                                 ok = ok && !desc;
                             }
                         } else if (kSums && peek_on && j == P.memo_pos && !mb) {
-                            // subtrees below this position already counted by some warp
-                            bool hit = false;
-                            unsigned long long hv = 0;
-                            if (ok) hit = lsum_peek(a.lsum_tab, a.lsum_mask, memo_key((uint32_t)ei, c), hv);
+                            // subtrees some warp expands already: only their weight is left to add
+                            uint32_t slot = kLsumNone;
+                            bool fresh = false;
+                            if (ok) slot = memo_slot(a, memo_key((uint32_t)ei, c), false, fresh);
+                            const bool hit = slot != kLsumNone;
                             unsigned long long wt = 1;
                             if (P.grouped) {
                                 wt = X.n - __shfl_sync(kFull, st_hs, j);
                                 if ((P.hit_mask >> j) & 1u) wt -= X.mult_lane(c, hit, lane);
                             }
-                            if (hit) cnt += hv * wt;
+                            if (hit) atomicAdd(a.memo_tab + 4 * (size_t)slot + 2, wt);
                             desc = ok && !hit;
                             ok = false;
                         } else {
@@ -2408,6 +2447,9 @@ struct cgb_handle {
     uint32_t pair_lane_max = kPairLaneMax;
     uint8_t* d_rev = nullptr;          // reverse direction of each direction
     uint32_t* d_touched = nullptr; size_t touched_cap = 0;  // footprint runs: record bit set
+    unsigned long long* d_memo = nullptr;  // subtree memos [memo_slots][4], sized with the record table
+    uint32_t* d_memo_list = nullptr;
+    uint32_t memo_slots = 0;
     unsigned long long* d_lsum = nullptr;  // level-sum table, sized with the record table
     uint32_t lsum_slots = 0;
     unsigned long long* d_wsum = nullptr; size_t wsum_cap = 0;  // dense level sums [n_wsum][dvcap]
@@ -2521,6 +2563,20 @@ cgb_status ensure_dvcap(cgb_handle* h, uint32_t dv) {
         CK(cudaMalloc(&h->d_lsum, (size_t)slots * 2 * sizeof(unsigned long long)));
         h->lsum_slots = slots;
     }
+    // subtree memos: up to 2^20 slots (32 B each), emptied by the launches that use them
+    slots = std::min(slots, 1u << 20);
+    if (slots > h->memo_slots) {
+        CK(cudaStreamSynchronize(h->stream));
+        if (h->d_memo) CK(cudaFree(h->d_memo));
+        if (h->d_memo_list) CK(cudaFree(h->d_memo_list));
+        h->d_memo = nullptr;
+        h->d_memo_list = nullptr;
+        h->memo_slots = 0;
+        CK(cudaMalloc(&h->d_memo, (size_t)slots * 4 * sizeof(unsigned long long)));
+        CK(cudaMalloc(&h->d_memo_list, (size_t)slots * sizeof(uint32_t)));
+        CK(cudaMemsetAsync(h->d_memo, 0, (size_t)slots * 4 * sizeof(unsigned long long), h->stream));
+        h->memo_slots = slots;
+    }
     return CGB_OK;
 }
 
@@ -2583,16 +2639,29 @@ cgb_status dense_level_sums(cgb_handle* h) {
     return CGB_OK;
 }
 
-// Level-sum table of a DFS launch (none when no plan uses level sums);
-// lsum_clear zeroes it on the stream before each launch.
-void lsum_bind(const cgb_handle* h, bool any, DfsArgs& da) {
-    const bool on = any && h->d_lsum;
+// Level-sum table of a DFS launch (none when no plan uses level sums), zeroed
+// by lsum_clear on the stream before each launch, and its subtree memos,
+// multiplied into the counts by memo_finish after it.
+void lsum_bind(const cgb_handle* h, bool any_sum, bool any_memo, DfsArgs& da) {
+    const bool on = any_sum && h->d_lsum;
     da.lsum_tab = on ? h->d_lsum : nullptr;
     da.lsum_mask = on ? h->lsum_slots - 1 : 0;
+    const bool memo = any_memo && h->d_memo;
+    da.memo_tab = memo ? h->d_memo : nullptr;
+    da.memo_mask = memo ? h->memo_slots - 1 : 0;
+    da.memo_list = h->d_memo_list;
 }
 cgb_status lsum_clear(cgb_handle* h, const DfsArgs& da) {
     if (da.lsum_tab)
         CK(cudaMemsetAsync(da.lsum_tab, 0, ((size_t)da.lsum_mask + 1) * 2 * sizeof(unsigned long long), h->stream));
+    return CGB_OK;
+}
+cgb_status memo_finish(cgb_handle* h, const DfsArgs& da) {
+    if (da.memo_tab) {
+        k_memo_finish<<<h->num_sms, 256, 0, h->stream>>>(da.memo_tab, da.memo_list, da.qctr + kQMemo, da.counts);
+        LAUNCHED();
+        CK(cudaGetLastError());
+    }
     return CGB_OK;
 }
 
@@ -2908,7 +2977,7 @@ void cgb_destroy(cgb_handle* h) {
                     h->d_edits_alt, h->d_runs[0], h->d_runs[1], h->d_runs[2],
                     h->d_dkeys, h->d_dkeys_alt, h->d_dval,
                     h->d_seed, h->d_tasks, h->d_temp, h->d_read_off, h->d_read, h->d_big_off, h->d_big_tile0, h->d_tiles,
-                    h->d_tile_state, h->d_qe_dirs, h->d_edge_ok,
+                    h->d_tile_state, h->d_memo, h->d_memo_list, h->d_qe_dirs, h->d_edge_ok,
                     h->d_vb, h->d_rb_slot, h->d_rb_sel, h->d_rb_bits, h->d_rb_new, h->d_rev, h->d_touched, h->d_plans,
                     h->d_vbplans, h->d_dir_edge, h->d_lsum, h->d_wsum, h->d_wjobs};
     for (void* p : ptrs)
@@ -3167,15 +3236,17 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
         }
         int bps = h->dfs_occupancy;
         if (h->cfg.dfs_blocks_per_sm) bps = std::min(bps, (int)h->cfg.dfs_blocks_per_sm);
-        bool any_sum = false;
-        for (uint32_t e = 0; e < h->q.qe; ++e)
-            any_sum |= (h->plans[e].sum_from != 0 && !h->plans[e].sum_dense) || h->plans[e].memo_from != 0;
+        bool any_sum = false, any_memo = false;
+        for (uint32_t e = 0; e < h->q.qe; ++e) {
+            any_sum |= h->plans[e].sum_from != 0 && !h->plans[e].sum_dense;
+            any_memo |= h->plans[e].memo_from != 0;
+        }
         da.wsum = nullptr;
         if (h->n_wsum && !da.vb && da.tail_cache) {
             if ((s = dense_level_sums(h)) != CGB_OK) return s;
             da.wsum = h->d_wsum;
         }
-        lsum_bind(h, any_sum, da);
+        lsum_bind(h, any_sum, any_memo, da);
         if ((s = lsum_clear(h, da)) != CGB_OK) return s;
         bool uses_sums = false;
         for (uint32_t e = 0; e < h->q.qe; ++e)
@@ -3187,6 +3258,7 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
         else k_dfs_count<false, false, false><<<grid, block, 0, h->stream>>>(da);
         LAUNCHED();
         CK(cudaGetLastError());
+        if ((s = memo_finish(h, da)) != CGB_OK) return s;
         CK(cudaEventRecord(h->ev[3], h->stream));
         if (footprint) {  // stats[4] := the launch's footprint (bytes of distinct records and lists)
             CK(cudaMemsetAsync(h->d_stats + 4, 0, sizeof(unsigned long long), h->stream));

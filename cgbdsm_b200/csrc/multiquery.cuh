@@ -408,7 +408,7 @@ DfsArgs mq_dfs_args(cgb_mq* m, const EdgePlan* plans, uint32_t G, uint64_t budge
     da.plans = plans;
     da.touched = nullptr;
     da.budget_ns = budget_ms * 1000000ull;
-    lsum_bind(h, true, da);
+    lsum_bind(h, true, true, da);
     da.wsum = nullptr;  // one-position (table) level sums only
     da.pair_lane_max = h->pair_lane_max;
     return da;
@@ -434,6 +434,7 @@ cgb_status mq_match_enqueue(cgb_mq* m, const EdgePlan* plans, const uint16_t* pa
     if (lsum_clear(h, da) != CGB_OK) return mq_fail(m, CGB_ERR_CUDA, "%s", h->err.c_str());
     k_dfs_count<true><<<h->num_sms * bps, kDfsWarps * 32, 0, h->stream>>>(da);
     LAUNCHED();
+    if (memo_finish(h, da) != CGB_OK) return mq_fail(m, CGB_ERR_CUDA, "%s", h->err.c_str());
     // fixed grid (grid-stride over the runs counted on the device): the step's
     // launch arguments do not depend on the batch size
     if (clear) {
@@ -475,7 +476,7 @@ cgb_status mq_match_all(cgb_mq* m, uint64_t n2) {
     put(&m->d_pair, sizeof(void*));
     if (m->gexec && kl == m->gkey_len && std::memcmp(key, m->gkey, kl) == 0) {
         MCK(cudaGraphLaunch(m->gexec, h->stream));
-        h->launches += 4;  // seed ranges, epoch, DFS, delta clear
+        h->launches += 5;  // seed ranges, epoch, DFS, memos, delta clear
         return CGB_OK;
     }
     if (m->gexec) {
@@ -574,6 +575,8 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
         Q.tuned_ms = best;
         m->plans_dirty = true;
     }
+    // a last trial that ran over its budget must not fail the batch
+    MCK(cudaMemsetAsync(h->d_scal + kCtlErr, 0, sizeof(unsigned long long), h->stream));
     MQ_TRY(mq_upload_plans(m));
     // the grid is timed again only once the plan count has doubled since
     // its last tuning (a registration alone does not pay for four launches

@@ -112,10 +112,9 @@ struct EdgePlan {
     // the range's core vertices share no label with prefix positions other
     // than memo_pos, no tail excludes such a position, and (grouped plans) no
     // position of the range is a hit position.  The count below depth
-    // memo_from is then a function of m[memo_pos] alone: the normal DFS
-    // counts it (unweighted, weighted once when complete) and, when none of
-    // it went to other warps, shares it through the level-sum table, once per
-    // (plan, vertex) and launch.  0: none.
+    // memo_from is then a function of m[memo_pos] alone: the DFS expands it
+    // once per (plan, vertex) and launch, unweighted, and every prefix adds
+    // its weight (the matcher's memo table).  0: none.
     uint8_t memo_from;
     uint8_t memo_pos;
     // Pair counting at the last core position j = n_core - 1: its two lists

@@ -1,0 +1,313 @@
+"""The matcher's and the index update's paths at the sizes where they can go
+wrong, against the C restatement (oracle/oracle.c) and plain set arithmetic.
+
+Exact equality throughout: counts, per-edge counts and keys are whole numbers.
+"""
+import json
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from cgbdsm_b200 import Engine, Gpma, MultiQuery
+from oracle import bind
+
+
+def _key(d, u, v):
+    return (np.uint64(d) << np.uint64(59)) | (np.uint64(u) << np.uint64(32)) | np.uint64(v)
+
+
+def _empty():
+    return np.zeros(0, np.uint64)
+
+
+# ---------------------------------------------------------------------------
+# index update: run lengths around the lane / warp / tile limits
+# ---------------------------------------------------------------------------
+# merged lengths at the edges of the three merges (32; 512) and of a tile
+# (2,816 entries), one and several tiles
+RUNS = [1, 31, 32, 33, 511, 512, 513, 2815, 2816, 2817, 5632, 5633, 9000]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("edits", [1, 2, 33, 700])
+def test_run_lengths_at_the_merge_limits(edits):
+    """One run per length in RUNS, updated by adds (new, present and repeated),
+    removes (present and absent) and keys both added and removed; the index
+    equals (index + ins) - del.  Twice, so that the second update also merges
+    runs the first one wrote."""
+    rng = np.random.default_rng(edits)
+    dv = 20000
+    old = {u: rng.choice(dv, n, replace=False) for u, n in enumerate(RUNS)}
+    init = np.array([_key(0, u, v) for u, vs in old.items() for v in vs], dtype=np.uint64)
+    eng = Engine()
+    eng.load_query(2, [(0, 1)], [0, 1])
+    eng.build_index(init, dv)
+    state = np.unique(init)
+    for _ in range(2):
+        ins, dele = [], []
+        for u, vs in old.items():
+            for v in rng.integers(0, dv, edits):
+                ins.append(_key(0, u, v))
+            for v in rng.choice(vs, min(len(vs), edits // 2 + 1)):
+                dele.append(_key(0, u, v))
+                ins.append(_key(0, u, v))  # removed although also added
+            ins.append(ins[-1])
+            dele.append(_key(0, u, int(rng.integers(0, dv))))
+        ins, dele = np.array(ins, np.uint64), np.array(dele, np.uint64)
+        rng.shuffle(ins)
+        rng.shuffle(dele)
+        eng.apply_batch(dv, ins, dele, _empty())
+        state = np.setdiff1d(np.union1d(state, ins), dele)
+        assert np.array_equal(np.sort(eng.read_index()), state)
+    eng.close()
+
+
+@pytest.mark.gpu
+def test_delta_merge_back_and_growing_ids():
+    """The sorted delta kept for the merge-back is packed again when the vertex
+    ids outgrow its bits (20 -> 5,000 vertices between batches)."""
+    eng = Engine()
+    eng.load_query(2, [(0, 1)], [0, 1])
+    eng.build_index(np.array([_key(0, 1, 2), _key(1, 2, 1)], np.uint64), 20)
+    delta = np.array([_key(0, 3, 4), _key(1, 4, 3), _key(0, 3, 4), _key(1, 4, 3)], np.uint64)  # repeated entries
+    eng.apply_batch(20, _empty(), _empty(), delta)
+    ins = np.array([_key(0, 4999, 17), _key(1, 17, 4999)], np.uint64)
+    eng.apply_batch(5000, ins, _empty(), _empty())
+    want = np.unique(np.concatenate([np.array([_key(0, 1, 2), _key(1, 2, 1)], np.uint64), delta, ins]))
+    assert np.array_equal(np.sort(eng.read_index()), want)
+    eng.close()
+
+
+# ---------------------------------------------------------------------------
+# per-candidate tails: several lists, shared labels, lists around 32 entries
+# ---------------------------------------------------------------------------
+PATTERNS = {
+    # square with a pendant: the counted vertex has two lists, one off the last core vertex
+    "square": ([0, 1, 0, 1, 2], [(0, 1), (1, 2), (2, 3), (3, 0), (0, 4)]),
+    # two counted vertices of one label on the same core vertices (inclusion-exclusion)
+    "twins": ([0, 1, 2, 2, 1], [(0, 1), (0, 2), (1, 2), (0, 3), (1, 3), (0, 4)]),
+    # three counted vertices of one label
+    "triplet": ([0, 0, 1, 1, 1], [(0, 1), (0, 2), (1, 2), (0, 3), (1, 3), (1, 4)]),
+    # diamond with tails whose label is the last core vertex's
+    "diamond": ([0, 1, 1, 0, 1], [(0, 1), (0, 2), (1, 2), (1, 3), (2, 3), (3, 4)]),
+    # a path whose labels repeat (level sums with prefix vertices subtracted)
+    "path": ([0, 1, 0, 1, 0], [(0, 1), (1, 2), (2, 3), (3, 4)]),
+    # a hub subtree shared by its prefixes (memo), below a pendant seed edge
+    "shared": ([0, 1, 2, 3, 3, 4], [(0, 1), (1, 2), (2, 3), (2, 4), (3, 5)]),
+}
+
+
+def _graph(rng, n, nlabels, hub_degree):
+    """Random labelled graph; vertex 0 of every label is a hub of hub_degree."""
+    lab = rng.integers(0, nlabels, n)
+    lab[:nlabels] = np.arange(nlabels)
+    pairs = {(int(min(a, b)), int(max(a, b))) for a, b in rng.integers(0, n, (4 * n, 2)) if a != b}
+    for h in range(nlabels):
+        for x in rng.choice(np.arange(nlabels, n), min(hub_degree, n - nlabels), replace=False):
+            pairs.add((h, int(x)))
+    return lab, np.array(sorted(pairs), dtype=np.int64)
+
+
+def _keys_of(orc, qe, ql, lab, pairs):
+    ks = []
+    for a, b in qe:
+        d0, d1 = orc.L.orc_dir(orc.h, a, b), orc.L.orc_dir(orc.h, b, a)
+        for x, y in pairs:
+            if lab[x] == ql[a] and lab[y] == ql[b]:
+                ks += [_key(d0, x, y), _key(d1, y, x)]
+            if lab[y] == ql[a] and lab[x] == ql[b]:
+                ks += [_key(d0, y, x), _key(d1, x, y)]
+    return np.array(ks, dtype=np.uint64)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hub_degree", [0, 31, 33, 120])
+@pytest.mark.parametrize("name", sorted(PATTERNS))
+def test_tails_per_candidate_match_restatement(name, hub_degree):
+    """Counts of two batches equal the restatement's (per query edge), in the
+    single-query engine and, in total, in the multi-query engine; then the
+    second batch's edges are deleted again (as many negative matches)."""
+    ql, qe = PATTERNS[name]
+    rng = np.random.default_rng(7 + hub_degree)
+    n, nlabels = 160, max(ql) + 1
+    lab, pairs = _graph(rng, n, nlabels, hub_degree)
+    rng.shuffle(pairs)
+    k = len(pairs) // 6
+    parts = [pairs[2 * k:], pairs[:k], pairs[k:2 * k]]
+    orc = bind.Oracle(len(ql), qe)
+    eng = Engine()
+    eng.load_query(len(ql), qe, ql)
+    init = _keys_of(orc, qe, ql, lab, parts[0])
+    orc.build(init, n)
+    eng.build_index(init, n)
+    m = MultiQuery(dfs_budget_ms=60000)
+    m.load_graph(lab.astype(np.uint32), parts[0].astype(np.uint32))
+    qid = m.register(len(ql), qe, ql)
+    for p in parts[1:]:
+        delta = _keys_of(orc, qe, ql, lab, p)
+        want = orc.batch(n, _empty(), _empty(), delta, None, bind.PER_EDGE)
+        assert eng.apply_batch(n, _empty(), _empty(), delta) == want
+        assert np.array_equal(eng.edge_counts(), orc.edge_counts())
+        pos, _ = m.apply_batch(ins=p.astype(np.uint32))
+        assert int(pos[qid]) == want
+    _, neg = m.apply_batch(dele=parts[2].astype(np.uint32))
+    assert int(neg[qid]) == want
+    eng.close()
+    m.close()
+
+
+# ---------------------------------------------------------------------------
+# packed-memory array: windows of one and of many leaves
+# ---------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,burst", [(0, 1), (31, 40), (1000, 33), (5000, 2000)])
+def test_gpma_windows_and_counts(n, burst):
+    """Inserts crowded into one stretch of keys (windows of many leaves) and
+    spread ones (single leaves), deletes, and both at once; contents and
+    counts per direction equal the set model's after every update."""
+    rng = np.random.default_rng(n + burst)
+    g = Gpma(3)
+    state = np.unique(np.array([_key(int(d), int(u), int(v)) for d, u, v in
+                                zip(rng.integers(0, 3, n), rng.integers(0, 500, n), rng.integers(0, 500, n))], np.uint64)) \
+        if n else _empty()
+    g.bulk_load(state)
+    for step in range(4):
+        crowd = np.array([_key(1, 250, 1000 + step * burst + i) for i in range(burst)], np.uint64)
+        spread = np.array([_key(int(d), int(u), int(v)) for d, u, v in
+                           zip(rng.integers(0, 3, burst), rng.integers(0, 500, burst), rng.integers(0, 500, burst))], np.uint64)
+        dele = rng.choice(state, len(state) // 4, replace=False) if len(state) else _empty()
+        ins = np.concatenate([crowd, spread, dele[:5]])
+        g.batch_update(ins, dele)
+        state = np.setdiff1d(np.union1d(state, ins), dele)
+        for d in range(3):
+            mine = state[(state >> np.uint64(59)) == d] & np.uint64((1 << 59) - 1)
+            assert np.array_equal(g.extract(d), mine), (step, d)
+        assert g.stats()["keys"] == len(state)
+    g.close()
+
+
+# ---------------------------------------------------------------------------
+# flat merge: tile edges (2,816 entries) and more than 32 tiles back to a prefix
+# ---------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_old,n_ins,n_del", [(2815, 1, 0), (2815, 1, 1), (2816, 0, 1), (5631, 3, 2), (0, 2817, 0),
+                                               (200_000, 5000, 5000)])
+def test_flat_merge_tile_edges(n_old, n_ins, n_del):
+    import torch
+
+    from cgbdsm_b200 import load_library
+
+    rng = np.random.default_rng(n_old)
+    dv = 3000
+    pool = np.unique(_key(0, 0, 0) + (rng.integers(0, 4, 2 * (n_old + n_ins) + 64).astype(np.uint64) << np.uint64(59))
+                     + (rng.integers(0, dv, 2 * (n_old + n_ins) + 64).astype(np.uint64) << np.uint64(32))
+                     + rng.integers(0, dv, 2 * (n_old + n_ins) + 64).astype(np.uint64))
+    pick = rng.permutation(len(pool))
+    old = np.sort(pool[pick[:n_old]])
+    ins = pool[pick[n_old:n_old + n_ins]]
+    dele = np.concatenate([rng.choice(old, n_del, replace=False) if n_old else _empty(), ins[:n_ins // 4]])[:max(n_del, 0)]
+    want = np.setdiff1d(np.union1d(old, ins), dele)
+
+    def dev(a):
+        return torch.from_numpy((a if len(a) else np.zeros(1, np.uint64)).view(np.int64)).cuda()
+
+    t_old, t_ins, t_del = dev(old), dev(ins), dev(dele)
+    out = torch.zeros(len(old) + len(ins) + 1, dtype=torch.int64, device="cuda")
+    out_n = torch.zeros(1, dtype=torch.int64, device="cuda")
+    st = load_library().cgb_merge_keys_noalloc(t_old.data_ptr(), len(old), t_ins.data_ptr(), len(ins), t_del.data_ptr(),
+                                               len(dele), dv, out.data_ptr(), out_n.data_ptr(), None)
+    torch.cuda.synchronize()
+    assert st == 0
+    got = out[:int(out_n.item())].cpu().numpy().view(np.uint64)
+    assert np.array_equal(got, want)
+
+
+# ---------------------------------------------------------------------------
+# planned subsets (no GPU)
+# ---------------------------------------------------------------------------
+SUBSETS_CPP = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <vector>
+#include "query.h"
+int main(int argc, char** argv) {  // qv qe fold labels... edges...
+    uint32_t qv = atoi(argv[1]), qe = atoi(argv[2]), fold = atoi(argv[3]);
+    std::vector<uint32_t> lab, edges;
+    for (uint32_t i = 0; i < qv; ++i) lab.push_back(atoi(argv[4 + i]));
+    for (uint32_t i = 0; i < 2 * qe; ++i) edges.push_back(atoi(argv[4 + qv + i]));
+    cgb::QueryMeta q;
+    if (!cgb::build_query_meta(qv, qe, edges.data(), lab.data(), q, cgb::kMaxQE).empty()) return 1;
+    float avg[cgb::kMaxDir];
+    for (float& x : avg) x = 1.f;
+    std::vector<cgb::EdgePlan> plans(cgb::kMaxQE);
+    cgb::plan_edges(q, avg, plans.data(), true, true, true, true, true, false, fold);
+    for (uint32_t e = 0; e < qe; ++e) {
+        const cgb::EdgePlan& p = plans[e];
+        std::printf("%u %u %u %u", p.n, p.n_core, p.n_sub, p.sub_base);
+        for (uint32_t j = 0; j <= p.n; ++j) std::printf(" %u", p.bn_off[j]);
+        for (uint32_t b = 0; b < p.bn_off[p.n]; ++b) std::printf(" %u", p.bn_pos[b]);
+        for (uint32_t j = 0; j < p.n; ++j) std::printf(" %u", p.tail_gid[j]);
+        for (uint32_t i = 0; i < p.n_sub; ++i) std::printf(" %u %u %u %u", p.sub_lists[i], p.sub_pos[i], p.sub_group[i], p.sub_kind[i]);
+        std::printf("\n");
+    }
+}
+"""
+
+
+def test_planned_subsets_cover_every_tail_group(tmp_path):
+    """Every tail label group of k members has its 2^k - 1 member subsets in an
+    order whose single members come first, each with the union of its members'
+    lists and owners; every tail vertex is in exactly one group."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    csrc = os.path.join(root, "cgbdsm_b200", "csrc")
+    src, exe = tmp_path / "subsets.cpp", tmp_path / "subsets"
+    src.write_text(SUBSETS_CPP)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", csrc, "-I", os.path.join(root, "include"), str(src),
+                    os.path.join(csrc, "query.cpp"), "-o", str(exe)], check=True)
+    cases = list(PATTERNS.values())
+    for s in ("c2", "c3"):
+        with open(os.path.join(root, "cgbdsm_b200", "data", f"queries_{s}.json")) as f:
+            cases += [(q["labels"], [tuple(e) for e in q["edges"]]) for q in json.load(f)["queries"]]
+    folded = 0
+    for labels, edges in cases:
+        for fold in (0, 3, 12):
+            args = [str(x) for x in (len(labels), len(edges), fold, *labels, *[v for e in edges for v in e])]
+            out = subprocess.run([str(exe), *args], check=True, capture_output=True, text=True).stdout
+            for line in out.splitlines():
+                f = [int(x) for x in line.split()]
+                n, nc, ns, base = f[:4]
+                off, f = f[4:5 + n], f[5 + n:]
+                pos, f = f[:off[n]], f[off[n]:]
+                gid, f = f[:n], f[n:]
+                subs = [f[4 * i:4 * i + 4] for i in range(ns)]
+                groups, t = [], nc
+                while t < n:
+                    e = t
+                    while e < n and gid[e] == gid[t]:
+                        e += 1
+                    groups.append(list(range(t, e)))
+                    t = e
+                i = 0
+                for g in groups:
+                    k = len(g)
+                    assert 1 <= k <= 3
+                    seen = []
+                    for lists, owners, group, kind in subs[i:i + 2 ** k - 1]:
+                        mask = kind & 7
+                        want = 0
+                        for mem in range(k):
+                            if mask >> mem & 1:
+                                for b in range(off[g[mem]], off[g[mem] + 1]):
+                                    want |= 1 << (b - base)
+                        assert lists == want and owners == sum(1 << x for x in {pos[base + b] for b in range(32) if want >> b & 1})
+                        assert owners & ~group == 0 and bool(kind & 0x10) == (k == 3)
+                        assert bool(kind & 8) == (len(seen) == 2 ** k - 2)
+                        if nc - 1 in [pos[base + b] for b in range(32) if want >> b & 1] and bin(want).count("1") > 1:
+                            folded += 1
+                        seen.append(mask)
+                    assert sorted(seen) == list(range(1, 2 ** k)) and sorted(seen[:k]) == [1 << x for x in range(k)]
+                    i += 2 ** k - 1
+                assert ns - i <= 1  # then the pair or the level sum
+    assert folded > 0
