@@ -35,7 +35,8 @@ def build(ref: bool = True, ref_tree: Optional[str] = None) -> None:
     given (ref_tree, else $CGB_REFERENCE_TREE) and present on this machine."""
     subprocess.run(["make", "-s", "-C", HERE, "oracle"], check=True)
     tree = ref_tree or REF_TREE
-    if ref and tree and os.path.isdir(tree):
+    # An empty or partial tree counts as absent: the prebuilt library stands.
+    if ref and tree and os.path.isfile(os.path.join(tree, "index", "calig.cpp")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={tree}"], check=True)
 
 
