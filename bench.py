@@ -352,8 +352,8 @@ def run_pipelines(names: list[str], args, rank: int, world: int, local: int, foo
                            "l2_throughput_pct_ncu": l2pct, "index_update_achieved_gbs": upd_gbs,
                            "index_update_frac": upd_gbs / peak if peak else None}
     else:
-        traffic, l2pct, src = _profiled("k_merge_runs", names[0])
-        out["roofline"] = {"kernel": "k_merge_runs / k_merge_big (index update)", "bound": "hbm",
+        traffic, l2pct, src = _profiled("k_merge", names[0])
+        out["roofline"] = {"kernel": "k_merge (index update)", "bound": "hbm",
                            "achieved": upd_gbs, "peak": peak, "unit": "GB/s",
                            "frac": upd_gbs / peak if peak else None, "peak_source": peak_kind,
                            "algorithmic_bytes": "8 B per edit + 4 B per old and new run word + 32 B per record",

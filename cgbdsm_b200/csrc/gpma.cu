@@ -12,7 +12,7 @@
 // slot is valid and holds x.
 //
 // Batch update, set semantics (index + ins) - del (the same as the engine's
-// k_merge_runs; the reference's GPMA is bulk-loaded once and never updated
+// k_merge; the reference's GPMA is bulk-loaded once and never updated
 // or read by its matcher, calig_helper_gpma.cu:284-296, 383-414, so its
 // update semantics are not a parity target):
 //   1. sort the edits (key, op), one effect per distinct key: a present key
