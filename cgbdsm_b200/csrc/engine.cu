@@ -2111,8 +2111,14 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                 if (lane == 0) count_tails(non);
             }
             if (nc == 2) break;
-            // a level whose prefix-only tail count is 0 adds nothing however it goes on
-            if (lane == j) st_next = node || (dead && !serial) ? glen : gnext + 32u;
+            // a level whose prefix-only tail count is 0 adds nothing however it goes
+            // on; neither do survivors buffered from this chunk (pair counting), and
+            // with st_next past the chunk their places could not be found again
+            if (lane == j) {
+                const bool done = node || (dead && !serial);
+                st_next = done ? glen : gnext + 32u;
+                if (kSums && done) st_ncand = st_pos;
+            }
             __syncwarp();
         }
         if (out_of_time) {

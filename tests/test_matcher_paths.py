@@ -158,6 +158,97 @@ def test_tails_per_candidate_match_restatement(name, hub_degree):
     m.close()
 
 
+# Triangle (1, 3, 4) whose vertex 1 also carries a counted pendant (2) and the
+# way to the seed: with no vertex of several lists kept in the tail, the last
+# level is one intersection per candidate (pair counting).
+PAIRED = ([0, 1, 2, 3, 4, 0], [(0, 1), (1, 2), (1, 3), (1, 4), (3, 4), (0, 5)])
+
+PAIR_CPP = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <vector>
+#include "query.h"
+int main(int argc, char** argv) {  // qv qe labels... edges...: plans with pair counting, per set of list lengths
+    uint32_t qv = atoi(argv[1]), qe = atoi(argv[2]);
+    std::vector<uint32_t> lab, edges;
+    for (uint32_t i = 0; i < qv; ++i) lab.push_back(atoi(argv[3 + i]));
+    for (uint32_t i = 0; i < 2 * qe; ++i) edges.push_back(atoi(argv[3 + qv + i]));
+    cgb::QueryMeta q;
+    if (!cgb::build_query_meta(qv, qe, edges.data(), lab.data(), q, cgb::kMaxQE).empty()) return 1;
+    for (int t = 0; t < 50; ++t) {
+        float avg[cgb::kMaxDir];
+        for (float& x : avg) x = 1.f + rand() % 100;
+        std::vector<cgb::EdgePlan> plans(cgb::kMaxQE);
+        cgb::plan_edges(q, avg, plans.data(), true, true, true, true, true, false, 0);
+        int n = 0;
+        for (uint32_t e = 0; e < qe; ++e) n += plans[e].pair_last;
+        std::printf("%d\n", n);
+    }
+}
+"""
+
+
+def _native(tmp_path, name, text, args):
+    """Output lines of a C++ program built with the planner."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    csrc = os.path.join(root, "cgbdsm_b200", "csrc")
+    src, exe = tmp_path / f"{name}.cpp", tmp_path / name
+    src.write_text(text)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", csrc, "-I", os.path.join(root, "include"), str(src),
+                    os.path.join(csrc, "query.cpp"), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe), *[str(x) for x in args]], check=True, capture_output=True,
+                          text=True).stdout.splitlines()
+
+
+def test_paired_pattern_plans_pair_counting(tmp_path):
+    """PAIRED reaches pair counting whatever the mean list lengths are, in the
+    plans that keep vertices with several lists out of the tail (a variant
+    the multi-query engine's autotuner always tries)."""
+    ql, qe = PAIRED
+    counts = _native(tmp_path, "pairs", PAIR_CPP, [len(ql), len(qe), *ql, *[v for e in qe for v in e]])
+    assert len(counts) == 50 and all(int(x) > 0 for x in counts)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lane_max", [0, 2])
+@pytest.mark.parametrize("pendants", [0, 3, 400])
+def test_pair_counting_beside_descent_and_empty_tails(lane_max, pendants, monkeypatch):
+    """With $CGB_PAIR_LANE_MAX a chunk holds candidates counted at once and
+    candidates left to the descent, in lists shorter than a chunk; a prefix
+    whose vertex has no pendant neighbour (all but `pendants` of them) has no
+    tail, and its chunks are left at once.  Every plan variant's count equals
+    the restatement's (the autotuner refuses variants that differ)."""
+    monkeypatch.setenv("CGB_PAIR_LANE_MAX", str(lane_max))
+    ql, qe = PAIRED
+    rng = np.random.default_rng(pendants)
+    n = 1500
+    lab = np.repeat(np.arange(5), n // 5)
+    rng.shuffle(lab)
+    by = [np.flatnonzero(lab == k) for k in range(5)]
+    pairs = set()
+    for x, y, m in [(0, 0, 900), (0, 1, 1500), (1, 3, 4000), (1, 4, 4000), (3, 4, 4000)]:
+        pairs |= {(int(a), int(b)) for a, b in zip(rng.choice(by[x], m), rng.choice(by[y], m)) if a != b}
+    for a in rng.choice(by[1], min(pendants, len(by[1])), replace=False):
+        pairs.add((int(a), int(rng.choice(by[2]))))
+    pairs = np.array(sorted({(min(p), max(p)) for p in pairs}), dtype=np.int64)
+    rng.shuffle(pairs)
+    k = len(pairs) // 5
+    parts = [pairs[2 * k:], pairs[:k], pairs[k:2 * k]]
+    orc = bind.Oracle(len(ql), qe)
+    orc.build(_keys_of(orc, qe, ql, lab, parts[0]), n)
+    m = MultiQuery(dfs_budget_ms=60000)
+    m.load_graph(lab.astype(np.uint32), parts[0].astype(np.uint32))
+    qid = m.register(len(ql), qe, ql)
+    total = 0
+    for p in parts[1:]:
+        want = orc.batch(n, _empty(), _empty(), _keys_of(orc, qe, ql, lab, p), None, bind.PER_EDGE)
+        pos, _ = m.apply_batch(ins=p.astype(np.uint32))
+        assert int(pos[qid]) == want
+        total += want
+    assert (total > 0) == (pendants > 0)
+    m.close()
+
+
 # ---------------------------------------------------------------------------
 # packed-memory array: windows of one and of many leaves
 # ---------------------------------------------------------------------------
