@@ -2254,6 +2254,7 @@ __global__ void k_vb_seed(const cgb::VbPlan* __restrict__ vbp, const uint8_t* __
     const uint64_t m = (1ull << B) - 1ull;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t k = dkeys[i];
+        if (k == ~0ull) continue;  // a key out of range: the batch is rejected after this step
         const uint32_t d = (uint32_t)(k >> (2 * B)), u = (uint32_t)((k >> B) & m);
         const uint32_t ei = dir_edge[d];
         const cgb::VbPlan& P = vbp[ei];

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 from cgbdsm_b200 import Engine, Gpma, MultiQuery
+from cgbdsm_b200.engine import FLAG_MASK_PRUNE, FLAG_VALID_BITS, CgbError
 from oracle import bind
 
 
@@ -77,6 +78,25 @@ def test_delta_merge_back_and_growing_ids():
     eng.apply_batch(5000, ins, _empty(), _empty())
     want = np.unique(np.concatenate([np.array([_key(0, 1, 2), _key(1, 2, 1)], np.uint64), delta, ins]))
     assert np.array_equal(np.sort(eng.read_index()), want)
+    eng.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flags", [0, FLAG_VALID_BITS, FLAG_MASK_PRUNE])
+@pytest.mark.parametrize("bad", [(3, 5, 6), (31, 5, 6), (0, 64, 6), (1, 5, 64), (31, (1 << 27) - 1, (1 << 27) - 1)])
+def test_out_of_range_delta_key_is_rejected(flags, bad):
+    """A delta key whose direction or vertex is out of range rejects the batch
+    (also where valid bits are computed, whose pass over the delta meets the
+    key's marker); the engine then matches the next batch as ever."""
+    eng = Engine(flags=flags)
+    eng.load_query(2, [(0, 1)], [0, 1])
+    eng.build_index(np.array([_key(0, 1, 2), _key(1, 2, 1)], np.uint64), 64)
+    good = [_key(0, 3, 4), _key(1, 4, 3), _key(0, 63, 62), _key(1, 62, 63)]
+    with pytest.raises(CgbError, match="out of range"):
+        eng.apply_batch(64, _empty(), _empty(), np.array([*good, _key(*bad)], np.uint64))
+    assert eng.apply_batch(64, _empty(), _empty(), np.array(good, np.uint64)) == 2
+    eng.apply_batch(64, _empty(), _empty(), _empty())
+    assert np.array_equal(np.sort(eng.read_index()), np.unique(np.array([_key(0, 1, 2), _key(1, 2, 1), *good], np.uint64)))
     eng.close()
 
 
