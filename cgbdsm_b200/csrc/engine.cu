@@ -1142,10 +1142,10 @@ __device__ __forceinline__ unsigned long long flat_lists(const EdgePlan& P, uint
 // outlive the index state they were computed on.  A lookup probes
 // kLsumProbes slots; a warp that finds its key busy or every probe taken by
 // other keys computes the value itself (nobody waits).
-// A slot is read and published by one 16-byte access (single-copy atomic), so
-// key and value need no order between them: relaxed, because an acquire at
-// device scope drops the SM's whole L1, which the searches of the other 31
-// resident warps live in.
+// A slot is claimed, read and published by 16-byte accesses alone (one memory
+// operation each, so that key and value need no order between them).  Relaxed:
+// an acquire at device scope drops the SM's whole L1, which the searches of
+// the other 31 resident warps live in.
 constexpr uint32_t kLsumProbes = 4;
 constexpr uint32_t kLsumNone = 0xffffffffu;
 
@@ -1158,6 +1158,14 @@ __device__ __forceinline__ void lsum_publish(unsigned long long* slot, unsigned 
     asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
                  ::"l"(slot), "l"((K << 1) | 1ull), "l"(v) : "memory");
 }
+// Claims an empty slot for K; otherwise false, and what the slot holds.
+__device__ __forceinline__ bool lsum_claim(unsigned long long* slot, unsigned long long K, unsigned long long& k,
+                                           unsigned long long& v) {
+    asm volatile("{\n\t.reg .b128 t, e, n;\n\tmov.b128 e, {%4, %4};\n\tmov.b128 n, {%3, %4};\n\t"
+                 "atom.relaxed.gpu.global.cas.b128 t, [%2], e, n;\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(k), "=l"(v) : "l"(slot), "l"(K << 1), "l"(0ull) : "memory");
+    return k == 0;
+}
 
 // One thread: the published value of K (hit = true), or the slot this
 // thread claimed for K (to publish into), or kLsumNone.
@@ -1168,10 +1176,7 @@ __device__ __forceinline__ uint32_t lsum_find(unsigned long long* tab, uint32_t 
         unsigned long long* slot = tab + 2 * (size_t)s;
         unsigned long long k, v;
         lsum_load(slot, k, v);
-        if (k == 0) {
-            if (atomicCAS(slot, 0ull, K << 1) == 0) return s;
-            lsum_load(slot, k, v);  // claimed or published meanwhile
-        }
+        if (k == 0 && lsum_claim(slot, K, k, v)) return s;
         if ((k >> 1) == K) {
             if (k & 1ull) {
                 hit = true;

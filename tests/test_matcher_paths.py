@@ -269,6 +269,51 @@ def test_pair_counting_beside_descent_and_empty_tails(lane_max, pendants, monkey
     m.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("hubs", [1, 3, 40])
+def test_level_sum_table_under_contention(hubs):
+    """Thousands of prefixes ask the level-sum table for the same few owners at
+    once: one of them claims the slot, the others find it busy or published.
+    Path 4-0-1-2-3 whose (0, 1) edges all end in `hubs` vertices; counts equal
+    the restatement's, in both engines."""
+    ql, qe = [0, 1, 2, 3, 4], [(0, 1), (1, 2), (2, 3), (0, 4)]
+    rng = np.random.default_rng(hubs)
+    n0 = 3000
+    v0 = np.arange(n0)
+    v1 = n0 + np.arange(hubs)
+    v2 = v1[-1] + 1 + np.arange(200)
+    v3 = v2[-1] + 1 + np.arange(60)
+    v4 = v3[-1] + 1 + np.arange(50)
+    n = int(v4[-1]) + 1
+    lab = np.zeros(n, np.int64)
+    for k, v in enumerate((v0, v1, v2, v3, v4)):
+        lab[v] = k
+    seeds = np.stack([v0, rng.choice(v1, n0)], 1)
+    rest = {(int(a), int(b)) for a, b in zip(rng.choice(v1, 40 * hubs), rng.choice(v2, 40 * hubs))}
+    rest |= {(int(a), int(b)) for a, b in zip(rng.choice(v2, 500), rng.choice(v3, 500))}
+    rest |= {(int(a), int(b)) for a, b in zip(rng.choice(v0, 4000), rng.choice(v4, 4000))}
+    rest = np.array(sorted(rest), dtype=np.int64)
+    orc = bind.Oracle(len(ql), qe)
+    init = _keys_of(orc, qe, ql, lab, rest)
+    delta = _keys_of(orc, qe, ql, lab, seeds)
+    orc.build(init, n)
+    want = orc.batch(n, _empty(), _empty(), delta, None, bind.PER_EDGE)
+    assert want > 0
+    eng = Engine()
+    eng.load_query(len(ql), qe, ql)
+    eng.build_index(init, n)
+    assert eng.apply_batch(n, _empty(), _empty(), delta) == want
+    eng.close()
+    m = MultiQuery(dfs_budget_ms=60000)
+    m.load_graph(lab.astype(np.uint32), rest.astype(np.uint32))
+    qid = m.register(len(ql), qe, ql)
+    pos, _ = m.apply_batch(ins=seeds.astype(np.uint32))
+    assert int(pos[qid]) == want
+    _, neg = m.apply_batch(dele=seeds.astype(np.uint32))
+    assert int(neg[qid]) == want
+    m.close()
+
+
 # ---------------------------------------------------------------------------
 # packed-memory array: windows of one and of many leaves
 # ---------------------------------------------------------------------------
