@@ -2547,8 +2547,38 @@ inline int grid_for(const cgb_handle* h, uint64_t n, int block = 256) {
     return (int)g;
 }
 
+// Level-sum table: about two slots per vertex, 2^12 to 2^24 slots (16 B each);
+// subtree memos: up to 2^20 slots (32 B each), emptied by the launches that
+// use them.  A table counts as there by its number of slots, which is set last:
+// after a failed allocation the next call tries again.
+cgb_status ensure_tables(cgb_handle* h) {
+    uint32_t slots = 1u << 12;
+    while (slots < (1u << 24) && slots < 2ull * h->dvcap) slots <<= 1;
+    if (slots > h->lsum_slots) {
+        h->lsum_slots = 0;
+        if (h->d_lsum) CK(cudaFree(h->d_lsum));
+        h->d_lsum = nullptr;
+        CK(cudaMalloc(&h->d_lsum, (size_t)slots * 2 * sizeof(unsigned long long)));
+        h->lsum_slots = slots;
+    }
+    slots = std::min(slots, 1u << 20);
+    if (slots > h->memo_slots) {
+        CK(cudaStreamSynchronize(h->stream));
+        h->memo_slots = 0;
+        if (h->d_memo) CK(cudaFree(h->d_memo));
+        h->d_memo = nullptr;
+        if (h->d_memo_list) CK(cudaFree(h->d_memo_list));
+        h->d_memo_list = nullptr;
+        CK(cudaMalloc(&h->d_memo, (size_t)slots * 4 * sizeof(unsigned long long)));
+        CK(cudaMalloc(&h->d_memo_list, (size_t)slots * sizeof(uint32_t)));
+        CK(cudaMemsetAsync(h->d_memo, 0, (size_t)slots * 4 * sizeof(unsigned long long), h->stream));
+        h->memo_slots = slots;
+    }
+    return CGB_OK;
+}
+
 cgb_status ensure_dvcap(cgb_handle* h, uint32_t dv) {
-    if (dv <= h->dvcap && h->rec) return CGB_OK;
+    if (dv <= h->dvcap && h->rec) return ensure_tables(h);
     uint32_t nc = std::max<uint32_t>(dv + dv / 4 + 1024, h->dvcap * 2);
     uint4* nr = nullptr;
     CK(cudaMalloc(&nr, (size_t)h->nd * nc * sizeof(uint4)));
@@ -2565,31 +2595,7 @@ cgb_status ensure_dvcap(cgb_handle* h, uint32_t dv) {
     h->dvcap = nc;
     h->rb_valid = false;  // the slot table and the bit sets follow the record layout
     h->rb_len_now = h->rb_min_len;
-    // level-sum table: about two slots per vertex, 2^12 to 2^24 slots (16 B each)
-    uint32_t slots = 1u << 12;
-    while (slots < (1u << 24) && slots < 2ull * nc) slots <<= 1;
-    if (slots > h->lsum_slots) {
-        if (h->d_lsum) CK(cudaFree(h->d_lsum));
-        h->d_lsum = nullptr;
-        h->lsum_slots = 0;
-        CK(cudaMalloc(&h->d_lsum, (size_t)slots * 2 * sizeof(unsigned long long)));
-        h->lsum_slots = slots;
-    }
-    // subtree memos: up to 2^20 slots (32 B each), emptied by the launches that use them
-    slots = std::min(slots, 1u << 20);
-    if (slots > h->memo_slots) {
-        CK(cudaStreamSynchronize(h->stream));
-        if (h->d_memo) CK(cudaFree(h->d_memo));
-        if (h->d_memo_list) CK(cudaFree(h->d_memo_list));
-        h->d_memo = nullptr;
-        h->d_memo_list = nullptr;
-        h->memo_slots = 0;
-        CK(cudaMalloc(&h->d_memo, (size_t)slots * 4 * sizeof(unsigned long long)));
-        CK(cudaMalloc(&h->d_memo_list, (size_t)slots * sizeof(uint32_t)));
-        CK(cudaMemsetAsync(h->d_memo, 0, (size_t)slots * 4 * sizeof(unsigned long long), h->stream));
-        h->memo_slots = slots;
-    }
-    return CGB_OK;
+    return ensure_tables(h);
 }
 
 // Dense level sums of every plan with sum_dense, children before parents
@@ -2655,10 +2661,10 @@ cgb_status dense_level_sums(cgb_handle* h) {
 // by lsum_clear on the stream before each launch, and its subtree memos,
 // multiplied into the counts by memo_finish after it.
 void lsum_bind(const cgb_handle* h, bool any_sum, bool any_memo, DfsArgs& da) {
-    const bool on = any_sum && h->d_lsum;
+    const bool on = any_sum && h->lsum_slots;
     da.lsum_tab = on ? h->d_lsum : nullptr;
     da.lsum_mask = on ? h->lsum_slots - 1 : 0;
-    const bool memo = any_memo && h->d_memo;
+    const bool memo = any_memo && h->memo_slots;
     da.memo_tab = memo ? h->d_memo : nullptr;
     da.memo_mask = memo ? h->memo_slots - 1 : 0;
     da.memo_list = h->d_memo_list;

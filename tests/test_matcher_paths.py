@@ -6,6 +6,7 @@ Exact equality throughout: counts, per-edge counts and keys are whole numbers.
 import json
 import os
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -378,6 +379,64 @@ def test_flat_merge_tile_edges(n_old, n_ins, n_del):
     assert st == 0
     got = out[:int(out_n.item())].cpu().numpy().view(np.uint64)
     assert np.array_equal(got, want)
+
+
+# ---------------------------------------------------------------------------
+# calls into the CUDA runtime that fail or that should not be made
+# ---------------------------------------------------------------------------
+RETRY_PY = r"""
+import sys
+import numpy as np
+from cgbdsm_b200 import Engine
+from cgbdsm_b200.engine import CgbError
+z = np.load(sys.argv[1])
+ql, qe, n = [int(x) for x in z["ql"]], [tuple(int(v) for v in e) for e in z["qe"]], int(z["n"])
+eng = Engine()
+eng.load_query(len(ql), qe, ql)
+try:
+    eng.build_index(z["init"], n)
+    print("no failure")
+except CgbError as e:
+    print("failed" if sys.argv[2] in str(e) else f"other failure: {e}")
+eng.build_index(z["init"], n)
+none = np.zeros(0, np.uint64)
+for k in range(2):
+    print(eng.apply_batch(n, none, none, z[f"delta{k}"]))
+"""
+
+
+def _with_shim(tmp_path, script, args, **env):
+    """Output lines of a Python script run with the runtime shim preloaded."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    so = tmp_path / "shim.so"
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", os.path.join(root, "tests", "native", "cudart_shim.c"), "-o", str(so),
+                    "-ldl"], check=True)
+    out = subprocess.run([sys.executable, "-c", script, *[str(x) for x in args]], check=True, capture_output=True, text=True,
+                         cwd=root, timeout=300, env={**os.environ, "LD_PRELOAD": str(so), "PYTHONPATH": root, **env}).stdout
+    return out.splitlines()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,what", [("d_memo_list", 4), ("d_memo", 32), ("d_lsum", 16)])
+def test_failed_table_allocation_is_retried(name, what, tmp_path):
+    """An allocation that fails while the matcher's tables are made (4,096
+    slots at this size) fails the call; the next one makes them, and counts on
+    a pattern with a subtree memo equal the restatement's."""
+    ql, qe = PATTERNS["shared"]
+    rng = np.random.default_rng(3)
+    n = 160
+    lab, pairs = _graph(rng, n, max(ql) + 1, 33)
+    rng.shuffle(pairs)
+    k = len(pairs) // 6
+    orc = bind.Oracle(len(ql), qe)
+    init = _keys_of(orc, qe, ql, lab, pairs[2 * k:])
+    deltas = [_keys_of(orc, qe, ql, lab, p) for p in (pairs[:k], pairs[k:2 * k])]
+    orc.build(init, n)
+    want = [orc.batch(n, _empty(), _empty(), d, None, bind.PER_EDGE) for d in deltas]
+    f = tmp_path / "in.npz"
+    np.savez(f, ql=ql, qe=qe, n=n, init=init, delta0=deltas[0], delta1=deltas[1])
+    got = _with_shim(tmp_path, RETRY_PY, [f, name], CGB_SHIM_FAIL_BYTES=str(4096 * what))
+    assert got == ["failed", str(want[0]), str(want[1])]
 
 
 # ---------------------------------------------------------------------------
