@@ -37,6 +37,7 @@
 
 #include "cgbdsm.h"
 #include "query.h"
+#include "seed_claim.h"
 
 using cgb::EdgePlan;
 using cgb::kMaxBN;
@@ -1243,7 +1244,7 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
     return x;
 }
 
-// Work units of the DFS: seeds (delta edges) from a counter, ranges handed
+// Work units of the DFS: seeds (delta edges; seed_claim.h), ranges handed
 // over inside a block through shared memory, and ranges handed to other blocks
 // through a ring of tasks in device memory.  A task is 16 words: w0 = ei |
 // depth << 16 | generator << 24, w1/w2 = [lo, hi) of the generator list, w3 =
@@ -1413,6 +1414,10 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     __shared__ uint32_t s_poller;                      // a warp of this block waits on the ring
     __shared__ uint32_t s_over;                        // the launch has no work left
     __shared__ unsigned long long s_live;              // unfinished units << 32 | finished, unreported
+    __shared__ uint32_t s_row;                         // the block's row of seeds
+    // lane 0's own (looked at between units only: registers are what the search is short of):
+    // where the next seed comes from, its row, this warp's bit of s_wait was set, ticket of the ring
+    __shared__ uint32_t s_acq[kDfsWarps][4];
     __shared__ unsigned long long s_stat[kDfsWarps][3];  // tail counts, bytes, busy cycles
 
     const uint32_t lane = threadIdx.x & 31;
@@ -1421,6 +1426,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     // launch tag of the task ring: a kernel argument, or (in a replayed CUDA
     // graph, whose arguments are fixed) a device word bumped before the launch
     const uint32_t epoch = a.epoch_ptr ? *(const volatile unsigned int*)a.epoch_ptr : a.epoch;
+    if (threadIdx.x == kDfsWarps * 32 - 1) s_row = atomicAdd(a.work_next + 1, 1u);  // beside the loads that follow
     if (!kMulti) {
         if (threadIdx.x <= a.qe) s_pre[threadIdx.x] = a.seed_pre[threadIdx.x];
         if (threadIdx.x < a.qe) s_lo[threadIdx.x] = a.seed_lo[threadIdx.x];
@@ -1432,6 +1438,9 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     if (threadIdx.x < kDfsWarps) {
         s_boxfull[threadIdx.x] = 0;
         s_stat[threadIdx.x][0] = s_stat[threadIdx.x][1] = s_stat[threadIdx.x][2] = 0;
+        s_acq[threadIdx.x][0] = cgb::kSeedFirst;
+        s_acq[threadIdx.x][2] = 0;
+        s_acq[threadIdx.x][3] = kNoTicket;
     }
     if (threadIdx.x == 0) {
         s_wait = s_poller = s_over = 0;
@@ -1474,16 +1483,13 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     const unsigned long long t_start = global_ns();
     uint32_t steps = 0;
     bool out_of_time = false;
-    bool no_seed = false;         // lane 0: every seed has been taken
-    bool waiting = false;         // lane 0: this warp's bit of s_wait was set
-    uint32_t ticket = kNoTicket;  // lane 0: ticket of the task ring this warp waits on
+    uint32_t &seeds = s_acq[w][0], &waiting = s_acq[w][2], &ticket = s_acq[w][3];
     uint32_t dirty = 0;  // shallowest position changed since the tail cache was filled (kClean: none)
     bool mb = false;              // counting (a part of) a subtree memo's S, unweighted, into mb_slot
     uint32_t mb_slot = kLsumNone;
     unsigned long long mb_base = 0;  // lane-local count when it was entered
     unsigned long long tail_k = 0;  // product of the tail groups that depend on the current prefix alone
     uint32_t idle_spins = 0;
-    bool first_seed = true;
     uint32_t kind = 0;
     uint32_t unit_clk = 0;  // kMulti: clock at the current unit's start
 
@@ -1503,15 +1509,13 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         kind = 0;
         uint32_t item = 0;
         if (lane == 0) {
-            if (!no_seed) {
-                // the first seed of every warp is fixed (no atomic when there are fewer seeds than warps)
-                item = first_seed ? blockIdx.x + gridDim.x * w : gridDim.x * kDfsWarps + atomicAdd(a.work_next, 1u);
-                first_seed = false;
+            if (seeds <= cgb::kSeedNext) {
+                item = cgb::seed_claim(seeds, s_acq[w][1], s_row, w, total, gridDim.x, kDfsWarps, a.steal != 0,
+                                       [&](uint32_t i, uint32_t n) { return atomicAdd(a.work_next + i, n); },
+                                       [&](uint32_t i) { return *(volatile unsigned int*)(a.work_next + i); });
                 if (item < total) {
                     kind = 1;
                     atomicAdd(&s_live, kLiveUnit);
-                } else {
-                    no_seed = true;
                 }
             }
             if (!kind) {
@@ -1563,6 +1567,15 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
         if (kind == 0) {
             __nanosleep(idle_spins < 16 ? 40u : 200u);
             ++idle_spins;
+            // rows left over now are those of blocks that cannot start
+            if ((idle_spins & 63u) == 16u && lane == 0 && seeds == cgb::kSeedLater && ticket == kNoTicket) {
+                if (*(volatile unsigned int*)(a.work_next + 1) >= gridDim.x) {
+                    seeds = cgb::kSeedNone;
+                } else if (!waiting || ((atomicAnd(&s_wait, ~(1u << w)) >> w) & 1u)) {
+                    waiting = false;  // (otherwise a busy warp is filling this warp's mailbox)
+                    seeds = cgb::kSeedNext;
+                }
+            }
             if ((idle_spins & 255u) == 0) {
                 const bool late = a.budget_ns && (global_ns() - t_start) > a.budget_ns;
                 if (__shfl_sync(kFull, late ? 1 : 0, 0)) { out_of_time = true; break; }
@@ -3246,7 +3259,8 @@ cgb_status cgb_apply_batch_device(cgb_handle* h, uint32_t dv_count, const uint64
         }
         da.budget_ns = h->cfg.dfs_budget_ms ? (unsigned long long)h->cfg.dfs_budget_ms * 1000000ull
                                             : 600ull * 1000000000ull;
-        // persistent grid: exactly the blocks that can be resident at once
+        // persistent grid: the blocks that an empty device holds at once (fewer may
+        // run while another handle's kernels do: seed_claim.h)
         if (h->dfs_occupancy == 0) {
             int occ = 0;
             CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_dfs_count<false>, kDfsWarps * 32, 0));

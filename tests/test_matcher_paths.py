@@ -12,12 +12,12 @@ import numpy as np
 import pytest
 
 from cgbdsm_b200 import Engine, Gpma, MultiQuery
-from cgbdsm_b200.engine import FLAG_MASK_PRUNE, FLAG_VALID_BITS, CgbError
+from cgbdsm_b200.engine import FLAG_MASK_PRUNE, FLAG_NO_STEAL, FLAG_VALID_BITS, CgbError
 from oracle import bind
 
 
 def _key(d, u, v):
-    return (np.uint64(d) << np.uint64(59)) | (np.uint64(u) << np.uint64(32)) | np.uint64(v)
+    return (np.uint64(d) << np.uint64(59)) | (np.asarray(u, np.uint64) << np.uint64(32)) | np.asarray(v, np.uint64)
 
 
 def _empty():
@@ -99,6 +99,43 @@ def test_out_of_range_delta_key_is_rejected(flags, bad):
     eng.apply_batch(64, _empty(), _empty(), _empty())
     assert np.array_equal(np.sort(eng.read_index()), np.unique(np.array([_key(0, 1, 2), _key(1, 2, 1), *good], np.uint64)))
     eng.close()
+
+
+# ---------------------------------------------------------------------------
+# seeds: how the launch's warps claim them
+# ---------------------------------------------------------------------------
+def test_seeds_are_claimed_by_whatever_part_of_the_grid_runs(tmp_path):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = tmp_path / "seed_claim"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-pthread", "-I", os.path.join(root, "cgbdsm_b200", "csrc"),
+                    os.path.join(root, "tests", "native", "seed_claim.cpp"), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], capture_output=True, text=True, timeout=300).stdout == "ok\n"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flags", [0, FLAG_NO_STEAL])
+@pytest.mark.parametrize("blocks", [0, 1])
+def test_seed_counts_around_the_grid(flags, blocks):
+    """As many seeds as blocks and as warps of the grid (148 SMs, 4 or 1 blocks
+    each, 8 warps), one fewer and one more; and several rounds of them.  Every
+    seed (x, y) of the path 0-1-2 counts y's neighbours of label 2."""
+    g = 148 * (blocks or 4)
+    n = 20000
+    rng = np.random.default_rng(g)
+    out = rng.integers(0, 4, 100)  # neighbours of label 2 of the vertices [10000, 10100)
+    qe, ql = [(0, 1), (1, 2)], [0, 1, 2]
+    orc = bind.Oracle(3, qe)
+    d = {(a, b): orc.L.orc_dir(orc.h, a, b) for x, y in qe for a, b in ((x, y), (y, x))}
+    init = [k for y, c in enumerate(out) for z in range(c)
+            for k in (_key(d[1, 2], 10000 + y, 11000 + z), _key(d[2, 1], 11000 + z, 10000 + y))]
+    for seeds in (1, g - 1, g, g + 1, 2 * g + 1, 8 * g - 1, 8 * g, 8 * g + 1, min(3 * 8 * g + 5, 9999)):
+        eng = Engine(flags=flags, dfs_blocks_per_sm=blocks)
+        eng.load_query(3, qe, ql)
+        eng.build_index(np.array(init, np.uint64), n)
+        y = rng.integers(0, 100, seeds)
+        delta = np.concatenate([_key(d[0, 1], np.arange(seeds), 10000 + y), _key(d[1, 0], 10000 + y, np.arange(seeds))])
+        assert eng.apply_batch(n, _empty(), _empty(), delta) == out[y].sum()
+        eng.close()
 
 
 # ---------------------------------------------------------------------------
