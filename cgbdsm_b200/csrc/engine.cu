@@ -2400,7 +2400,7 @@ struct cgb_handle {
     cgb_config cfg{};
     int device = 0;
     int num_sms = 148;
-    int clock_khz = 0;
+    int clock_khz = 0;      // asked for by the multi-query autotuner: a slow query
     int dfs_occupancy = 0;  // resident DFS blocks per SM
     uint32_t dfs_epoch = 0; // launch counter used as the task ready tag
     cudaStream_t stream = nullptr;
@@ -2972,7 +2972,6 @@ cgb_status cgb_create(const cgb_config* cfg, cgb_handle** out) {
 #define CKC(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { *out = h; return fail(h, CGB_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); } } while (0)
     CKC(cudaSetDevice(h->device));
     CKC(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device));
-    CKC(cudaDeviceGetAttribute(&h->clock_khz, cudaDevAttrClockRate, h->device));
     CKC(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
     CKC(cudaMalloc(&h->d_scal, kCtlWords * sizeof(unsigned long long)));

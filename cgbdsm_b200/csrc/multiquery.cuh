@@ -522,6 +522,7 @@ cgb_status mq_autotune(cgb_mq* m, uint64_t n2) {
     cgb_handle* h = m->h;
     const int occ = mq_occupancy(m);
     if (m->bps == 0) m->bps = m->cfg.dfs_blocks_per_sm ? std::min<int>(occ, m->cfg.dfs_blocks_per_sm) : occ;
+    if (h->clock_khz == 0) MCK(cudaDeviceGetAttribute(&h->clock_khz, cudaDevAttrClockRate, h->device));
     float ms = 0;
     bool any_new = false;
     const size_t live = std::count_if(m->queries.begin(), m->queries.end(), [](const cgb_mq::Query& q) { return q.live; });

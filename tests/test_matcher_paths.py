@@ -476,6 +476,27 @@ def test_failed_table_allocation_is_retried(name, what, tmp_path):
     assert got == ["failed", str(want[0]), str(want[1])]
 
 
+CREATE_PY = r"""
+import os, sys
+from cgbdsm_b200 import Engine, MultiQuery
+e, m = Engine(), MultiQuery(dfs_budget_ms=60000)
+print(open(os.environ["CGB_SHIM_ATTR_LOG"]).read().split())
+m.load_graph([0, 1, 0, 1], [(0, 1)])
+q = m.register(2, [(0, 1)], [0, 1])
+print(int(m.apply_batch(ins=[(2, 3), (0, 3)])[0][q]))
+print(open(os.environ["CGB_SHIM_ATTR_LOG"]).read().split())
+"""
+
+
+@pytest.mark.gpu
+def test_creating_an_engine_asks_for_no_clock_rate(tmp_path):
+    """The clock rate (attribute 13), slow to read, is asked for by the
+    autotuner alone, not by creating a handle."""
+    created, count, tuned = _with_shim(tmp_path, CREATE_PY, [], CGB_SHIM_ATTR_LOG=str(tmp_path / "attrs"))
+    assert "'13'" not in created and "'16'" in created
+    assert count == "2" and tuned.count("'13'") == 1
+
+
 # ---------------------------------------------------------------------------
 # planned subsets (no GPU)
 # ---------------------------------------------------------------------------
