@@ -2444,7 +2444,8 @@ struct cgb_handle {
     uint32_t* d_big_tile0 = nullptr; size_t big_tile0_cap = 0;
     uint2* d_tiles = nullptr; size_t tiles_cap = 0;
     unsigned long long* d_tile_state = nullptr; size_t tile_state_cap = 0;
-    uint64_t unsynced_edits = 0;  // edits merged since h_live was read
+    uint64_t unsynced_edits = 0;  // edits merged since h_live and h_pool_top were read
+    unsigned long long unsynced_need = 0;  // pool words those merges take at most
     uint64_t* d_dkeys = nullptr; uint64_t* d_dkeys_alt = nullptr; size_t dkeys_cap = 0;
     uint32_t* d_dval = nullptr;
     uint32_t* d_seed = nullptr;  // [0..kMaxQE) lo, [kMaxQE..2kMaxQE+1) pre
@@ -2749,19 +2750,37 @@ cgb_status compact_pool(cgb_handle* h, unsigned long long new_cap) {
     }
     h->h_pool_top = live;
     h->h_live = (long long)live;
+    h->unsynced_edits = 0;
+    h->unsynced_need = 0;
     unsigned long long sc[2] = {live, live};  // kCtlPoolTop, kCtlLive
     CK(cudaMemcpyAsync(h->d_scal, sc, sizeof(sc), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     return CGB_OK;
 }
 
-// Ensures the pool can absorb a merge of n_edits edits in the worst case.
+cgb_status sync_scalars(cgb_handle* h);
+
+// Ensures the pool can absorb a merge of n_edits edits in the worst case: every
+// run is written anew.  The pool's top is known as of the last read-back; the
+// merges enqueued since count by their own worst case, and where that says no
+// the pool is asked.
 cgb_status reserve_pool(cgb_handle* h, uint64_t n_edits) {
-    const unsigned long long need = (unsigned long long)std::max<long long>(h->h_live, 0) + 4ull * n_edits + 64;
-    if (h->h_pool_top + need <= h->pool_cap) return CGB_OK;
+    cgb_status s;
+    auto need = [&] {
+        return (unsigned long long)std::max<long long>(h->h_live, 0) + 4ull * (h->unsynced_edits + n_edits) + 64;
+    };
+    if (h->unsynced_need && h->h_pool_top + h->unsynced_need + need() > h->pool_cap &&
+        (s = sync_scalars(h)) != CGB_OK)
+        return s;
+    if (h->h_pool_top + h->unsynced_need + need() <= h->pool_cap) {
+        h->unsynced_need += need();
+        return CGB_OK;
+    }
     unsigned long long cap = h->pool_cap;
-    while ((unsigned long long)std::max<long long>(h->h_live, 0) + need > cap * 3 / 4) cap = cap * 2;
-    return compact_pool(h, cap);
+    while ((unsigned long long)std::max<long long>(h->h_live, 0) + need() > cap * 3 / 4) cap = cap * 2;
+    if ((s = compact_pool(h, cap)) != CGB_OK) return s;
+    h->unsynced_need = need();
+    return CGB_OK;
 }
 
 // Sorts packed keys in place (alt buffer used as ping-pong); returns sorted pointer.
@@ -2929,6 +2948,7 @@ cgb_status sync_scalars(cgb_handle* h) {
     h->h_pool_top = h->h_scal[kCtlPoolTop];
     h->h_live = (long long)h->h_scal[kCtlLive];
     h->unsynced_edits = 0;
+    h->unsynced_need = 0;
     return CGB_OK;
 }
 

@@ -101,6 +101,33 @@ def test_out_of_range_delta_key_is_rejected(flags, bad):
     eng.close()
 
 
+@pytest.mark.gpu
+def test_two_merges_of_a_batch_near_the_end_of_the_pool():
+    """A deletion batch merges the pending insertions and then its own edits,
+    both rewriting nearly every run.  In a pool that has room for either merge
+    but not for both (one of these sizes, after some batches) no batch is lost:
+    counts equal those of an engine whose pool is large."""
+    rng = np.random.default_rng(11)
+    hubs, leaves = 64, 8000
+    lab = np.array([0] * hubs + [1] * leaves, np.uint32)
+    pick = np.argsort(rng.random((leaves, hubs)), axis=1)[:, :12]  # distinct hubs of every leaf
+
+    def edges(cols):
+        return np.array([(pick[x, c], hubs + x) for x in range(leaves) for c in cols], np.uint32)
+
+    engines = []
+    for words in (0, *range(520_000, 1_000_000, 60_000)):
+        m = MultiQuery(dfs_budget_ms=60000, pool_words=words)
+        m.load_graph(lab, edges(range(8)))
+        engines.append((m, m.register(3, [(0, 1), (1, 2)], [1, 0, 1])))
+    batches = [edges([8 + i]) for i in range(4)]
+    for b in batches:
+        got = [[int(x) for x in (m.apply_batch(ins=b)[0][q], m.apply_batch(dele=b)[1][q])] for m, q in engines]
+        assert got[0][0] == got[0][1] > 0 and all(g == got[0] for g in got)
+    for m, _ in engines:
+        m.close()
+
+
 # ---------------------------------------------------------------------------
 # seeds: how the launch's warps claim them
 # ---------------------------------------------------------------------------
