@@ -2608,6 +2608,7 @@ cgb_status ensure_dvcap(cgb_handle* h, uint32_t dv) {
     h->rec = nr;
     h->dvcap = nc;
     h->rb_valid = false;  // the slot table and the bit sets follow the record layout
+    h->wjobs_for = nullptr;  // so do the arrays in the level-sum jobs, wherever d_wsum lies
     h->rb_len_now = h->rb_min_len;
     return ensure_tables(h);
 }

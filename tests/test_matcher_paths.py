@@ -503,6 +503,50 @@ def test_failed_table_allocation_is_retried(name, what, tmp_path):
     assert got == ["failed", str(want[0]), str(want[1])]
 
 
+GROWING_PY = r"""
+import sys
+import numpy as np
+from cgbdsm_b200 import Engine
+z = np.load(sys.argv[1])
+none = np.zeros(0, np.uint64)
+eng = Engine()
+eng.load_query(6, [(k, k + 1) for k in range(5)], list(range(6)))
+eng.build_index(z["init"], int(z["ids"][0]))
+for i, n in enumerate(z["ids"]):
+    print(eng.apply_batch(int(n), none, none, z[f"delta{i}"]))
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ids", [(300, 5000), (300, 2000, 9000, 40000)])
+def test_dense_level_sums_with_growing_ids(ids, tmp_path):
+    """A tree of labels of their own (dense level sums) whose vertex ids outgrow
+    the record table between matched batches, with an allocator that hands
+    the sums' block out again for their larger arrays: the jobs follow the
+    table's width, not the block's address.  Counts equal the restatement's."""
+    ql, qe = list(range(6)), [(k, k + 1) for k in range(5)]
+    rng = np.random.default_rng(len(ids))
+
+    def some(n, lo, m):
+        pairs = {(6 * (int(a) // 6) + x, 6 * (int(b) // 6) + y)
+                 for x, y in qe for a, b in zip(rng.integers(lo, n - 6, m), rng.integers(0, n - 6, m))}
+        return _keys_of(orc, qe, ql, np.arange(n) % 6, np.array(sorted(pairs), dtype=np.int64))
+
+    orc = bind.Oracle(len(ql), qe)
+    init = some(ids[0], 0, 400)
+    orc.build(init, ids[0])
+    seen, deltas, want = init, {}, []
+    for i, n in enumerate(ids):
+        keys = np.setdiff1d(some(n, ids[i - 1] if i else 0, 300), seen)
+        seen = np.union1d(seen, keys)
+        deltas[f"delta{i}"] = keys
+        want.append(orc.batch(n, _empty(), _empty(), keys, None, bind.PER_EDGE))
+    assert all(w > 0 for w in want)
+    f = tmp_path / "in.npz"
+    np.savez(f, ids=ids, init=init, **deltas)
+    assert _with_shim(tmp_path, GROWING_PY, [f], CGB_SHIM_REUSE="1") == [str(w) for w in want]
+
+
 CREATE_PY = r"""
 import os, sys
 from cgbdsm_b200 import Engine, MultiQuery
