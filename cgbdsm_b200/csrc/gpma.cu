@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "cgbdsm.h"
+#include "kept_buffers.h"
 
 namespace {
 
@@ -375,11 +376,9 @@ struct cgb_gpma {
     uint64_t* d_off = nullptr; uint64_t* d_cap = nullptr; uint32_t* d_h = nullptr; uint64_t* d_leaf0 = nullptr;
     unsigned long long* d_scal = nullptr;  // [0] n_ins, [1] n_win, [2] resize|err<<1 (u32 pair), [3..] hist
     void* temp = nullptr; size_t temp_cap = 0;
-    // per-call buffers, kept between calls (galloc, reclaim): a call's 16
-    // cudaMalloc and cudaFree took 14 of a 100k + 100k update's 17 ms
-    struct Buf { void* p; size_t bytes; bool used; };
-    std::vector<Buf> bufs;
-    size_t call_bytes = 0;    // handed out since the last reclaim
+    // per-call buffers, kept between calls: a call's 16 cudaMalloc and cudaFree
+    // took 14 of a 100k + 100k update's 17 ms
+    cgb::KeptBuffers bufs;
     uint64_t stats[6] = {0, 0, 0, 0, 0, 0};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
 };
@@ -405,24 +404,16 @@ cgb_status gfail(cgb_gpma* g, cgb_status s, const char* fmt, ...) {
 
 unsigned grid_of(uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, 148ull * 16)); }
 
-// A buffer of n T for the current call: the smallest kept one that holds it
-// without wasting more than three quarters, else a new one.
+// A buffer of n T for the current call.
 template <typename T>
 cgb_status galloc(cgb_gpma* g, T*& p, uint64_t n) {
-    const size_t need = std::max<uint64_t>(n, 1) * sizeof(T);
-    cgb_gpma::Buf* best = nullptr;
-    for (auto& b : g->bufs)
-        if (!b.used && b.bytes >= need && b.bytes <= 4 * need + (1u << 20) && (!best || b.bytes < best->bytes)) best = &b;
-    if (!best) {
-        const size_t bytes = need + need / 4;
+    cudaError_t e = cudaSuccess;
+    p = (T*)g->bufs.take(std::max<uint64_t>(n, 1) * sizeof(T), [&](size_t bytes) {
         void* q = nullptr;
-        GCK(cudaMalloc(&q, bytes));
-        g->bufs.push_back({q, bytes, false});
-        best = &g->bufs.back();
-    }
-    best->used = true;
-    g->call_bytes += best->bytes;
-    p = (T*)best->p;
+        e = cudaMalloc(&q, bytes);
+        return e == cudaSuccess ? q : nullptr;
+    }, [](void* q) { cudaFree(q); });
+    GCK(e);
     return CGB_OK;
 }
 
@@ -445,23 +436,9 @@ void free_structure(cgb_gpma* g) {
     g->leaf_ins = nullptr; g->leaf_dir = nullptr;
 }
 
-// Returns the call's buffers to the handle.  What is kept is bounded by twice
-// what the call used (at least 64 MiB): the largest go first.  all: frees all.
-void reclaim(cgb_gpma* g, bool all = false) {
-    size_t total = 0;
-    for (auto& b : g->bufs) {
-        b.used = false;
-        total += b.bytes;
-    }
-    const size_t keep = all ? 0 : std::max<size_t>(2 * g->call_bytes, 64u << 20);
-    g->call_bytes = 0;
-    if (total <= keep) return;
-    std::sort(g->bufs.begin(), g->bufs.end(), [](const cgb_gpma::Buf& x, const cgb_gpma::Buf& y) { return x.bytes < y.bytes; });
-    while (!g->bufs.empty() && total > keep) {
-        total -= g->bufs.back().bytes;
-        cudaFree(g->bufs.back().p);
-        g->bufs.pop_back();
-    }
+// Returns the call's buffers to the handle.
+void reclaim(cgb_gpma* g) {
+    g->bufs.give_back([](void* p) { cudaFree(p); });
 }
 
 // The caller's key arrays may come from work queued on the default stream.
@@ -596,7 +573,7 @@ void cgb_gpma_destroy(cgb_gpma* g) {
     cudaSetDevice(g->device);
     if (g->stream) cudaStreamSynchronize(g->stream);
     free_structure(g);
-    reclaim(g, true);
+    g->bufs.release_all([](void* p) { cudaFree(p); });
     for (void* p : {(void*)g->d_off, (void*)g->d_cap, (void*)g->d_h, (void*)g->d_leaf0, (void*)g->d_scal, g->temp})
         if (p) cudaFree(p);
     if (g->e0) cudaEventDestroy(g->e0);

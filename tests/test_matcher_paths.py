@@ -409,6 +409,14 @@ def test_gpma_windows_and_counts(n, burst):
     g.close()
 
 
+def test_buffers_kept_between_calls(tmp_path):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = tmp_path / "kept"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", os.path.join(root, "cgbdsm_b200", "csrc"),
+                    os.path.join(root, "tests", "native", "kept_buffers.cpp"), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], capture_output=True, text=True, timeout=60).stdout == "ok\n"
+
+
 # ---------------------------------------------------------------------------
 # flat merge: tile edges (2,816 entries) and more than 32 tiles back to a prefix
 # ---------------------------------------------------------------------------
