@@ -3477,10 +3477,22 @@ cgb_status cgb_read_index(cgb_handle* h, uint64_t* out, uint64_t cap, uint64_t* 
     cgb_status s;
     if ((s = flush_pending(h)) != CGB_OK) return s;
     const uint64_t n = (uint64_t)h->nd * h->dv;
-    // offsets of the runs and the key buffer stay with the handle (the key
-    // buffer up to kReadKeep): allocating them took 1 of a small index's 1.2 ms
-    if ((s = grow(h, h->d_read_off, h->read_off_cap, n + 1)) != CGB_OK) return s;
-    unsigned long long* offs = h->d_read_off;
+    // the offsets of the runs and the key buffer stay with the handle up to
+    // kReadKeep words each (allocating them took 1 of a small index's 1.2 ms);
+    // larger ones are the call's own
+    constexpr size_t kReadKeep = (64u << 20) / sizeof(uint64_t);
+    struct Own {
+        void* p = nullptr;
+        ~Own() { if (p) cudaFree(p); }
+    } own_off, own_keys;
+    unsigned long long* offs = nullptr;
+    if (n + 1 > kReadKeep) {
+        CK(cudaMalloc(&own_off.p, (n + 1) * sizeof(unsigned long long)));
+        offs = (unsigned long long*)own_off.p;
+    } else {
+        if ((s = grow(h, h->d_read_off, h->read_off_cap, n + 1)) != CGB_OK) return s;
+        offs = h->d_read_off;
+    }
     k_rec_lens<<<grid_for(h, n + 1), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, offs);
     LAUNCHED();
     size_t tb = 0;
@@ -3494,23 +3506,18 @@ cgb_status cgb_read_index(cgb_handle* h, uint64_t* out, uint64_t cap, uint64_t* 
     *n_out = total;
     if (out && cap < total) return fail(h, CGB_ERR_ARG, "output capacity %llu < %llu", (unsigned long long)cap, total);
     if (out && total > 0) {
-        constexpr size_t kReadKeep = (64u << 20) / sizeof(uint64_t);
+        uint64_t* keys = nullptr;
         if (total > kReadKeep) {
-            uint64_t* d_out = nullptr;
-            CK(cudaMalloc(&d_out, total * sizeof(uint64_t)));
-            k_dump<<<grid_for(h, n * 32), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, h->pool, offs, d_out);
-            LAUNCHED();
-            cudaError_t e = cudaMemcpyAsync(out, d_out, total * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-            cudaFree(d_out);
-            CK(e);
+            CK(cudaMalloc(&own_keys.p, total * sizeof(uint64_t)));
+            keys = (uint64_t*)own_keys.p;
         } else {
             if ((s = grow(h, h->d_read, h->read_cap, (size_t)total)) != CGB_OK) return s;
-            k_dump<<<grid_for(h, n * 32), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, h->pool, offs, h->d_read);
-            LAUNCHED();
-            CK(cudaMemcpyAsync(out, h->d_read, total * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
-            CK(cudaStreamSynchronize(h->stream));
+            keys = h->d_read;
         }
+        k_dump<<<grid_for(h, n * 32), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, h->pool, offs, keys);
+        LAUNCHED();
+        CK(cudaMemcpyAsync(out, keys, total * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
     }
     return CGB_OK;
 }

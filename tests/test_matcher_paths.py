@@ -128,6 +128,24 @@ def test_two_merges_of_a_batch_near_the_end_of_the_pool():
         m.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("dv", [1000, 2_100_000, 5_000_000])
+def test_reading_the_index_keeps_no_large_buffer(dv):
+    """A read-back of an index whose run offsets (4 directions, 8 bytes a
+    vertex) are beyond 64 MiB holds none of its memory afterwards."""
+    import torch
+
+    eng = Engine()
+    eng.load_query(3, [(0, 1), (1, 2)], [0, 1, 2])
+    keys = np.unique(np.array([_key(d, u, v) for d, u, v in [(0, 1, 2), (1, 2, 1), (3, dv - 1, 7), (2, 7, dv - 1)]], np.uint64))
+    eng.build_index(keys, dv)
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        assert np.array_equal(np.sort(eng.read_index()), keys)
+    assert free - torch.cuda.mem_get_info()[0] <= 110 << 20  # kept: offsets up to 64 MiB and half as much again
+    eng.close()
+
+
 # ---------------------------------------------------------------------------
 # seeds: how the launch's warps claim them
 # ---------------------------------------------------------------------------
