@@ -1037,7 +1037,7 @@ __device__ __forceinline__ unsigned long long flat_lists(const EdgePlan& P, uint
                                                          const uint4* bn, const uint4* __restrict__ rec,
                                                          uint32_t dvcap, const uint32_t* __restrict__ pool,
                                                          const uint32_t* __restrict__ dval, uint32_t lane,
-                                                         uint32_t& bytes, const RB& rb) {
+                                                         uint32_t& n_words, const RB& rb) {
     // this lane's shortest list: record fields x, y, z, length, bn index
     uint32_t gx = 0, gy = 0, gz = 0, glen = 0xffffffffu, gq = 0;
     for (uint32_t b = lists; b; b &= b - 1) {
@@ -1050,7 +1050,7 @@ __device__ __forceinline__ unsigned long long flat_lists(const EdgePlan& P, uint
             r = rec[at];
             if (!P.bn_dvis[q]) r.w = 0;
             rb.touch(at);
-            bytes += 16;
+            n_words += 4;
         }
         if (r.y + r.w < glen) {
             glen = r.y + r.w;
@@ -1088,7 +1088,7 @@ __device__ __forceinline__ unsigned long long flat_lists(const EdgePlan& P, uint
             uint32_t x = 0;
             if (ok) {
                 x = off < oy ? __ldg(pool + ox + off) : __ldg(dval + oz + (off - oy));
-                bytes += 4;
+                n_words += 1;
             }
             if (sum) {
                 unsigned long long v = ok ? sum_lens(P, rec, dvcap, x, rb) : 0ull;
@@ -1122,7 +1122,7 @@ __device__ __forceinline__ unsigned long long flat_lists(const EdgePlan& P, uint
                             if (!P.bn_dvis[q]) r.w = 0;
                             sl = rb.slot_at(at);
                         }
-                        bytes += 32u * (33u - __clz(r.y | 1u));
+                        n_words += 8u * (33u - __clz(r.y | 1u));
                         ok = rb.has_slot(sl, r, pool, dval, x);
                     }
                 }
@@ -1471,13 +1471,15 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
     unsigned long long cnt = 0;  // lane-local partial count of the current edge
     // statistics: 32-bit counts in registers; tail counts and bytes (seed keys,
     // records, list words, probe sectors) gathered in shared memory, bytes
-    // from a per-lane count emptied every 64 steps and at every unit's end
-    uint32_t n_seeds = 0, n_chunks = 0, n_tested = 0, n_tasks = 0, n_bytes = 0;
+    // from a per-lane count of 4-byte words emptied every 64 steps and at every
+    // unit's end (2^32 words a lane: some ten seconds of one warp's search)
+    uint32_t n_seeds = 0, n_chunks = 0, n_tested = 0, n_tasks = 0, n_words = 0;
     auto count_tails = [&](uint32_t v) { s_stat[w][0] += v; };
     auto flush_bytes = [&]() {
-        const uint32_t b = __reduce_add_sync(kFull, n_bytes >> 2);
-        n_bytes &= 3u;
-        if (lane == 0) s_stat[w][1] += 4ull * b;
+        // in two halves: 32 lanes' sum has more than 32 bits
+        const uint32_t lo = __reduce_add_sync(kFull, n_words & 0xffffu), hi = __reduce_add_sync(kFull, n_words >> 16);
+        n_words = 0;
+        if (lane == 0) s_stat[w][1] += 4ull * lo + ((unsigned long long)hi << 18);
     };
     int cur_ei = -1;
     const unsigned long long t_start = global_ns();
@@ -1614,7 +1616,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
             if (lane == 0) {
                 m[0] = (uint32_t)((key >> a.B) & vmask);
                 m[1] = grouped_at(ei) ? kNoVertex : (uint32_t)(key & vmask);
-                n_bytes += 8;
+                n_words += 2;
             }
         } else {
             // lane 0 saw the ticket's ready tag, or its mailbox full: the task's words are published
@@ -1663,7 +1665,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
             X.x = a.dval + xr.z;
             X.n = xr.w;
             if (X.n <= 32 && lane < X.n) X.xv = __ldg(X.x + lane);
-            if (lane == 0) n_bytes += 16 + 4 * min(X.n, 32u);
+            if (lane == 0) n_words += 4 + min(X.n, 32u);
         }
         // set up depth j: resolve BN records, choose the shortest list as generator
         auto setup = [&](uint32_t j) {
@@ -1678,7 +1680,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                 bn[k] = r;
                 rb.note(k, at);
                 len = r.y + r.w;
-                n_bytes += 16;
+                n_words += 4;
             }
             // shortest list, lowest lane on ties: one redux over (length << 5 | lane)
             // (lengths are below 2^27; a longer one is only a worse generator)
@@ -1797,7 +1799,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                                 const uint32_t p = P.bn_pos[P.bn_off[lane]];
                                 if (p < j) {
                                     v0 = __ldg(a.wsum + (size_t)(P.wslot + lane - j) * a.dvcap + m[p]);
-                                    n_bytes += 8;
+                                    n_words += 2;
                                 }
                             }
                             for (int o = 16; o > 0; o >>= 1) v0 *= __shfl_xor_sync(kFull, v0, o);
@@ -1911,7 +1913,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                     ok = idx < glen;
                     if (ok) {
                         c = idx < gr.y ? __ldg(a.pool + gr.x + idx) : __ldg(a.dval + gr.z + (idx - gr.y));
-                        n_bytes += 4;
+                        n_words += 1;
                         for (uint32_t t = 0; t < j; ++t) ok &= (c != m[t]);
                         if (ok && a.vb)  // the valid bits are a sound superset: a clear bit cannot match
                             ok = (__ldg(a.vb + ((size_t)ei * a.qv + P.vs[j]) * a.vb_stride + (c >> 5)) >> (c & 31)) & 1u;
@@ -1925,7 +1927,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                         for (uint32_t k = o0; k < o1 && ok; ++k) {
                             if (k == o0 + g) continue;
                             const uint4 r = bn[k];
-                            n_bytes += 32u * (33u - __clz(r.y | 1u));
+                            n_words += 8u * (33u - __clz(r.y | 1u));
                             ok = rb.has(k, r, a.pool, a.dval, c);
                         }
                         ++n_tested;
@@ -2002,7 +2004,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                         if (!P.bn_dvis[k]) r.w = 0;
                         bn[k] = r;
                         rb.note(k, at);
-                        n_bytes += 16;
+                        n_words += 4;
                     }
                     __syncwarp();
                 }
@@ -2053,7 +2055,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                                     if (!P.bn_dvis[q]) r.w = 0;
                                     if (ex) sl = rb.slot_at(at);
                                     rb.touch(at);
-                                    n_bytes += 16;
+                                    n_words += 4;
                                 }
                                 v = (unsigned long long)r.y + r.w;
                                 for (uint32_t e = stat ? ex & dmask : ex; e; e &= e - 1) {
@@ -2067,7 +2069,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                                 }
                             } else {
                                 v = flat_lists(P, lists, fd, is_sum, fon, fc, stat ? ex & dmask : ex, m, bn, a.rec, a.dvcap,
-                                               a.pool, a.dval, lane, n_bytes, rb);
+                                               a.pool, a.dval, lane, n_words, rb);
                             }
                             if (stat) {
                                 v = __shfl_sync(kFull, v, 0);
@@ -2096,7 +2098,7 @@ __global__ void __launch_bounds__(kDfsWarps * 32, 4) k_dfs_count(DfsArgs a) {
                             bool in = true;
                             for (uint32_t b = lists; b && in; b &= b - 1) {
                                 const uint32_t q = P.sub_base + __ffs(b) - 1;
-                                n_bytes += 32u * (33u - __clz(bn[q].y | 1u));
+                                n_words += 8u * (33u - __clz(bn[q].y | 1u));
                                 in = rb.has(q, bn[q], a.pool, a.dval, c);
                             }
                             v -= in ? 1ull : 0ull;

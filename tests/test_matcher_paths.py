@@ -397,6 +397,33 @@ def test_level_sum_table_under_contention(hubs):
     m.close()
 
 
+@pytest.mark.gpu
+def test_byte_count_of_long_walks():
+    """The statistics' bytes of one warp's 64 steps go beyond 2^34: 2,100
+    candidates with 1,600 common neighbours each, counted as a group of three:
+    seven walks a candidate, over 2, 4 or 6 lists."""
+    K, T = 2100, 1600
+    ql, qe = [0, 1, 2, 3, 3, 3], [(0, 1), (0, 2), (1, 3), (1, 4), (1, 5), (2, 3), (2, 4), (2, 5)]
+    orc = bind.Oracle(len(ql), qe)
+    d = {(a, b): orc.L.orc_dir(orc.h, a, b) for x, y in qe for a, b in ((x, y), (y, x))}
+    v0, v1, c, t = 0, 1, 2 + np.arange(K), 2 + K + np.arange(T)
+    cc, tt = np.repeat(c, T), np.tile(t, K)
+    keys = []
+    for a, b, x, y in [(0, 2, np.full(K, v0), c)] + [(1, k, np.full(T, v1), t) for k in (3, 4, 5)] + \
+            [(2, k, cc, tt) for k in (3, 4, 5)]:
+        keys += [_key(d[a, b], x, y), _key(d[b, a], y, x)]
+    eng = Engine(flags=FLAG_NO_STEAL, dfs_budget_ms=60000)
+    eng.load_query(len(ql), qe, ql)
+    eng.build_index(np.concatenate(keys), 2 + K + T)
+    delta = np.array([_key(d[0, 1], v0, v1), _key(d[1, 0], v1, v0)], np.uint64)
+    assert eng.apply_batch(2 + K + T, _empty(), _empty(), delta) == K * T * (T - 1) * (T - 2)
+    # per common neighbour: its entry in every walk, and searches in the walks' other lists
+    want = K * T * (7 * 4 + (3 * 1 + 3 * 3 + 1 * 5) * 32 * (33 - (32 - T.bit_length())))
+    assert want * 60 // 64 > 1 << 34
+    assert want <= eng.stats()["match_bytes"] < want * 1.01
+    eng.close()
+
+
 # ---------------------------------------------------------------------------
 # packed-memory array: windows of one and of many leaves
 # ---------------------------------------------------------------------------
