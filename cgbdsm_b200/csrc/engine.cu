@@ -35,6 +35,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "alloc_count.h"
 #include "cgbdsm.h"
 #include "query.h"
 #include "seed_claim.h"
@@ -2540,7 +2541,7 @@ cgb_status grow(cgb_handle* h, T*& p, size_t& cap, size_t need) {
     size_t nc = std::max<size_t>(need + need / 2, 1024);
     if (p) CK(cudaFree(p));
     p = nullptr;
-    CK(cudaMalloc(&p, nc * sizeof(T)));
+    CK(cgb::device_malloc(&p, nc * sizeof(T)));
     cap = nc;
     return CGB_OK;
 }
@@ -2550,7 +2551,7 @@ cgb_status grow_temp(cgb_handle* h, size_t need) {
     size_t nc = std::max<size_t>(need + need / 2, 1 << 20);
     if (h->d_temp) CK(cudaFree(h->d_temp));
     h->d_temp = nullptr;
-    CK(cudaMalloc(&h->d_temp, nc));
+    CK(cgb::device_malloc(&h->d_temp, nc));
     h->temp_cap = nc;
     return CGB_OK;
 }
@@ -2574,7 +2575,7 @@ cgb_status ensure_tables(cgb_handle* h) {
         h->lsum_slots = 0;
         if (h->d_lsum) CK(cudaFree(h->d_lsum));
         h->d_lsum = nullptr;
-        CK(cudaMalloc(&h->d_lsum, (size_t)slots * 2 * sizeof(unsigned long long)));
+        CK(cgb::device_malloc(&h->d_lsum, (size_t)slots * 2 * sizeof(unsigned long long)));
         h->lsum_slots = slots;
     }
     slots = std::min(slots, 1u << 20);
@@ -2585,8 +2586,8 @@ cgb_status ensure_tables(cgb_handle* h) {
         h->d_memo = nullptr;
         if (h->d_memo_list) CK(cudaFree(h->d_memo_list));
         h->d_memo_list = nullptr;
-        CK(cudaMalloc(&h->d_memo, (size_t)slots * 4 * sizeof(unsigned long long)));
-        CK(cudaMalloc(&h->d_memo_list, (size_t)slots * sizeof(uint32_t)));
+        CK(cgb::device_malloc(&h->d_memo, (size_t)slots * 4 * sizeof(unsigned long long)));
+        CK(cgb::device_malloc(&h->d_memo_list, (size_t)slots * sizeof(uint32_t)));
         CK(cudaMemsetAsync(h->d_memo, 0, (size_t)slots * 4 * sizeof(unsigned long long), h->stream));
         h->memo_slots = slots;
     }
@@ -2597,7 +2598,7 @@ cgb_status ensure_dvcap(cgb_handle* h, uint32_t dv) {
     if (dv <= h->dvcap && h->rec) return ensure_tables(h);
     uint32_t nc = std::max<uint32_t>(dv + dv / 4 + 1024, h->dvcap * 2);
     uint4* nr = nullptr;
-    CK(cudaMalloc(&nr, (size_t)h->nd * nc * sizeof(uint4)));
+    CK(cgb::device_malloc(&nr, (size_t)h->nd * nc * sizeof(uint4)));
     CK(cudaMemsetAsync(nr, 0, (size_t)h->nd * nc * sizeof(uint4), h->stream));
     if (h->rec) {
         k_copy_rows<<<grid_for(h, (uint64_t)h->nd * h->dv), 256, 0, h->stream>>>(h->rec, h->dvcap, nr, nc, h->nd,
@@ -2659,7 +2660,7 @@ cgb_status dense_level_sums(cgb_handle* h) {
         }
         if (h->d_wjobs) CK(cudaFree(h->d_wjobs));
         h->d_wjobs = nullptr;
-        CK(cudaMalloc(&h->d_wjobs, std::max<size_t>(all.size(), 1) * sizeof(WsumJob)));
+        CK(cgb::device_malloc(&h->d_wjobs, std::max<size_t>(all.size(), 1) * sizeof(WsumJob)));
         CK(cudaMemcpy(h->d_wjobs, all.data(), all.size() * sizeof(WsumJob), cudaMemcpyHostToDevice));
         h->wjobs_for = h->d_wsum;
     }
@@ -2708,8 +2709,8 @@ cgb_status compact_pool(cgb_handle* h, unsigned long long new_cap) {
     uint32_t* sizes = nullptr;
     unsigned long long* offs = nullptr;
     unsigned long long live = 0;
-    CK(cudaMalloc(&sizes, std::max<uint64_t>(n, 1) * sizeof(uint32_t)));
-    CK(cudaMalloc(&offs, (n + 1) * sizeof(unsigned long long)));
+    CK(cgb::device_malloc(&sizes, std::max<uint64_t>(n, 1) * sizeof(uint32_t)));
+    CK(cgb::device_malloc(&offs, (n + 1) * sizeof(unsigned long long)));
     CK(cudaMemsetAsync(offs, 0, (n + 1) * sizeof(unsigned long long), h->stream));
     if (n > 0) {
         k_rec_sizes<<<grid_for(h, n), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, sizes);
@@ -2732,7 +2733,7 @@ cgb_status compact_pool(cgb_handle* h, unsigned long long new_cap) {
     } else {
         if (h->pool_alt) CK(cudaFree(h->pool_alt));
         h->pool_alt = nullptr;
-        CK(cudaMalloc(&dst, new_cap * sizeof(uint32_t)));
+        CK(cgb::device_malloc(&dst, new_cap * sizeof(uint32_t)));
     }
     if (n > 0) {
         k_compact<<<grid_for(h, n * 32), 256, 0, h->stream>>>(h->rec, h->dvcap, h->dv, h->nd, h->pool, dst, offs);
@@ -2809,9 +2810,9 @@ cgb_status ensure_edit_buffers(cgb_handle* h, uint64_t n) {
     for (auto& p : h->d_runs) p = nullptr;
     h->d_edits = h->d_edits_alt = nullptr;
     h->edits_cap = 0;
-    CK(cudaMalloc(&h->d_edits, nc * sizeof(uint64_t)));
-    CK(cudaMalloc(&h->d_edits_alt, nc * sizeof(uint64_t)));
-    for (auto& p : h->d_runs) CK(cudaMalloc(&p, nc * sizeof(uint2)));
+    CK(cgb::device_malloc(&h->d_edits, nc * sizeof(uint64_t)));
+    CK(cgb::device_malloc(&h->d_edits_alt, nc * sizeof(uint64_t)));
+    for (auto& p : h->d_runs) CK(cgb::device_malloc(&p, nc * sizeof(uint2)));
     h->edits_cap = nc;
     return CGB_OK;
 }
@@ -2827,10 +2828,10 @@ cgb_status ensure_delta_buffers(cgb_handle* h, uint64_t n) {
     h->d_dkeys = h->d_dkeys_alt = h->d_pending = nullptr;
     h->d_dval = nullptr;
     h->dkeys_cap = h->pending_cap = 0;
-    CK(cudaMalloc(&h->d_pending, nc * sizeof(uint64_t)));
-    CK(cudaMalloc(&h->d_dkeys, nc * sizeof(uint64_t)));
-    CK(cudaMalloc(&h->d_dkeys_alt, nc * sizeof(uint64_t)));
-    CK(cudaMalloc(&h->d_dval, nc * sizeof(uint32_t)));
+    CK(cgb::device_malloc(&h->d_pending, nc * sizeof(uint64_t)));
+    CK(cgb::device_malloc(&h->d_dkeys, nc * sizeof(uint64_t)));
+    CK(cgb::device_malloc(&h->d_dkeys_alt, nc * sizeof(uint64_t)));
+    CK(cgb::device_malloc(&h->d_dval, nc * sizeof(uint32_t)));
     h->dkeys_cap = h->pending_cap = nc;
     return CGB_OK;
 }
@@ -2997,25 +2998,25 @@ cgb_status cgb_create(const cgb_config* cfg, cgb_handle** out) {
     CKC(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device));
     CKC(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
-    CKC(cudaMalloc(&h->d_scal, kCtlWords * sizeof(unsigned long long)));
+    CKC(cgb::device_malloc(&h->d_scal, kCtlWords * sizeof(unsigned long long)));
     CKC(cudaMemset(h->d_scal, 0, kCtlWords * sizeof(unsigned long long)));
     h->d_rb_ctr = (unsigned int*)(h->d_scal + kCtlRbClaimed);
     h->d_list_ctr = (unsigned int*)(h->d_scal + kCtlList);
     h->d_stats = h->d_scal + kCtlStats;
     h->d_counts = h->d_scal + kCtlCounts;
     h->d_qctr = (unsigned int*)(h->d_scal + kCtlQueue);
-    CKC(cudaMalloc(&h->d_self, sizeof(unsigned int)));
+    CKC(cgb::device_malloc(&h->d_self, sizeof(unsigned int)));
     CKC(cudaMemset(h->d_self, 0, sizeof(unsigned int)));
     CKC(cudaMallocHost(&h->h_scal, kCtlWords * sizeof(unsigned long long)));
-    CKC(cudaMalloc(&h->d_rev, kMaxDir));
-    CKC(cudaMalloc(&h->d_seed, (3 * kMaxQE + 2) * sizeof(uint32_t)));
-    CKC(cudaMalloc(&h->d_tasks, (size_t)kTaskCap * kTaskWords * sizeof(uint32_t)));
+    CKC(cgb::device_malloc(&h->d_rev, kMaxDir));
+    CKC(cgb::device_malloc(&h->d_seed, (3 * kMaxQE + 2) * sizeof(uint32_t)));
+    CKC(cgb::device_malloc(&h->d_tasks, (size_t)kTaskCap * kTaskWords * sizeof(uint32_t)));
     CKC(cudaMemset(h->d_tasks, 0, (size_t)kTaskCap * kTaskWords * sizeof(uint32_t)));
-    CKC(cudaMalloc(&h->d_qe_dirs, 2 * kMaxQE));
-    CKC(cudaMalloc(&h->d_edge_ok, kMaxQE));
-    CKC(cudaMalloc(&h->d_plans, sizeof(EdgePlan) * kMaxQE));
-    CKC(cudaMalloc(&h->d_vbplans, sizeof(cgb::VbPlan) * kMaxQE));
-    CKC(cudaMalloc(&h->d_dir_edge, kMaxDir));
+    CKC(cgb::device_malloc(&h->d_qe_dirs, 2 * kMaxQE));
+    CKC(cgb::device_malloc(&h->d_edge_ok, kMaxQE));
+    CKC(cgb::device_malloc(&h->d_plans, sizeof(EdgePlan) * kMaxQE));
+    CKC(cgb::device_malloc(&h->d_vbplans, sizeof(cgb::VbPlan) * kMaxQE));
+    CKC(cgb::device_malloc(&h->d_dir_edge, kMaxDir));
     for (auto& ev : h->ev) CKC(cudaEventCreate(&ev));
 #undef CKC
     *out = h;
@@ -3131,7 +3132,7 @@ cgb_status cgb_build_index(cgb_handle* h, const uint64_t* keys, uint64_t n, uint
     // out-of-place merges write every touched run anew, so the pool carries
     // headroom for many batches between compactions (HBM is plentiful)
     if (cap == 0) cap = std::max<unsigned long long>(4ull * n + (128ull << 20), 192ull << 20);
-    CK(cudaMalloc(&h->pool, cap * sizeof(uint32_t)));
+    CK(cgb::device_malloc(&h->pool, cap * sizeof(uint32_t)));
     h->pool_cap = cap;
     h->h_pool_top = 0;
     h->h_live = 0;
@@ -3431,7 +3432,7 @@ cgb_status cgb_check_symmetry(cgb_handle* h, uint64_t* n_asym) {
     cgb_status s;
     if ((s = flush_pending(h)) != CGB_OK) return s;
     unsigned long long* d_bad = nullptr;
-    CK(cudaMalloc(&d_bad, sizeof(unsigned long long)));
+    CK(cgb::device_malloc(&d_bad, sizeof(unsigned long long)));
     CK(cudaMemsetAsync(d_bad, 0, sizeof(unsigned long long), h->stream));
     const uint64_t n = (uint64_t)h->nd * h->dv;
     if (n) {
@@ -3489,7 +3490,7 @@ cgb_status cgb_read_index(cgb_handle* h, uint64_t* out, uint64_t cap, uint64_t* 
     } own_off, own_keys;
     unsigned long long* offs = nullptr;
     if (n + 1 > kReadKeep) {
-        CK(cudaMalloc(&own_off.p, (n + 1) * sizeof(unsigned long long)));
+        CK(cgb::device_malloc(&own_off.p, (n + 1) * sizeof(unsigned long long)));
         offs = (unsigned long long*)own_off.p;
     } else {
         if ((s = grow(h, h->d_read_off, h->read_off_cap, n + 1)) != CGB_OK) return s;
@@ -3510,7 +3511,7 @@ cgb_status cgb_read_index(cgb_handle* h, uint64_t* out, uint64_t cap, uint64_t* 
     if (out && total > 0) {
         uint64_t* keys = nullptr;
         if (total > kReadKeep) {
-            CK(cudaMalloc(&own_keys.p, total * sizeof(uint64_t)));
+            CK(cgb::device_malloc(&own_keys.p, total * sizeof(uint64_t)));
             keys = (uint64_t*)own_keys.p;
         } else {
             if ((s = grow(h, h->d_read, h->read_cap, (size_t)total)) != CGB_OK) return s;

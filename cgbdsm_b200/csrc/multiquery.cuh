@@ -288,13 +288,13 @@ cgb_status mq_grow_plans(cgb_mq* m, size_t need) {
     void* olds[] = {m->d_plans, m->d_pair, m->d_seed, m->d_counts, m->d_tplans, m->d_tpair};
     for (void* p : olds) if (p) MCK(cudaFree(p));
     if (m->h_counts) MCK(cudaFreeHost(m->h_counts));
-    MCK(cudaMalloc(&m->d_plans, nc * sizeof(EdgePlan)));
-    MCK(cudaMalloc(&m->d_pair, nc * sizeof(uint16_t)));
-    MCK(cudaMalloc(&m->d_seed, (2 * nc + 2) * sizeof(uint32_t)));
-    MCK(cudaMalloc(&m->d_counts, nc * sizeof(unsigned long long)));
+    MCK(cgb::device_malloc(&m->d_plans, nc * sizeof(EdgePlan)));
+    MCK(cgb::device_malloc(&m->d_pair, nc * sizeof(uint16_t)));
+    MCK(cgb::device_malloc(&m->d_seed, (2 * nc + 2) * sizeof(uint32_t)));
+    MCK(cgb::device_malloc(&m->d_counts, nc * sizeof(unsigned long long)));
     MCK(cudaMallocHost(&m->h_counts, nc * sizeof(unsigned long long)));
-    MCK(cudaMalloc(&m->d_tplans, kMaxQE * sizeof(EdgePlan)));
-    MCK(cudaMalloc(&m->d_tpair, kMaxQE * sizeof(uint16_t)));
+    MCK(cgb::device_malloc(&m->d_tplans, kMaxQE * sizeof(EdgePlan)));
+    MCK(cgb::device_malloc(&m->d_tpair, kMaxQE * sizeof(uint16_t)));
     m->plan_cap = nc;
     return CGB_OK;
 }
@@ -347,8 +347,8 @@ cgb_status mq_prepare_delta(cgb_mq* m, const uint32_t* pairs, uint64_t mpairs, b
         if (m->d_sel) MCK(cudaFree(m->d_sel));
         if (m->d_keep) MCK(cudaFree(m->d_keep));
         m->sel_cap = std::max<size_t>(n + n / 2, 1 << 16);
-        MCK(cudaMalloc(&m->d_sel, m->sel_cap * sizeof(uint64_t)));
-        MCK(cudaMalloc(&m->d_keep, m->sel_cap));
+        MCK(cgb::device_malloc(&m->d_sel, m->sel_cap * sizeof(uint64_t)));
+        MCK(cgb::device_malloc(&m->d_keep, m->sel_cap));
     }
     k_mq_pack<<<grid_for(h, mpairs), 256, 0, h->stream>>>(pairs, mpairs, h->d_vlabel, h->dv, B, h->lb, h->d_dkeys,
                                                           d_err);
@@ -492,6 +492,7 @@ cgb_status mq_match_all(cgb_mq* m, uint64_t n2) {
         return s;
     }
     MCK(e);
+    cgb::device_allocs().fetch_add(1, std::memory_order_relaxed);  // the executable graph's own memory
     e = cudaGraphInstantiate(&m->gexec, g, 0);
     cudaGraphDestroy(g);
     MCK(e);
@@ -661,8 +662,8 @@ cgb_status cgb_mq_create(const cgb_mq_config* cfg, cgb_mq** out) {
         return s;
     }
     m->h->mq = true;
-    MCK(cudaMalloc(&m->d_nsel, sizeof(int)));
-    MCK(cudaMalloc(&m->h->d_epoch, sizeof(unsigned int)));
+    MCK(cgb::device_malloc(&m->d_nsel, sizeof(int)));
+    MCK(cgb::device_malloc(&m->h->d_epoch, sizeof(unsigned int)));
     MCK(cudaMemset(m->h->d_epoch, 0, sizeof(unsigned int)));
     for (auto& e : m->ev) MCK(cudaEventCreate(&e));
     return CGB_OK;
@@ -714,19 +715,19 @@ cgb_status cgb_mq_load_graph(cgb_mq* m, uint32_t n, const uint32_t* labels, uint
     // query-independent plan for the engine's own structures: none (plans per query)
     h->dv = n;
     MQ_TRY(ensure_dvcap(h, n));
-    MCK(cudaMalloc(&h->d_vlabel, std::max<uint32_t>(n, 1)));
+    MCK(cgb::device_malloc(&h->d_vlabel, std::max<uint32_t>(n, 1)));
     MCK(cudaMemcpy(h->d_vlabel, lab8.data(), n, cudaMemcpyHostToDevice));
     // index keys of every edge, both directions
     const uint64_t nk = 2 * num_edges;
     unsigned long long cap = m->cfg.pool_words;
     if (cap == 0) cap = std::max<unsigned long long>(nk + nk / 2 + (128ull << 20), 192ull << 20);
-    MCK(cudaMalloc(&h->pool, cap * sizeof(uint32_t)));
+    MCK(cgb::device_malloc(&h->pool, cap * sizeof(uint32_t)));
     h->pool_cap = cap;
     h->h_pool_top = 0;
     h->h_live = 0;
     MCK(cudaMemsetAsync(h->d_scal, 0, kCtlWords * sizeof(unsigned long long), h->stream));
     uint32_t* d_edges = nullptr;
-    MCK(cudaMalloc(&d_edges, std::max<uint64_t>(num_edges, 1) * 2 * sizeof(uint32_t)));
+    MCK(cgb::device_malloc(&d_edges, std::max<uint64_t>(num_edges, 1) * 2 * sizeof(uint32_t)));
     if (num_edges) MCK(cudaMemcpyAsync(d_edges, edges, num_edges * 8, cudaMemcpyHostToDevice, h->stream));
     cgb_status s = CGB_OK;
     if ((s = grow(h, h->d_keys_in, h->keys_in_cap, std::max<uint64_t>(nk, 1))) == CGB_OK) {
@@ -745,7 +746,7 @@ cgb_status cgb_mq_load_graph(cgb_mq* m, uint32_t n, const uint32_t* labels, uint
     unsigned long long* d_st = nullptr;
     std::vector<unsigned long long> cnt((size_t)L * L), nodes((size_t)L * L);
     if (s == CGB_OK) {
-        MCK(cudaMalloc(&d_st, 2 * (size_t)L * L * sizeof(unsigned long long)));
+        MCK(cgb::device_malloc(&d_st, 2 * (size_t)L * L * sizeof(unsigned long long)));
         MCK(cudaMemsetAsync(d_st, 0, 2 * (size_t)L * L * sizeof(unsigned long long), h->stream));
         if (num_edges) {
             k_mq_label_stats<<<grid_for(h, num_edges), 256, 0, h->stream>>>(d_edges, num_edges, h->d_vlabel, L, d_st);
@@ -944,7 +945,7 @@ cgb_status cgb_mq_apply_batch(cgb_mq* m, const uint32_t* ins, uint64_t n_ins, co
     if (2 * n > m->pairs_cap || !m->d_pairs) {
         if (m->d_pairs) MCK(cudaFree(m->d_pairs));
         m->pairs_cap = std::max<uint64_t>(2 * n + n, 1 << 16);
-        MCK(cudaMalloc(&m->d_pairs, m->pairs_cap * sizeof(uint32_t)));
+        MCK(cgb::device_malloc(&m->d_pairs, m->pairs_cap * sizeof(uint32_t)));
     }
     if (n_ins) MCK(cudaMemcpyAsync(m->d_pairs, ins, n_ins * 8, cudaMemcpyHostToDevice, h->stream));
     if (n_del) MCK(cudaMemcpyAsync(m->d_pairs + 2 * n_ins, del, n_del * 8, cudaMemcpyHostToDevice, h->stream));

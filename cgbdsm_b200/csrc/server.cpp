@@ -41,6 +41,7 @@
 #include <thread>
 #include <vector>
 
+#include "alloc_count.h"
 #include "cgbdsm.h"
 #include "staging_ring.h"
 
@@ -97,6 +98,7 @@ struct cgb_server {
     uint32_t live = 0;
     uint64_t used_seen = 0;   // device memory in use when last asked (scheduler thread)
     double used_at = -1;      // and when
+    uint64_t allocs_seen = 0; // engine allocations up to then
     // stats
     uint64_t batches_done = 0, edges_done = 0, rejected = 0;
     double busy_ms = 0;
@@ -158,17 +160,21 @@ void complete(cgb_server* s, const std::shared_ptr<Req>& r) {
 // Device memory in use, for the admission of a batch that needs `need` bytes
 // (scheduler thread).  The driver's answer takes about half a millisecond, as
 // long as a small batch, so the last one stands for kMemoryCheckMs while the
-// budget is a quarter away; near the limit every batch asks.
+// engine has allocated nothing and the budget is a quarter away; near the limit
+// every batch asks.  What others allocate on the device is seen by the next
+// answer.
 constexpr double kMemoryCheckMs = 20.0;
 uint64_t memory_used(cgb_server* s, uint64_t need) {
     const double now = s->now_ms();
-    if (s->used_at >= 0 && now - s->used_at < kMemoryCheckMs &&
+    const uint64_t allocs = cgb::device_allocs().load(std::memory_order_relaxed);
+    if (s->used_at >= 0 && now - s->used_at < kMemoryCheckMs && allocs == s->allocs_seen &&
         s->used_seen + need <= s->base_used + s->budget - s->budget / 4)
         return s->used_seen;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     s->used_seen = (uint64_t)(total_b - free_b);
     s->used_at = now;
+    s->allocs_seen = allocs;
     return s->used_seen;
 }
 

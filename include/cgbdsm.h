@@ -415,7 +415,10 @@ void* cgb_mq_stream(const cgb_mq* m);
  * Admission by HBM budget: an update batch's edge pairs must fit a device
  * staging ring (they are copied as soon as space frees, on a copy stream, so
  * the copies of waiting batches overlap the running batch), and its working
- * set must fit the budget (else its result is CGB_ERR_LIMIT).
+ * set must fit the budget (else its result is CGB_ERR_LIMIT).  The memory in
+ * use is asked of the driver again after every allocation of the engine, every
+ * 20 ms, and before every batch when less than a quarter of the budget is
+ * left; what other programs allocate in between is not seen until then.
  * ------------------------------------------------------------------------ */
 typedef struct cgb_server cgb_server;
 

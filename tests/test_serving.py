@@ -100,3 +100,22 @@ def test_deletion_batches_and_oversize_rejection():
     assert int(r[0]["pos"][0]) == int(p0[qid])
     assert int(r[2]["pos"][0]) == int(p1[qid])
     assert int(r[3]["neg"][0]) == int(n3[qid])
+
+
+def test_budget_sees_what_the_batch_before_allocated():
+    """Two large batches at once: each fits the budget, but not beside the
+    buffers that the first one made the engine allocate; the second is refused
+    although its turn comes within milliseconds of the first's check."""
+    n, k = 100_000, 400_000
+    rng = np.random.default_rng(4)
+    e = np.unique(rng.integers(0, n, (2 * k + 50_000, 2)).astype(np.uint32), axis=0)
+    e = e[e[:, 0] < e[:, 1]]
+    while len(e) < 2 * k:
+        more = rng.integers(0, n, (k, 2)).astype(np.uint32)
+        e = np.unique(np.concatenate([e, more[more[:, 0] < more[:, 1]]]), axis=0)
+    rng.shuffle(e)
+    srv = Server(np.zeros(n, np.uint32), np.array([(0, 1)], np.uint32), staging_bytes=8 << 20, hbm_budget_bytes=64 << 20)
+    t = [srv.submit_batch(ins=e[:k]), srv.submit_batch(ins=e[k:2 * k])]
+    r = [srv.wait(x) for x in t]
+    srv.close()
+    assert [x["status"] for x in r] == [0, 4]
