@@ -219,13 +219,18 @@ __global__ void __launch_bounds__(kThreads) k_na_merge(Merged M, uint32_t ntiles
                 if (pre) break;
                 at -= 32;
             }
-            if (gave_up && lane == 0) atomicOr(err, 2u);
+            if (gave_up && lane == 0) {
+                atomicOr(err, 2u);
+                __threadfence();  // before this tile's count: the last tile reads the error behind it
+            }
         }
         if (lane == 0) {
             atomicExch(state + tile, kPrefix | (base + all));
             s_base = base;
-            if (tile == ntiles - 1)
+            if (tile == ntiles - 1) {
+                __threadfence();
                 *out_n = *(volatile unsigned int*)err ? ~0ull : (uint64_t)(base + all);
+            }
         }
     }
     __syncthreads();  // every entry of the tile is in registers: its memory takes the output
