@@ -851,8 +851,13 @@ __global__ void k_asymmetry(const uint4* __restrict__ rec, uint32_t dvcap, uint3
 // ---------------------------------------------------------------------------
 // persistent warp DFS (count only)
 // ---------------------------------------------------------------------------
-// DFS queue counters (words); the polled ones on lines of their own
-constexpr uint32_t kQReserved = 0, kQTickets = 1, kQDone = 32, kQBusy = 40, kQMemo = 44, kQWords = 64;
+// DFS queue counters (words), on 128-byte lines by who looks at them: tasks and
+// tickets (every donor), finished units (every waiting block), and what only
+// those that add to it touch
+constexpr uint32_t kQReserved = 0, kQTickets = 1, kQDone = 32, kQMemo = 64, kQBusy = 66, kQWords = 96;
+static_assert(kQDone / 32 != kQReserved / 32 && kQDone / 32 != kQMemo / 32 && kQMemo / 32 != kQReserved / 32 &&
+                  kQBusy % 2 == 0 && kQBusy + 2 <= kQWords,
+              "polled counters share no line with others; kQBusy holds 64 bits");
 struct DfsArgs {
     const uint4* rec;
     uint32_t dvcap;
