@@ -1287,13 +1287,6 @@ __device__ __forceinline__ void add_release(unsigned int* p, unsigned int v) {
 
 constexpr uint32_t kTaskWords = 16;
 constexpr uint32_t kTaskMemo = 15;  // word of a task: memo slot its counts go to (no prefix reaches position 11)
-// Tail vertices with up to this many lists stay in the tail where they hang off
-// the last core vertex (single-query engine).  R-MAT 1M/10M, 9-vertex dense,
-// matching per batch: none 14.4 ms, up to three lists 14.0, all 16.4 (four
-// lists: enumerating the vertex narrows its candidates list by list, which the
-// per-candidate count does not share between candidates); R-MAT 100k/1M, a
-// 6-vertex sparse pattern: none 0.50 ms, up to three 0.26.
-constexpr uint32_t kFoldLists = 3;
 constexpr unsigned long long kLiveUnit = 1ull << 32;  // one unfinished unit in s_live
 constexpr uint32_t kNoTicket = 0xffffffffu;
 
@@ -3109,7 +3102,7 @@ cgb_status cgb_build_index(cgb_handle* h, const uint64_t* keys, uint64_t n, uint
     for (uint32_t d = 0; d < h->nd; ++d) avg[d] = nodes[d] ? (float)card[d] / (float)nodes[d] : 0.f;
     cgb::plan_edges(h->q, avg, h->plans, !(h->cfg.flags & CGB_FLAG_ENUMERATE_TAIL),
                     !(h->cfg.flags & CGB_FLAG_PLAIN_CORE_ORDER), !(h->cfg.flags & CGB_FLAG_NO_SEED_GROUPS),
-                    !(h->cfg.flags & CGB_FLAG_WARP_TAIL), !(h->cfg.flags & CGB_FLAG_NO_LEVEL_SUM), true, kFoldLists);
+                    !(h->cfg.flags & CGB_FLAG_WARP_TAIL), !(h->cfg.flags & CGB_FLAG_NO_LEVEL_SUM), true, cgb::kFoldLists);
     h->n_wsum = 0;
     h->wjobs_for = nullptr;  // the plans changed: rebuild the level-sum jobs
     for (uint32_t e = 0; e < h->q.qe; ++e)

@@ -269,7 +269,7 @@ void mq_plan(const cgb_mq* m, cgb_mq::Query& Q, uint32_t variant) {
     float avg[kMaxDir];
     for (uint32_t d = 0; d < q.nd; ++d) avg[d] = m->avg[q.labels[q.dir_src[d]] * m->L + q.labels[q.dir_dst[d]]];
     cgb::plan_edges(q, avg, Q.plans, true, !(variant & kVarPlainCore), !(variant & kVarNoSeedGroups), true, true, false,
-                    (variant & kVarNoFold) ? 0u : kMaxQV);
+                    (variant & kVarNoFold) ? 0u : cgb::kFoldListsMulti);
     for (uint32_t ei = 0; ei < q.qe; ++ei) {
         EdgePlan& P = Q.plans[ei];
         for (uint32_t j = 2; j < P.n; ++j)

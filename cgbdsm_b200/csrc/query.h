@@ -90,18 +90,15 @@ struct EdgePlan {
     //     before the launch (children first) into array wslot + k - sum_from.
     uint16_t sum_tails;
     uint16_t sum_same;  // positions < j whose vertex can lie in G (same label)
-    // tail_lane: each lane evaluates its own candidate's tail count at the
-    // last core position.  1: no tail list hangs off the last core vertex,
+    // tail_lane: how the tail depends on the candidate of the last core position
+    // (every lane counts its own candidate's, whatever this says; the level
+    // sums need 1, 2 or a constant tail).  1: no tail list hangs off the last core vertex,
     // so a candidate changes the tail count only by lying in prefix-only
     // lists (same label).  2: as 1, except for tail vertices whose only list
     // hangs off the last core vertex and whose label group they form alone:
     // such a count is the length of the candidate's list minus the excluded
-    // prefix vertices in it.  0: the warp counts one embedding at a time.
+    // prefix vertices in it.  0: otherwise, or a constant tail (tail_const).
     uint8_t tail_lane;
-    // tail_dep: the deepest core position below n_core - 1 that a tail count
-    // reads (a list's owner or an excluded vertex); a prefix change at a
-    // deeper position leaves every prefix-only tail count as it was.
-    uint8_t tail_dep;
     uint8_t sum_from;   // 0: no level sums
     uint8_t sum_dense;
     uint8_t wslot;
@@ -185,12 +182,21 @@ std::string parse_query_file(const std::string& path, std::vector<uint32_t>& lab
 // analytic_tail = false keeps every vertex in the enumerated core.
 // pick_last = true puts the core vertex with the fewest tail neighbours last.
 // group_pendant = true groups the seeds of edges with a pendant endpoint
-// (EdgePlan::grouped; needs labels).  lane_tail = false leaves tail_lane 0;
+// (EdgePlan::grouped; needs labels).  lane_tail = false leaves tail_lane 0 and has
+// the tails counted one embedding at a time (kPlanWarpTail);
 // level_sum = false leaves sum_from 0; dense_sums = false allows only the
 // one-position (table) level sums.  wslot is left 0 (the engine assigns it).
 // fold_lists: a tail vertex with two to fold_lists lists stays in the tail even
 // where it hangs off the last core vertex (its intersections are then counted
 // per candidate of that vertex); below 2: none does.
+// Engines' values: the single-query engine's.  R-MAT 1M/10M, 9-vertex dense,
+// matching per batch: none 14.4 ms, up to three lists 14.0, all 16.4 (four
+// lists: enumerating the vertex narrows its candidates list by list, which the
+// per-candidate count does not share between candidates); R-MAT 100k/1M, a
+// 6-vertex sparse pattern: none 0.50 ms, up to three 0.26.  The multi-query
+// engine keeps them all (64 queries: none 44 ms, up to three 33-37, all 31) or,
+// in one of the variants its autotuner tries per query, none.
+constexpr uint32_t kFoldLists = 3, kFoldListsMulti = kMaxQV;
 void plan_edges(const QueryMeta& q, const float* avg_deg, EdgePlan* plans, bool analytic_tail = true,
                 bool pick_last = true, bool group_pendant = true, bool lane_tail = true, bool level_sum = true,
                 bool dense_sums = false, uint32_t fold_lists = 0);

@@ -1,7 +1,9 @@
 // Prints the matching plans cgb::plan_edges makes for a query file (one line
 // per query edge, space-separated fields and '|'-separated arrays), with the
 // single-query engine's options (dense level sums on) or, with a second
-// argument "mq", the multi-query engine's (one-position level sums only).
+// argument "mq", the multi-query engine's (one-position level sums only), or
+// "mq_no_fold", those of its plan variant that keeps vertices with several lists
+// out of the tail where they hang off the last core vertex.
 // Mean list lengths are taken as 1 for every direction.
 #include <cstdio>
 #include <string>
@@ -15,7 +17,8 @@ int main(int argc, char** argv) {
     uint32_t qv = 0;
     std::string err = cgb::parse_query_file(argv[1], labels, edges, qv);
     if (!err.empty()) { std::printf("error %s\n", err.c_str()); return 1; }
-    const bool mq = argc > 2 && std::string(argv[2]) == "mq";
+    const bool no_fold = argc > 2 && std::string(argv[2]) == "mq_no_fold";
+    const bool mq = no_fold || (argc > 2 && std::string(argv[2]) == "mq");
     cgb::QueryMeta q;
     err = cgb::build_query_meta(qv, (uint32_t)(edges.size() / 2), edges.data(), labels.data(), q,
                                 mq ? cgb::kMaxQE : cgb::kMaxQEKeyed);
@@ -23,7 +26,8 @@ int main(int argc, char** argv) {
     float avg[cgb::kMaxDir];
     for (float& x : avg) x = 1.f;
     std::vector<cgb::EdgePlan> plans(cgb::kMaxQE);
-    cgb::plan_edges(q, avg, plans.data(), true, true, true, true, true, !mq);
+    cgb::plan_edges(q, avg, plans.data(), true, true, true, true, true, !mq,
+                    no_fold ? 0 : mq ? cgb::kFoldListsMulti : cgb::kFoldLists);
     for (uint32_t ei = 0; ei < q.qe; ++ei) {
         const cgb::EdgePlan& p = plans[ei];
         std::printf("%u %u %u %u %u %u %u %u %u %u %u %u %u %u %u %u |", ei, p.n, p.n_core, p.sum_from, p.sum_dense,

@@ -43,7 +43,7 @@ def dump(tmp_path_factory):
                     "-o", exe], check=True)
     counter = [0]
 
-    def run(labels, edges, mq=False):
+    def run(labels, edges, mq=False, fold=True):
         counter[0] += 1
         qp = str(d / f"q{counter[0]}.graph")
         with open(qp, "w") as f:
@@ -51,7 +51,7 @@ def dump(tmp_path_factory):
                 f.write(f"v {i} {lb}\n")
             for a, b in edges:
                 f.write(f"e {a} {b} 0\n")
-        out = subprocess.run([exe, qp] + (["mq"] if mq else []), capture_output=True, text=True, check=True).stdout
+        out = subprocess.run([exe, qp] + (["mq" if fold else "mq_no_fold"] if mq else []), capture_output=True, text=True, check=True).stdout
         plans = []
         for line in out.splitlines():
             head, vs, off, pos, excl, gid = line.split("|")
@@ -107,7 +107,7 @@ def check_plan(p, labels):
         assert p["sum_same"] == sum(1 << t for t in range(j) if lab[t] == lab[j])
     m, key = p["memo_from"], p["memo_pos"]
     if m:
-        assert key < m and m + 2 <= nc
+        assert key < m < nc
         assert not (p["grouped"] and key < 2)
         inside = lambda x: x == key or x >= m  # noqa: E731
         for k in range(m, nc):
@@ -137,7 +137,12 @@ def test_headline_patterns_plan_their_shortcuts(dump):
     sparse = dump(*C3_SPARSE)
     memo = [(p["ei"], p["memo_from"], p["memo_pos"]) for p in sparse if p["memo_from"]]
     assert memo == [(1, 3, 2)]  # edge (0, 2): the subtree below the hub vertex 1
-    assert sparse[1]["pair_last"]  # and its last level is one intersection per lane
+    assert sparse[1]["nc"] == 4  # vertex 6 (two lists) is counted, not enumerated
+    # where it is enumerated its level is one intersection per lane (pair counting)
+    plain = dump(*C3_SPARSE, mq=True, fold=False)
+    assert plain[1]["nc"] == 5 and plain[1]["pair_last"] and not any(p["pair_last"] for p in sparse)
+    for p in plain:
+        check_plan(p, C3_SPARSE[0])
     for labels, edges, plans in [(*C3_TREE, tree), (*C3_SPARSE, sparse)]:
         for p in plans:
             check_plan(p, labels)
@@ -151,16 +156,16 @@ def test_query_set_plans_meet_their_conditions(dump, qset):
     seen = Counter()
     for q in qs:
         edges = [tuple(e) for e in q["edges"]]
-        for mq in (False, True):
+        for mq, fold in ((False, True), (True, True), (True, False)):
             if not mq and len(edges) > 16:
                 continue
-            for p in dump(q["labels"], edges, mq=mq):
+            for p in dump(q["labels"], edges, mq=mq, fold=fold):
                 check_plan(p, q["labels"])
                 seen["dense"] += p["dense"]
                 seen["one"] += bool(p["sum_from"]) and not p["dense"]
                 seen["memo"] += bool(p["memo_from"])
                 seen["pair"] += p["pair_last"]
-    assert seen["one"] > 0, seen
+    assert seen["one"] > 0 and seen["memo"] > 0 and seen["pair"] > 0, seen
 
 
 def test_parity_workload_plans_meet_their_conditions(dump, tmp_path):
