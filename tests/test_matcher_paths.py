@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from cgbdsm_b200 import Engine, Gpma, MultiQuery
-from cgbdsm_b200.engine import FLAG_MASK_PRUNE, FLAG_NO_STEAL, FLAG_VALID_BITS, CgbError
+from cgbdsm_b200.engine import FLAG_FORCE_SPLIT, FLAG_MASK_PRUNE, FLAG_NO_STEAL, FLAG_VALID_BITS, CgbError
 from oracle import bind
 
 
@@ -421,6 +421,44 @@ def test_byte_count_of_long_walks():
     want = K * T * (7 * 4 + (3 * 1 + 3 * 3 + 1 * 5) * 32 * (33 - (32 - T.bit_length())))
     assert want * 60 // 64 > 1 << 34
     assert want <= eng.stats()["match_bytes"] < want * 1.01
+    eng.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flags", [0, FLAG_FORCE_SPLIT, FLAG_NO_STEAL])
+@pytest.mark.parametrize("hub_degree", [10, 90])
+def test_subtree_memos_while_work_is_shared(flags, hub_degree):
+    """A plan with a subtree memo (asserted), whose one expansion per vertex is
+    handed to other warps part by part (every chunk of it under
+    FLAG_FORCE_SPLIT, asserted) while prefixes add their weights: counts per
+    query edge equal the restatement's, batch after batch."""
+    ql, qe = [0, 1, 2, 3, 4, 5, 1], [(0, 1), (0, 2), (1, 3), (1, 4), (1, 5), (1, 6), (5, 6)]
+    rng = np.random.default_rng(hub_degree)
+    n = 900
+    lab = rng.choice(6, n, p=[0.25, 0.3, 0.2, 0.05, 0.05, 0.15])
+    pairs = {(int(min(p)), int(max(p))) for p in rng.integers(0, n, (10 * n, 2)) if p[0] != p[1]}
+    for h in np.flatnonzero(lab == 1)[:5]:
+        pairs |= {(int(min(h, x)), int(max(h, x))) for x in rng.choice(n, hub_degree, replace=False) if x != h}
+    pairs = np.array(sorted(pairs), dtype=np.int64)
+    rng.shuffle(pairs)
+    k = len(pairs) // 5
+    orc = bind.Oracle(len(ql), qe)
+    eng = Engine(flags=flags, dfs_budget_ms=60000)
+    eng.load_query(len(ql), qe, ql)
+    init = _keys_of(orc, qe, ql, lab, pairs[2 * k:])
+    orc.build(init, n)
+    eng.build_index(init, n)
+    assert any(eng.plan_info(e)["memo_from"] for e in range(len(qe)))
+    tasks = total = 0
+    for p in (pairs[:k], pairs[k:2 * k]):
+        delta = _keys_of(orc, qe, ql, lab, p)
+        want = orc.batch(n, _empty(), _empty(), delta, None, bind.PER_EDGE)
+        assert eng.apply_batch(n, _empty(), _empty(), delta) == want
+        assert np.array_equal(eng.edge_counts(), orc.edge_counts())
+        tasks += eng.stats()["stolen_tasks"]
+        total += want
+    assert total > 0
+    assert (tasks == 0) if flags == FLAG_NO_STEAL else (tasks > 0 or flags == 0)
     eng.close()
 
 
