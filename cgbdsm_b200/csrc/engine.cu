@@ -869,7 +869,7 @@ struct DfsArgs {
     const uint32_t* seed_lo;
     const uint32_t* seed_pre;
     unsigned long long* counts;  // [qe]
-    unsigned int* work_next;
+    unsigned int* work_next;     // [0] seeds claimed behind the rows, [1] rows of seeds taken (seed_claim.h)
     unsigned int* err;
     unsigned long long* stats;   // [8]: seeds, chunks, tested, tails, algorithmic bytes read, .., .., stolen tasks
     unsigned long long budget_ns;  // per-launch wall-clock budget (0 = unlimited)
