@@ -603,7 +603,9 @@ def test_pair_counting_mixed_with_descent(lane_max, workdir, tmp_path, monkeypat
     not count a chunk's candidates twice.  With the bound at 0 or 2 every
     chunk mixes both kinds, and every chunk is shared (FLAG_FORCE_SPLIT):
     counts equal the reference's on C1 and on the benchmark's sparse
-    pattern (single-query and multi-query engine)."""
+    pattern (single-query and multi-query engine).  Only a plan variant of the
+    multi-query autotuner enumerates such levels (the other plans count the
+    vertex in the tail); the autotuner refuses variants whose counts differ."""
     if not bind.have_ref():
         pytest.skip("oracle/_ref/libcgbref.so not built")
     from cgbdsm_b200 import MultiQuery

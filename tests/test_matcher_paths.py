@@ -183,6 +183,41 @@ def test_seed_counts_around_the_grid(flags, blocks):
         eng.close()
 
 
+@pytest.mark.gpu
+def test_engines_side_by_side_on_one_device():
+    """Three engines fed by three threads at once, each with as many matcher
+    blocks as an empty device holds: every batch ends, with its count."""
+    import threading
+
+    ql, qe = PATTERNS["shared"]
+    rng = np.random.default_rng(12)
+    n = 400
+    lab, pairs = _graph(rng, n, max(ql) + 1, 120)
+    rng.shuffle(pairs)
+    k = len(pairs) // 10
+    orc = bind.Oracle(len(ql), qe)
+    init = _keys_of(orc, qe, ql, lab, pairs[6 * k:])
+    deltas = [_keys_of(orc, qe, ql, lab, pairs[i * k:(i + 1) * k]) for i in range(6)]
+    orc.build(init, n)
+    want = [orc.batch(n, _empty(), _empty(), d, None, bind.PER_EDGE) for d in deltas]
+    got = [[], [], []]
+
+    def run(out):
+        for _ in range(5):
+            eng = Engine(dfs_budget_ms=20000)
+            eng.load_query(len(ql), qe, ql)
+            eng.build_index(init, n)
+            out.append([eng.apply_batch(n, _empty(), _empty(), d) for d in deltas])
+            eng.close()
+
+    threads = [threading.Thread(target=run, args=(g,)) for g in got]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert got == [[want] * 5] * 3
+
+
 # ---------------------------------------------------------------------------
 # per-candidate tails: several lists, shared labels, lists around 32 entries
 # ---------------------------------------------------------------------------
